@@ -501,6 +501,12 @@ static void launch_zcol(Grid& g, View<const typename CELL::T> in, View<typename 
 
 void launch_jacobi7(Grid& g, int steps)
 {
+    // the timeout tests' switch (lgd_gpu_test_bounded_waits) is about the TMA
+    // kernel's waits: a grid under it keeps that kernel
+    if (g.variant == 0 && g.test_wait_cycles == 0 && g.test_skip_plane == 0 && jacobi7_f64_applicable(g)) {
+        for (int s = 0; s < steps; ++s) launch_jacobi7_f64(g);
+        return;
+    }
     if ((g.variant == 0 || g.variant == 6) && tma_applicable(g)) {
         // temporal blocking: passes of `depth` steps, then one shorter pass
         // for the remainder (single steps go through the one-step kernel)

@@ -164,6 +164,9 @@ struct Grid {
     int tbmap_rows[2];
 };
 
+// the IEEE FP64 Jacobi kernel (k_fp64.cu)
+bool jacobi7_f64_applicable(const Grid& g);
+void launch_jacobi7_f64(Grid& g);
 bool tma_applicable(const Grid& g);
 void launch_jacobi7_tma(Grid& g);
 bool varcoef_tma_applicable(const Grid& g);

@@ -1,0 +1,39 @@
+"""The IEEE FP64 Jacobi kernel (csrc/k_fp64.cu) against the oracle, bit for
+bit, at the sizes and values where it can go wrong: planes around one CTA of
+128 cells, z chunks that end short, values that leave the integer product's
+range, and non-zero edges."""
+import numpy as np
+import pytest
+
+import oracle
+from libgeodecomp_gb300 import lgd, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def run(u0, steps, edge=0.0):
+    with lgd.Grid(lgd.CELL_JACOBI7_F64, u0.shape, edge=(edge, 0, 0, 0)) as g:
+        g.upload(0, u0)
+        g.step(steps)
+        return g.download(0)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 127), (2, 16, 8), (3, 43, 3), (17, 1, 129), (9, 33, 31), (130, 96, 64)])
+@pytest.mark.parametrize("edge", [0.0, -0.5])
+def test_shapes(shape, edge):
+    u0 = workloads.jacobi_initial(shape[2], shape[1], shape[0], seed=51)
+    np.testing.assert_array_equal(run(u0, 5, edge), oracle.jacobi7(u0, 5, edge=edge))
+
+
+@pytest.mark.parametrize("scale", [1e-323, 3e-308, 1e-300, 1.0, 1e300, 2e307])
+def test_value_ranges(scale):
+    """Subnormals, the ends of the exponent range, negative values, zeros and
+    sums whose significand makes the product a tie."""
+    rng = np.random.default_rng(5)
+    u0 = (rng.uniform(-1.0, 1.0, (7, 12, 40)) * scale).astype(np.float64)
+    u0[2] = 0.0
+    u0[4] = scale * 0.25
+    with np.errstate(over="ignore", invalid="ignore"):
+        ref = oracle.jacobi7(u0, 3)
+    out = run(u0, 3)
+    np.testing.assert_array_equal(out.view(np.uint64), ref.view(np.uint64))
