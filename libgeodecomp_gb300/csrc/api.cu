@@ -222,14 +222,15 @@ static void lower_fix_exp(Grid& g)
 }
 
 // --------------------------------------------------------------- helpers
-// Reads (and clears) the device error word that kernels with bounded waits
-// set when a wait gave up; call after the stream is synchronised.
+// Reads (and clears) the error word that kernels with bounded waits set when
+// a wait gave up; call after the stream is synchronised.  The word lives in
+// mapped host memory: kernels only ever write it, and only on a failure, and
+// the check is a host load (a copy from the device took 14 us per call).
 static void check_device_error(Grid& g)
 {
-    int e = 0;
-    LGD_CHECK_CUDA(cudaMemcpy(&e, g.d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (e) {
-        LGD_CHECK_CUDA(cudaMemset(g.d_err, 0, sizeof(int)));
+    volatile int *e = g.d_err;
+    if (*e) {
+        *e = 0;
         throw Error(LGD_ERR_TIMEOUT, "a device-side wait gave up; the last step's results are incomplete");
     }
 }
@@ -268,6 +269,87 @@ static void xfer_init(Grid& g)
         LGD_CHECK_CUDA(cudaEventCreateWithFlags(&g.xfer_ev[k], cudaEventDisableTiming));
     }
     g.xfer_ready = true;
+}
+
+// Dense rows <-> pitched rows on the device, one 4-byte word (W = 4: rows of
+// a multiple of 4 bytes, aligned) or one pitched word of single bytes (W = 1)
+// per thread.  The copy engine moves rows that are not a multiple of its
+// burst far below the link's rate (59 MB in rows of 1300 B: 1.96 ms up as a
+// pitched copy, 0.33 ms as one dense copy and this kernel).
+template<int W, bool TO_PITCHED>
+__global__ void __launch_bounds__(256)
+repitch_kernel(unsigned char *dense, unsigned char *pitched, unsigned words, unsigned row_bytes, long long rows,
+               long long pitch)
+{
+    const long long total = (long long)words * rows;
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < total; i += gridDim.x * 256ll) {
+        const long long r = i / words;
+        const unsigned off = (unsigned)(i - r * words) * 4u;
+        unsigned char *d = dense + r * row_bytes + off;
+        unsigned char *p = pitched + r * pitch + off;
+        if (W == 4) {
+            if (TO_PITCHED) *reinterpret_cast<uint32_t *>(p) = *reinterpret_cast<const uint32_t *>(d);
+            else *reinterpret_cast<uint32_t *>(d) = *reinterpret_cast<const uint32_t *>(p);
+        } else {
+            const unsigned n = min(4u, row_bytes - off);
+            for (unsigned k = 0; k < n; ++k) {
+                if (TO_PITCHED) p[k] = d[k];
+                else d[k] = p[k];
+            }
+        }
+    }
+}
+
+static void repitch(Grid& g, void *dense, void *pitched, size_t row_bytes, long long rows, size_t pitch,
+                    bool to_pitched)
+{
+    const bool wide = row_bytes % 4 == 0 && (uintptr_t)dense % 4 == 0;
+    const unsigned words = (unsigned)((row_bytes + 3) / 4);
+    const unsigned blocks = (unsigned)std::min<long long>(152LL * 32, ((long long)words * rows + 255) / 256);
+    unsigned char *d = (unsigned char *)dense, *p = (unsigned char *)pitched;
+    if (wide && to_pitched) {
+        repitch_kernel<4, true><<<blocks, 256, 0, g.stream>>>(d, p, words, (unsigned)row_bytes, rows, (long long)pitch);
+    } else if (wide) {
+        repitch_kernel<4, false><<<blocks, 256, 0, g.stream>>>(d, p, words, (unsigned)row_bytes, rows, (long long)pitch);
+    } else if (to_pitched) {
+        repitch_kernel<1, true><<<blocks, 256, 0, g.stream>>>(d, p, words, (unsigned)row_bytes, rows, (long long)pitch);
+    } else {
+        repitch_kernel<1, false><<<blocks, 256, 0, g.stream>>>(d, p, words, (unsigned)row_bytes, rows, (long long)pitch);
+    }
+    check_launch("row copy");
+    ++g.launches;
+}
+
+// Host <-> grid copy of one member: rows that fill their pitch go as one
+// dense copy, others through a bounded staging buffer and repitch.
+constexpr size_t HOST_STAGE_BYTES = 64u << 20;
+constexpr size_t REPITCH_MAX_ROW = 1u << 30;        // repitch_kernel numbers a row's words in 32 bits
+
+static void host_copy(Grid& g, int member, void *buf, void *host, bool to_grid)
+{
+    const size_t row_bytes = (size_t)g.desc.nx * g.m[member].elem;
+    const size_t pitch = g.pitch_bytes[member];
+    const size_t rows = (size_t)g.desc.ny * g.desc.nz;
+    const cudaMemcpyKind kind = to_grid ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+    if (row_bytes == pitch || rows == 1) {
+        LGD_CHECK_CUDA(cudaMemcpyAsync(to_grid ? buf : host, to_grid ? host : buf, row_bytes * rows, kind, g.stream));
+        return;
+    }
+    if (row_bytes > REPITCH_MAX_ROW) {
+        LGD_CHECK_CUDA(cudaMemcpy2DAsync(to_grid ? buf : host, to_grid ? pitch : row_bytes, to_grid ? host : buf,
+                                         to_grid ? row_bytes : pitch, row_bytes, rows, kind, g.stream));
+        return;
+    }
+    const size_t chunk = std::min(rows, std::max<size_t>(1, HOST_STAGE_BYTES / row_bytes));
+    unsigned char *stage = (unsigned char *)staging(g, chunk * row_bytes);
+    for (size_t r = 0; r < rows; r += chunk) {
+        const size_t n = std::min(chunk, rows - r);
+        unsigned char *h = (unsigned char *)host + r * row_bytes;
+        unsigned char *p = (unsigned char *)buf + r * pitch;
+        if (to_grid) LGD_CHECK_CUDA(cudaMemcpyAsync(stage, h, n * row_bytes, kind, g.stream));
+        repitch(g, stage, p, row_bytes, (long long)n, pitch, to_grid);
+        if (!to_grid) LGD_CHECK_CUDA(cudaMemcpyAsync(h, stage, n * row_bytes, kind, g.stream));
+    }
 }
 
 static Grid& grid_of(lgd_handle *h)
@@ -401,8 +483,9 @@ static void create_grid(const lgd_grid_desc *desc, size_t record_bytes, const vo
         LGD_CHECK_CUDA(cudaGetDevice(&g.device));
         try {
             LGD_CHECK_CUDA(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
-            LGD_CHECK_CUDA(cudaMalloc(&g.d_err, sizeof(int)));
-            LGD_CHECK_CUDA(cudaMemsetAsync(g.d_err, 0, sizeof(int), g.stream));
+            // unified addressing: the host pointer is the device's, too
+            LGD_CHECK_CUDA(cudaHostAlloc(&g.d_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+            *g.d_err = 0;
             for (int m = 0; m < ci.n_members; ++m) {
                 g.m[m].elem = ci.elem[m];
                 g.m[m].is_static = ci.is_static[m];
@@ -436,7 +519,7 @@ static void create_grid(const lgd_grid_desc *desc, size_t record_bytes, const vo
                     if (g.m[m].buf[b]) cudaFree(g.m[m].buf[b]);
                 }
             }
-            if (g.d_err) cudaFree(g.d_err);
+            if (g.d_err) cudaFreeHost(g.d_err);
             if (g.d_fixmax) cudaFree(g.d_fixmax);
             if (g.d_edge_record) cudaFree(g.d_edge_record);
             std::free(g.edge_record);
@@ -588,7 +671,7 @@ int lgd_gpu_destroy(lgd_handle *h)
         if (g.d_streaks) cudaFree(g.d_streaks);
         if (g.d_streak_prefix) cudaFree(g.d_streak_prefix);
         if (g.d_partials) cudaFree(g.d_partials);
-        if (g.d_err) cudaFree(g.d_err);
+        if (g.d_err) cudaFreeHost(g.d_err);
         if (g.d_fixmax) cudaFree(g.d_fixmax);
         if (g.d_edge_record) cudaFree(g.d_edge_record);
         std::free(g.edge_record);
@@ -684,9 +767,7 @@ int lgd_gpu_upload(lgd_handle *h, int member, int which, const void *host, size_
             }
             return;
         }
-        LGD_CHECK_CUDA(cudaMemcpy2DAsync(member_buf(g, member, which), g.pitch_bytes[member], host,
-                                         (size_t)g.desc.nx * helem, (size_t)g.desc.nx * helem, rows,
-                                         cudaMemcpyHostToDevice, g.stream));
+        host_copy(g, member, member_buf(g, member, which), const_cast<void *>(host), true);
         LGD_CHECK_CUDA(cudaStreamSynchronize(g.stream));
     });
 }
@@ -729,9 +810,7 @@ int lgd_gpu_download(lgd_handle *h, int member, int which, void *host, size_t by
             check_device_error(g);
             return;
         }
-        LGD_CHECK_CUDA(cudaMemcpy2DAsync(host, (size_t)g.desc.nx * helem, member_buf(g, member, which),
-                                         g.pitch_bytes[member], (size_t)g.desc.nx * helem, rows,
-                                         cudaMemcpyDeviceToHost, g.stream));
+        host_copy(g, member, member_buf(g, member, which), host, false);
         LGD_CHECK_CUDA(cudaStreamSynchronize(g.stream));
         check_device_error(g);
     });
@@ -929,12 +1008,24 @@ static void device_copy(lgd_handle *h, int member, int which, void *dev, size_t 
     LGD_REQUIRE(bytes == n * elem, LGD_ERR_INVALID, "byte count does not match the grid");
     const size_t rows = (size_t)g.desc.ny * g.desc.nz;
     const size_t row_bytes = (size_t)g.desc.nx * elem;
-    if (to_grid) {
-        LGD_CHECK_CUDA(cudaMemcpy2DAsync(member_buf(g, member, which), g.pitch_bytes[member], dev, row_bytes, row_bytes,
-                                         rows, cudaMemcpyDeviceToDevice, g.stream));
+    void *buf = member_buf(g, member, which);
+    if (row_bytes == g.pitch_bytes[member]) {
+        LGD_CHECK_CUDA(cudaMemcpyAsync(to_grid ? buf : dev, to_grid ? dev : buf, bytes, cudaMemcpyDeviceToDevice, g.stream));
     } else {
-        LGD_CHECK_CUDA(cudaMemcpy2DAsync(dev, row_bytes, member_buf(g, member, which), g.pitch_bytes[member], row_bytes,
-                                         rows, cudaMemcpyDeviceToDevice, g.stream));
+        // the row kernel reads memory of this device; anything else (another
+        // device's, a host pointer) stays with the copy engine
+        cudaPointerAttributes attr;
+        const bool local = cudaPointerGetAttributes(&attr, dev) == cudaSuccess &&
+                           attr.type == cudaMemoryTypeDevice && attr.device == g.device;
+        const size_t pitch = g.pitch_bytes[member];
+        if (local && row_bytes <= REPITCH_MAX_ROW) {
+            repitch(g, dev, buf, row_bytes, (long long)rows, pitch, to_grid);
+        } else {
+            cudaGetLastError();
+            LGD_CHECK_CUDA(cudaMemcpy2DAsync(to_grid ? buf : dev, to_grid ? pitch : row_bytes, to_grid ? dev : buf,
+                                             to_grid ? row_bytes : pitch, row_bytes, rows, cudaMemcpyDeviceToDevice,
+                                             g.stream));
+        }
     }
     LGD_CHECK_CUDA(cudaStreamSynchronize(g.stream));
 }
