@@ -30,9 +30,10 @@ namespace fp64k {
 constexpr int THREADS = 128;
 
 __global__ void __launch_bounds__(THREADS, 16)
-jacobi7_f64_kernel(const double *__restrict__ in, double *__restrict__ out, long pitch, int nx, int ny, int nz,
+jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, int nz,
                    int zchunk, double edge)
 {
+    dependent_start();
     const unsigned cells = (unsigned)nx * (unsigned)ny;         // below 2^31 (host rule)
     const unsigned c = blockIdx.x * THREADS + threadIdx.x;
     if (c >= cells) return;
@@ -44,15 +45,15 @@ jacobi7_f64_kernel(const double *__restrict__ in, double *__restrict__ out, long
     const bool has_n = y > 0, has_s = y + 1 < ny, has_w = x > 0, has_e = x + 1 < nx;
     const double *p = in + (long)z0 * plane + (long)y * pitch + x;
     double *o = out + (long)z0 * plane + (long)y * pitch + x;
-    double b = z0 > 0 ? __ldg(p - plane) : edge;
-    double m = __ldg(p);
+    double b = z0 > 0 ? *(p - plane) : edge;
+    double m = *p;
 #pragma unroll 1
     for (int z = z0; z < z1; ++z) {
-        const double t = z + 1 < nz ? __ldg(p + plane) : edge;
-        const double n = has_n ? __ldg(p - pitch) : edge;
-        const double s = has_s ? __ldg(p + pitch) : edge;
-        const double e = has_e ? __ldg(p + 1) : edge;
-        const double w = has_w ? __ldg(p - 1) : edge;
+        const double t = z + 1 < nz ? *(p + plane) : edge;
+        const double n = has_n ? *(p - pitch) : edge;
+        const double s = has_s ? *(p + pitch) : edge;
+        const double e = has_e ? *(p + 1) : edge;
+        const double w = has_w ? *(p - 1) : edge;
         double acc = __dadd_rn(m, n);
         acc = __dadd_rn(acc, s);
         acc = __dadd_rn(acc, e);
@@ -95,8 +96,8 @@ void launch_jacobi7_f64(Grid& g)
     while (zchunk > 1 && xy * ((g.desc.nz + zchunk - 1) / zchunk) < 40LL * sms) zchunk /= 2;
     zchunk = std::max(zchunk, (g.desc.nz + 65534) / 65535);
     const dim3 grid((unsigned)xy, (unsigned)((g.desc.nz + zchunk - 1) / zchunk));
-    fp64k::jacobi7_f64_kernel<<<grid, fp64k::THREADS, 0, g.stream>>>(
-        (const double *)g.m[0].buf[g.cur], (double *)g.m[0].buf[1 - g.cur], (long)(g.pitch_bytes[0] / 8), g.desc.nx,
+    launch_dependent(
+        fp64k::jacobi7_f64_kernel, grid, fp64k::THREADS, 0, g.stream, (const double *)g.m[0].buf[g.cur], (double *)g.m[0].buf[1 - g.cur], (long)(g.pitch_bytes[0] / 8), g.desc.nx,
         g.desc.ny, g.desc.nz, zchunk, g.desc.edge[0]);
     check_launch("jacobi7 f64");
     ++g.launches;

@@ -158,6 +158,9 @@ jacobi7_tb_kernel(const __grid_constant__ CUtensorMap in_map, typename CELL::T *
         for (int s = 0; s < G::S; ++s) mbar_init(smem_addr(&bars[s]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_fail = 0;
+    }
+    dependent_start();
+    if (tid == 0) {
         const int first = min(G::D, nq);
         for (int q = 0; q < first; ++q) {
             const uint32_t bar = smem_addr(&bars[q % G::S]);
@@ -371,8 +374,8 @@ static void launch_tb_typed(Grid& g, int dtype)
     const int zchunk = pick_zchunk_tb((long long)bx * by, g.desc.nz, resident, 2 * TB);
     const int zsplit = (g.desc.nz + zchunk - 1) / zchunk;
     const CUtensorMap *map = reinterpret_cast<const CUtensorMap *>(g.tbmap[src]);
-    tbk::jacobi7_tb_kernel<CELL, TB, WY, ROWS><<<dim3(bx, by, zsplit), G::THREADS, G::SMEM, g.stream>>>(
-        *map, (T *)g.m[0].buf[1 - src], (long)(g.pitch_bytes[0] / sizeof(T)), g.desc.nx, g.desc.ny, g.desc.nz, zchunk,
+    launch_dependent(
+        tbk::jacobi7_tb_kernel<CELL, TB, WY, ROWS>, dim3(bx, by, zsplit), G::THREADS, G::SMEM, g.stream, *map, (T *)g.m[0].buf[1 - src], (long)(g.pitch_bytes[0] / sizeof(T)), g.desc.nx, g.desc.ny, g.desc.nz, zchunk,
         g.d_err);
 }
 

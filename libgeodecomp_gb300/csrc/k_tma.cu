@@ -87,6 +87,9 @@ jacobi7_tma_kernel(const __grid_constant__ CUtensorMap in_map, typename CELL::T 
         for (int s = 0; s < S; ++s) mbar_init(smem_addr(&bars[s]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_fail = 0;
+    }
+    dependent_start();
+    if (tid == 0) {
         const int first = min(D, nplanes - 1);
         for (int q = 0; q <= first; ++q) {
             if (q == skip) continue;
@@ -270,6 +273,9 @@ varcoef_tma_kernel(const __grid_constant__ vc::Maps maps, R *__restrict__ out, l
         for (int s = 0; s < VC_S; ++s) mbar_init(smem_addr(&bars[s]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_fail = 0;
+    }
+    dependent_start();
+    if (tid == 0) {
         const int first = min(VC_D, nplanes - 1);
         for (int q = 0; q <= first; ++q) issue(q);
         s_issued = first + 1;
@@ -555,8 +561,8 @@ static void launch_tma_typed(Grid& g, CUtensorMapDataType dt)
     }
     zsplit = (g.desc.nz + zchunk - 1) / zchunk;
     const CUtensorMap *map = reinterpret_cast<const CUtensorMap *>(g.tmap[src]);
-    tmak::jacobi7_tma_kernel<CELL><<<dim3(bx, by, zsplit), tmak::THREADS, smem, g.stream>>>(
-        *map, (T *)g.m[0].buf[1 - src], (long)(g.pitch_bytes[0] / sizeof(T)), g.desc.nx, g.desc.ny, g.desc.nz, zchunk,
+    launch_dependent(
+        tmak::jacobi7_tma_kernel<CELL>, dim3(bx, by, zsplit), tmak::THREADS, smem, g.stream, *map, (T *)g.m[0].buf[1 - src], (long)(g.pitch_bytes[0] / sizeof(T)), g.desc.nx, g.desc.ny, g.desc.nz, zchunk,
         g.d_err, g.test_wait_cycles > 0 ? g.test_wait_cycles : tmak::WAIT_CYCLES, g.test_skip_plane - 1);
 }
 
@@ -602,8 +608,8 @@ static void launch_varcoef_tma_typed(Grid& g, CUtensorMapDataType dt)
     const int by = (g.desc.ny + tmak::TY - 1) / tmak::TY;
     const int zchunk = tmak::pick_zchunk((long long)bx * by, g.desc.nz, resident);
     const int zsplit = (g.desc.nz + zchunk - 1) / zchunk;
-    tmak::varcoef_tma_kernel<R><<<dim3(bx, by, zsplit), tmak::THREADS, smem, g.stream>>>(
-        *maps, (R *)g.m[0].buf[1 - src], (long)(g.pitch_bytes[0] / sizeof(R)), g.desc.nx, g.desc.ny, g.desc.nz,
+    launch_dependent(
+        tmak::varcoef_tma_kernel<R>, dim3(bx, by, zsplit), tmak::THREADS, smem, g.stream, *maps, (R *)g.m[0].buf[1 - src], (long)(g.pitch_bytes[0] / sizeof(R)), g.desc.nx, g.desc.ny, g.desc.nz,
         g.desc.periodic, zchunk, g.d_err);
 }
 

@@ -132,7 +132,7 @@ sell_diffusion_kernel(const int *__restrict__ chunk_offset, const int *__restric
 template<typename R, bool EXACT, int D>
 __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offset, const int *__restrict__ row_length,
                                               const R *__restrict__ values, const int *__restrict__ column,
-                                              const R *__restrict__ x, R *__restrict__ xn, int C, int row, int chunk)
+                                              const R *x, R *xn, int C, int row, int chunk)
 {
     const long long cbase = chunk_offset[chunk];
     const long long base = cbase + (row - chunk * C);
@@ -155,7 +155,7 @@ __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offs
     for (int k = 0; k < len; k += D) {
         R g[D];
 #pragma unroll
-        for (int j = 0; j < D; ++j) g[j] = (k + j < len) ? __ldg(x + cc[j]) : (R)0;
+        for (int j = 0; j < D; ++j) g[j] = (k + j < len) ? x[cc[j]] : (R)0;
         R nw[D];
         int nc[D];
 #pragma unroll
@@ -194,8 +194,9 @@ template<typename R, bool EXACT, int D, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 sell_diffusion_pipe_kernel(const int *__restrict__ chunk_offset, const int *__restrict__ row_length,
                            const R *__restrict__ values, const int *__restrict__ column,
-                           const R *__restrict__ x, R *__restrict__ xn, int n, int C, int row_begin, int row_end)
+                           const R *x, R *xn, int n, int C, int row_begin, int row_end)
 {
+    dependent_start();
     const int row = row_begin + blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= row_end) return;
     sell_pipe_row<R, EXACT, D>(chunk_offset, row_length, values, column, x, xn, C, row, row / C);
@@ -240,8 +241,8 @@ template<typename R, bool EXACT, int D, int THREADS>
 static void launch_pipe(Sell& s, int row_begin, int row_end, const R *x, R *xn, const R *vals)
 {
     const int blocks = (row_end - row_begin + THREADS - 1) / THREADS;
-    sell_diffusion_pipe_kernel<R, EXACT, D, THREADS><<<blocks, THREADS, 0, s.stream>>>(
-        s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.n, s.C, row_begin, row_end);
+    launch_dependent(
+        sell_diffusion_pipe_kernel<R, EXACT, D, THREADS>, dim3(blocks), THREADS, 0, s.stream, s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.n, s.C, row_begin, row_end);
 }
 
 template<typename R, bool EXACT>
