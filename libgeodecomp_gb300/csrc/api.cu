@@ -676,6 +676,7 @@ int lgd_gpu_destroy(lgd_handle *h)
         if (g.d_edge_record) cudaFree(g.d_edge_record);
         std::free(g.edge_record);
         if (g.d_stage) cudaFree(g.d_stage);
+        if (g.d_bits) cudaFree(g.d_bits);
         if (g.xfer_ready) {
             cudaStreamSynchronize(g.xfer_stream);
             for (int k = 0; k <= XFER_CHUNKS; ++k) cudaEventDestroy(g.xfer_ev[k]);

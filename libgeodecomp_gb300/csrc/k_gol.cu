@@ -290,6 +290,12 @@ gol_bits_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int n
 // generations per bit-sliced pass when none are requested
 constexpr int GOL_BITS_DEFAULT_DEPTH = 16;
 
+// generations of a call from which the packed board pays for packing and
+// unpacking: on a torus of aligned rows (the alternative is a bit-sliced pass
+// over bytes), and on other boards (one launch per generation)
+constexpr int GOL_PACK_MIN_TORUS = 17;
+constexpr int GOL_PACK_MIN = 4;
+
 bool gol_tb_applicable(const Grid& g)
 {
     return g.desc.cell == LGD_CELL_GOL_U8 && (g.desc.periodic & 3) == 3 && g.desc.nz == 1 && g.desc.nx % 16 == 0 &&
@@ -444,10 +450,26 @@ static void prepare_gol_kernels()
     });
 }
 
+static void gol_single(Grid& g, int steps);
+
 void launch_gol(Grid& g, int steps)
 {
     prepare_gol_kernels();
     LGD_REQUIRE(g.desc.nz == 1, LGD_ERR_INVALID, "Game of Life grids are 2D (nz = 1)");
+    // no depth asked for: packed passes (k_golpack.cu).  Boards that only the
+    // byte-wise kernel served before take their first generation with it: it
+    // counts cells by their byte values, so bytes other than 0 and 1 keep
+    // their meaning, and leaves 0 and 1 behind
+    const bool aligned_torus = gol_tb_applicable(g);
+    if (g.variant == 0 && g.time_block == 0 && steps >= (aligned_torus ? GOL_PACK_MIN_TORUS : GOL_PACK_MIN) &&
+        gol_packed_applicable(g)) {
+        if (!aligned_torus) {
+            gol_single(g, 1);
+            --steps;
+        }
+        launch_gol_packed(g, steps);
+        return;
+    }
     // temporal blocking on the torus: bit-sliced passes (rows of a
     // multiple of 32 cells, up to 32 generations) or byte passes (rows of a
     // multiple of 16 cells, up to 12; variant 1 forces these for
@@ -457,13 +479,18 @@ void launch_gol(Grid& g, int steps)
         if (depth > 1) {
             while (steps >= 2) steps -= gol_bits_pass(g, std::min(depth, steps), g.tb_shape);
         }
-    } else if (g.variant <= 1 && gol_tb_applicable(g)) {
+    } else if (g.variant <= 1 && aligned_torus) {
         const int depth = (g.time_block == 0) ? 8 : std::min(g.time_block, 12);
         if (depth > 1) {
             while (steps >= 2) steps -= gol_tb_pass(g, std::min(depth, steps), g.tb_shape);
         }
     }
+    gol_single(g, steps);
+}
 
+// one generation per launch, on bytes
+static void gol_single(Grid& g, int steps)
+{
     const bool swar = ((g.desc.periodic & 3) == 3) && (g.desc.nx % 16 == 0) && (g.pitch_bytes[0] % 16 == 0);
     const long pitch = (long)g.pitch_bytes[0];
     for (int s = 0; s < steps; ++s) {

@@ -195,6 +195,7 @@ struct Grid {
     alignas(64) unsigned char vtmap[2][6 * 128];
     bool vtmap_ready[2];
     void *vtmap_base[2][2];
+    uint32_t *d_bits;       // Game of Life: the packed board, two buffers (k_golpack.cu; from the first use on)
     // temporal-blocking kernel: one tensor map per buffer (box 64 x rows)
     alignas(64) unsigned char tbmap[2][128];
     bool tbmap_ready[2];
@@ -224,6 +225,8 @@ void encode_tensor_map(void *map, int dtype, int rank, void *base, const uint64_
 // kernels, one entry per cell family (implemented in k_*.cu)
 void launch_jacobi7(Grid& g, int steps);
 void launch_gol(Grid& g, int steps);
+bool gol_packed_applicable(const Grid& g);
+void launch_gol_packed(Grid& g, int steps);
 void launch_varcoef(Grid& g, int steps);
 void launch_region(Grid& g, const int *d_streaks, const long long *d_prefix, int n_streaks, long long cells,
                    unsigned nano_step);
