@@ -292,8 +292,10 @@ constexpr int GOL_BITS_DEFAULT_DEPTH = 16;
 
 // generations of a call from which the packed board pays for packing and
 // unpacking: on a torus of aligned rows (the alternative is a bit-sliced pass
-// over bytes), and on other boards (one launch per generation)
-constexpr int GOL_PACK_MIN_TORUS = 17;
+// over bytes), and on other boards (one launch per generation).  us per call,
+// packed against not: 8192^2 x 4 43 / 38, x 8 54 / 54, x 16 70 / 100; 1024^2 x
+// 4 11 / 15, x 16 12 / 83; 1001 x 777 x 4 17 / 34
+constexpr int GOL_PACK_MIN_TORUS = 6;
 constexpr int GOL_PACK_MIN = 4;
 
 bool gol_tb_applicable(const Grid& g)

@@ -21,8 +21,10 @@
 // T <= 32, lanes 1 .. 30 are right and are stored.
 //
 // Bound by the ALU pipe (64 lanes per clock and SM): 16 instructions per word
-// allow 38 T cell updates per second on 152 SMs; the rim and the SMs' uneven
-// shares take 15-30% of that.
+// allow 38 T cell updates per second on 152 SMs.  A pass of 16 generations of
+// 8192^2 takes 44 us (24 T updates per second; gol_bits_kernel: 99 us); the
+// rest goes to the rim (6% of rows, 5% of words), 144 of 152 SMs at work, and
+// four warps per SM quarter that do not always have an instruction ready.
 #include <algorithm>
 
 #include "lgd_internal.h"
@@ -150,31 +152,47 @@ gol_pack_kernel(const uint32_t *in, uint32_t *out, Board b, int T, int out_rows)
     const int fill = b.nx - p;                                  // cells up to the row's end
     const bool wraps = (b.periodic & 1) && fill < 32;
 
+    // rows first .. first + R - 1 of the board (rowin: those that exist); all
+    // loads of a kind are in flight together, and only windows that reach
+    // around a row's end load more than one word per row
     uint32_t v[R];
     uint32_t rowin[CUBE ? (R + 31) / 32 : 1] = {};
-    int y = y0 - T + warp * R;                                  // board row of the lane's first row
+    int first = y0 - T + warp * R;
     if (b.periodic & 2) {
-        y %= b.ny;
-        if (y < 0) y += b.ny;
+        first %= b.ny;
+        if (first < 0) first += b.ny;
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-        uint32_t x = 0;
-        const bool inside = !CUBE || (unsigned)y < (unsigned)b.ny;
-        if (inside) {
-            const uint32_t *row = in + (long long)y * b.wpitch;
-            x = row[wl];
-            if (sh) x = __funnelshift_r(x, has_hi ? row[wl + 1] : 0u, sh);
-            if (wraps) x |= row[0] << fill;
-        }
+    auto row_of = [&](int r) -> const uint32_t * {
+        int y = first + r;
         if (CUBE) {
-            x = (x & colmask) | (b.edge & ~colmask);
-            if (!inside) x = b.edge;
+            if ((b.periodic & 2) && y >= b.ny) y %= b.ny;
+            y = min(max(y, 0), b.ny - 1);
+        } else if (y >= b.ny) {
+            y -= b.ny;
+            if (y >= b.ny) y %= b.ny;
+        }
+        return in + (long long)y * b.wpitch;
+    };
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = row_of(r)[wl];
+    if (__any_sync(0xffffffffu, sh != 0)) {
+        const int wh = has_hi ? wl + 1 : wl;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const uint32_t *row = row_of(r);
+            const uint32_t hi = row[wh], start = row[0];
+            uint32_t x = __funnelshift_r(v[r], has_hi ? hi : 0u, sh);
+            if (wraps) x |= start << fill;
+            v[r] = x;
+        }
+    }
+    if (CUBE) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const bool inside = (b.periodic & 2) || (unsigned)(first + r) < (unsigned)b.ny;
+            v[r] = inside ? (v[r] & colmask) | (b.edge & ~colmask) : b.edge;
             if (inside) rowin[r / 32] |= 1u << (r % 32);
         }
-        v[r] = x;
-        ++y;
-        if ((b.periodic & 2) && y >= b.ny) y = 0;
     }
 
     for (int t = 0; t < T; ++t) {
@@ -216,36 +234,42 @@ gol_pack_kernel(const uint32_t *in, uint32_t *out, Board b, int T, int out_rows)
     }
 }
 
-// Tile height and generations per pass.  Modelled time of a generation: the
-// busiest SM's rows at 16 ALU instructions and 2 shuffles per row and warp
-// (about 9 clocks with four quarters working), at least the time one warp
-// takes alone (its instructions and the exchange); a pass adds its launch,
-// load and store.
+// Tile height and generations per pass, by a model fitted to a sweep of all of
+// them on boards from 300^2 to 8192^2 (it finds the sweep's best or one within
+// 5%).  A generation takes the busiest SM's rows at 4.45 ns each (its four
+// quarters in step: the warps of the fullest count), or one warp's chain of
+// rows, 18 ns each, whichever is longer, and 45 ns of exchange; a pass adds
+// its launch, loads and stores.
 struct Plan {
     int R, W, T, out_rows;
+    int per_sm;                             // CTAs on the busiest SM
     double ns;                              // per generation
 };
 
-constexpr int ROWS[] = {8, 16, 24, 34};     // compiled tile rows per lane (34: 16 warps hold 512 + 2 * 16 rows)
+constexpr int SM_SMEM = 224 * 1024;         // shared memory of an SM to divide up, at most
+constexpr int CTA_SMEM = 12 * 1024;         // static (the rim) and reserved shared memory of a CTA
+
+constexpr int ROWS[] = {8, 12, 16, 24, 34};     // compiled rows per lane (34: 16 warps hold 512 + 2 * 16 rows)
 
 static Plan plan(int nx, int ny, int sms, int steps)
 {
-    Plan best = {8, 4, 1, 1, 1e300};
+    Plan best = {8, 4, 1, 1, 1, 1e300};
     const long long xt = (nx + OUT_WORDS * 32 - 1) / (OUT_WORDS * 32);
     for (int R : ROWS) {
-        for (int W : {4, 8, 16}) {
-            for (int T : {4, 8, 12, 16, 24, 32}) {
+        for (int W = 4; W <= MAX_WARPS; ++W) {
+            for (int T = 4; T <= MAX_T; T += 4) {
                 const int room = W * R - 2 * T;
-                if (room < 4) continue;
+                if (room < 4) break;
                 // even bands: no tile is nearly empty
                 const long long bands = (ny + room - 1) / room;
                 if (bands > 65535) continue;
                 const int out_rows = (int)((ny + bands - 1) / bands);
                 const long long per_sm = (xt * bands + sms - 1) / sms;
-                const double gen = std::max(per_sm * W * R * 4.5, R * 12.0 + 60.0);
+                const double rows = (double)((per_sm * W + 3) / 4 * 4) * R;
+                const double gen = std::max(rows * 4.45, R * 18.0) + 45.0;
                 const int passes = (steps + T - 1) / T;
-                const double ns = (passes * 2500.0 + gen * steps) / steps;
-                if (ns < best.ns * 0.999) best = {R, W, T, out_rows, ns};
+                const double ns = (passes * (1600.0 + 100.0 * R) + gen * steps) / steps;
+                if (ns < best.ns * 0.999) best = {R, W, T, out_rows, (int)per_sm, ns};
             }
         }
     }
@@ -260,11 +284,26 @@ static void launch_pass(Grid& g, const Board& b, const Plan& p, int T, const uin
     void (*fn)(const uint32_t *, uint32_t *, Board, int, int) = nullptr;
     switch (p.R) {
     case 8: fn = gol_pack_kernel<8, CUBE>; break;
+    case 12: fn = gol_pack_kernel<12, CUBE>; break;
     case 16: fn = gol_pack_kernel<16, CUBE>; break;
     case 24: fn = gol_pack_kernel<24, CUBE>; break;
     default: fn = gol_pack_kernel<34, CUBE>; break;
     }
-    launch_dependent(fn, grid, 32u * p.W, 0, g.stream, in, out, b, T, p.out_rows);
+    // Shared memory that only the plan's share of CTAs fits on an SM with: a
+    // dependent launch is placed while the pass before still runs, and would
+    // pile its CTAs on the SMs that happen to have room (8192^2: 144 CTAs of
+    // one per SM, 90 us per pass of 16 piled up, 55 us spread)
+    static PerDevice<bool> setup;
+    setup.get([] {
+        for (const void *f : {(const void *)gol_pack_kernel<8, CUBE>, (const void *)gol_pack_kernel<12, CUBE>,
+                              (const void *)gol_pack_kernel<16, CUBE>, (const void *)gol_pack_kernel<24, CUBE>,
+                              (const void *)gol_pack_kernel<34, CUBE>}) {
+            LGD_CHECK_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM - CTA_SMEM));
+        }
+        return true;
+    });
+    const size_t smem = (size_t)std::max(0, std::min(SM_SMEM - CTA_SMEM, SM_SMEM / p.per_sm - CTA_SMEM));
+    launch_dependent(fn, grid, 32u * p.W, smem, g.stream, in, out, b, T, p.out_rows);
 }
 
 }  // namespace golp
