@@ -45,6 +45,7 @@ struct Sell {
     void *d_values;         // total, FP64 or FP32
     int *d_column;          // total
     void *d_x[2];           // rows_padded each
+    double *d_stage;        // n values on their way between host and device (from the first copy on)
     int *d_perm;            // physical -> logical (n), or null
     int cur;
     int variant;            // kernel variant, see lgd_sell_set_variant
@@ -202,6 +203,72 @@ sell_diffusion_pipe_kernel(const int *__restrict__ chunk_offset, const int *__re
     sell_pipe_row<R, EXACT, D>(chunk_offset, row_length, values, column, x, xn, C, row, row / C);
 }
 
+// L lanes per row, for matrices that leave the GPU's warps idle: a row is a
+// chain of dependent memory trips (len / D of them with one lane per row, and
+// a chunk's longest row holds its warp), so the lanes of a team load and
+// gather every L-th slot each and every lane sums all of them in slot order
+// from the others' registers - the same additions in the same order as above.
+// FP32 only: the L-fold repeated additions would fill the FP64 pipe.
+// Measured, FP32, us per step against the better single-lane form: 2000 nodes
+// 4.1 / 5.8, 20000 7.0 / 7.2, 100003 9.9 / 11.2, 300000 21.1 / 20.4.
+template<bool EXACT, int L, int D, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+sell_diffusion_team_kernel(const int *__restrict__ chunk_offset, const int *__restrict__ row_length,
+                           const float *__restrict__ values, const int *__restrict__ column, const float *x, float *xn,
+                           int C, int row_begin, int row_end)
+{
+    dependent_start();
+    const int t = blockIdx.x * THREADS + threadIdx.x;
+    const int q = t % L;
+    const int row = min(row_begin + t / L, row_end - 1);            // idle teams repeat the last row (all lanes shuffle)
+    const int chunk = row / C;
+    const int len = row_length[row];
+    const float xr = x[row];
+    const float *v = values + (long long)chunk_offset[chunk] + (row - chunk * C);
+    const int *c = column + (long long)chunk_offset[chunk] + (row - chunk * C);
+    // rounds of the warp's longest row
+    const int longest = __reduce_max_sync(0xffffffffu, len);
+    const int team = (threadIdx.x & 31) / L * L;
+    float w[D];
+    int cc[D];
+    auto load = [&](int k0, float (&lw)[D], int (&lc)[D]) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            const int k = k0 + j * L + q;
+            lw[j] = 0.f;
+            lc[j] = 0;
+            if (k < len) {
+                lw[j] = __ldg(v + (long long)k * C);
+                lc[j] = __ldg(c + (long long)k * C);
+            }
+        }
+    };
+    load(0, w, cc);
+    float acc = 0.f;
+    for (int k0 = 0; k0 < longest; k0 += D * L) {
+        float g[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) g[j] = (k0 + j * L + q < len) ? x[cc[j]] : 0.f;
+        float nw[D];
+        int nc[D];
+        load(k0 + D * L, nw, nc);
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+#pragma unroll
+            for (int s = 0; s < L; ++s) {
+                const float gs = __shfl_sync(0xffffffffu, g[j], team + s);
+                const float ws = __shfl_sync(0xffffffffu, w[j], team + s);
+                if (k0 + j * L + s < len) acc = madd<float, EXACT>(acc, gs, ws);
+            }
+            w[j] = nw[j];
+            cc[j] = nc[j];
+        }
+    }
+    if (q == 0 && row_begin + t / L < row_end) {
+        xn[row] = EXACT ? __fadd_rn(__fmul_rn(0.1f, xr), acc) : 0.1f * xr + acc;
+    }
+}
+
 template<typename R>
 __global__ void permute_in_kernel(const double *logical, const int *perm, R *phys, int n)
 {
@@ -233,6 +300,7 @@ static void sell_free(Sell& s)
     cudaFree(s.d_column);
     cudaFree(s.d_x[0]);
     cudaFree(s.d_x[1]);
+    cudaFree(s.d_stage);
     cudaFree(s.d_perm);
     if (s.stream) cudaStreamDestroy(s.stream);
 }
@@ -243,6 +311,18 @@ static void launch_pipe(Sell& s, int row_begin, int row_end, const R *x, R *xn, 
     const int blocks = (row_end - row_begin + THREADS - 1) / THREADS;
     launch_dependent(
         sell_diffusion_pipe_kernel<R, EXACT, D, THREADS>, dim3(blocks), THREADS, 0, s.stream, s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.n, s.C, row_begin, row_end);
+}
+
+constexpr int SELL_TEAM_MAX_ROWS = 200000;
+constexpr int SELL_DEEP_MAX_ROWS = 600000;
+
+template<bool EXACT>
+static void launch_team(Sell& s, int row_begin, int row_end, const float *x, float *xn, const float *vals)
+{
+    constexpr int L = 4, D = 4, THREADS = 128;
+    const int blocks = (int)(((long long)(row_end - row_begin) * L + THREADS - 1) / THREADS);
+    launch_dependent(sell_diffusion_team_kernel<EXACT, L, D, THREADS>, dim3(blocks), THREADS, 0, s.stream,
+                     s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.C, row_begin, row_end);
 }
 
 template<typename R, bool EXACT>
@@ -263,7 +343,18 @@ static void launch_sell_typed(Sell& s, int row_begin, int row_end)
     case 3: launch_pipe<R, EXACT, 4, 64>(s, row_begin, row_end, x, xn, vals); break;
     case 4: launch_pipe<R, EXACT, 4, 256>(s, row_begin, row_end, x, xn, vals); break;
     case 5: launch_pipe<R, EXACT, 8, 64>(s, row_begin, row_end, x, xn, vals); break;
-    default: launch_pipe<R, EXACT, 4, 128>(s, row_begin, row_end, x, xn, vals); break;
+    default:
+        // small matrices: teams of lanes (FP32), deeper pipelines (FP64;
+        // 20000 nodes 8.6 us per step against 10.2, 400000 27.2 against
+        // 29.3, one million 61.6 against 60.6)
+        if (sizeof(R) == 4 && row_end - row_begin <= SELL_TEAM_MAX_ROWS) {
+            launch_team<EXACT>(s, row_begin, row_end, (const float *)x, (float *)xn, (const float *)vals);
+        } else if (row_end - row_begin <= SELL_DEEP_MAX_ROWS) {
+            launch_pipe<R, EXACT, 8, 64>(s, row_begin, row_end, x, xn, vals);
+        } else {
+            launch_pipe<R, EXACT, 4, 128>(s, row_begin, row_end, x, xn, vals);
+        }
+        break;
     }
 }
 
@@ -945,8 +1036,10 @@ static void sell_copy_x(Sell& s, int which, double *host, size_t bytes, bool up,
     LGD_REQUIRE(host != nullptr, LGD_ERR_INVALID, "null host buffer");
     LGD_REQUIRE(bytes == sizeof(double) * (size_t)s.n, LGD_ERR_INVALID, "byte count must be n doubles");
     LGD_REQUIRE(!logical || s.d_perm != nullptr, LGD_ERR_INVALID, "no permutation was given at create");
-    double *tmp = nullptr;
-    LGD_CHECK_CUDA(cudaMallocAsync(&tmp, bytes, s.stream));
+    // kept by the handle: a pool allocation per copy cost 200 us, most of a
+    // copy of 100000 nodes
+    if (s.d_stage == nullptr) LGD_CHECK_CUDA(cudaMalloc(&s.d_stage, bytes));
+    double *tmp = s.d_stage;
     void *x = s.d_x[which ? 1 - s.cur : s.cur];
     const int *perm = logical ? s.d_perm : nullptr;
     const int blocks = std::min(152 * 8, (s.n + 255) / 256);
@@ -967,7 +1060,6 @@ static void sell_copy_x(Sell& s, int which, double *host, size_t bytes, bool up,
     }
     check_launch("sell permute");
     ++s.launches;
-    LGD_CHECK_CUDA(cudaFreeAsync(tmp, s.stream));
     LGD_CHECK_CUDA(cudaStreamSynchronize(s.stream));
 }
 

@@ -222,3 +222,28 @@ def test_renumbering_needs_host_arrays():
     t = [torch.as_tensor(a, device="cuda") for a in (rp, col.astype(np.int32), w)]
     with pytest.raises(lgd.LGDError):
         lgd.SellGrid.from_csr(1000, t[0], t[1], t[2], 32, 256, device=True, renumber=True)
+
+
+@pytest.mark.parametrize("n", [1, 5, 31, 33, 257, 4099])
+@pytest.mark.parametrize("C,sigma", [(32, 256), (8, 64), (3, 7)])
+@pytest.mark.parametrize("exact", [False, True])
+def test_sell_teams_equal_one_lane_per_row(n, C, sigma, exact):
+    """FP32 matrices of few rows run several lanes per row (variant 0); the
+    sums are the one-lane kernel's (variant 4), bit for bit: ragged and empty
+    rows, row counts off the team and chunk sizes, a row range."""
+    rng = np.random.default_rng(n)
+    deg = rng.integers(0, min(n, 70) + 1, n)
+    row_ptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int64)
+    col = np.concatenate([np.sort(rng.choice(n, d, replace=False)) for d in deg] + [np.zeros(0)]).astype(np.int32)
+    w = rng.random(row_ptr[-1]) * 0.02
+    x0 = rng.random(n)
+    out = []
+    for variant in (0, 4):
+        with lgd.SellGrid.from_csr(n, row_ptr, col, w, C, sigma, precision=4, exact=exact) as g:
+            g.set_variant(variant)
+            g.upload(x0)
+            g.step(3)
+            g.update_rows(n // 3, n)
+            out += [g.download(), g.download(which=1)]
+    np.testing.assert_array_equal(out[0], out[2])
+    np.testing.assert_array_equal(out[1], out[3])
