@@ -348,13 +348,16 @@ int lgd_gpu_launch_count(lgd_handle *h, uint64_t *count);
 
 /* Temporal blocking depth used by lgd_gpu_step (time steps fused into one
  * pass over memory): 0 = library default (3 for LGD_CELL_JACOBI7_F32, 2 for
- * LGD_CELL_JACOBI7_F64_FIX, 16 for LGD_CELL_GOL_U8 with rows of a multiple
- * of 32 cells, 8 for other Game of Life torus grids, 1 for the others),
+ * LGD_CELL_JACOBI7_F64_FIX, 2 for LGD_CELL_VARCOEF_F32 on a torus with rows of
+ * a multiple of 16 bytes, passes of up to 32 generations on packed rows for
+ * calls of several generations of LGD_CELL_GOL_U8, 1 for the others),
  * 1 = one step per pass, 2 .. LGD_TB_MAX_DEPTH.  It applies to
  *   - the FP32 Jacobi cell (at most 4; results bit-identical for every depth)
  *     and the fixed-point Jacobi cell (at most 2: its pass sums two steps
  *     exactly and rounds once) on 3D cube grids with a zero edge cell, under
  *     kernel variants 0 and 6;
+ *   - the FP32 var-coef cell on such a torus (at most 2; bit-identical) under
+ *     variant 0;
  *   - Game of Life on a torus (cells 0 or 1; bit-identical): rows of a
  *     multiple of 32 cells run bit-sliced passes (32 cells per 32-bit word;
  *     depths 2, 4, 6, 8, 12, 16, 24, 32) under kernel variant 0, rows of a

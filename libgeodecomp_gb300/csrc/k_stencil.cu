@@ -693,6 +693,9 @@ void launch_varcoef(Grid& g, int steps)
     // default: the TMA kernel for FP32 cells (HBM-bound); FP64 cells are
     // bound by the FP64 rate, where the register kernel measured faster
     const bool tma = (g.variant == 6) || (g.variant == 0 && g.desc.cell == LGD_CELL_VARCOEF_F32);
+    if (g.variant == 0 && g.time_block != 1 && varcoef_tb2_applicable(g)) {
+        for (; steps >= 2; steps -= 2) launch_varcoef_tb2(g);
+    }
     if (tma && varcoef_tma_applicable(g)) {
         for (int s = 0; s < steps; ++s) launch_varcoef_tma(g);
         return;

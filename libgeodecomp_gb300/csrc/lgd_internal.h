@@ -210,6 +210,9 @@ bool tma_applicable(const Grid& g);
 void launch_jacobi7_tma(Grid& g);
 bool varcoef_tma_applicable(const Grid& g);
 void launch_varcoef_tma(Grid& g);
+// two var-coef steps per pass (k_vctb.cu)
+bool varcoef_tb2_applicable(const Grid& g);
+void launch_varcoef_tb2(Grid& g);
 // temporal blocking (k_tb.cu): depth time steps per pass, 2 .. LGD_TB_MAX_DEPTH
 bool tb_applicable(const Grid& g);
 int tb_default_depth(const Grid& g);
