@@ -1,406 +1,405 @@
-// Surrogate convolution C -> C (C = 24) on the fifth-generation tensor
-// cores: tcgen05.mma with BF16 operands in shared memory and the FP32
-// accumulator in tensor memory.
+// The surrogate's 3^3 convolutions (C = 24) on the fifth-generation tensor
+// cores: tcgen05.mma with BF16 operands in shared memory and FP32 accumulators
+// in tensor memory.  One kernel, four input forms:
+//   MID    24 channels, ghosted BF16 activations (layers 2 and 3, and the
+//          input gradients of layers 2 and 3 with mirrored weights);
+//   FIRST  the fields u and kappa in FP32 (layer 1; rounded to BF16 here);
+//   LAST   24 channels -> 1 (layer 4);
+//   DLAST  the loss gradient 2 (du - target) / N, one channel (the input
+//          gradient of layer 4);
+// and three epilogues: ACT (bias, GELU, ghosted BF16 output, optionally the
+// FP32 pre-activations for the backward pass), GRAD (times GELU'(z), ghosted
+// BF16 output, bias gradient), OUT (FP32 du, or u += du).
 //
-// Activations for this path are "ghosted": BF16 [batch][nz+2][ny+2][nx+2][32],
-// the torus' wrapped neighbours stored in a one-voxel ghost layer (written
-// by the producing layer's epilogue), channels 24..31 zero.  A CTA owns a
-// 128 x 2 tile of output voxels of every plane of its z chunk and keeps:
-//   - the layer's weights, 27 taps x 32 x 32 BF16 (54 KiB, one bulk copy),
-//     as the MMA's B operand in the canonical K-major layout without
-//     swizzle: element (tap, cin, cout) at ((tap * 4 + cin / 8) * 32 + cout)
-//     * 16 B + cin % 8;
-//   - a ring of five input planes, each 4 channel groups x 4 rows x 130
-//     voxels x 8 channels, laid out [group][row][voxel][8 ch], i.e. voxels
-//     16 B apart: the canonical K-major layout of the A operand (8-voxel core
-//     matrices 128 B apart = SBO, channel groups one group block apart =
-//     LBO).  A tap shifts the A start address by whole voxels (16 B) and
-//     rows; no data moves.
-// Warp-specialised pipeline, no CTA-wide barrier inside the plane loop:
-//   - warps 9..12 (loaders) copy input planes into the ring with cp.async,
-//     16 B per request, each warp instruction 32 consecutive voxels of one
-//     channel group (the four groups of a voxel back to back, so the three
-//     re-reads of a 64-byte voxel hit L1); two planes in flight, each
-//     published to the MMA thread through the slot's "full" mbarrier (after
-//     a generic-to-async proxy fence) before the loader waits for the next
-//     free slot.  (A tensor-map copy would land the same
-//     layout, but its 16-byte box rows run at about one row per 7.5 cycles
-//     per SM, four times slower than the MMAs.)
-//   - warp 0, one thread: per output plane i it waits for input planes
-//     i .. i+2 and for the epilogue to have emptied TMEM accumulator buffer
-//     i % 2, issues 2 rows x 27 taps x 2 K-steps of M=128 (voxels), N=32
-//     (output channels), K=16 MMAs into that buffer and commits them to the
-//     buffer's mbarrier and to the "empty" mbarrier of input plane i's slot
-//     (plane i has no later reader);
-//   - warps 1..8 (the epilogue): each owns one TMEM lane quarter (32 voxels)
-//     and one output row; per plane it waits for the commit, reads its 32
-//     accumulator columns (tcgen05.ld), hands the buffer back and then
-//     applies bias, GELU, BF16 rounding and stores the voxel and its ghost
-//     copies.
+// Why this shape.  An MMA of 128 voxels x N x 16 reads 4 KB of A and 32 N
+// bytes of B from shared memory at 128 B per clock; with N = 24 (one tap at a
+// time) that read, not the multiplication, sets the time (2160 clocks per 128
+// voxels and layer).  So the three taps in z become N: when input plane q
+// arrives, the nine taps in (y, x) of all three output planes q - 2, q - 1, q
+// it reaches are multiplied at once, into three adjacent accumulators of 24
+// columns (N = 80).  An accumulator is complete after three input planes; the
+// epilogue reads it and puts the bias back into it, for the plane that takes
+// its place (three slots in rotation: the weights are stored twice over, so
+// that the rotation is a start address).  K runs over 9 taps x 24 channels =
+// 27 groups of 8; a K-step's two groups come from two taps, so that only the
+// last tap needs a zero group: 14 K-steps, 728 clocks of operand reads per 128
+// voxels (FIRST and DLAST: the three taps in x sit in the 8 channels of a
+// group, 2 K-steps).  And an input plane is used up at once: two or three
+// slots of input suffice.
+//
+// A CTA owns TXW x TY = 512 output voxels of every plane of its z chunk: four
+// accumulator tiles of 128 voxels (128 x 1, 64 x 2 or 32 x 4 each).  A plane
+// of input sits in shared memory as [channel group][row][8 voxels + 2 halo]
+// x 16 B: every 8-voxel core matrix brings its own halo, so tap (dy, dx) of
+// any tile is a start address and M may span rows.
+//   - warp 0, one thread: issues the MMAs, tile by tile;
+//   - warps 1 .. 16: epilogue of tile (w - 1) / 4, lane quarter w % 4;
+//   - warps 17 .. 20: fill the input slots (cp.async; FIRST and DLAST build
+//     their groups from the FP32 fields).
 // Every wait is bounded and gives up early once another role has failed; a
 // CTA that gives up sets the error word, lets its copies and MMAs finish and
 // frees its tensor memory.
-#include <cuda.h>
-#include <cuda_bf16.h>
+#include <algorithm>
 
 #include "lgd_internal.h"
+#include "tc_common.cuh"
+#include "conv_tc.h"
 
 namespace lgd {
 namespace sur {
-
 namespace tc {
 
-constexpr int TXO = 128;                    // output voxels per row tile (MMA M)
-constexpr int TYO = 2;                      // output rows per tile
-constexpr int R = TYO + 2;                  // halo rows per plane
-constexpr int HXV = TXO + 2;                // halo voxels per row
-constexpr int CP = 32;                      // channels stored per voxel
-constexpr int G = CP / 8;                   // 16-byte channel groups
-constexpr int GROUP_BYTES = R * HXV * 16;   // 8320
-constexpr int SLOT = G * GROUP_BYTES;       // 33280
-constexpr int S = 5;                        // ring slots
-constexpr int W_BYTES = 27 * G * CP * 16;   // 55296
-constexpr int SMEM = 128 + W_BYTES + S * SLOT;
-constexpr int EPI_WARPS = 8;                // epilogue warps: 4 lane quarters x 2 rows
-constexpr int LOAD_WARPS = 4;               // cp.async loaders
-constexpr int LOAD0 = 1 + EPI_WARPS;        // first loader warp
+enum { MID = 0, FIRST = 1, LAST = 2, DLAST = 3 };
+enum { ACT = 0, GRAD = 1, OUT = 2 };
+
+constexpr int TILES = 4;                    // accumulator tiles of 128 voxels per CTA
+constexpr int EPI_WARPS = 16;
+constexpr int LOAD_WARPS = 4;
 constexpr int THREADS = 32 * (1 + EPI_WARPS + LOAD_WARPS);
-constexpr int TMEM_COLS = 128;              // 2 buffers x 2 rows x 32 columns
-constexpr long long WAIT_CYCLES = 4000000000LL;
+constexpr int LOAD0 = 1 + EPI_WARPS;
+constexpr int S = 3;                        // input slots
 
-// kind::f16 instruction descriptor: FP32 accumulator, BF16 A and B, both
-// K-major, N = 32, M = 128
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(CP >> 3) << 17) | ((uint32_t)(TXO >> 4) << 24);
-
-__device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// shared-memory matrix descriptor, no swizzle: start, leading (K) and
-// stride (M/N) byte offsets in 16-byte units, descriptor version 1
-__device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile(
-        "{\n"
-        " .reg .pred p;\n"
-        " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        " selp.u32 %0, 1, 0, p;\n"
-        "}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
-{
-    if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try(bar, parity)) {
-        if (clock64() - t0 > WAIT_CYCLES) return false;
-    }
-    return true;
-}
-
-__device__ __forceinline__ void tma_4d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, int c3, uint32_t bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];" ::"r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-        : "memory");
-}
-
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void mma(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t acc)
-{
-    asm volatile(
-        "{\n"
-        " .reg .pred p;\n"
-        " setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(dtmem),
-        "l"(a), "l"(b), "r"(IDESC), "r"(acc)
-        : "memory");
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// 32 consecutive accumulator columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
-{
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
-
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
-{
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(lo)) |
-           ((uint32_t)__bfloat16_as_ushort(__float2bfloat16(hi)) << 16);
-}
-
-struct Params {
-    int nx, ny, nz, batch, zchunk;
+template<int SRC, int TXW>
+struct Geo {
+    static constexpr bool WIDE = SRC == MID || SRC == LAST;     // 24 channels with halo, else one built group
+    static constexpr int TY = 512 / TXW;
+    static constexpr int ROWS = TY + 2;
+    static constexpr int NG = TXW / 8;
+    static constexpr int VOX = WIDE ? 10 : 8;                   // voxels stored per group of 8
+    static constexpr int GS = VOX * 16;                         // bytes of a group (SBO)
+    static constexpr int ROWP = NG * GS;
+    static constexpr int CGS = ROWS * ROWP;                     // channel-group stride
+    static constexpr int SLOT = (WIDE ? 3 : 1) * CGS;
+    static constexpr int KSTEPS = WIDE ? 14 : 2;
+    static constexpr int N = SRC == LAST ? 16 : 80;
+    static constexpr int KS_BYTES = SRC == LAST ? 2 * 2 * 128 : 2 * 16 * 128;     // B of one K-step
+    static constexpr int W_BYTES = KSTEPS * KS_BYTES * (SRC == LAST ? 3 : 1);
+    static constexpr int TCOLS = SRC == LAST ? 16 : 128;        // columns between tiles
+    static constexpr int TMEM = SRC == LAST ? 64 : 512;
+    static constexpr int SMEM = 128 + W_BYTES + S * SLOT;
 };
 
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+struct Params {
+    Shape s;
+    int zchunk;
+    const bf16 *in;             // MID, LAST: ghosted
+    const float *f0, *f1;       // FIRST: u, kappa; DLAST: du, target
+    float scale;                // DLAST: 2 / N
+    const bf16 *w;              // packed weights
+    const float *bias;          // ACT, OUT
+    bf16 *out;                  // ACT, GRAD: ghosted
+    float *z;                   // ACT: pre-activations out (or null); GRAD: in
+    float *db;                  // GRAD: bias gradient, added to
+    float *fout;                // OUT
+    int add;                    // OUT: add to fout
+    int *err;
+};
+
+// position of voxel (x, y) of plane z in the pre-activations: FP32
+// [batch][nz][ny][6][nx][4], the float4 of channels 4 c .. 4 c + 3 at + c * nx
+__device__ __forceinline__ long long z_at(const Shape& s, int b, int z, int y, int x)
 {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+    return ((((long long)b * s.nz + z) * s.ny + y) * 6) * s.nx + x;
 }
 
-// bounded wait that also gives up as soon as another role has failed
-__device__ __forceinline__ bool mbar_wait_or_fail(uint32_t bar, uint32_t parity, volatile int *fail)
-{
-    if (mbar_try(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try(bar, parity)) {
-        if (*fail || clock64() - t0 > WAIT_CYCLES) return false;
-    }
-    return true;
-}
-
+template<int SRC, int EPI, int TXW>
 __global__ void __launch_bounds__(THREADS, 1)
-conv_tc_kernel(const __nv_bfloat16 *__restrict__ in, const __nv_bfloat16 *__restrict__ wpacked,
-               const float *__restrict__ bias, __nv_bfloat16 *__restrict__ out, Params p, int *err)
+conv_tc_kernel(const Params p)
 {
+    typedef Geo<SRC, TXW> G;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_w;
-    __shared__ __align__(8) uint64_t bar_full[S];     // input plane in its slot (one arrive per loader warp)
-    __shared__ __align__(8) uint64_t bar_empty[S];    // input slot no longer read (MMA commit)
-    __shared__ __align__(8) uint64_t bar_mma[2];      // accumulator buffer written (MMA commit)
-    __shared__ __align__(8) uint64_t bar_free[2];     // accumulator buffer read by the epilogue
+    __shared__ __align__(8) uint64_t bar_full[S];       // input plane in its slot (one arrive per loader warp)
+    __shared__ __align__(8) uint64_t bar_empty[S];      // input slot no longer read (MMA commit)
+    __shared__ __align__(8) uint64_t bar_mma[TILES];    // a plane's MMAs of the tile done
+    __shared__ __align__(8) uint64_t bar_free[TILES];   // its completed accumulator read and started over
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
+    __shared__ float s_db[24];
     volatile int *fail = &s_fail;
 
     unsigned char *smem = smem_raw + ((128 - (saddr(smem_raw) & 127)) & 127);
     unsigned char *wsm = smem;
-    unsigned char *ring = smem + W_BYTES;
+    unsigned char *ring = smem + G::W_BYTES;
 
+    const Shape s = p.s;
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
-    const int x0 = blockIdx.x * TXO;
-    const int y0 = blockIdx.y * TYO;
-    const int zsplit = (p.nz + p.zchunk - 1) / p.zchunk;
+    const int x0 = blockIdx.x * TXW;
+    const int y0 = blockIdx.y * G::TY;
+    const int zsplit = (s.nz + p.zchunk - 1) / p.zchunk;
     const int b = blockIdx.z / zsplit;
     const int z0 = (blockIdx.z % zsplit) * p.zchunk;
-    const int z1 = min(z0 + p.zchunk, p.nz);
-    const int n = z1 - z0;                  // output planes; input planes q = 0 .. n+1
-    const int zg0 = b * (p.nz + 2) + z0;    // ghosted z of input plane q = 0
+    const int n = min(z0 + p.zchunk, s.nz) - z0;        // output planes j = 0 .. n - 1; input planes q = 0 .. n + 1
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s_tmem)),
-                     "r"(TMEM_COLS)
+                     "r"(G::TMEM)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // MMA-thread state (thread 0 only)
-    int waited = 0;         // input planes waited for
-    int committed = 0;      // output planes whose MMAs were committed
-    bool w_ready = false;
     if (tid == 0) {
         s_fail = 0;
         mbar_init(saddr(&bar_w), 1);
-        for (int s = 0; s < S; ++s) {
-            mbar_init(saddr(&bar_full[s]), LOAD_WARPS);
-            mbar_init(saddr(&bar_empty[s]), 1);
+        for (int i = 0; i < S; ++i) {
+            mbar_init(saddr(&bar_full[i]), LOAD_WARPS);
+            mbar_init(saddr(&bar_empty[i]), 1);
         }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(saddr(&bar_mma[s]), 1);
-            mbar_init(saddr(&bar_free[s]), EPI_WARPS);
+        for (int i = 0; i < TILES; ++i) {
+            mbar_init(saddr(&bar_mma[i]), 1);
+            mbar_init(saddr(&bar_free[i]), 4);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        mbar_expect_tx(saddr(&bar_w), W_BYTES);
-        bulk_copy(saddr(wsm), wpacked, W_BYTES, saddr(&bar_w));
+    }
+    if (EPI == GRAD && tid < 24) s_db[tid] = 0.f;
+    dependent_start();
+    if (tid == 0) {
+        mbar_expect_tx(saddr(&bar_w), G::W_BYTES);
+        bulk_copy(saddr(wsm), p.w, G::W_BYTES, saddr(&bar_w));
     }
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = s_tmem;
+    int committed = 0;                                  // thread 0: tiles committed, over all planes
+    bool w_ready = false;
 
     if (warp == 0) {
         if (lane == 0) {
-            bool ok = mbar_wait_or_fail(saddr(&bar_w), 0, fail);
+            bool ok = mbar_wait(saddr(&bar_w), 0, fail);
             w_ready = ok;
-            const uint32_t rbase = saddr(ring);
-            const uint64_t wd = sdesc(saddr(wsm), CP * 16, 128);
-            for (int i = 0; ok && i < n; ++i) {
-                while (ok && waited <= i + 2) {
-                    ok = mbar_wait_or_fail(saddr(&bar_full[waited % S]), (uint32_t)((waited / S) & 1), fail);
-                    if (ok) ++waited;
-                }
-                if (ok && i >= 2) ok = mbar_wait_or_fail(saddr(&bar_free[i & 1]), (uint32_t)(((i - 2) >> 1) & 1), fail);
+            const uint32_t rbase = saddr(ring), wbase = saddr(wsm);
+            constexpr uint32_t ID = idesc(128, G::N, false);
+            for (int q = 0; ok && q < n + 2; ++q) {
+                ok = mbar_wait(saddr(&bar_full[q % S]), (uint32_t)((q / S) & 1), fail);
                 if (!ok) break;
                 fence_after();
-                // descriptors: one base per input slot, every MMA adds a
-                // compile-time offset (16-byte units) to the address field
-                // (addresses stay below 2^18, so nothing carries out of it)
-                uint64_t sd[3];
-                const int i_slot = i % S;
+                const uint32_t slot = rbase + (uint32_t)((q % S) * G::SLOT);
+                // the block order of the three accumulators (see pack_kernel)
+                const uint32_t rot = (uint32_t)((3 - q % 3) % 3);
+                const uint64_t wd = SRC == LAST ? sdesc(wbase + rot * (G::KSTEPS * G::KS_BYTES), 2 * 128, 128)
+                                                : sdesc(wbase + rot * 3 * 128, 16 * 128, 128);
+                // a K-step's descriptor: start and leading offset of its two
+                // groups (compile-time), added to the tile's base
+                const uint64_t base = sdesc(slot, 0, G::GS);
 #pragma unroll
-                for (int dz = 0; dz < 3; ++dz) {
-                    const int sl = (i_slot + dz >= S) ? i_slot + dz - S : i_slot + dz;
-                    sd[dz] = sdesc(rbase + (uint32_t)(sl * SLOT), GROUP_BYTES, 128);
-                }
+                for (int m = 0; m < TILES; ++m) {
+                    ok = mbar_wait(saddr(&bar_free[m]), (uint32_t)(q & 1), fail);
+                    if (!ok) break;
+                    fence_after();
+                    const uint32_t d = tmem + (uint32_t)(m * G::TCOLS);
 #pragma unroll
-                for (int r = 0; r < TYO; ++r) {
-                    const uint32_t d = tmem + (uint32_t)((i & 1) * 64 + r * 32);
-#pragma unroll
-                    for (int tap = 0; tap < 27; ++tap) {
-                        const int dz = tap / 9, dy = (tap / 3) % 3, dx = tap % 3;
-#pragma unroll
-                        for (int s = 0; s < 2; ++s) {
-                            const uint64_t a = sd[dz] + (uint64_t)(((2 * s) * R + r + dy) * HXV + dx);
-                            const uint64_t bw = wd + (uint64_t)((tap * G + 2 * s) * CP);
-                            mma(d, a, bw, (tap | s) ? 1u : 0u);
+                    for (int k = 0; k < G::KSTEPS; ++k) {
+                        uint32_t first, lead;           // bytes
+                        if (G::WIDE) {
+                            if (k < 12) {               // taps 2 (k / 3) and 2 (k / 3) + 1, channel group k % 3
+                                const int ta = 2 * (k / 3), tb = ta + 1;
+                                const int oa = (ta / 3) * G::ROWP + (ta % 3) * 16;
+                                const int ob = (tb / 3) * G::ROWP + (tb % 3) * 16;
+                                first = (uint32_t)(oa + (k % 3) * G::CGS);
+                                lead = (uint32_t)(ob - oa);
+                            } else {                    // tap 8: groups 0, 1 and 1 (zero weights), 2
+                                first = (uint32_t)(2 * G::ROWP + 2 * 16 + (k - 12) * G::CGS);
+                                lead = (uint32_t)G::CGS;
+                            }
+                        } else {                        // rows 0, 1 and 1 (zero weights), 2
+                            first = (uint32_t)(k * G::ROWP);
+                            lead = (uint32_t)G::ROWP;
                         }
+                        const uint64_t a = base + ((uint64_t)(lead >> 4) << 16) + (uint64_t)((first + m * 16 * G::GS) >> 4);
+                        mma(d, a, wd + (uint64_t)((k * G::KS_BYTES) >> 4), ID, 1u);
                     }
+                    mma_commit(saddr(&bar_mma[m]));
+                    ++committed;
                 }
-                mma_commit(saddr(&bar_mma[i & 1]));
-                mma_commit(saddr(&bar_empty[i % S]));     // plane i has no later reader
-                committed = i + 1;
+                if (!ok) break;
+                mma_commit(saddr(&bar_empty[q % S]));
             }
             if (!ok) s_fail = 1;
         }
         __syncwarp();
     } else if (warp >= LOAD0) {
-        // loaders: input plane q into slot q % S, [group][row][voxel][8 ch]
         const int lt = tid - LOAD0 * 32;
-        const long long gnx = p.nx + 2;
         int published = 0;
         bool ok = true;
-        auto publish = [&](int upto) {          // planes published .. upto-1 have landed
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        auto publish = [&](int upto) {
+            fence_async_proxy();
             __syncwarp();
             for (; published < upto; ++published) {
                 if (lane == 0) mbar_arrive(saddr(&bar_full[published % S]));
             }
         };
-        for (int q = 0; q <= n + 1; ++q) {
-            const int slot = q % S;
-            // publish what has landed before waiting for a slot: plane q-2
-            // (all groups but the newest are complete), so the MMAs of the
-            // plane that frees this slot never wait on this loader
-            if (q >= 2) {
+        for (int q = 0; q < n + 2; ++q) {
+            // publish what has landed before waiting for a slot: the MMAs that
+            // free it never wait on this loader
+            if (G::WIDE && q >= 2) {
                 asm volatile("cp.async.wait_group 1;" ::: "memory");
                 publish(q - 1);
             }
             if (q >= S) {
-                const bool got = mbar_wait_or_fail(saddr(&bar_empty[slot]), (uint32_t)(((q - S) / S) & 1), fail);
+                const bool got = mbar_wait(saddr(&bar_empty[q % S]), (uint32_t)(((q - S) / S) & 1), fail);
                 if (!__all_sync(0xffffffffu, got)) {
                     ok = false;
                     break;
                 }
             }
-            unsigned char *dst = ring + slot * SLOT;
-            const long long base = ((long long)(zg0 + q) * (p.ny + 2) + y0) * gnx + x0;   // ghosted voxel (row 0, voxel 0)
-            for (int v = lt; v < R * HXV; v += LOAD_WARPS * 32) {
-                const int yy = v / HXV;
-                const int xx = v - yy * HXV;
-                const __nv_bfloat16 *src = in + (base + (long long)yy * gnx + xx) * CP;
+            const uint32_t slot = saddr(ring) + (uint32_t)((q % S) * G::SLOT);
+            if (G::WIDE) {
+                constexpr int PER_ROW = G::NG * 10;
+                for (int v = lt; v < G::ROWS * PER_ROW; v += LOAD_WARPS * 32) {
+                    const int r = v / PER_ROW;
+                    const int i = v - r * PER_ROW;              // group i / 10, voxel i % 10 of it
+                    const int gy = min(y0 + r, s.ny + 1);       // ghosted row (rows past the grid: any)
+                    const bf16 *src = p.in + (ghost_row(s, b, z0 + q, gy) * (s.nx + 2) + x0 + (i / 10) * 8 + i % 10) * 8;
+                    const uint32_t d = slot + (uint32_t)(r * G::ROWP + i * 16);
 #pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const uint32_t d = saddr(dst + ((g * R + yy) * HXV + xx) * 16);
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src + 8 * g) : "memory");
+                    for (int c = 0; c < 3; ++c) copy16(d + c * G::CGS, src + (long long)c * (s.nx + 2) * 8);
                 }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            } else {
+                int z = z0 - 1 + q;
+                z = z < 0 ? z + s.nz : (z >= s.nz ? z - s.nz : z);
+                for (int v = lt; v < G::ROWS * TXW; v += LOAD_WARPS * 32) {
+                    const int r = v / TXW;
+                    const int x = x0 + v % TXW;
+                    int y = y0 - 1 + r;
+                    y = y < 0 ? y + s.ny : (y >= s.ny ? (y - s.ny) % s.ny : y);
+                    const int xw = x == 0 ? s.nx - 1 : x - 1;
+                    const int xe = x == s.nx - 1 ? 0 : x + 1;
+                    const long long row = (((long long)b * s.nz + z) * s.ny + y) * s.nx;
+                    const float *a = p.f0 + row, *c = p.f1 + row;
+                    uint4 w;
+                    if (SRC == FIRST) {
+                        w = make_uint4(pack_bf16(a[xw], c[xw]), pack_bf16(a[x], c[x]), pack_bf16(a[xe], c[xe]), 0u);
+                    } else {
+                        w = make_uint4(pack_bf16(p.scale * (a[xw] - c[xw]), p.scale * (a[x] - c[x])),
+                                       pack_bf16(p.scale * (a[xe] - c[xe]), 0.f), 0u, 0u);
+                    }
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(slot + (uint32_t)(v * 16)), "r"(w.x),
+                                 "r"(w.y), "r"(w.z), "r"(w.w)
+                                 : "memory");
+                }
+                publish(q + 1);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (G::WIDE) asm volatile("cp.async.wait_all;" ::: "memory");
         if (ok) publish(n + 2);
         else if (lane == 0) s_fail = 1;
     } else {
-        // epilogue: lane quarter qd (TMEM lanes 32 qd .. 32 qd + 31 = voxels),
-        // output row r of the tile
-        const int qd = warp & 3;
-        const int r = (warp - 1) >> 2;
-        const int x = x0 + qd * 32 + lane;
-        const int y = y0 + r;
-        int xs[3], ys[3];         // an axis of extent 1 has both ghost copies
-        int nxs = 1, nys = 1;
-        xs[0] = x + 1;
-        if (x == 0) xs[nxs++] = p.nx + 1;
-        if (x == p.nx - 1) xs[nxs++] = 0;
-        ys[0] = y + 1;
-        if (y == 0) ys[nys++] = p.ny + 1;
-        if (y == p.ny - 1) ys[nys++] = 0;
-        float bv[24];
+        const int m = (warp - 1) >> 2;                  // tile
+        const int qd = warp & 3;                        // lane quarter this warp may read
+        const int vt = m * 128 + qd * 32 + lane;        // voxel of the CTA's 512
+        const int x = x0 + vt % TXW;
+        const int y = y0 + vt / TXW;
+        const bool live = y < s.ny;
+        const uint32_t acc = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(m * G::TCOLS);
+        float db[EPI == GRAD ? 24 : 1] = {};
+        const float b1 = EPI == OUT ? __ldg(p.bias) : 0.f;
+        // accumulator slot (columns) j % 3 starts at the bias (OUT adds it at the end)
+        auto restart = [&](int slot) {
+            if constexpr (EPI == OUT) {
+                tmem_st1(acc + (uint32_t)slot, 0.f);
+            } else {
 #pragma unroll
-        for (int c = 0; c < 24; ++c) bv[c] = __ldg(bias + c);
-        for (int j = 0; j < n; ++j) {
-            const bool ok = mbar_wait_or_fail(saddr(&bar_mma[j & 1]), (uint32_t)((j >> 1) & 1), fail);
+                for (int c = 0; c < 3; ++c) {
+                    float v[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[i] = EPI == ACT ? __ldg(p.bias + c * 8 + i) : 0.f;
+                    tmem_st8(acc + (uint32_t)(slot * 24 + c * 8), v);
+                }
+            }
+            tmem_st_wait();
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(saddr(&bar_free[m]));
+        };
+        restart(0);
+        for (int q = 0; q < n + 2; ++q) {
+            const bool ok = mbar_wait(saddr(&bar_mma[m]), (uint32_t)(q & 1), fail);
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) s_fail = 1;
                 break;
             }
             fence_after();
-            float v[32];
-            tmem_ld32(tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)((j & 1) * 64 + r * 32), v);
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(saddr(&bar_free[j & 1]));
-            uint32_t w[12];
-#pragma unroll
-            for (int c = 0; c < 12; ++c) w[c] = pack_bf16(gelu(v[2 * c] + bv[2 * c]), gelu(v[2 * c + 1] + bv[2 * c + 1]));
-            const int zz = z0 + j;
-            int zs[3];
-            int nzs = 1;
-            zs[0] = zz + 1;
-            if (zz == 0) zs[nzs++] = p.nz + 1;
-            if (zz == p.nz - 1) zs[nzs++] = 0;
-            for (int a = 0; a < nzs; ++a) {
-                for (int bb = 0; bb < nys; ++bb) {
-                    for (int c = 0; c < nxs; ++c) {
-                        const long long vox =
-                            (((long long)b * (p.nz + 2) + zs[a]) * (p.ny + 2) + ys[bb]) * (p.nx + 2) + xs[c];
-                        uint4 *o = reinterpret_cast<uint4 *>(out + vox * CP);
-                        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-                        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
-                        o[2] = make_uint4(w[8], w[9], w[10], w[11]);
-                        o[3] = make_uint4(0u, 0u, 0u, 0u);
-                    }
+            const int slot = (q + 1) % 3;               // output q - 2 is complete, q + 1 takes its place
+            const int z = z0 + q - 2;
+            if constexpr (EPI == OUT) {
+                const float v = tmem_ld1(acc + (uint32_t)slot);
+                restart(slot);
+                if (q >= 2 && live) {
+                    float *o = p.fout + (((long long)b * s.nz + z) * s.ny + y) * s.nx + x;
+                    if (p.add) *o += v + b1;
+                    else *o = v + b1;
                 }
+            } else {
+                float v[24];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    float t[8];
+                    tmem_ld8(acc + (uint32_t)(slot * 24 + c * 8), t);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[c * 8 + i] = t[i];
+                }
+                restart(slot);
+                if (q < 2 || !live) continue;
+                if constexpr (EPI == ACT) {
+                    if (p.z) {
+                        float4 *zp = reinterpret_cast<float4 *>(p.z) + z_at(s, b, z, y, x);
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) {
+                            zp[(long long)c * s.nx] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < 24; ++c) v[c] = gelu(v[c]);
+                } else {
+                    const float4 *zp = reinterpret_cast<const float4 *>(p.z) + z_at(s, b, z, y, x);
+#pragma unroll
+                    for (int c = 0; c < 6; ++c) {
+                        const float4 t = zp[(long long)c * s.nx];
+                        v[4 * c] *= gelu_grad(t.x);
+                        v[4 * c + 1] *= gelu_grad(t.y);
+                        v[4 * c + 2] *= gelu_grad(t.z);
+                        v[4 * c + 3] *= gelu_grad(t.w);
+                    }
+#pragma unroll
+                    for (int c = 0; c < 24; ++c) db[c] += v[c];
+                }
+                uint4 w[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    w[c] = make_uint4(pack_bf16(v[8 * c], v[8 * c + 1]), pack_bf16(v[8 * c + 2], v[8 * c + 3]),
+                                      pack_bf16(v[8 * c + 4], v[8 * c + 5]), pack_bf16(v[8 * c + 6], v[8 * c + 7]));
+                }
+                // the voxel and its ghost copies (an axis of extent 1 has both)
+                auto put = [&](int gz, int gy, int gx) {
+                    uint4 *o = reinterpret_cast<uint4 *>(p.out) + ghost_row(s, b, gz, gy) * (s.nx + 2) + gx;
+                    o[0] = w[0];
+                    o[s.nx + 2] = w[1];
+                    o[2 * (s.nx + 2)] = w[2];
+                };
+                auto put_x = [&](int gz, int gy) {
+                    put(gz, gy, x + 1);
+                    if (x == 0) put(gz, gy, s.nx + 1);
+                    if (x == s.nx - 1) put(gz, gy, 0);
+                };
+                auto put_y = [&](int gz) {
+                    put_x(gz, y + 1);
+                    if (y == 0) put_x(gz, s.ny + 1);
+                    if (y == s.ny - 1) put_x(gz, 0);
+                };
+                put_y(z + 1);
+                if (z == 0) put_y(s.nz + 1);
+                if (z == s.nz - 1) put_y(0);
+            }
+        }
+        if constexpr (EPI == GRAD) {
+#pragma unroll
+            for (int c = 0; c < 24; ++c) {
+                float t = db[c];
+                for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+                if (lane == 0) atomicAdd(&s_db[c], t);
             }
         }
     }
@@ -408,91 +407,222 @@ conv_tc_kernel(const __nv_bfloat16 *__restrict__ in, const __nv_bfloat16 *__rest
     fence_before();
     __syncthreads();            // every role has left its loop; no copy is in flight
     fence_after();
+    if (EPI == GRAD && tid < 24) atomicAdd(p.db + tid, s_db[tid]);
     if (s_fail) {
         // report, then wait (bounded) for the MMAs and the weight copy
         if (tid == 0) {
-            atomicExch(err, 1);
-            if (committed > 0) mbar_wait(saddr(&bar_mma[(committed - 1) & 1]), ((committed - 1) >> 1) & 1);
-            if (!w_ready) mbar_wait(saddr(&bar_w), 0);
+            atomicExch(p.err, 1);
+            for (int m = 0; m < TILES; ++m) {
+                const int c = (committed + TILES - 1 - m) / TILES;      // commits of this tile
+                if (c > 0) mbar_wait(saddr(&bar_mma[m]), (uint32_t)((c - 1) & 1), nullptr);
+            }
+            if (!w_ready) mbar_wait(saddr(&bar_w), 0, nullptr);
         }
         fence_before();
         __syncthreads();
         fence_after();
     }
     if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G::TMEM) : "memory");
     }
 }
 
-// FP32 W[tap][cin][cout] (cin = cout = 24) -> BF16 B operand layout
-__global__ void pack_tc_weights_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ out)
+// Weights of one convolution as the MMA's B operand, K-major without swizzle:
+// [K-step][group 0, 1][N group of 8][8 columns][8 k].  Columns: blocks of 24
+// output channels in the z-tap order 0, 2, 1, 0, 2 (and 8 zeros); at input
+// plane q the accumulators 0, 1, 2 take taps (q - s) mod 3, which is the
+// window of three blocks that starts at block (3 - q % 3) % 3.  LAST has one
+// output channel: columns 0, 1, 2 are the accumulators, one copy per rotation.
+// W: FP32 [tap][cin][cout]; mirror: the input-gradient convolution (taps
+// mirrored, channel roles swapped).
+__global__ void pack_kernel(const float *w, bf16 *out, int src, int mirror)
 {
-    const int total = 27 * G * CP * 8;
+    const int ksteps = src == MID || src == LAST ? 14 : 2;
+    const int ng = src == LAST ? 2 : 16;
+    const int copies = src == LAST ? 3 : 1;
+    const int total = copies * ksteps * 2 * ng * 64;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const int k8 = i & 7;
-        const int co = (i >> 3) & (CP - 1);
-        const int g = (i >> 8) & (G - 1);
-        const int tap = i >> 10;
-        const int ci = g * 8 + k8;
-        const float v = (ci < 24 && co < 24) ? w[(tap * 24 + ci) * 24 + co] : 0.f;
+        const int col = ((i >> 6) % ng) * 8 + ((i >> 3) & 7);
+        const int half = (i / (64 * ng)) & 1;
+        const int ks = (i / (128 * ng)) % ksteps;
+        const int rot = i / (128 * ng * ksteps);
+        int dz = -1, co = 0;
+        if (src == LAST) {
+            if (col < 3) {
+                const int order[5] = {0, 2, 1, 0, 2};
+                dz = order[rot + col];
+            }
+        } else if (col < 120) {
+            const int order[5] = {0, 2, 1, 0, 2};
+            dz = order[col / 24];
+            co = col % 24;
+        }
+        int tap = -1, ci = 0;                       // tap in (y, x), input channel
+        if (src == MID || src == LAST) {
+            if (ks < 12) {
+                tap = 2 * (ks / 3) + half;
+                ci = (ks % 3) * 8 + k8;
+            } else if (!(ks == 13 && half == 0)) {
+                tap = 8;
+                ci = (ks - 12 + half) * 8 + k8;
+            }
+        } else {
+            const int dy = ks + half;               // ks 1, half 0 repeats row 1 with zero weights
+            if (!(ks == 1 && half == 0)) {
+                if (src == FIRST && k8 < 6) {
+                    tap = dy * 3 + k8 / 2;
+                    ci = k8 & 1;
+                } else if (src == DLAST && k8 < 3) {
+                    tap = dy * 3 + k8;
+                }
+            }
+        }
+        float v = 0.f;
+        if (dz >= 0 && tap >= 0) {
+            const int t = dz * 9 + tap;
+            if (src == MID) v = mirror ? w[((26 - t) * 24 + co) * 24 + ci] : w[(t * 24 + ci) * 24 + co];
+            else if (src == LAST) v = w[t * 24 + ci];
+            else if (src == FIRST) v = w[(t * 2 + ci) * 24 + co];
+            else v = w[(26 - t) * 24 + co];
+        }
         out[i] = __float2bfloat16(v);
     }
 }
 
-}  // namespace tc
-
-bool tc_applicable(int nx, int ny, int channels)
+// planes per CTA: waves of one CTA per SM times planes per CTA (two of them
+// halo, and about two planes' time to start and to drain)
+static int pick_zchunk(long long xy, int nz, int sms)
 {
-    return channels == 24 && nx % tc::TXO == 0 && ny % tc::TYO == 0;
-}
-
-size_t tc_weight_bytes() { return tc::W_BYTES; }
-
-void tc_pack_weights(const float *w, void *out, cudaStream_t stream)
-{
-    tc::pack_tc_weights_kernel<<<27, 256, 0, stream>>>(w, (__nv_bfloat16 *)out);
-    check_launch("pack tensor-core weights");
-}
-
-// one C -> C layer: ghosted BF16 in -> ghosted BF16 out (GELU(conv + bias))
-void tc_conv(void *map_cache, const void *in, void *out, const void *wpacked, const float *bias, int nx, int ny, int nz,
-             int batch, cudaStream_t stream, int *d_err)
-{
-    static PerDevice<long long> setup;
-    const long long resident = setup.get([] {
-        LGD_CHECK_CUDA(cudaFuncSetAttribute(tc::conv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::SMEM));
-        int dev = 0, sms = 0;
-        LGD_CHECK_CUDA(cudaGetDevice(&dev));
-        LGD_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        return (long long)sms;
-    });
-    (void)map_cache;
-    // z chunks: whole waves of one CTA per SM
-    const long long xy = (long long)(nx / tc::TXO) * (ny / tc::TYO) * batch;
     int best_chunk = nz;
     double best = 1e300;
-    for (int split = 1; split <= std::max(1, nz / 4); ++split) {
+    for (int split = 1; split <= std::max(1, nz / 2); ++split) {
         const int chunk = (nz + split - 1) / split;
-        const int s = (nz + chunk - 1) / chunk;
-        const long long waves = (xy * s + resident - 1) / resident;
-        const double t = (double)waves * (chunk + 2);
+        const int c = (nz + chunk - 1) / chunk;
+        const double t = (double)((xy * c + sms - 1) / sms) * (chunk + 4);
         if (t < best * 0.999) {
             best = t;
             best_chunk = chunk;
         }
     }
-    tc::Params p;
-    p.nx = nx;
-    p.ny = ny;
-    p.nz = nz;
-    p.batch = batch;
-    p.zchunk = best_chunk;
-    const int zsplit = (nz + best_chunk - 1) / best_chunk;
-    dim3 grid(nx / tc::TXO, ny / tc::TYO, batch * zsplit);
-    tc::conv_tc_kernel<<<grid, tc::THREADS, tc::SMEM, stream>>>((const __nv_bfloat16 *)in,
-                                                                 (const __nv_bfloat16 *)wpacked, bias,
-                                                                 (__nv_bfloat16 *)out, p, d_err);
+    return best_chunk;
+}
+
+template<int SRC, int EPI, int TXW>
+static void run(Params p, cudaStream_t stream)
+{
+    typedef Geo<SRC, TXW> G;
+    static PerDevice<int> setup;
+    const int sms = setup.get([] {
+        auto *fn = conv_tc_kernel<SRC, EPI, TXW>;
+        LGD_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM));
+        int dev = 0, count = 0;
+        LGD_CHECK_CUDA(cudaGetDevice(&dev));
+        LGD_CHECK_CUDA(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev));
+        return count;
+    });
+    const int bx = p.s.nx / TXW, by = (p.s.ny + G::TY - 1) / G::TY;
+    p.zchunk = pick_zchunk((long long)bx * by * p.s.batch, p.s.nz, sms);
+    const int zsplit = (p.s.nz + p.zchunk - 1) / p.zchunk;
+    launch_dependent(conv_tc_kernel<SRC, EPI, TXW>, dim3(bx, by, p.s.batch * zsplit), THREADS, G::SMEM, stream, p);
     check_launch("tensor-core convolution");
+}
+
+template<int SRC, int EPI>
+static void run_any(const Params& p, cudaStream_t stream)
+{
+    if (p.s.nx % 128 == 0) run<SRC, EPI, 128>(p, stream);
+    else if (p.s.nx % 64 == 0) run<SRC, EPI, 64>(p, stream);
+    else run<SRC, EPI, 32>(p, stream);
+}
+
+}  // namespace tc
+
+using namespace tc;
+
+bool tc_applicable(int nx, int ny, int channels)
+{
+    return channels == 24 && nx % 32 == 0 && ny >= 1;
+}
+
+static const size_t PACKED = 14 * 2 * 16 * 64;      // elements of the largest packed operand
+
+TcWeights tc_alloc_weights(bool training)
+{
+    TcWeights w = {};
+    bf16 *base = nullptr;
+    LGD_CHECK_CUDA(cudaMalloc(&base, (training ? 7 : 4) * PACKED * sizeof(bf16)));
+    w.base = base;
+    for (int l = 0; l < 4; ++l) w.fwd[l] = base + l * PACKED;
+    if (training) {
+        for (int l = 1; l < 4; ++l) w.grad[l] = base + (3 + l) * PACKED;
+    }
+    return w;
+}
+
+void tc_free_weights(TcWeights& w) { cudaFree(w.base); }
+
+int tc_pack_weights(const float *const layer[4], const TcWeights& w, cudaStream_t stream)
+{
+    const int src[4] = {FIRST, MID, MID, LAST};
+    int launches = 0;
+    for (int l = 0; l < 4; ++l, ++launches) pack_kernel<<<56, 256, 0, stream>>>(layer[l], (bf16 *)w.fwd[l], src[l], 0);
+    if (w.grad[1]) {
+        const int gsrc[4] = {0, MID, MID, DLAST};
+        for (int l = 1; l < 4; ++l, ++launches) {
+            pack_kernel<<<56, 256, 0, stream>>>(layer[l], (bf16 *)w.grad[l], gsrc[l], 1);
+        }
+    }
+    check_launch("pack tensor-core weights");
+    return launches;
+}
+
+size_t tc_ghost_bytes(int nx, int ny, int nz, int batch)
+{
+    return (size_t)batch * (nz + 2) * (ny + 2) * 3 * (nx + 2) * 16;
+}
+
+void tc_layer1(const float *u, const float *k, const void *w, const float *bias, void *out, float *z, const int dims[4],
+               int *err, cudaStream_t stream)
+{
+    Params p = {};
+    p.s = {dims[0], dims[1], dims[2], dims[3]};
+    p.f0 = u;
+    p.f1 = k;
+    p.w = (const bf16 *)w;
+    p.bias = bias;
+    p.out = (bf16 *)out;
+    p.z = z;
+    p.err = err;
+    run_any<FIRST, ACT>(p, stream);
+}
+
+void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, float *z, const int dims[4], int *err,
+                  cudaStream_t stream)
+{
+    Params p = {};
+    p.s = {dims[0], dims[1], dims[2], dims[3]};
+    p.in = (const bf16 *)in;
+    p.w = (const bf16 *)w;
+    p.bias = bias;
+    p.out = (bf16 *)out;
+    p.z = z;
+    p.err = err;
+    run_any<MID, ACT>(p, stream);
+}
+
+void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, const int dims[4], int *err,
+                   cudaStream_t stream)
+{
+    Params p = {};
+    p.s = {dims[0], dims[1], dims[2], dims[3]};
+    p.in = (const bf16 *)in;
+    p.w = (const bf16 *)w;
+    p.bias = bias;
+    p.fout = out;
+    p.add = add ? 1 : 0;
+    p.err = err;
+    run_any<LAST, OUT>(p, stream);
 }
 
 }  // namespace sur

@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "lgd_internal.h"
+#include "conv_tc.h"
 #include "../../include/lgd_surrogate.h"
 
 namespace lgd {
@@ -66,10 +67,9 @@ struct Geo {
 };
 
 // Halo tile of the layer input for the CTA at (x0, y0, z, b): (TX+2) x 6 x 3
-// voxels, wrapped on the torus, CIN BF16 channels each (CIN even).  GIN:
-// the input is ghosted ([batch][nz+2][ny+2][nx+2][32], the wrapped
-// neighbours stored in the ghost layer), else dense [V][CIN].
-template<int CIN, int TX, bool GIN = false>
+// voxels, wrapped on the torus, CIN BF16 channels each (CIN even), from dense
+// [V][CIN].
+template<int CIN, int TX>
 __device__ __forceinline__ void load_halo(uint32_t *halo, const bf16 *__restrict__ in, const Geo& g, int x0, int y0,
                                           int z, int b)
 {
@@ -87,52 +87,19 @@ __device__ __forceinline__ void load_halo(uint32_t *halo, const bf16 *__restrict
         int gx = x0 - 1 + hx;
         int gy = y0 - 1 + hy;
         int gz = z - 1 + hz;
-        if (GIN) {
-            const long long v = (((long long)b * (g.nz + 2) + gz + 1) * (g.ny + 2) + gy + 1) * (g.nx + 2) + gx + 1;
-            halo[i] = src[v * 16 + w];
-        } else {
-            gx = (gx < 0) ? gx + g.nx : (gx >= g.nx ? gx - g.nx : gx);
-            gy = (gy < 0) ? gy + g.ny : (gy >= g.ny ? gy - g.ny : gy);
-            gz = (gz < 0) ? gz + g.nz : (gz >= g.nz ? gz - g.nz : gz);
-            const long long v = (((long long)b * g.nz + gz) * g.ny + gy) * g.nx + gx;
-            halo[i] = src[v * WORDS + w];
-        }
-    }
-}
-
-// BF16 pair (channels co, co+1) of voxel (x, y, z, b) into a ghosted
-// activation buffer, at its own position and its ghost copies
-__device__ __forceinline__ void store_ghosted(bf16 *__restrict__ out, const Geo& g, int x, int y, int z, int b, int co,
-                                              uint32_t pair)
-{
-    int xs[3], ys[3], zs[3];
-    int nxs = 1, nys = 1, nzs = 1;
-    xs[0] = x + 1;
-    if (x == 0) xs[nxs++] = g.nx + 1;
-    if (x == g.nx - 1) xs[nxs++] = 0;
-    ys[0] = y + 1;
-    if (y == 0) ys[nys++] = g.ny + 1;
-    if (y == g.ny - 1) ys[nys++] = 0;
-    zs[0] = z + 1;
-    if (z == 0) zs[nzs++] = g.nz + 1;
-    if (z == g.nz - 1) zs[nzs++] = 0;
-    for (int a = 0; a < nzs; ++a) {
-        for (int c = 0; c < nys; ++c) {
-            for (int d = 0; d < nxs; ++d) {
-                const long long v = (((long long)b * (g.nz + 2) + zs[a]) * (g.ny + 2) + ys[c]) * (g.nx + 2) + xs[d];
-                *reinterpret_cast<uint32_t *>(out + v * 32 + co) = pair;
-            }
-        }
+        gx = (gx < 0) ? gx + g.nx : (gx >= g.nx ? gx - g.nx : gx);
+        gy = (gy < 0) ? gy + g.ny : (gy >= g.ny ? gy - g.ny : gy);
+        gz = (gz < 0) ? gz + g.nz : (gz >= g.nz ? gz - g.nz : gz);
+        const long long v = (((long long)b * g.nz + gz) * g.ny + gy) * g.nx + gx;
+        halo[i] = src[v * WORDS + w];
     }
 }
 
 // ------------------------------------------------------------ forward conv
 // MODE 0: out_h = gelu(acc + bias) in BF16 (COUT even), out_z = acc + bias
 //         in FP32 when non-null.  MODE 1: out_f = acc (+ bias when
-//         non-null) in FP32 for co < COUT.  MODE 2: as MODE 0 without
-//         out_z, into a ghosted buffer (own position and ghost copies).
-// GIN: the input is ghosted (see load_halo).
-template<int CIN, int COUT, int TX, int MODE, bool GIN = false>
+//         non-null) in FP32 for co < COUT.
+template<int CIN, int COUT, int TX, int MODE>
 __global__ void __launch_bounds__(THREADS)
 conv_fwd_kernel(const bf16 *__restrict__ in, const uint2 *__restrict__ wfrag, const float *__restrict__ bias, Geo g,
                 bf16 *__restrict__ out_h, float *__restrict__ out_z, float *__restrict__ out_f)
@@ -146,14 +113,12 @@ conv_fwd_kernel(const bf16 *__restrict__ in, const uint2 *__restrict__ wfrag, co
     extern __shared__ uint32_t smem[];
     uint32_t *halo = smem;                                        // 3 * HY * HX * CIN / 2 words
     uint2 *wsm = reinterpret_cast<uint2 *>(smem + ((3 * HY * HX * CIN / 2 + 3) & ~3));   // 16-byte aligned
-    // MODE 2: the tile's output voxels, 16 words (32 BF16 channels) each
-    uint32_t *otile = reinterpret_cast<uint32_t *>(wsm + KS * NT * 32);
 
     const int x0 = blockIdx.x * TX;
     const int y0 = blockIdx.y * TYT;
     const int z = blockIdx.z % g.nz;
     const int b = blockIdx.z / g.nz;
-    load_halo<CIN, TX, GIN>(halo, in, g, x0, y0, z, b);
+    load_halo<CIN, TX>(halo, in, g, x0, y0, z, b);
     for (int i = threadIdx.x; i < KS * NT * 32; i += THREADS) wsm[i] = wfrag[i];
     __syncthreads();
 
@@ -225,57 +190,9 @@ conv_fwd_kernel(const bf16 *__restrict__ in, const uint2 *__restrict__ wfrag, co
                         *reinterpret_cast<uint32_t *>(out_h + v * COUT + co) =
                             pack2(__float2bfloat16(gelu_f(z0)), __float2bfloat16(gelu_f(z1)));
                     }
-                } else if (MODE == 2) {
-                    const int vt = warp * TX + (x - x0);
-                    if (co < COUT) {
-                        const float z0 = r0 + bias[co];
-                        const float z1 = r1 + bias[co + 1];
-                        otile[vt * 16 + co / 2] = pack2(__float2bfloat16(gelu_f(z0)), __float2bfloat16(gelu_f(z1)));
-                    } else if (co < 32) {
-                        otile[vt * 16 + co / 2] = 0u;
-                    }
                 } else {
                     if (co < COUT) out_f[v * COUT + co] = r0 + (bias ? bias[co] : 0.f);
                     if (co + 1 < COUT) out_f[v * COUT + co + 1] = r1 + (bias ? bias[co + 1] : 0.f);
-                }
-            }
-        }
-    }
-    if (MODE == 2) {
-        // channels COUT .. 31 of the staged voxels (the n-tiles stop at COUT)
-        for (int i = threadIdx.x; i < TYT * TX * (16 - NT * 4); i += THREADS) {
-            const int per = 16 - NT * 4;
-            otile[(i / per) * 16 + NT * 4 + i % per] = 0u;
-        }
-        __syncthreads();
-        // one 64-byte record per voxel, at its position and its ghost copies
-        for (int vt = threadIdx.x; vt < TYT * TX; vt += THREADS) {
-            const uint4 *src = reinterpret_cast<const uint4 *>(otile + vt * 16);
-            const uint4 q0 = src[0], q1 = src[1], q2 = src[2], q3 = src[3];
-            const int x = x0 + vt % TX;
-            const int yv = y0 + vt / TX;
-            int xs[3], ys[3], zs[3];     // an axis of extent 1 has both ghost copies
-            int nxs = 1, nys = 1, nzs = 1;
-            xs[0] = x + 1;
-            if (x == 0) xs[nxs++] = g.nx + 1;
-            if (x == g.nx - 1) xs[nxs++] = 0;
-            ys[0] = yv + 1;
-            if (yv == 0) ys[nys++] = g.ny + 1;
-            if (yv == g.ny - 1) ys[nys++] = 0;
-            zs[0] = z + 1;
-            if (z == 0) zs[nzs++] = g.nz + 1;
-            if (z == g.nz - 1) zs[nzs++] = 0;
-            for (int a = 0; a < nzs; ++a) {
-                for (int c = 0; c < nys; ++c) {
-                    for (int d = 0; d < nxs; ++d) {
-                        const long long v =
-                            (((long long)b * (g.nz + 2) + zs[a]) * (g.ny + 2) + ys[c]) * (g.nx + 2) + xs[d];
-                        uint4 *o = reinterpret_cast<uint4 *>(out_h + v * 32);
-                        o[0] = q0;
-                        o[1] = q1;
-                        o[2] = q2;
-                        o[3] = q3;
-                    }
                 }
             }
         }
@@ -540,36 +457,23 @@ struct Net {
     int t;              // Adam step
     cudaStream_t stream;
     uint64_t launches;
-    // tensor-core (tcgen05) inference path: C = 24, nx % 128 == 0, ny even,
-    // no training buffers; layers 2 and 3 on tcgen05, 1 and 4 on mma.sync
+    // tensor-core (tcgen05) path: C = 24, no training buffers (conv_tc.cu)
     bool fast;
     int variant;        // 0: tcgen05 path where it applies; 1: mma.sync for every layer
-    bf16 *hg[2];        // ghosted activations [batch][nz+2][ny+2][nx+2][32]
-    void *wtc[2];       // weights of layers 2 and 3 in the tcgen05 B layout
-    int *d_err;         // bounded waits of the tcgen05 kernel
-    alignas(64) unsigned char tmap[128];
+    void *hg[2];        // ghosted activations
+    TcWeights wtc;      // weights in the tcgen05 operand layout
+    int *d_err;         // bounded waits of the tcgen05 kernels
 };
-
-bool tc_applicable(int nx, int ny, int channels);
-size_t tc_weight_bytes();
-void tc_pack_weights(const float *w, void *out, cudaStream_t stream);
-void tc_conv(void *map_cache, const void *in, void *out, const void *wpacked, const float *bias, int nx, int ny, int nz,
-             int batch, cudaStream_t stream, int *d_err);
-bool last_conv_applicable(int nx, int ny, int channels);
-void last_conv(const void *h, const float *w, const float *bias, float *out, bool add_to_u, int nx, int ny, int nz,
-               int batch, cudaStream_t stream);
 
 static int layer_frag_words(int cin, int cout)
 {
     return ceil_div(27 * cin, 16) * ceil_div(cout, 8) * 32;
 }
 
-template<int CIN, int COUT, int TX, int MODE = 0>
+template<int CIN, int COUT, int TX>
 static size_t fwd_smem()
 {
-    // MODE 2 adds the staged output tile (TYT x TX voxels x 32 BF16 channels)
-    return (size_t)(((3 * (TYT + 2) * (TX + 2) * CIN / 2 + 3) & ~3) * 4 + layer_frag_words(CIN, COUT) * 8) +
-           (MODE == 2 ? (size_t)TYT * TX * 64 : 0);
+    return (size_t)(((3 * (TYT + 2) * (TX + 2) * CIN / 2 + 3) & ~3) * 4 + layer_frag_words(CIN, COUT) * 8);
 }
 
 template<int CIN, int COUT, int TX>
@@ -578,18 +482,18 @@ static size_t wgrad_smem()
     return (size_t)(3 * (TYT + 2) * (TX + 2) * CIN / 2) * 4 + (size_t)TYT * TX * ((COUT + 1) & ~1) * 2;
 }
 
-template<int CIN, int COUT, int TX, int MODE, bool GIN = false>
+template<int CIN, int COUT, int TX, int MODE>
 static void run_fwd(Net& n, const bf16 *in, const uint2 *frag, const float *bias, bf16 *oh, float *oz, float *of)
 {
-    const size_t sm = fwd_smem<CIN, COUT, TX, MODE>();
+    const size_t sm = fwd_smem<CIN, COUT, TX>();
     static PerDevice<bool> setup;             // per instantiation, per device
     setup.get([sm] {
-        LGD_CHECK_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<CIN, COUT, TX, MODE, GIN>,
+        LGD_CHECK_CUDA(cudaFuncSetAttribute(conv_fwd_kernel<CIN, COUT, TX, MODE>,
                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         return true;
     });
     dim3 grid(n.g.nx / TX, n.g.ny / TYT, n.g.nz * n.g.batch);
-    conv_fwd_kernel<CIN, COUT, TX, MODE, GIN><<<grid, THREADS, sm, n.stream>>>(in, frag, bias, n.g, oh, oz, of);
+    conv_fwd_kernel<CIN, COUT, TX, MODE><<<grid, THREADS, sm, n.stream>>>(in, frag, bias, n.g, oh, oz, of);
     check_launch("conv forward");
     ++n.launches;
 }
@@ -627,38 +531,35 @@ static void repack(Net& n)
     }
     check_launch("pack fragments");
     if (n.fast) {
-        tc_pack_weights(n.params + n.L[1].w_off, n.wtc[0], n.stream);
-        tc_pack_weights(n.params + n.L[2].w_off, n.wtc[1], n.stream);
-        n.launches += 2;
+        const float *w[4];
+        for (int l = 0; l < 4; ++l) w[l] = n.params + n.L[l].w_off;
+        n.launches += tc_pack_weights(w, n.wtc, n.stream);
     }
 }
 
-// Inference with the tcgen05 layers: input packing, layer 1 (mma.sync) into
-// a ghosted buffer, layers 2 and 3 on tcgen05 between the two ghosted
-// buffers, layer 4 from the ghosted buffer into du (the tap-product kernel
-// of conv_last.cu where the tile fits, else mma.sync).  With add_to_u the
-// last layer adds its result to u instead (u <- u + du, the residual step).
-// Returns whether it did.
-template<int TX>
-static bool forward_fast_impl(Net& n, const float *u, const float *k, float *du, bool add_to_u)
+// Inference on the tensor cores: four launches, the activations between two
+// ghosted buffers.  With add_to_u the last layer adds its result to u instead
+// (u <- u + du, the residual step).
+static void forward_fast(Net& n, const float *u, const float *k, float *du, bool add_to_u)
 {
-    pack_input_kernel<<<grid_blocks(n.V), 256, 0, n.stream>>>(u, k, n.x0, n.V);
-    ++n.launches;
-    run_fwd<2, 24, TX, 2>(n, n.x0, n.L[0].frag, n.params + n.L[0].b_off, n.hg[0], nullptr, nullptr);
-    tc_conv(n.tmap, n.hg[0], n.hg[1], n.wtc[0], n.params + n.L[1].b_off, n.g.nx, n.g.ny, n.g.nz, n.g.batch, n.stream,
-            n.d_err);
-    ++n.launches;
-    tc_conv(n.tmap, n.hg[1], n.hg[0], n.wtc[1], n.params + n.L[2].b_off, n.g.nx, n.g.ny, n.g.nz, n.g.batch, n.stream,
-            n.d_err);
-    ++n.launches;
-    if (last_conv_applicable(n.g.nx, n.g.ny, n.C)) {
-        last_conv(n.hg[0], n.params + n.L[3].w_off, n.params + n.L[3].b_off, add_to_u ? const_cast<float *>(u) : du,
-                  add_to_u, n.g.nx, n.g.ny, n.g.nz, n.g.batch, n.stream);
-        ++n.launches;
-        return add_to_u;
-    }
-    run_fwd<24, 1, TX, 1, true>(n, n.hg[0], n.L[3].frag, n.params + n.L[3].b_off, nullptr, nullptr, du);
-    return false;
+    const int dims[4] = {n.g.nx, n.g.ny, n.g.nz, n.g.batch};
+    const float *bias[4];
+    for (int l = 0; l < 4; ++l) bias[l] = n.params + n.L[l].b_off;
+    tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], nullptr, dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], nullptr, dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], n.hg[0], nullptr, dims, n.d_err, n.stream);
+    tc_layer_last(n.hg[0], n.wtc.fwd[3], bias[3], add_to_u ? const_cast<float *>(u) : du, add_to_u, dims, n.d_err,
+                  n.stream);
+    n.launches += 4;
+}
+
+// buffers of the mma.sync path, made when it first runs
+static void ensure_dense(Net& n)
+{
+    if (n.x0) return;
+    LGD_CHECK_CUDA(cudaMalloc(&n.x0, sizeof(bf16) * 2 * n.V));
+    const int nh = n.training ? 3 : 2;
+    for (int i = 0; i < nh; ++i) LGD_CHECK_CUDA(cudaMalloc(&n.h[i], sizeof(bf16) * n.C * n.V));
 }
 
 // the network's channel count is a template parameter of the kernels; the
@@ -718,8 +619,10 @@ static void backward_impl(Net& n, const float *target, double *loss_out)
 static bool forward(Net& n, const float *u, const float *k, float *du, bool add_to_u = false)
 {
     if (n.fast && n.variant == 0) {
-        return n.TX == 64 ? forward_fast_impl<64>(n, u, k, du, add_to_u) : forward_fast_impl<32>(n, u, k, du, add_to_u);
+        forward_fast(n, u, k, du, add_to_u);
+        return add_to_u;
     }
+    ensure_dense(n);
     if (n.C == 24) {
         if (n.TX == 64) forward_impl<24, 64>(n, u, k, du); else forward_impl<24, 32>(n, u, k, du);
     } else {
@@ -760,8 +663,7 @@ static void net_free(Net& n)
     cudaFree(n.d_loss);
     cudaFree(n.hg[0]);
     cudaFree(n.hg[1]);
-    cudaFree(n.wtc[0]);
-    cudaFree(n.wtc[1]);
+    tc_free_weights(n.wtc);
     cudaFree(n.d_err);
     if (n.stream) cudaStreamDestroy(n.stream);
 }
@@ -838,9 +740,6 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
                 LGD_CHECK_CUDA(cudaMalloc(&L.frag_t, sizeof(uint2) * L.frag_t_n));
             }
             const long long V = n->V;
-            LGD_CHECK_CUDA(cudaMalloc(&n->x0, sizeof(bf16) * 2 * V));
-            const int nh = n->training ? 3 : 2;
-            for (int i = 0; i < nh; ++i) LGD_CHECK_CUDA(cudaMalloc(&n->h[i], sizeof(bf16) * C * V));
             LGD_CHECK_CUDA(cudaMalloc(&n->du, sizeof(float) * V));
             if (n->training) {
                 for (int i = 0; i < 3; ++i) LGD_CHECK_CUDA(cudaMalloc(&n->zb[i], sizeof(float) * C * V));
@@ -857,13 +756,8 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
             }
             n->fast = !n->training && tc_applicable(nx, ny, C);
             if (n->fast) {
-                const size_t gbytes = (size_t)batch * (nz + 2) * (ny + 2) * (nx + 2) * 32 * sizeof(bf16);
-                for (int i = 0; i < 2; ++i) {
-                    LGD_CHECK_CUDA(cudaMalloc(&n->hg[i], gbytes));
-                    // channels 24..31 stay zero (layer 1 writes only 0..23)
-                    LGD_CHECK_CUDA(cudaMemsetAsync(n->hg[i], 0, gbytes, n->stream));
-                    LGD_CHECK_CUDA(cudaMalloc(&n->wtc[i], tc_weight_bytes()));
-                }
+                for (int i = 0; i < 2; ++i) LGD_CHECK_CUDA(cudaMalloc(&n->hg[i], tc_ghost_bytes(nx, ny, nz, batch)));
+                n->wtc = tc_alloc_weights(false);
                 LGD_CHECK_CUDA(cudaMalloc(&n->d_err, sizeof(int)));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->d_err, 0, sizeof(int), n->stream));
             }
