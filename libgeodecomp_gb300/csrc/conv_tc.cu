@@ -32,7 +32,7 @@
 // of input sits in shared memory as [channel group][row][8 voxels + 2 halo]
 // x 16 B: every 8-voxel core matrix brings its own halo, so tap (dy, dx) of
 // any tile is a start address and M may span rows.
-//   - warp 0, one thread: issues the MMAs, tile by tile;
+//   - warp 0: issues the MMAs, tile by tile;
 //   - warps 1 .. 16: epilogue of tile (w - 1) / 4, lane quarter w % 4;
 //   - warps 17 .. 20: fill the input slots (cp.async; FIRST and DLAST build
 //     their groups from the FP32 fields).
@@ -162,62 +162,60 @@ conv_tc_kernel(const Params p)
     __syncthreads();
     fence_after();
     const uint32_t tmem = s_tmem;
-    int committed = 0;                                  // thread 0: tiles committed, over all planes
+    int committed = 0;                                  // warp 0: tiles committed, over all planes
     bool w_ready = false;
 
     if (warp == 0) {
-        if (lane == 0) {
-            bool ok = mbar_wait(saddr(&bar_w), 0, fail);
-            w_ready = ok;
-            const uint32_t rbase = saddr(ring), wbase = saddr(wsm);
-            constexpr uint32_t ID = idesc(128, G::N, false);
-            for (int q = 0; ok && q < n + 2; ++q) {
-                ok = mbar_wait(saddr(&bar_full[q % S]), (uint32_t)((q / S) & 1), fail);
+        bool ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_w), 0, fail));
+        w_ready = ok;
+        const uint32_t rbase = saddr(ring), wbase = saddr(wsm);
+        constexpr uint32_t ID = idesc(128, G::N, false);
+        constexpr uint32_t HI_A = desc_hi(G::GS), HI_B = desc_hi(128);
+        for (int q = 0; ok && q < n + 2; ++q) {
+            ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_full[q % S]), (uint32_t)((q / S) & 1), fail));
+            if (!ok) break;
+            fence_after();
+            const uint32_t a0 = desc_lo(rbase + (uint32_t)((q % S) * G::SLOT), 0);
+            // the block order of the three accumulators (see pack_kernel)
+            const uint32_t rot = (uint32_t)((3 - q % 3) % 3);
+            const uint32_t b0 = SRC == LAST ? desc_lo(wbase + rot * (G::KSTEPS * G::KS_BYTES), 2 * 128)
+                                            : desc_lo(wbase + rot * 3 * 128, 16 * 128);
+            for (int m = 0; m < TILES; ++m) {
+                ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_free[m]), (uint32_t)(q & 1), fail));
                 if (!ok) break;
                 fence_after();
-                const uint32_t slot = rbase + (uint32_t)((q % S) * G::SLOT);
-                // the block order of the three accumulators (see pack_kernel)
-                const uint32_t rot = (uint32_t)((3 - q % 3) % 3);
-                const uint64_t wd = SRC == LAST ? sdesc(wbase + rot * (G::KSTEPS * G::KS_BYTES), 2 * 128, 128)
-                                                : sdesc(wbase + rot * 3 * 128, 16 * 128, 128);
-                // a K-step's descriptor: start and leading offset of its two
-                // groups (compile-time), added to the tile's base
-                const uint64_t base = sdesc(slot, 0, G::GS);
-#pragma unroll
-                for (int m = 0; m < TILES; ++m) {
-                    ok = mbar_wait(saddr(&bar_free[m]), (uint32_t)(q & 1), fail);
-                    if (!ok) break;
-                    fence_after();
+                if (elect_one()) {
                     const uint32_t d = tmem + (uint32_t)(m * G::TCOLS);
+                    const uint32_t am = a0 + (uint32_t)(m * G::GS);         // 16 groups, in 16-byte units
 #pragma unroll
                     for (int k = 0; k < G::KSTEPS; ++k) {
-                        uint32_t first, lead;           // bytes
+                        int first, lead;                // start and leading offset of the step's two groups, bytes
                         if (G::WIDE) {
                             if (k < 12) {               // taps 2 (k / 3) and 2 (k / 3) + 1, channel group k % 3
                                 const int ta = 2 * (k / 3), tb = ta + 1;
                                 const int oa = (ta / 3) * G::ROWP + (ta % 3) * 16;
                                 const int ob = (tb / 3) * G::ROWP + (tb % 3) * 16;
-                                first = (uint32_t)(oa + (k % 3) * G::CGS);
-                                lead = (uint32_t)(ob - oa);
+                                first = oa + (k % 3) * G::CGS;
+                                lead = ob - oa;
                             } else {                    // tap 8: groups 0, 1 and 1 (zero weights), 2
-                                first = (uint32_t)(2 * G::ROWP + 2 * 16 + (k - 12) * G::CGS);
-                                lead = (uint32_t)G::CGS;
+                                first = 2 * G::ROWP + 2 * 16 + (k - 12) * G::CGS;
+                                lead = G::CGS;
                             }
                         } else {                        // rows 0, 1 and 1 (zero weights), 2
-                            first = (uint32_t)(k * G::ROWP);
-                            lead = (uint32_t)G::ROWP;
+                            first = k * G::ROWP;
+                            lead = G::ROWP;
                         }
-                        const uint64_t a = base + ((uint64_t)(lead >> 4) << 16) + (uint64_t)((first + m * 16 * G::GS) >> 4);
-                        mma(d, a, wd + (uint64_t)((k * G::KS_BYTES) >> 4), ID, 1u);
+                        mma<true>(d, desc(am + (uint32_t)((first >> 4) + ((lead >> 4) << 16)), HI_A),
+                                  desc(b0 + (uint32_t)((k * G::KS_BYTES) >> 4), HI_B), ID);
                     }
                     mma_commit(saddr(&bar_mma[m]));
-                    ++committed;
+                    if (m == TILES - 1) mma_commit(saddr(&bar_empty[q % S]));
                 }
-                if (!ok) break;
-                mma_commit(saddr(&bar_empty[q % S]));
+                __syncwarp();
+                ++committed;
             }
-            if (!ok) s_fail = 1;
         }
+        if (!ok && lane == 0) s_fail = 1;
         __syncwarp();
     } else if (warp >= LOAD0) {
         const int lt = tid - LOAD0 * 32;
@@ -258,27 +256,52 @@ conv_tc_kernel(const Params p)
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
             } else {
+                // a warp builds the groups of 32 consecutive voxels: neighbours
+                // by shuffle, the two beyond the ends by the end lanes; the
+                // loads of all its segments are in flight together
+                constexpr int SEGS = G::ROWS * TXW / 32;
+                constexpr int PER = (SEGS + LOAD_WARPS - 1) / LOAD_WARPS;
                 int z = z0 - 1 + q;
                 z = z < 0 ? z + s.nz : (z >= s.nz ? z - s.nz : z);
-                for (int v = lt; v < G::ROWS * TXW; v += LOAD_WARPS * 32) {
-                    const int r = v / TXW;
-                    const int x = x0 + v % TXW;
+                float va[PER], vc[PER], ea[PER], ec[PER];
+#pragma unroll
+                for (int i = 0; i < PER; ++i) {
+                    const int seg = (lt >> 5) + i * LOAD_WARPS;
+                    const int r = min(seg * 32 / TXW, G::ROWS - 1);
+                    const int x = x0 + seg * 32 % TXW + lane;
                     int y = y0 - 1 + r;
                     y = y < 0 ? y + s.ny : (y >= s.ny ? (y - s.ny) % s.ny : y);
-                    const int xw = x == 0 ? s.nx - 1 : x - 1;
-                    const int xe = x == s.nx - 1 ? 0 : x + 1;
                     const long long row = (((long long)b * s.nz + z) * s.ny + y) * s.nx;
-                    const float *a = p.f0 + row, *c = p.f1 + row;
-                    uint4 w;
-                    if (SRC == FIRST) {
-                        w = make_uint4(pack_bf16(a[xw], c[xw]), pack_bf16(a[x], c[x]), pack_bf16(a[xe], c[xe]), 0u);
-                    } else {
-                        w = make_uint4(pack_bf16(p.scale * (a[xw] - c[xw]), p.scale * (a[x] - c[x])),
-                                       pack_bf16(p.scale * (a[xe] - c[xe]), 0.f), 0u, 0u);
+                    va[i] = p.f0[row + x];
+                    vc[i] = p.f1[row + x];
+                    const int e = lane == 0 ? (x == 0 ? s.nx - 1 : x - 1) : (x == s.nx - 1 ? 0 : x + 1);
+                    ea[i] = ec[i] = 0.f;
+                    if (lane == 0 || lane == 31) {
+                        ea[i] = p.f0[row + e];
+                        ec[i] = p.f1[row + e];
                     }
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(slot + (uint32_t)(v * 16)), "r"(w.x),
-                                 "r"(w.y), "r"(w.z), "r"(w.w)
-                                 : "memory");
+                }
+#pragma unroll
+                for (int i = 0; i < PER; ++i) {
+                    const int seg = (lt >> 5) + i * LOAD_WARPS;
+                    uint32_t mid, edge;                 // FIRST: the pair (u, kappa); DLAST: the gradient
+                    if (SRC == FIRST) {
+                        mid = pack_bf16(va[i], vc[i]);
+                        edge = pack_bf16(ea[i], ec[i]);
+                    } else {
+                        mid = pack_bf16(p.scale * (va[i] - vc[i]), 0.f);
+                        edge = pack_bf16(p.scale * (ea[i] - ec[i]), 0.f);
+                    }
+                    uint32_t w = __shfl_up_sync(0xffffffffu, mid, 1);
+                    uint32_t e = __shfl_down_sync(0xffffffffu, mid, 1);
+                    if (lane == 0) w = edge;
+                    if (lane == 31) e = edge;
+                    const uint4 g = SRC == FIRST ? make_uint4(w, mid, e, 0u) : make_uint4(w | (mid << 16), e, 0u, 0u);
+                    if (SEGS % LOAD_WARPS == 0 || seg < SEGS) {
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(slot + (uint32_t)((seg * 32 + lane) * 16)),
+                                     "r"(g.x), "r"(g.y), "r"(g.z), "r"(g.w)
+                                     : "memory");
+                    }
                 }
                 publish(q + 1);
             }

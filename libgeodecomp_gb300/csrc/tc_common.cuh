@@ -17,13 +17,8 @@ constexpr long long WAIT_CYCLES = 4000000000LL;     // about two seconds
 
 __device__ __forceinline__ uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// matrix descriptor, no swizzle, in 16-byte units: start address, leading and
-// stride offsets, descriptor version 1
-__device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo)
-{
-    return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
-}
+// Matrix descriptors (no swizzle): start address, leading and stride offsets in
+// 16-byte units, descriptor version 1; see desc_lo and desc_hi.
 
 // kind::f16 instruction descriptor: FP32 accumulator, BF16 operands; mn: both
 // operands with M / N contiguous instead of K
@@ -33,15 +28,45 @@ __host__ __device__ constexpr uint32_t idesc(int m, int n, bool mn)
            ((uint32_t)(m >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t id, uint32_t acc)
+// One lane of a converged warp.  The MMA warp runs its loop with all lanes and
+// elects one around each batch of MMAs: loop variables and descriptors then
+// stay in uniform registers.  Under a branch on the lane number every MMA
+// first moves its operands there, and with the epilogue warps competing for
+// issue slots an MMA of 52 clocks took 107.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t r;
+    asm volatile(
+        "{\n"
+        " .reg .pred p;\n"
+        " elect.sync _|p, 0xffffffff;\n"
+        " selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(r));
+    return r != 0;
+}
+
+// descriptors as their low words (start address and leading offset, which
+// change from MMA to MMA) and constant high words; ACC: add to D
+__device__ __forceinline__ uint64_t desc(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
+
+__host__ __device__ constexpr uint32_t desc_hi(uint32_t sbo) { return ((sbo >> 4) & 0x3FFFu) | (1u << 14); }
+
+__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo)
+{
+    return ((addr >> 4) & 0x3FFFu) | (((lbo >> 4) & 0x3FFFu) << 16);
+}
+
+template<bool ACC>
+__device__ __forceinline__ void mma(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t id)
 {
     asm volatile(
         "{\n"
         " .reg .pred p;\n"
-        " setp.ne.b32 p, %4, 0;\n"
+        " setp.eq.u32 p, 1, %4;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
         "}\n" ::"r"(dtmem),
-        "l"(a), "l"(b), "r"(id), "r"(acc)
+        "l"(a), "l"(b), "r"(id), "n"(ACC ? 1 : 0)
         : "memory");
 }
 
