@@ -66,13 +66,14 @@ int lgd_net_synchronize(lgd_net *h);
 int lgd_net_stream(lgd_net *h, void **stream);
 int lgd_net_launch_count(lgd_net *h, uint64_t *count);
 
-/* Inference path: 0 (default) runs the two C -> C layers on the tcgen05
- * tensor cores (TMA-fed input planes, accumulators in tensor memory) when
- * the handle has no training buffers, C = 24, nx is a multiple of 128 and
- * ny even; 1 runs every layer on the mma.sync kernels (the training
- * path's).  Results agree to BF16 rounding of the activations. */
+/* Kernels of the 24-channel network: 0 (default) runs every convolution, of
+ * the backward pass too, on the tcgen05 tensor cores (accumulators in tensor
+ * memory); 1 runs every layer on the mma.sync kernels, whose buffers are made
+ * at its first use.  A backward pass takes the path of the forward pass
+ * before it.  Results agree to BF16 rounding of the activations.  Other
+ * channel counts run mma.sync. */
 int lgd_net_set_variant(lgd_net *h, int variant);
-/* *yes = 1 when forward / advance run the tcgen05 layers. */
+/* *yes = 1 when the handle's passes run the tcgen05 kernels. */
 int lgd_net_uses_tensor_core_path(lgd_net *h, int *yes);
 
 #ifdef __cplusplus

@@ -648,5 +648,35 @@ void tc_layer_last(const void *in, const void *w, const float *bias, float *out,
     run_any<LAST, OUT>(p, stream);
 }
 
+void tc_grad_mid(const void *dz, const void *w, const float *z, void *out, float *db, const int dims[4], int *err,
+                 cudaStream_t stream)
+{
+    Params p = {};
+    p.s = {dims[0], dims[1], dims[2], dims[3]};
+    p.in = (const bf16 *)dz;
+    p.w = (const bf16 *)w;
+    p.z = const_cast<float *>(z);
+    p.out = (bf16 *)out;
+    p.db = db;
+    p.err = err;
+    run_any<MID, GRAD>(p, stream);
+}
+
+void tc_grad_last(const float *du, const float *target, float scale, const void *w, const float *z, void *out, float *db,
+                  const int dims[4], int *err, cudaStream_t stream)
+{
+    Params p = {};
+    p.s = {dims[0], dims[1], dims[2], dims[3]};
+    p.f0 = du;
+    p.f1 = target;
+    p.scale = scale;
+    p.w = (const bf16 *)w;
+    p.z = const_cast<float *>(z);
+    p.out = (bf16 *)out;
+    p.db = db;
+    p.err = err;
+    run_any<DLAST, GRAD>(p, stream);
+}
+
 }  // namespace sur
 }  // namespace lgd

@@ -32,6 +32,27 @@ void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, f
 void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, const int dims[4], int *err,
                    cudaStream_t stream);
 
+// input gradients: dz of the layer below = conv_t(dz) * GELU'(z), ghosted, and
+// its sum over the voxels added to db.  The last layer's takes the loss
+// gradient scale * (du - target) itself
+void tc_grad_mid(const void *dz, const void *w, const float *z, void *out, float *db, const int dims[4], int *err,
+                 cudaStream_t stream);
+void tc_grad_last(const float *du, const float *target, float scale, const void *w, const float *z, void *out, float *db,
+                  const int dims[4], int *err, cudaStream_t stream);
+
+// weight gradients of layer 0 (x0: BF16 pairs u, kappa; dz), 1 and 2 (h the
+// layer's input, dz), 3 (h, du, target, scale): each CTA's share into its
+// slice of partials (tc_partial_floats); returns the CTAs.  tc_wgrad_reduce
+// sums all layers' shares into grads.
+size_t tc_partial_floats();
+int tc_wgrad(int layer, const void *h, const void *x0, const void *dz, const float *du, const float *target, float scale,
+             float *partials, const int dims[4], int *err, cudaStream_t stream);
+void tc_wgrad_reduce(const float *partials, const int ctas[4], const long long w_off[4], float *grads,
+                     cudaStream_t stream);
+
+// floats of a layer's pre-activations
+inline size_t tc_z_floats(int nx, int ny, int nz, int batch) { return (size_t)nx * ny * nz * batch * 24; }
+
 }  // namespace sur
 }  // namespace lgd
 

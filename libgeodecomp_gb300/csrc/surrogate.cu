@@ -333,7 +333,8 @@ __global__ void gelu_bwd_kernel(const float *__restrict__ dh, const float *__res
 }
 
 // MSE loss of du against target: g = 2 (du - t) / N as the BF16 gradient of
-// the last layer ([V][2], channel 1 zero), db4 += sum g, loss += sum diff^2
+// the last layer ([V][2], channel 1 zero; or null), db4 += sum g, loss += sum
+// diff^2
 __global__ void loss_kernel(const float *__restrict__ du, const float *__restrict__ target, bf16 *__restrict__ dz4,
                             float *__restrict__ db4, double *__restrict__ loss, long long nvox)
 {
@@ -347,7 +348,7 @@ __global__ void loss_kernel(const float *__restrict__ du, const float *__restric
         l += (double)d * d;
         const float gv = scale * d;
         gs += gv;
-        *reinterpret_cast<uint32_t *>(dz4 + 2 * v) = pack2(__float2bfloat16(gv), __float2bfloat16(0.f));
+        if (dz4) *reinterpret_cast<uint32_t *>(dz4 + 2 * v) = pack2(__float2bfloat16(gv), __float2bfloat16(0.f));
     }
     sl[threadIdx.x] = l;
     sg[threadIdx.x] = gs;
@@ -457,10 +458,15 @@ struct Net {
     int t;              // Adam step
     cudaStream_t stream;
     uint64_t launches;
-    // tensor-core (tcgen05) path: C = 24, no training buffers (conv_tc.cu)
+    // tensor-core (tcgen05) path: C = 24 (conv_tc.cu, wgrad_tc.cu)
     bool fast;
+    bool fast_forward;  // the last forward pass took it (the backward pass follows)
     int variant;        // 0: tcgen05 path where it applies; 1: mma.sync for every layer
-    void *hg[2];        // ghosted activations
+    void *hg[3];        // ghosted activations (two without training)
+    void *dzg[2];       // ghosted gradients (training)
+    float *zt[3];       // pre-activations (training)
+    uint32_t *xt;       // BF16 pairs (u, kappa) of the last forward pass (training)
+    float *part;        // weight-gradient shares of the CTAs (training)
     TcWeights wtc;      // weights in the tcgen05 operand layout
     int *d_err;         // bounded waits of the tcgen05 kernels
 };
@@ -537,20 +543,66 @@ static void repack(Net& n)
     }
 }
 
-// Inference on the tensor cores: four launches, the activations between two
-// ghosted buffers.  With add_to_u the last layer adds its result to u instead
-// (u <- u + du, the residual step).
+// waits for the stream, then reports (and clears) a wait that gave up
+static void sync_and_check(Net& n)
+{
+    LGD_CHECK_CUDA(cudaStreamSynchronize(n.stream));
+    volatile int *e = n.d_err;
+    if (e && *e) {
+        *e = 0;
+        throw Error(LGD_ERR_TIMEOUT, "a tensor-core kernel gave up waiting for its copies or MMAs");
+    }
+}
+
+// The forward pass on the tensor cores: four launches, the activations between
+// two ghosted buffers (three when training, which also keeps the
+// pre-activations and the packed input).  With add_to_u the last layer adds its
+// result to u instead (u <- u + du, the residual step).
 static void forward_fast(Net& n, const float *u, const float *k, float *du, bool add_to_u)
 {
     const int dims[4] = {n.g.nx, n.g.ny, n.g.nz, n.g.batch};
     const float *bias[4];
     for (int l = 0; l < 4; ++l) bias[l] = n.params + n.L[l].b_off;
-    tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], nullptr, dims, n.d_err, n.stream);
-    tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], nullptr, dims, n.d_err, n.stream);
-    tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], n.hg[0], nullptr, dims, n.d_err, n.stream);
-    tc_layer_last(n.hg[0], n.wtc.fwd[3], bias[3], add_to_u ? const_cast<float *>(u) : du, add_to_u, dims, n.d_err,
-                  n.stream);
+    void *h3 = n.training ? n.hg[2] : n.hg[0];
+    if (n.training) {
+        pack_input_kernel<<<grid_blocks(n.V), 256, 0, n.stream>>>(u, k, (bf16 *)n.xt, n.V);
+        ++n.launches;
+    }
+    tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], n.zt[0], dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], n.zt[1], dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], h3, n.zt[2], dims, n.d_err, n.stream);
+    tc_layer_last(h3, n.wtc.fwd[3], bias[3], add_to_u ? const_cast<float *>(u) : du, add_to_u, dims, n.d_err, n.stream);
     n.launches += 4;
+}
+
+// The backward pass on the tensor cores.  Every input gradient comes out of
+// its convolution already multiplied by GELU' and with its bias gradient; the
+// weight gradients leave each CTA's share, summed at the end.
+static void backward_fast(Net& n, const float *target, double *loss_out)
+{
+    const int dims[4] = {n.g.nx, n.g.ny, n.g.nz, n.g.batch};
+    const float scale = 2.0f / (float)n.V;
+    LGD_CHECK_CUDA(cudaMemsetAsync(n.grads, 0, sizeof(float) * n.P, n.stream));
+    LGD_CHECK_CUDA(cudaMemsetAsync(n.d_loss, 0, sizeof(double), n.stream));
+    loss_kernel<<<grid_blocks(n.V), 256, 0, n.stream>>>(n.du, target, nullptr, n.grads + n.L[3].b_off, n.d_loss, n.V);
+    check_launch("loss");
+    int ctas[4];
+    ctas[3] = tc_wgrad(3, n.hg[2], nullptr, nullptr, n.du, target, scale, n.part, dims, n.d_err, n.stream);
+    tc_grad_last(n.du, target, scale, n.wtc.grad[3], n.zt[2], n.dzg[0], n.grads + n.L[2].b_off, dims, n.d_err, n.stream);
+    ctas[2] = tc_wgrad(2, n.hg[1], nullptr, n.dzg[0], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
+    tc_grad_mid(n.dzg[0], n.wtc.grad[2], n.zt[1], n.dzg[1], n.grads + n.L[1].b_off, dims, n.d_err, n.stream);
+    ctas[1] = tc_wgrad(1, n.hg[0], nullptr, n.dzg[1], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
+    tc_grad_mid(n.dzg[1], n.wtc.grad[1], n.zt[0], n.dzg[0], n.grads + n.L[0].b_off, dims, n.d_err, n.stream);
+    ctas[0] = tc_wgrad(0, nullptr, n.xt, n.dzg[0], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
+    const long long off[4] = {n.L[0].w_off, n.L[1].w_off, n.L[2].w_off, n.L[3].w_off};
+    tc_wgrad_reduce(n.part, ctas, off, n.grads, n.stream);
+    n.launches += 9;
+    if (loss_out) {
+        double l = 0.0;
+        LGD_CHECK_CUDA(cudaMemcpyAsync(&l, n.d_loss, sizeof(double), cudaMemcpyDeviceToHost, n.stream));
+        sync_and_check(n);
+        *loss_out = l / (double)n.V;
+    }
 }
 
 // buffers of the mma.sync path, made when it first runs
@@ -560,6 +612,12 @@ static void ensure_dense(Net& n)
     LGD_CHECK_CUDA(cudaMalloc(&n.x0, sizeof(bf16) * 2 * n.V));
     const int nh = n.training ? 3 : 2;
     for (int i = 0; i < nh; ++i) LGD_CHECK_CUDA(cudaMalloc(&n.h[i], sizeof(bf16) * n.C * n.V));
+    if (n.training) {
+        for (int i = 0; i < 3; ++i) LGD_CHECK_CUDA(cudaMalloc(&n.zb[i], sizeof(float) * n.C * n.V));
+        LGD_CHECK_CUDA(cudaMalloc(&n.dh, sizeof(float) * n.C * n.V));
+        LGD_CHECK_CUDA(cudaMalloc(&n.dzb, sizeof(bf16) * n.C * n.V));
+        LGD_CHECK_CUDA(cudaMalloc(&n.dz4, sizeof(bf16) * 2 * n.V));
+    }
 }
 
 // the network's channel count is a template parameter of the kernels; the
@@ -618,7 +676,8 @@ static void backward_impl(Net& n, const float *target, double *loss_out)
 // (returns true when it did)
 static bool forward(Net& n, const float *u, const float *k, float *du, bool add_to_u = false)
 {
-    if (n.fast && n.variant == 0) {
+    n.fast_forward = n.fast && n.variant == 0;
+    if (n.fast_forward) {
         forward_fast(n, u, k, du, add_to_u);
         return add_to_u;
     }
@@ -633,6 +692,11 @@ static bool forward(Net& n, const float *u, const float *k, float *du, bool add_
 
 static void backward(Net& n, const float *target, double *loss)
 {
+    if (n.fast_forward) {
+        backward_fast(n, target, loss);
+        return;
+    }
+    ensure_dense(n);
     if (n.C == 24) {
         if (n.TX == 64) backward_impl<24, 64>(n, target, loss); else backward_impl<24, 32>(n, target, loss);
     } else {
@@ -661,10 +725,16 @@ static void net_free(Net& n)
     cudaFree(n.dzb);
     cudaFree(n.dz4);
     cudaFree(n.d_loss);
-    cudaFree(n.hg[0]);
-    cudaFree(n.hg[1]);
+    for (int i = 0; i < 3; ++i) {
+        cudaFree(n.hg[i]);
+        cudaFree(n.zt[i]);
+    }
+    cudaFree(n.dzg[0]);
+    cudaFree(n.dzg[1]);
+    cudaFree(n.xt);
+    cudaFree(n.part);
     tc_free_weights(n.wtc);
-    cudaFree(n.d_err);
+    if (n.d_err) cudaFreeHost(n.d_err);
     if (n.stream) cudaStreamDestroy(n.stream);
 }
 
@@ -742,24 +812,30 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
             const long long V = n->V;
             LGD_CHECK_CUDA(cudaMalloc(&n->du, sizeof(float) * V));
             if (n->training) {
-                for (int i = 0; i < 3; ++i) LGD_CHECK_CUDA(cudaMalloc(&n->zb[i], sizeof(float) * C * V));
                 LGD_CHECK_CUDA(cudaMalloc(&n->grads, sizeof(float) * n->P));
                 LGD_CHECK_CUDA(cudaMalloc(&n->m, sizeof(float) * n->P));
                 LGD_CHECK_CUDA(cudaMalloc(&n->v, sizeof(float) * n->P));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->grads, 0, sizeof(float) * n->P, n->stream));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->m, 0, sizeof(float) * n->P, n->stream));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->v, 0, sizeof(float) * n->P, n->stream));
-                LGD_CHECK_CUDA(cudaMalloc(&n->dh, sizeof(float) * C * V));
-                LGD_CHECK_CUDA(cudaMalloc(&n->dzb, sizeof(bf16) * C * V));
-                LGD_CHECK_CUDA(cudaMalloc(&n->dz4, sizeof(bf16) * 2 * V));
                 LGD_CHECK_CUDA(cudaMalloc(&n->d_loss, sizeof(double)));
             }
-            n->fast = !n->training && tc_applicable(nx, ny, C);
+            n->fast = tc_applicable(nx, ny, C);
             if (n->fast) {
-                for (int i = 0; i < 2; ++i) LGD_CHECK_CUDA(cudaMalloc(&n->hg[i], tc_ghost_bytes(nx, ny, nz, batch)));
-                n->wtc = tc_alloc_weights(false);
-                LGD_CHECK_CUDA(cudaMalloc(&n->d_err, sizeof(int)));
-                LGD_CHECK_CUDA(cudaMemsetAsync(n->d_err, 0, sizeof(int), n->stream));
+                const size_t gbytes = tc_ghost_bytes(nx, ny, nz, batch);
+                for (int i = 0; i < (n->training ? 3 : 2); ++i) LGD_CHECK_CUDA(cudaMalloc(&n->hg[i], gbytes));
+                if (n->training) {
+                    for (int i = 0; i < 2; ++i) LGD_CHECK_CUDA(cudaMalloc(&n->dzg[i], gbytes));
+                    for (int i = 0; i < 3; ++i) {
+                        LGD_CHECK_CUDA(cudaMalloc(&n->zt[i], sizeof(float) * tc_z_floats(nx, ny, nz, batch)));
+                    }
+                    LGD_CHECK_CUDA(cudaMalloc(&n->xt, sizeof(uint32_t) * V));
+                    LGD_CHECK_CUDA(cudaMalloc(&n->part, sizeof(float) * tc_partial_floats()));
+                }
+                n->wtc = tc_alloc_weights(n->training);
+                // mapped host memory: written by a failing kernel, read by the host
+                LGD_CHECK_CUDA(cudaHostAlloc(&n->d_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+                *n->d_err = 0;
             }
             repack(*n);
             LGD_CHECK_CUDA(cudaStreamSynchronize(n->stream));
@@ -804,7 +880,7 @@ int lgd_net_get_params(lgd_net *h, float *host, size_t count)
         Net& n = net_of(h);
         LGD_REQUIRE(host != nullptr && (long long)count == n.P, LGD_ERR_INVALID, "parameter count mismatch");
         LGD_CHECK_CUDA(cudaMemcpyAsync(host, n.params, sizeof(float) * count, cudaMemcpyDeviceToHost, n.stream));
-        LGD_CHECK_CUDA(cudaStreamSynchronize(n.stream));
+        sync_and_check(n);
     });
 }
 
@@ -815,7 +891,7 @@ int lgd_net_get_grads(lgd_net *h, float *host, size_t count)
         LGD_REQUIRE(n.training, LGD_ERR_INVALID, "network was created without training buffers");
         LGD_REQUIRE(host != nullptr && (long long)count == n.P, LGD_ERR_INVALID, "parameter count mismatch");
         LGD_CHECK_CUDA(cudaMemcpyAsync(host, n.grads, sizeof(float) * count, cudaMemcpyDeviceToHost, n.stream));
-        LGD_CHECK_CUDA(cudaStreamSynchronize(n.stream));
+        sync_and_check(n);
     });
 }
 
@@ -886,15 +962,7 @@ int lgd_net_synchronize(lgd_net *h)
 {
     return guard([&] {
         Net& n = net_of(h);
-        LGD_CHECK_CUDA(cudaStreamSynchronize(n.stream));
-        if (n.d_err) {
-            int e = 0;
-            LGD_CHECK_CUDA(cudaMemcpy(&e, n.d_err, sizeof(int), cudaMemcpyDeviceToHost));
-            if (e) {
-                LGD_CHECK_CUDA(cudaMemset(n.d_err, 0, sizeof(int)));
-                throw Error(LGD_ERR_TIMEOUT, "tensor-core convolution gave up waiting for its copies or MMAs");
-            }
-        }
+        sync_and_check(n);
     });
 }
 

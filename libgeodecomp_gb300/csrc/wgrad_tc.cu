@@ -1,0 +1,492 @@
+// Weight gradients of the surrogate's 3^3 convolutions (C = 24) on the
+// fifth-generation tensor cores: dW[tap][ci][co] = sum over the voxels v of
+// h[v + tap][ci] * dz[v][co], a contraction over the voxels.
+//
+// Operands lie in shared memory with the channels contiguous (16 bytes = 8
+// channels of a voxel, voxels 16 bytes apart), which is the tensor core's
+// MN-major form with K = voxels: a unit of eight M or N elements per (row,
+// channel group), all units a constant stride apart, and a tap in x is a start
+// address.  Per MMA (K = 16 voxels):
+//   CC (layers 2, 3)  M = 16 units = five rows of h and a third (120 of the
+//                     128 rows of D used), N = two rows of dz (48): the pairs
+//                     (row of h, row of dz) with h at most one row away give
+//                     the taps in y, so that one MMA serves all three.  Nine
+//                     accumulators of 48 columns: taps in z times taps in x;
+//   L (layer 4)       the same h against two rows of the loss gradient, its
+//                     three x neighbours in one unit: N = 16, three
+//                     accumulators;
+//   F (layer 1)       M = 16 rows of x0 (u, kappa of the three x neighbours in
+//                     one unit) against four rows of dz: N = 96, three
+//                     accumulators.
+// The accumulators (FP32, tensor memory) stay for all of a CTA's voxels; at
+// the end it folds them into one dW and writes that to its own slice of a
+// buffer, which reduce_kernel adds up in a fixed order.  The mma.sync kernel
+// before took its operands from shared memory two bytes at a time and added
+// every tile's dW to the gradient with atomics.
+//
+// CTAs are persistent over (column of TXW x TY voxels, z chunk) items and
+// march each in z: h plane q meets dz planes q - 2, q - 1, q (two slots of h,
+// four of dz).  Warp 0 issues the MMAs, warps 1 .. 4 clear the accumulators
+// first and fold them at the end, warps 5 .. 12 fill the slots.  Waits are
+// bounded as in conv_tc.cu.
+#include <algorithm>
+
+#include "lgd_internal.h"
+#include "tc_common.cuh"
+#include "conv_tc.h"
+
+namespace lgd {
+namespace sur {
+namespace tc {
+
+enum { CC = 0, FL = 1, LL = 2 };            // layers 2 and 3; first; last
+
+constexpr int WG_LOADERS = 8;
+constexpr int WG_THREADS = 32 * (5 + WG_LOADERS);
+constexpr int SH = 2, SD = 4;               // slots of h and dz
+
+template<int MODE, int TXW>
+struct WGeo {
+    static constexpr int TY = 512 / TXW;
+    static constexpr int ROWS = TY + 2;
+    static constexpr int NG = TXW / 8;
+    static constexpr int GS = MODE == FL ? 128 : 160;           // bytes of an 8-voxel group of h (with halo)
+    static constexpr int UA = NG * GS;                          // M unit stride
+    static constexpr int UPR = MODE == FL ? 1 : 3;              // M units per row
+    static constexpr int HSLOT = ROWS * UPR * UA;
+    static constexpr int UB = TXW * 16;                         // N unit stride
+    static constexpr int NPR = MODE == LL ? 1 : 3;              // N units per row
+    static constexpr int DSLOT = TY * NPR * UB;
+    static constexpr int YB = MODE == FL ? 4 : 2;               // dz rows per MMA
+    static constexpr int N = YB * NPR * 8;                      // 48, 96, 16
+    static constexpr int DX = MODE == CC ? 3 : 1;
+    static constexpr int TMEM = MODE == CC ? 512 : (MODE == FL ? 512 : 64);
+    static constexpr int CIN = MODE == FL ? 2 : 24;
+    static constexpr int COUT = MODE == LL ? 1 : 24;
+    static constexpr int OUT = 27 * CIN * COUT;
+    static constexpr int RING = SH * HSLOT + SD * DSLOT;
+    // M always spans 16 units: the last MMA of a slot reads past it
+    static constexpr int REACH = SH * HSLOT + 16 * UA;
+    static constexpr int USED = RING > REACH ? RING : REACH;
+    static constexpr int SMEM = 128 + (USED > OUT * 4 ? USED : OUT * 4);
+};
+
+struct WParams {
+    Shape s;
+    int zchunk, items;
+    const bf16 *h;              // CC, LL: ghosted activations
+    const uint32_t *x0;         // FL: BF16 pairs (u, kappa) [batch][nz][ny][nx]
+    const bf16 *dz;             // CC, FL: ghosted
+    const float *du, *target;   // LL
+    float scale;                // LL: 2 / N
+    float *part;                // [gridDim.x][OUT]
+    int *err;
+};
+
+__device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void *src, bool copy)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(copy ? 16 : 0) : "memory");
+}
+
+__device__ __forceinline__ void st_shared16(uint32_t dst, uint4 v)
+{
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+template<int MODE, int TXW>
+__global__ void __launch_bounds__(WG_THREADS, 1)
+wgrad_tc_kernel(const WParams p)
+{
+    typedef WGeo<MODE, TXW> G;
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[SH];      // a step's h and dz planes there (one arrive per loader warp)
+    __shared__ __align__(8) uint64_t bar_empty[SH];     // h slot no longer read
+    __shared__ __align__(8) uint64_t bar_dempty[SD];    // dz slot no longer read
+    __shared__ __align__(8) uint64_t bar_clear;         // accumulators cleared
+    __shared__ __align__(8) uint64_t bar_done;          // all MMAs done
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_fail;
+    __shared__ int s_bad;       // the fold gave up (set by its own warps only, so that they agree)
+    volatile int *fail = &s_fail;
+
+    unsigned char *smem = smem_raw + ((128 - (saddr(smem_raw) & 127)) & 127);
+    const uint32_t hring = saddr(smem);
+    const uint32_t dring = hring + SH * G::HSLOT;
+
+    const Shape s = p.s;
+    const int tid = threadIdx.x;
+    const int warp = tid >> 5;
+    const int lane = tid & 31;
+    const int bx = s.nx / TXW, by = (s.ny + G::TY - 1) / G::TY;
+    const int zsplit = (s.nz + p.zchunk - 1) / p.zchunk;
+
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&s_tmem)),
+                     "r"(G::TMEM)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 0) {
+        s_fail = 0;
+        s_bad = 0;
+        for (int i = 0; i < SH; ++i) {
+            mbar_init(saddr(&bar_full[i]), WG_LOADERS);
+            mbar_init(saddr(&bar_empty[i]), 1);
+        }
+        for (int i = 0; i < SD; ++i) mbar_init(saddr(&bar_dempty[i]), 1);
+        mbar_init(saddr(&bar_clear), 4);
+        mbar_init(saddr(&bar_done), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    dependent_start();
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = s_tmem;
+
+    // item -> column and z range; the same walk in every role
+    struct Item {
+        int x0, y0, b, z0, n;
+    };
+    auto item_of = [&](int it) {
+        Item t;
+        const int col = it / zsplit;
+        t.x0 = col % bx * TXW;
+        t.y0 = col / bx % by * G::TY;
+        t.b = col / (bx * by);
+        t.z0 = it % zsplit * p.zchunk;
+        t.n = min(t.z0 + p.zchunk, s.nz) - t.z0;
+        return t;
+    };
+
+    if (warp == 0) {
+        bool ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_clear), 0, fail));
+        fence_after();
+        constexpr uint32_t ID = idesc(128, G::N, true);
+        constexpr uint32_t HI_A = desc_hi(G::UA), HI_B = desc_hi(G::UB);
+        int step = 0;               // h planes so far
+        int dbase = 0;              // dz planes of the items before this one
+        for (int it = blockIdx.x; ok && it < p.items; it += gridDim.x) {
+            const Item t = item_of(it);
+            for (int q = 0; ok && q < t.n + 2; ++q, ++step) {
+                ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_full[step % SH]), (uint32_t)((step / SH) & 1), fail));
+                if (!ok) break;
+                fence_after();
+                const uint32_t a0 = desc_lo(hring + (uint32_t)((step % SH) * G::HSLOT), G::GS);
+                for (int dz = 0; dz < 3; ++dz) {
+                    const int j = q - dz;
+                    if (j < 0 || j >= t.n) continue;
+                    const uint32_t b0 = desc_lo(dring + (uint32_t)(((dbase + j) % SD) * G::DSLOT), 128);
+                    for (int y = 0; y < G::TY; y += G::YB) {
+                        if (elect_one()) {
+                            const uint32_t ay = a0 + (uint32_t)((y * G::UPR * G::UA) >> 4);
+                            const uint32_t bw = b0 + (uint32_t)((y * G::NPR * G::UB) >> 4);
+                            const uint32_t d = tmem + (uint32_t)(dz * G::DX * G::N);
+#pragma unroll
+                            for (int dx = 0; dx < G::DX; ++dx) {
+                                // CC: tap dx; LL: the centre voxel; FL: x taps sit in the unit
+                                const int shift = MODE == CC ? dx : (MODE == LL ? 1 : 0);
+#pragma unroll
+                                for (int k = 0; k < TXW / 16; ++k) {
+                                    mma<true>(d + (uint32_t)(dx * G::N), desc(ay + (uint32_t)((2 * k * G::GS) / 16 + shift), HI_A),
+                                              desc(bw + (uint32_t)(2 * k * 8), HI_B), ID);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                    }
+                }
+                if (elect_one()) {
+                    mma_commit(saddr(&bar_empty[step % SH]));
+                    if (q >= 2) mma_commit(saddr(&bar_dempty[(dbase + q - 2) % SD]));
+                }
+                __syncwarp();
+            }
+            dbase += t.n;
+        }
+        if (elect_one()) mma_commit(saddr(&bar_done));
+        if (!ok && lane == 0) s_fail = 1;
+        __syncwarp();
+    } else if (warp >= 5) {
+        const int lt = tid - 5 * 32;
+        constexpr int LT = WG_LOADERS * 32;
+        bool ok = true;
+        int step = 0, dcount = 0;
+        int published = 0;
+        auto publish = [&](int upto) {
+            fence_async_proxy();
+            __syncwarp();
+            for (; published < upto; ++published) {
+                if (lane == 0) mbar_arrive(saddr(&bar_full[published % SH]));
+            }
+        };
+        for (int it = blockIdx.x; ok && it < p.items; it += gridDim.x) {
+            const Item t = item_of(it);
+            for (int q = 0; q < t.n + 2; ++q, ++step) {
+                bool got = true;
+                if (step >= SH) {
+                    // the step before has landed meanwhile: hand it over first
+                    asm volatile("cp.async.wait_all;" ::: "memory");
+                    publish(step);
+                    got = mbar_wait(saddr(&bar_empty[step % SH]), (uint32_t)(((step - SH) / SH) & 1), fail);
+                }
+                const bool has_dz = q < t.n;
+                if (has_dz && dcount >= SD) {
+                    got = got && mbar_wait(saddr(&bar_dempty[dcount % SD]), (uint32_t)(((dcount - SD) / SD) & 1), fail);
+                }
+                if (!__all_sync(0xffffffffu, got)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t hs = hring + (uint32_t)((step % SH) * G::HSLOT);
+                const uint32_t ds = dring + (uint32_t)((dcount % SD) * G::DSLOT);
+                if (MODE == FL) {
+                    int z = t.z0 - 1 + q;
+                    z = z < 0 ? z + s.nz : (z >= s.nz ? z - s.nz : z);
+                    for (int v = lt; v < G::ROWS * TXW; v += LT) {
+                        const int r = v / TXW;
+                        const int x = t.x0 + v % TXW;
+                        int y = t.y0 - 1 + r;
+                        y = y < 0 ? y + s.ny : (y >= s.ny ? (y - s.ny) % s.ny : y);
+                        const uint32_t *row = p.x0 + (((long long)t.b * s.nz + z) * s.ny + y) * s.nx;
+                        st_shared16(hs + (uint32_t)(v * 16), make_uint4(row[x == 0 ? s.nx - 1 : x - 1], row[x],
+                                                                        row[x == s.nx - 1 ? 0 : x + 1], 0u));
+                    }
+                } else {
+                    constexpr int PER_ROW = G::NG * 10;
+                    for (int v = lt; v < G::ROWS * PER_ROW; v += LT) {
+                        const int r = v / PER_ROW;
+                        const int i = v - r * PER_ROW;
+                        const int gy = min(t.y0 + r, s.ny + 1);
+                        const bf16 *src =
+                            p.h + (ghost_row(s, t.b, t.z0 + q, gy) * (s.nx + 2) + t.x0 + (i / 10) * 8 + i % 10) * 8;
+                        const uint32_t d = hs + (uint32_t)(r * 3 * G::UA + i * 16);
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) copy16(d + c * G::UA, src + (long long)c * (s.nx + 2) * 8);
+                    }
+                }
+                if (has_dz) {
+                    // rows past the grid count nothing
+                    for (int v = lt; v < G::TY * TXW; v += LT) {
+                        const int r = v / TXW;
+                        const int x = t.x0 + v % TXW;
+                        const int y = t.y0 + r;
+                        const bool in = y < s.ny;
+                        const uint32_t d = ds + (uint32_t)(r * G::NPR * G::UB + v % TXW * 16);
+                        if (MODE == LL) {
+                            // taps dx = 0, 1, 2 of voxel x of h meet g at x + 1, x, x - 1
+                            uint4 g = make_uint4(0u, 0u, 0u, 0u);
+                            if (in) {
+                                const long long row = (((long long)t.b * s.nz + t.z0 + q) * s.ny + y) * s.nx;
+                                const int xw = x == 0 ? s.nx - 1 : x - 1, xe = x == s.nx - 1 ? 0 : x + 1;
+                                g.x = pack_bf16(p.scale * (p.du[row + xe] - p.target[row + xe]),
+                                                p.scale * (p.du[row + x] - p.target[row + x]));
+                                g.y = pack_bf16(p.scale * (p.du[row + xw] - p.target[row + xw]), 0.f);
+                            }
+                            st_shared16(d, g);
+                        } else {
+                            const bf16 *src =
+                                p.dz + (ghost_row(s, t.b, t.z0 + q + 1, in ? y + 1 : 0) * (s.nx + 2) + x + 1) * 8;
+#pragma unroll
+                            for (int c = 0; c < 3; ++c) {
+                                copy16_or_zero(d + c * G::UB, src + (long long)c * (s.nx + 2) * 8, in);
+                            }
+                        }
+                    }
+                    ++dcount;
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (ok) publish(step);
+        else if (lane == 0) s_fail = 1;
+    } else {
+        // warps 1 .. 4: lane quarter warp % 4
+        const int qd = warp & 3;
+        const uint32_t acc = tmem + ((uint32_t)(qd * 32) << 16);
+        const float zero[8] = {};
+        for (int c = 0; c < 3 * G::DX * G::N; c += 8) tmem_st8(acc + (uint32_t)c, zero);
+        tmem_st_wait();
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(saddr(&bar_clear));
+        const bool done = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_done), 0, fail));
+        fence_after();
+        if (!done && lane == 0) s_fail = s_bad = 1;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (!s_bad) {
+            // every copy has been read by an MMA: the ring becomes dW
+            float *dw = reinterpret_cast<float *>(smem);
+            const int ft = (warp - 1) * 32 + lane;
+            for (int i = ft; i < G::OUT; i += 128) dw[i] = 0.f;
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            const int m = qd * 32 + lane;               // row of D: unit m / 8, element m % 8
+            const int w = MODE == FL ? m / 8 : m / 24;  // row of h
+            const int e = MODE == FL ? m % 8 : m % 24;  // FL: 2 dx + channel; else input channel
+            // rounds over the dz row: one contribution per dW element each
+            for (int y = 0; y < G::YB; ++y) {
+                const int dy = w - y;
+                const bool use = dy >= 0 && dy < 3 && (MODE != FL || e < 6);
+                for (int dz = 0; dz < 3; ++dz) {
+#pragma unroll
+                    for (int dx = 0; dx < G::DX; ++dx) {
+#pragma unroll
+                        for (int c = 0; c < G::NPR; ++c) {
+                            float v[8];
+                            __syncwarp();
+                            tmem_ld8(acc + (uint32_t)((dz * G::DX + dx) * G::N + (y * G::NPR + c) * 8), v);
+#pragma unroll
+                            for (int i = 0; i < 8 && use; ++i) {
+                                if (MODE == LL) {
+                                    if (i < 3) dw[((dz * 3 + dy) * 3 + i) * 24 + e] += v[i];
+                                } else if (MODE == FL) {
+                                    dw[(((dz * 3 + dy) * 3 + e / 2) * 2 + e % 2) * 24 + c * 8 + i] += v[i];
+                                } else {
+                                    dw[(((dz * 3 + dy) * 3 + dx) * 24 + e) * 24 + c * 8 + i] += v[i];
+                                }
+                            }
+                        }
+                    }
+                }
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+            }
+            float *out = p.part + (long long)blockIdx.x * G::OUT;
+            for (int i = ft; i < G::OUT; i += 128) out[i] = dw[i];
+        }
+    }
+
+    fence_before();
+    __syncthreads();
+    fence_after();
+    if (s_fail) {
+        // report, then wait (bounded) for the MMAs in flight
+        if (tid == 0) {
+            atomicExch(p.err, 1);
+            mbar_wait(saddr(&bar_done), 0, nullptr);
+        }
+        fence_before();
+        __syncthreads();
+        fence_after();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G::TMEM) : "memory");
+    }
+}
+
+// grads[off + i] = the sum of the CTAs' dW, in the CTAs' order
+struct RParams {
+    const float *part[4];
+    int ctas[4], n[4];
+    long long off[4];
+};
+
+__global__ void __launch_bounds__(256)
+reduce_kernel(const RParams p, float *grads)
+{
+    dependent_start();
+    const int l = blockIdx.y;
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < p.n[l]; i += gridDim.x * 256) {
+        const float *q = p.part[l] + i;
+        float a = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < p.ctas[l]; ++c) a += q[(long long)c * p.n[l]];
+        grads[p.off[l] + i] = a;
+    }
+}
+
+static int sm_count()
+{
+    static PerDevice<int> setup;
+    return setup.get([] {
+        int dev = 0, count = 0;
+        LGD_CHECK_CUDA(cudaGetDevice(&dev));
+        LGD_CHECK_CUDA(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev));
+        return count;
+    });
+}
+
+template<int MODE, int TXW>
+static int run_w(WParams p, cudaStream_t stream)
+{
+    typedef WGeo<MODE, TXW> G;
+    static PerDevice<bool> setup;
+    setup.get([] {
+        LGD_CHECK_CUDA(cudaFuncSetAttribute(wgrad_tc_kernel<MODE, TXW>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM));
+        return true;
+    });
+    const int sms = sm_count();
+    const long long cols = (long long)(p.s.nx / TXW) * ((p.s.ny + G::TY - 1) / G::TY) * p.s.batch;
+    double best = 1e300;
+    for (int split = 1; split <= std::max(1, p.s.nz / 2); ++split) {
+        const int chunk = (p.s.nz + split - 1) / split;
+        const long long items = cols * ((p.s.nz + chunk - 1) / chunk);
+        const double t = (double)((items + sms - 1) / sms) * (chunk + 2);
+        if (t < best * 0.999) {
+            best = t;
+            p.zchunk = chunk;
+            p.items = (int)items;
+        }
+    }
+    const int ctas = std::min(sms, p.items);
+    launch_dependent(wgrad_tc_kernel<MODE, TXW>, dim3(ctas), WG_THREADS, G::SMEM, stream, p);
+    check_launch("tensor-core weight gradient");
+    return ctas;
+}
+
+template<int MODE>
+static int run_w_any(const WParams& p, cudaStream_t stream)
+{
+    if (p.s.nx % 128 == 0) return run_w<MODE, 128>(p, stream);
+    if (p.s.nx % 64 == 0) return run_w<MODE, 64>(p, stream);
+    return run_w<MODE, 32>(p, stream);
+}
+
+}  // namespace tc
+
+using namespace tc;
+
+// elements of a layer's dW, and of all layers' partial buffers
+static const int DW[4] = {27 * 2 * 24, 27 * 24 * 24, 27 * 24 * 24, 27 * 24};
+
+size_t tc_partial_floats()
+{
+    return (size_t)sm_count() * (DW[0] + DW[1] + DW[2] + DW[3]);
+}
+
+int tc_wgrad(int layer, const void *h, const void *x0, const void *dz, const float *du, const float *target, float scale,
+             float *partials, const int dims[4], int *err, cudaStream_t stream)
+{
+    WParams p = {};
+    p.s = {dims[0], dims[1], dims[2], dims[3]};
+    p.h = (const bf16 *)h;
+    p.x0 = (const uint32_t *)x0;
+    p.dz = (const bf16 *)dz;
+    p.du = du;
+    p.target = target;
+    p.scale = scale;
+    size_t off = 0;
+    for (int l = 0; l < layer; ++l) off += (size_t)sm_count() * DW[l];
+    p.part = partials + off;
+    p.err = err;
+    if (layer == 0) return run_w_any<FL>(p, stream);
+    if (layer == 3) return run_w_any<LL>(p, stream);
+    return run_w_any<CC>(p, stream);
+}
+
+void tc_wgrad_reduce(const float *partials, const int ctas[4], const long long w_off[4], float *grads, cudaStream_t stream)
+{
+    RParams r;
+    size_t off = 0;
+    for (int l = 0; l < 4; ++l) {
+        r.part[l] = partials + off;
+        r.ctas[l] = ctas[l];
+        r.n[l] = DW[l];
+        r.off[l] = w_off[l];
+        off += (size_t)sm_count() * DW[l];
+    }
+    launch_dependent(reduce_kernel, dim3((DW[1] + 255) / 256, 4), 256u, 0, stream, r, grads);
+    check_launch("weight gradient sum");
+}
+
+}  // namespace sur
+}  // namespace lgd

@@ -151,8 +151,7 @@ class SurrogateNet:
         return n.value
 
     def set_variant(self, variant: int):
-        """0: tcgen05 layers where they apply (inference, C = 24, nx % 128 == 0,
-        ny even); 1: mma.sync for every layer."""
+        """0: tcgen05 kernels for every convolution (24 channels); 1: mma.sync."""
         lgd.check(self._L.lgd_net_set_variant(self._h, variant))
 
     def uses_tensor_core_path(self) -> bool:
