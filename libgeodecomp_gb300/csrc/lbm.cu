@@ -80,9 +80,10 @@ struct Lbm {
     int depth;
     int tb_shape;
     int tb_ctas;
-    int4 *d_cols;
+    int4 *d_cols;       // (instance, x0 | y0 << 16, z0, z1)
     int n_cols;
     int cols_shape;
+    double *d_stage;    // conversion staging of uploads and downloads (FP32; from the first one on)
 };
 
 // D3Q19 directions in the reference's naming order: C, N, E, W, S, T, B,
@@ -214,17 +215,37 @@ struct PullAll<R, 19, IDX, NC, INTERIOR> {
     static __device__ __forceinline__ void run(const R *, IDX, IDX, int, int, int, int, R, R *) {}
 };
 
-// BGK collision, operation order of the oracle's lgd_d3q19_collide; put(i,
-// v) stores post-collision population i
-// e * u for a direction component e in {-1, 0, 1} known at compile time:
-// u, -u, or u * 0 (kept as a multiplication, so that the sign of a zero
-// product is the IEEE product's) - bit for bit the product (R)e * u
-template<typename R>
-__device__ __forceinline__ R mul_dir(int e, R u)
+// e . u for one of a pair of opposite directions, components added in the
+// oracle's order (x, y, z).  Its zero components drop out: adding 0 * u does
+// not change a sum but for the sign of a zero, which d + eu and eu * eu below
+// do not see.
+template<typename R, int I>
+__device__ __forceinline__ R dot_dir(R ux, R uy, R uz)
 {
-    return e == 1 ? u : (e == -1 ? -u : LbmArith<R>::mul((R)0, u));
+    typedef LbmArith<R> A;
+    const R x = Q<I>::ex == 1 ? ux : -ux, y = Q<I>::ey == 1 ? uy : -uy, z = Q<I>::ez == 1 ? uz : -uz;
+    if (Q<I>::ex == 0 && Q<I>::ey == 0) return z;
+    if (Q<I>::ex == 0) return Q<I>::ez == 0 ? y : A::add(y, z);
+    if (Q<I>::ey == 0) return Q<I>::ez == 0 ? x : A::add(x, z);
+    return A::add(x, y);
 }
 
+// directions I and its opposite: e . u is the exact negative and its square
+// the same, so both are taken once (D3Q19: 9 pairs; the collision was a third
+// longer with 18 separate directions)
+template<typename R, int I, typename PUT>
+__device__ __forceinline__ void collide_pair(const R *f, R keep, R w1, R w2, R d, R ux, R uy, R uz, PUT put)
+{
+    typedef LbmArith<R> A;
+    const R wi = (I < 7) ? w1 : w2;
+    const R eu = dot_dir<R, I>(ux, uy, uz);
+    const R sq = A::mul((R)1.5, A::mul(eu, eu));
+    put(I, A::add(A::mul(keep, f[I]), A::mul(wi, A::add(A::add(d, eu), sq))));
+    put(Q<I>::opp, A::add(A::mul(keep, f[Q<I>::opp]), A::mul(wi, A::add(A::sub(d, eu), sq))));
+}
+
+// BGK collision, operation order of the oracle's lgd_d3q19_collide; put(i,
+// v) stores post-collision population i
 template<typename R, typename PUT>
 __device__ __forceinline__ void collide_to(const R *f, R omega, PUT put)
 {
@@ -247,13 +268,15 @@ __device__ __forceinline__ void collide_to(const R *f, R omega, PUT put)
     const R w1 = A::mul(omega, (R)(1.0 / 6.0));
     const R w2 = A::mul(omega, (R)(1.0 / 12.0));
     put(0, A::add(A::mul(keep, f[0]), A::mul(omega, d)));
-#pragma unroll
-    for (int i = 1; i < 19; ++i) {
-        // eu = ex * ux + ey * uy + ez * uz, evaluated as the oracle does
-        const R eu = A::add(A::add(mul_dir<R>(dir_ex(i), ux), mul_dir<R>(dir_ey(i), uy)), mul_dir<R>(dir_ez(i), uz));
-        const R wi = (i < 7) ? w1 : w2;
-        put(i, A::add(A::mul(keep, f[i]), A::mul(wi, A::add(A::add(d, eu), A::mul((R)1.5, A::mul(eu, eu))))));
-    }
+    collide_pair<R, 1>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 2>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 5>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 7>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 8>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 11>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 12>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 15>(f, keep, w1, w2, d, ux, uy, uz, put);
+    collide_pair<R, 16>(f, keep, w1, w2, d, ux, uy, uz, put);
 }
 
 template<typename R, typename IDX, int NC>
@@ -343,7 +366,7 @@ __global__ void lbm_single_kernel(const LbmInstance *__restrict__ inst, int j, c
 
 // ------------------------------------------------ two steps per launch
 // Temporal blocking of depth 2.  A work item is a column of one instance:
-// TX x TY cells of every z plane.  The CTA marches z; at each plane it
+// TX x TY cells of the z planes of its chunk.  The CTA marches z; at each plane it
 // first computes step 1 for the tile plus a one-cell rim (the cells whose
 // populations step 2 pulls), pulling from the input grid and keeping the 19
 // post-collision populations in a ring of three planes in shared memory,
@@ -413,14 +436,16 @@ lbm_tb2_kernel(const LbmInstance *__restrict__ inst, const int4 *__restrict__ it
         const int4 w = items[it];
         const LbmInstance in = inst[w.x];
         const int L = in.L;
-        const int x0 = w.y;
-        const int y0 = w.z;
+        const int x0 = w.y & 0xffff;
+        const int y0 = w.y >> 16;
+        const int z0 = w.z;             // step 2 computes planes z0 .. z1 - 1, step 1 one more on either side
+        const int z1 = w.w;
         const IDX n3 = ((IDX)L * L * L + 31) & ~(IDX)31;
         const R *src = A + in.base;
         R *dst = B + in.base;
         const R omega = (sizeof(R) == 8) ? (R)in.omega : (R)in.omega_f;
         const R lid = (sizeof(R) == 8) ? (R)in.lid : (R)in.lid_f;
-        for (int z = 0; z <= L; ++z) {
+        for (int z = max(z0 - 1, 0); z <= z1; ++z) {
             if (z < L) {
                 // step 1 at plane z: the tile and its rim, inside the instance
                 R *plane = ring + (z % 3) * 19 * G::HC;
@@ -441,7 +466,7 @@ lbm_tb2_kernel(const LbmInstance *__restrict__ inst, const int4 *__restrict__ it
                 }
             }
             __syncthreads();
-            if (z >= 1) {
+            if (z > z0) {
                 // step 2 at plane z - 1: the tile, from the ring
                 const int zz = z - 1;
                 const int tx = tid % TX;
@@ -473,6 +498,57 @@ __global__ void lbm_rest_kernel(const LbmInstance *__restrict__ inst, int count,
         for (int i = 1; i < 7; ++i) A[in.base + i * P + c] = (R)(1.0 / 18.0);
         for (int i = 7; i < 19; ++i) A[in.base + i * P + c] = (R)(1.0 / 36.0);
     }
+}
+
+// FP32 populations of one instance <-> dense doubles, values first .. first + n
+template<bool TO_HOST>
+__global__ void __launch_bounds__(256)
+convert_kernel(float *f, double *dense, unsigned n3, long long pitch, long long first, long long n)
+{
+    for (long long k = blockIdx.x * 256ll + threadIdx.x; k < n; k += gridDim.x * 256ll) {
+        const long long i = (first + k) / n3;
+        float *p = f + i * pitch + (first + k - i * n3);
+        if (TO_HOST) dense[k] = *p;
+        else *p = (float)dense[k];
+    }
+}
+
+// Host copy of one instance as 19 * L^3 doubles.  FP32 populations convert on
+// the device in bounded chunks (on one host core the conversion took 0.5 ns a
+// value, ten times the copy).
+constexpr long long CONVERT_CHUNK = 8ll << 20;
+
+static void copy_instance(Lbm& e, const LbmInstance& in, size_t n3, double *host, bool up)
+{
+    if (e.precision == 8) {
+        double *d = (double *)e.buf[e.cur] + in.base;
+        if (up) {
+            LGD_CHECK_CUDA(cudaMemcpy2DAsync(d, (size_t)in.pitch * 8, host, n3 * 8, n3 * 8, 19, cudaMemcpyHostToDevice,
+                                             e.stream));
+        } else {
+            LGD_CHECK_CUDA(cudaMemcpy2DAsync(host, n3 * 8, d, (size_t)in.pitch * 8, n3 * 8, 19, cudaMemcpyDeviceToHost,
+                                             e.stream));
+        }
+        LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
+        return;
+    }
+    if (e.d_stage == nullptr) LGD_CHECK_CUDA(cudaMalloc(&e.d_stage, CONVERT_CHUNK * sizeof(double)));
+    float *f = (float *)e.buf[e.cur] + in.base;
+    const long long total = 19ll * (long long)n3;
+    for (long long first = 0; first < total; first += CONVERT_CHUNK) {
+        const long long n = std::min(CONVERT_CHUNK, total - first);
+        const unsigned blocks = (unsigned)std::min<long long>(152 * 16, (n + 255) / 256);
+        if (up) {
+            LGD_CHECK_CUDA(cudaMemcpyAsync(e.d_stage, host + first, n * 8, cudaMemcpyHostToDevice, e.stream));
+            convert_kernel<false><<<blocks, 256, 0, e.stream>>>(f, e.d_stage, (unsigned)n3, in.pitch, first, n);
+        } else {
+            convert_kernel<true><<<blocks, 256, 0, e.stream>>>(f, e.d_stage, (unsigned)n3, in.pitch, first, n);
+            LGD_CHECK_CUDA(cudaMemcpyAsync(host + first, e.d_stage, n * 8, cudaMemcpyDeviceToHost, e.stream));
+        }
+        check_launch("lbm conversion");
+        ++e.launches;
+    }
+    LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
 }
 
 static Lbm& lbm_of(lgd_lbm *h)
@@ -592,11 +668,21 @@ static void build_cols(Lbm& e, int shape)
     std::vector<int> order(e.count);
     for (int j = 0; j < e.count; ++j) order[j] = j;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return e.inst[a].L > e.inst[b].L; });
+    // z chunks: the columns of a small ensemble are too few for the GPU and its
+    // largest instances' would run alone at the end; about four items per
+    // resident CTA, chunks of at least 16 planes (two more for step 1)
+    long long planes = 0;
+    for (const LbmInstance& in : e.inst) planes += (long long)((in.L + TX - 1) / TX) * ((in.L + TY - 1) / TY) * in.L;
+    const long long chunk = std::max(16ll, planes / (16ll * e.sms));
     std::vector<int4> cols;
     for (int j : order) {
         const int L = e.inst[j].L;
-        for (int y0 = 0; y0 < L; y0 += TY) {
-            for (int x0 = 0; x0 < L; x0 += TX) cols.push_back(make_int4(j, x0, y0, 0));
+        const int split = (int)std::max(1ll, (L + chunk / 2) / chunk);
+        const int zc = (L + split - 1) / split;
+        for (int z0 = 0; z0 < L; z0 += zc) {
+            for (int y0 = 0; y0 < L; y0 += TY) {
+                for (int x0 = 0; x0 < L; x0 += TX) cols.push_back(make_int4(j, x0 | y0 << 16, z0, std::min(L, z0 + zc)));
+            }
         }
     }
     if (e.d_cols) cudaFree(e.d_cols);
@@ -789,6 +875,7 @@ static void lbm_free(Lbm& e)
     cudaFree(e.d_inst);
     cudaFree(e.d_items);
     cudaFree(e.d_cols);
+    cudaFree(e.d_stage);
     cudaFree(e.d_counter);
     if (e.stream) cudaStreamDestroy(e.stream);
 }
@@ -1070,17 +1157,7 @@ int lgd_lbm_download(lgd_lbm *h, int instance, double *f, size_t bytes)
         const size_t n = 19ull * in.L * in.L * in.L;
         LGD_REQUIRE(f != nullptr && bytes == n * sizeof(double), LGD_ERR_INVALID, "buffer must hold 19 * L^3 doubles");
         const size_t n3 = n / 19;
-        if (e.precision == 8) {
-            LGD_CHECK_CUDA(cudaMemcpy2DAsync(f, n3 * 8, (const double *)e.buf[e.cur] + in.base, (size_t)in.pitch * 8,
-                                             n3 * 8, 19, cudaMemcpyDeviceToHost, e.stream));
-            LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
-        } else {
-            std::vector<float> tmp(n);
-            LGD_CHECK_CUDA(cudaMemcpy2DAsync(tmp.data(), n3 * 4, (const float *)e.buf[e.cur] + in.base,
-                                             (size_t)in.pitch * 4, n3 * 4, 19, cudaMemcpyDeviceToHost, e.stream));
-            LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
-            for (size_t i = 0; i < n; ++i) f[i] = tmp[i];
-        }
+        copy_instance(e, in, n3, f, false);
     });
 }
 
@@ -1093,16 +1170,7 @@ int lgd_lbm_upload(lgd_lbm *h, int instance, const double *f, size_t bytes)
         const size_t n = 19ull * in.L * in.L * in.L;
         LGD_REQUIRE(f != nullptr && bytes == n * sizeof(double), LGD_ERR_INVALID, "buffer must hold 19 * L^3 doubles");
         const size_t n3 = n / 19;
-        if (e.precision == 8) {
-            LGD_CHECK_CUDA(cudaMemcpy2DAsync((double *)e.buf[e.cur] + in.base, (size_t)in.pitch * 8, f, n3 * 8, n3 * 8, 19,
-                                             cudaMemcpyHostToDevice, e.stream));
-            LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
-        } else {
-            std::vector<float> tmp(f, f + n);
-            LGD_CHECK_CUDA(cudaMemcpy2DAsync((float *)e.buf[e.cur] + in.base, (size_t)in.pitch * 4, tmp.data(), n3 * 4,
-                                             n3 * 4, 19, cudaMemcpyHostToDevice, e.stream));
-            LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
-        }
+        copy_instance(e, in, n3, const_cast<double *>(f), true);
     });
 }
 
