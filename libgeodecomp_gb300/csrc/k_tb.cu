@@ -130,7 +130,7 @@ struct TBOps<Jacobi7FixTwoStepT<NONNEG> > {
 };
 
 template<typename CELL, int TB, int WY, int ROWS>
-__global__ void __launch_bounds__(32 * WY)
+__global__ void __launch_bounds__(32 * WY, WY <= 8 ? 2 : 1)
 jacobi7_tb_kernel(const __grid_constant__ CUtensorMap in_map, typename CELL::T *__restrict__ out, long pitch, int nx,
                   int ny, int nz, int zchunk, int *err)
 {
@@ -243,7 +243,9 @@ jacobi7_tb_kernel(const __grid_constant__ CUtensorMap in_map, typename CELL::T *
                     for (int r = 0; r < ROWS; ++r) {
                         v[t][P][r][0] = res[r][0];
                         v[t][P][r][1] = res[r][1];
-                        st_pair<T>(dst + ((r0 + r) * BW + cx) * (int)sizeof(T), res[r][0], res[r][1]);
+                        if (r == 0 || r == ROWS - 1) {          // the rows other warps read
+                            st_pair<T>(dst + ((r0 + r) * BW + cx) * (int)sizeof(T), res[r][0], res[r][1]);
+                        }
                     }
                 } else {
 #pragma unroll
@@ -251,7 +253,9 @@ jacobi7_tb_kernel(const __grid_constant__ CUtensorMap in_map, typename CELL::T *
                         const bool yin = zin && ((ymask >> r) & 1u);
                         v[t][P][r][0] = (yin && xin0) ? res[r][0] : T(0);
                         v[t][P][r][1] = (yin && xin1) ? res[r][1] : T(0);
-                        st_pair<T>(dst + ((r0 + r) * BW + cx) * (int)sizeof(T), v[t][P][r][0], v[t][P][r][1]);
+                        if (r == 0 || r == ROWS - 1) {
+                            st_pair<T>(dst + ((r0 + r) * BW + cx) * (int)sizeof(T), v[t][P][r][0], v[t][P][r][1]);
+                        }
                     }
                 }
             } else if (xout) {
@@ -334,22 +338,31 @@ static long long tb_resident()
 
 // Planes per CTA: minimise waves of resident CTAs times input planes per CTA
 // (the chunk plus the 2 TB halo planes); chunks of at least 8 planes.
-static int pick_zchunk_tb(long long xy, int nz, long long resident, int halo)
+struct TbPlan {
+    int zchunk;
+    double planes;          // of the launch: waves times planes per CTA
+};
+
+static TbPlan plan_tb(long long xy, int nz, long long resident, int halo)
 {
-    int best_chunk = nz;
-    double best = 1e300;
+    TbPlan best = {nz, 1e300};
     const int max_split = std::max(1, nz / 8);
     for (int split = 1; split <= max_split; ++split) {
         const int chunk = (nz + split - 1) / split;
         const int s = (nz + chunk - 1) / chunk;
         const long long waves = (xy * s + resident - 1) / resident;
         const double t = (double)waves * (chunk + halo);
-        if (t < best * 0.999) {
-            best = t;
-            best_chunk = chunk;
-        }
+        if (t < best.planes * 0.999) best = {chunk, t};
     }
-    return best_chunk;
+    return best;
+}
+
+template<typename CELL, int TB, int WY, int ROWS>
+static TbPlan plan_tb_typed(const Grid& g)
+{
+    typedef tbk::Geo<typename CELL::T, TB, WY, ROWS> G;
+    const long long xy = (long long)((g.desc.nx + G::OX - 1) / G::OX) * ((g.desc.ny + G::OY - 1) / G::OY);
+    return plan_tb(xy, g.desc.nz, tb_resident<CELL, TB, WY, ROWS>(), 2 * TB);
 }
 
 template<typename CELL, int TB, int WY, int ROWS>
@@ -368,10 +381,9 @@ static void launch_tb_typed(Grid& g, int dtype)
         g.tbmap_base[src] = base;
         g.tbmap_rows[src] = G::BH;
     }
-    const long long resident = tb_resident<CELL, TB, WY, ROWS>();
     const int bx = (g.desc.nx + G::OX - 1) / G::OX;
     const int by = (g.desc.ny + G::OY - 1) / G::OY;
-    const int zchunk = pick_zchunk_tb((long long)bx * by, g.desc.nz, resident, 2 * TB);
+    const int zchunk = plan_tb_typed<CELL, TB, WY, ROWS>(g).zchunk;
     const int zsplit = (g.desc.nz + zchunk - 1) / zchunk;
     const CUtensorMap *map = reinterpret_cast<const CUtensorMap *>(g.tbmap[src]);
     launch_dependent(
@@ -407,12 +419,8 @@ int tb_default_depth(const Grid& g)
     return g.desc.cell == LGD_CELL_JACOBI7_F32 ? 3 : 2;
 }
 
-// One pass of depth steps with box shape `shape` (0 = the fastest measured
-// on GB300 for the cell and depth; 1, 2 = alternatives; warps x rows per
-// warp; a shape that does not exist for a depth runs shape 0):
-//   fixed point  depth 2 (exact two-step sums, one rounding): 16x4, 8x4, 16x2
-//   FP32         depth 2: 8x4, 16x4, 16x2     depth 3: 16x4, 8x4, 16x2
-//                depth 4: 16x4, 8x4, 16x2
+// One pass of depth steps with box shape `shape`: 1 = 8 x 4 (warps x rows per
+// warp), 2 = 16 x 2, 0 = the best of these and 16 x 4 for the grid.
 // every pass kernel set up once, on the first pass of any grid
 static void prepare_tb_kernels()
 {
@@ -437,6 +445,20 @@ static void prepare_tb_kernels()
     });
 }
 
+// The shape of a pass when none is asked for: the least of waves times planes
+// per CTA times the measured time of a plane (us, all CTAs of an SM at work).
+// 8 x 4 boxes run two to an SM, whose phases between barriers overlap: 512^3
+// fixed point 241 us per step against 257 for 16 x 4, 302 for 16 x 2; FP32 at
+// depth 3 113 / 109 / 153; 16 x 2 wins where bands of 64 rows leave the GPU
+// idle (64^3 fixed point 5.7 us against 7.4 and 9.3).
+template<typename CELL, int TB>
+static int best_shape(const Grid& g, double us16x4, double us8x4, double us16x2)
+{
+    const double t[3] = {plan_tb_typed<CELL, TB, 16, 4>(g).planes * us16x4, plan_tb_typed<CELL, TB, 8, 4>(g).planes * us8x4,
+                         plan_tb_typed<CELL, TB, 16, 2>(g).planes * us16x2};
+    return (int)(std::min_element(t, t + 3) - t);
+}
+
 void launch_jacobi7_tb(Grid& g, int depth, int shape)
 {
     prepare_tb_kernels();
@@ -445,6 +467,7 @@ void launch_jacobi7_tb(Grid& g, int depth, int shape)
     if (g.desc.cell == LGD_CELL_JACOBI7_F64_FIX) {
         LGD_REQUIRE(depth == 2, LGD_ERR_INVALID, "the fixed-point cell fuses two steps per pass");
         // grids without negative values skip the sign handling (same results)
+        if (shape == 0) shape = best_shape<Jacobi7FixTwoStepNonNeg, 2>(g, 1.69, 1.54, 0.99);
         if (g.fix_nonneg) {
             switch (shape) {
             case 1: launch_tb_typed<Jacobi7FixTwoStepNonNeg, 2, 8, 4>(g, i64); break;
@@ -459,20 +482,22 @@ void launch_jacobi7_tb(Grid& g, int depth, int shape)
             }
         }
     } else if (g.desc.cell == LGD_CELL_JACOBI7_F32) {
+        if (shape == 0) {
+            shape = depth == 2   ? best_shape<Jacobi7F32, 2>(g, 0.76, 0.74, 0.48)
+                    : depth == 3 ? best_shape<Jacobi7F32, 3>(g, 1.00, 0.96, 0.68)
+                                 : best_shape<Jacobi7F32, 4>(g, 1.37, 1.30, 0.90);
+        }
         switch (depth * 10 + shape) {
-        case 21: launch_tb_typed<Jacobi7F32, 2, 16, 4>(g, f32); break;
+        case 20: launch_tb_typed<Jacobi7F32, 2, 16, 4>(g, f32); break;
+        case 21: launch_tb_typed<Jacobi7F32, 2, 8, 4>(g, f32); break;
         case 22: launch_tb_typed<Jacobi7F32, 2, 16, 2>(g, f32); break;
+        case 30: launch_tb_typed<Jacobi7F32, 3, 16, 4>(g, f32); break;
         case 31: launch_tb_typed<Jacobi7F32, 3, 8, 4>(g, f32); break;
         case 32: launch_tb_typed<Jacobi7F32, 3, 16, 2>(g, f32); break;
+        case 40: launch_tb_typed<Jacobi7F32, 4, 16, 4>(g, f32); break;
         case 41: launch_tb_typed<Jacobi7F32, 4, 8, 4>(g, f32); break;
         case 42: launch_tb_typed<Jacobi7F32, 4, 16, 2>(g, f32); break;
-        default:
-            switch (depth) {
-            case 2: launch_tb_typed<Jacobi7F32, 2, 8, 4>(g, f32); break;
-            case 3: launch_tb_typed<Jacobi7F32, 3, 16, 4>(g, f32); break;
-            case 4: launch_tb_typed<Jacobi7F32, 4, 16, 4>(g, f32); break;
-            default: throw Error(LGD_ERR_INVALID, "temporal blocking depth out of range");
-            }
+        default: throw Error(LGD_ERR_INVALID, "temporal blocking depth out of range");
         }
     } else {
         throw Error(LGD_ERR_UNSUPPORTED, "temporal blocking serves the fixed-point and FP32 Jacobi cells");
