@@ -7,9 +7,10 @@
 //   LAST   24 channels -> 1 (layer 4);
 //   DLAST  the loss gradient 2 (du - target) / N, one channel (the input
 //          gradient of layer 4);
-// and three epilogues: ACT (bias, GELU, ghosted BF16 output, optionally the
-// FP32 pre-activations for the backward pass), GRAD (times GELU'(z), ghosted
-// BF16 output, bias gradient), OUT (FP32 du, or u += du).
+// and three epilogues: ACT (bias, GELU, ghosted BF16 output; when training also
+// GELU' in FP32 for the backward pass, from the same terms), GRAD
+// (times the saved GELU', ghosted BF16 output, bias gradient), OUT (FP32 du, or
+// u += du).
 //
 // Why this shape.  An MMA of 128 voxels x N x 16 reads 4 KB of A and 32 N
 // bytes of B from shared memory at 128 B per clock; with N = 24 (one tap at a
@@ -88,16 +89,16 @@ struct Params {
     const bf16 *w;              // packed weights
     const float *bias;          // ACT, OUT
     bf16 *out;                  // ACT, GRAD: ghosted
-    float *z;                   // ACT: pre-activations out (or null); GRAD: in
+    float *g;                   // ACT: GELU' of the pre-activations out (or null); GRAD: in
     float *db;                  // GRAD: bias gradient, added to
     float *fout;                // OUT
     int add;                    // OUT: add to fout
     int *err;
 };
 
-// position of voxel (x, y) of plane z in the pre-activations: FP32
+// position of voxel (x, y) of plane z in the saved GELU': FP32
 // [batch][nz][ny][6][nx][4], the float4 of channels 4 c .. 4 c + 3 at + c * nx
-__device__ __forceinline__ long long z_at(const Shape& s, int b, int z, int y, int x)
+__device__ __forceinline__ long long g_at(const Shape& s, int b, int z, int y, int x)
 {
     return ((((long long)b * s.nz + z) * s.ny + y) * 6) * s.nx + x;
 }
@@ -367,24 +368,38 @@ conv_tc_kernel(const Params p)
                 restart(slot);
                 if (q < 2 || !live) continue;
                 if constexpr (EPI == ACT) {
-                    if (p.z) {
-                        float4 *zp = reinterpret_cast<float4 *>(p.z) + z_at(s, b, z, y, x);
+                    if (p.g) {
+                        // training: GELU' for the backward pass, beside GELU
+                        float4 *gp = reinterpret_cast<float4 *>(p.g) + g_at(s, b, z, y, x);
 #pragma unroll
                         for (int c = 0; c < 6; ++c) {
-                            zp[(long long)c * s.nx] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                            float2 h0, h1, g0, g1;
+                            gelu_pair<true>(make_float2(v[4 * c], v[4 * c + 1]), h0, g0);
+                            gelu_pair<true>(make_float2(v[4 * c + 2], v[4 * c + 3]), h1, g1);
+                            gp[(long long)c * s.nx] = make_float4(g0.x, g0.y, g1.x, g1.y);
+                            v[4 * c] = h0.x;
+                            v[4 * c + 1] = h0.y;
+                            v[4 * c + 2] = h1.x;
+                            v[4 * c + 3] = h1.y;
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 12; ++c) {
+                            float2 h, g;
+                            gelu_pair<false>(make_float2(v[2 * c], v[2 * c + 1]), h, g);
+                            v[2 * c] = h.x;
+                            v[2 * c + 1] = h.y;
                         }
                     }
-#pragma unroll
-                    for (int c = 0; c < 24; ++c) v[c] = gelu(v[c]);
                 } else {
-                    const float4 *zp = reinterpret_cast<const float4 *>(p.z) + z_at(s, b, z, y, x);
+                    const float4 *gp = reinterpret_cast<const float4 *>(p.g) + g_at(s, b, z, y, x);
 #pragma unroll
                     for (int c = 0; c < 6; ++c) {
-                        const float4 t = zp[(long long)c * s.nx];
-                        v[4 * c] *= gelu_grad(t.x);
-                        v[4 * c + 1] *= gelu_grad(t.y);
-                        v[4 * c + 2] *= gelu_grad(t.z);
-                        v[4 * c + 3] *= gelu_grad(t.w);
+                        const float4 t = gp[(long long)c * s.nx];
+                        v[4 * c] *= t.x;
+                        v[4 * c + 1] *= t.y;
+                        v[4 * c + 2] *= t.z;
+                        v[4 * c + 3] *= t.w;
                     }
 #pragma unroll
                     for (int c = 0; c < 24; ++c) db[c] += v[c];
@@ -605,7 +620,7 @@ size_t tc_ghost_bytes(int nx, int ny, int nz, int batch)
     return (size_t)batch * (nz + 2) * (ny + 2) * 3 * (nx + 2) * 16;
 }
 
-void tc_layer1(const float *u, const float *k, const void *w, const float *bias, void *out, float *z, const int dims[4],
+void tc_layer1(const float *u, const float *k, const void *w, const float *bias, void *out, float *gelu_grad, const int dims[4],
                int *err, cudaStream_t stream)
 {
     Params p = {};
@@ -615,12 +630,12 @@ void tc_layer1(const float *u, const float *k, const void *w, const float *bias,
     p.w = (const bf16 *)w;
     p.bias = bias;
     p.out = (bf16 *)out;
-    p.z = z;
+    p.g = gelu_grad;
     p.err = err;
     run_any<FIRST, ACT>(p, stream);
 }
 
-void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, float *z, const int dims[4], int *err,
+void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, float *gelu_grad, const int dims[4], int *err,
                   cudaStream_t stream)
 {
     Params p = {};
@@ -629,7 +644,7 @@ void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, f
     p.w = (const bf16 *)w;
     p.bias = bias;
     p.out = (bf16 *)out;
-    p.z = z;
+    p.g = gelu_grad;
     p.err = err;
     run_any<MID, ACT>(p, stream);
 }
@@ -648,21 +663,21 @@ void tc_layer_last(const void *in, const void *w, const float *bias, float *out,
     run_any<LAST, OUT>(p, stream);
 }
 
-void tc_grad_mid(const void *dz, const void *w, const float *z, void *out, float *db, const int dims[4], int *err,
+void tc_grad_mid(const void *dz, const void *w, const float *gelu_grad, void *out, float *db, const int dims[4], int *err,
                  cudaStream_t stream)
 {
     Params p = {};
     p.s = {dims[0], dims[1], dims[2], dims[3]};
     p.in = (const bf16 *)dz;
     p.w = (const bf16 *)w;
-    p.z = const_cast<float *>(z);
+    p.g = const_cast<float *>(gelu_grad);
     p.out = (bf16 *)out;
     p.db = db;
     p.err = err;
     run_any<MID, GRAD>(p, stream);
 }
 
-void tc_grad_last(const float *du, const float *target, float scale, const void *w, const float *z, void *out, float *db,
+void tc_grad_last(const float *du, const float *target, float scale, const void *w, const float *gelu_grad, void *out, float *db,
                   const int dims[4], int *err, cudaStream_t stream)
 {
     Params p = {};
@@ -671,7 +686,7 @@ void tc_grad_last(const float *du, const float *target, float scale, const void 
     p.f1 = target;
     p.scale = scale;
     p.w = (const bf16 *)w;
-    p.z = const_cast<float *>(z);
+    p.g = const_cast<float *>(gelu_grad);
     p.out = (bf16 *)out;
     p.db = db;
     p.err = err;

@@ -23,21 +23,22 @@ void tc_free_weights(TcWeights& w);
 int tc_pack_weights(const float *const layer[4], const TcWeights& w, cudaStream_t stream);   // launches made
 
 // layer 1 (u, kappa -> 24), layers 2 and 3 (24 -> 24): ghosted BF16 output;
-// z (or null) receives the pre-activations for the backward pass
-void tc_layer1(const float *u, const float *k, const void *w, const float *bias, void *out, float *z, const int dims[4],
+// gelu_grad (or null) receives GELU' of the pre-activations for the backward
+// pass
+void tc_layer1(const float *u, const float *k, const void *w, const float *bias, void *out, float *gelu_grad, const int dims[4],
                int *err, cudaStream_t stream);
-void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, float *z, const int dims[4], int *err,
+void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, float *gelu_grad, const int dims[4], int *err,
                   cudaStream_t stream);
 // layer 4 (24 -> 1): out = conv + bias, or out += that
 void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, const int dims[4], int *err,
                    cudaStream_t stream);
 
-// input gradients: dz of the layer below = conv_t(dz) * GELU'(z), ghosted, and
+// input gradients: dz of the layer below = conv_t(dz) * gelu_grad, ghosted, and
 // its sum over the voxels added to db.  The last layer's takes the loss
 // gradient scale * (du - target) itself
-void tc_grad_mid(const void *dz, const void *w, const float *z, void *out, float *db, const int dims[4], int *err,
+void tc_grad_mid(const void *dz, const void *w, const float *gelu_grad, void *out, float *db, const int dims[4], int *err,
                  cudaStream_t stream);
-void tc_grad_last(const float *du, const float *target, float scale, const void *w, const float *z, void *out, float *db,
+void tc_grad_last(const float *du, const float *target, float scale, const void *w, const float *gelu_grad, void *out, float *db,
                   const int dims[4], int *err, cudaStream_t stream);
 
 // weight gradients of layer 0 (x0: BF16 pairs u, kappa; dz), 1 and 2 (h the
@@ -50,8 +51,8 @@ int tc_wgrad(int layer, const void *h, const void *x0, const void *dz, const flo
 void tc_wgrad_reduce(const float *partials, const int ctas[4], const long long w_off[4], float *grads,
                      cudaStream_t stream);
 
-// floats of a layer's pre-activations
-inline size_t tc_z_floats(int nx, int ny, int nz, int batch) { return (size_t)nx * ny * nz * batch * 24; }
+// floats of a layer's gelu_grad
+inline size_t tc_gelu_grad_floats(int nx, int ny, int nz, int batch) { return (size_t)nx * ny * nz * batch * 24; }
 
 }  // namespace sur
 }  // namespace lgd

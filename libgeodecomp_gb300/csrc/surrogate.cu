@@ -345,7 +345,7 @@ __global__ void loss_kernel(const float *__restrict__ du, const float *__restric
     const float scale = 2.0f / (float)nvox;
     for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvox; v += (long long)gridDim.x * blockDim.x) {
         const float d = du[v] - target[v];
-        l += (double)d * d;
+        l = fma((double)d, (double)d, l);
         const float gv = scale * d;
         gs += gv;
         if (dz4) *reinterpret_cast<uint32_t *>(dz4 + 2 * v) = pack2(__float2bfloat16(gv), __float2bfloat16(0.f));
@@ -464,7 +464,7 @@ struct Net {
     int variant;        // 0: tcgen05 path where it applies; 1: mma.sync for every layer
     void *hg[3];        // ghosted activations (two without training)
     void *dzg[2];       // ghosted gradients (training)
-    float *zt[3];       // pre-activations (training)
+    float *gt[3];       // GELU' of the pre-activations (training)
     uint32_t *xt;       // BF16 pairs (u, kappa) of the last forward pass (training)
     float *part;        // weight-gradient shares of the CTAs (training)
     TcWeights wtc;      // weights in the tcgen05 operand layout
@@ -555,8 +555,8 @@ static void sync_and_check(Net& n)
 }
 
 // The forward pass on the tensor cores: four launches, the activations between
-// two ghosted buffers (three when training, which also keeps the
-// pre-activations and the packed input).  With add_to_u the last layer adds its
+// two ghosted buffers (three when training, which also keeps GELU' and the
+// packed input).  With add_to_u the last layer adds its
 // result to u instead (u <- u + du, the residual step).
 static void forward_fast(Net& n, const float *u, const float *k, float *du, bool add_to_u)
 {
@@ -568,9 +568,9 @@ static void forward_fast(Net& n, const float *u, const float *k, float *du, bool
         pack_input_kernel<<<grid_blocks(n.V), 256, 0, n.stream>>>(u, k, (bf16 *)n.xt, n.V);
         ++n.launches;
     }
-    tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], n.zt[0], dims, n.d_err, n.stream);
-    tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], n.zt[1], dims, n.d_err, n.stream);
-    tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], h3, n.zt[2], dims, n.d_err, n.stream);
+    tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], n.gt[0], dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], n.gt[1], dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], h3, n.gt[2], dims, n.d_err, n.stream);
     tc_layer_last(h3, n.wtc.fwd[3], bias[3], add_to_u ? const_cast<float *>(u) : du, add_to_u, dims, n.d_err, n.stream);
     n.launches += 4;
 }
@@ -588,11 +588,11 @@ static void backward_fast(Net& n, const float *target, double *loss_out)
     check_launch("loss");
     int ctas[4];
     ctas[3] = tc_wgrad(3, n.hg[2], nullptr, nullptr, n.du, target, scale, n.part, dims, n.d_err, n.stream);
-    tc_grad_last(n.du, target, scale, n.wtc.grad[3], n.zt[2], n.dzg[0], n.grads + n.L[2].b_off, dims, n.d_err, n.stream);
+    tc_grad_last(n.du, target, scale, n.wtc.grad[3], n.gt[2], n.dzg[0], n.grads + n.L[2].b_off, dims, n.d_err, n.stream);
     ctas[2] = tc_wgrad(2, n.hg[1], nullptr, n.dzg[0], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
-    tc_grad_mid(n.dzg[0], n.wtc.grad[2], n.zt[1], n.dzg[1], n.grads + n.L[1].b_off, dims, n.d_err, n.stream);
+    tc_grad_mid(n.dzg[0], n.wtc.grad[2], n.gt[1], n.dzg[1], n.grads + n.L[1].b_off, dims, n.d_err, n.stream);
     ctas[1] = tc_wgrad(1, n.hg[0], nullptr, n.dzg[1], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
-    tc_grad_mid(n.dzg[1], n.wtc.grad[1], n.zt[0], n.dzg[0], n.grads + n.L[0].b_off, dims, n.d_err, n.stream);
+    tc_grad_mid(n.dzg[1], n.wtc.grad[1], n.gt[0], n.dzg[0], n.grads + n.L[0].b_off, dims, n.d_err, n.stream);
     ctas[0] = tc_wgrad(0, nullptr, n.xt, n.dzg[0], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
     const long long off[4] = {n.L[0].w_off, n.L[1].w_off, n.L[2].w_off, n.L[3].w_off};
     tc_wgrad_reduce(n.part, ctas, off, n.grads, n.stream);
@@ -727,7 +727,7 @@ static void net_free(Net& n)
     cudaFree(n.d_loss);
     for (int i = 0; i < 3; ++i) {
         cudaFree(n.hg[i]);
-        cudaFree(n.zt[i]);
+        cudaFree(n.gt[i]);
     }
     cudaFree(n.dzg[0]);
     cudaFree(n.dzg[1]);
@@ -827,7 +827,7 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
                 if (n->training) {
                     for (int i = 0; i < 2; ++i) LGD_CHECK_CUDA(cudaMalloc(&n->dzg[i], gbytes));
                     for (int i = 0; i < 3; ++i) {
-                        LGD_CHECK_CUDA(cudaMalloc(&n->zt[i], sizeof(float) * tc_z_floats(nx, ny, nz, batch)));
+                        LGD_CHECK_CUDA(cudaMalloc(&n->gt[i], sizeof(float) * tc_gelu_grad_floats(nx, ny, nz, batch)));
                     }
                     LGD_CHECK_CUDA(cudaMalloc(&n->xt, sizeof(uint32_t) * V));
                     LGD_CHECK_CUDA(cudaMalloc(&n->part, sizeof(float) * tc_partial_floats()));

@@ -176,11 +176,45 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
            ((uint32_t)__bfloat16_as_ushort(__float2bfloat16(hi)) << 16);
 }
 
-__device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
-
-__device__ __forceinline__ float gelu_grad(float z)
+// GELU(z) = z Phi(z) of two values, and GELU'(z) = Phi(z) + z phi(z) where
+// asked for, each from packed FMAs, one reciprocal and one exponential:
+//   |z| < 1   Phi = 1/2 + z Q(z^2), Q of degree 4 (largest error 7e-9)
+//   else      Phi(-|z|) = exp(-z^2 / 2) t P(t) with t = 1 / (1 + p |z|): the
+//             function exp(z^2 / 2) Phi(-z) / t is smooth in t, and P its
+//             polynomial of degree 6 (relative error 8e-8 up to z = 14; p chosen
+//             for the smallest)
+// Both are least-squares fits with weights moved towards the largest error until
+// that stopped falling.  erff and expf took twice the instructions, which set the
+// time of a layer's epilogue.
+template<bool GRAD>
+__device__ __forceinline__ void gelu_pair(float2 z, float2& h, float2& g)
 {
-    return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * expf(-0.5f * z * z) * 0.39894228040143268f;
+    constexpr float P = 0.395f;
+    constexpr float C[7] = {0.15760743f, 0.15697990f, 0.13892886f, 0.052616711f,
+                            0.11542270f, -0.18699883f, 0.065657586f};
+    constexpr float Q[5] = {0.39894220f, -0.066488728f, 0.0099641671f, -0.0011653511f, 0.000092468512f};
+    const float2 d = __ffma2_rn(make_float2(fabsf(z.x), fabsf(z.y)), make_float2(P, P), make_float2(1.0f, 1.0f));
+    const float2 s = __fmul2_rn(z, z);
+    const float2 q = __fmul2_rn(s, make_float2(-0.72134752f, -0.72134752f));        // -z^2 / (2 ln 2)
+    float2 t, e;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(d.x));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(d.y));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(q.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(q.y));
+    float2 p = make_float2(C[6], C[6]), r = make_float2(Q[4], Q[4]);
+#pragma unroll
+    for (int i = 5; i >= 0; --i) p = __ffma2_rn(p, t, make_float2(C[i], C[i]));
+#pragma unroll
+    for (int i = 3; i >= 0; --i) r = __ffma2_rn(r, s, make_float2(Q[i], Q[i]));
+    r = __ffma2_rn(r, z, make_float2(0.5f, 0.5f));
+    const float2 te = __fmul2_rn(t, e);
+    // Phi = te P below -1, 1 - te P above 1
+    float2 phi = make_float2(z.x >= 0.0f ? fmaf(-p.x, te.x, 1.0f) : p.x * te.x,
+                             z.y >= 0.0f ? fmaf(-p.y, te.y, 1.0f) : p.y * te.y);
+    phi.x = s.x < 1.0f ? r.x : phi.x;
+    phi.y = s.y < 1.0f ? r.y : phi.y;
+    h = __fmul2_rn(z, phi);
+    if (GRAD) g = __ffma2_rn(__fmul2_rn(e, make_float2(0.39894228f, 0.39894228f)), z, phi);
 }
 
 // Ghosted activations of the tensor-core path: BF16

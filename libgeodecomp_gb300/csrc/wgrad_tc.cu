@@ -380,17 +380,29 @@ struct RParams {
     long long off[4];
 };
 
+// a warp's lanes take 32 consecutive elements, the eight warps every eighth CTA
 __global__ void __launch_bounds__(256)
 reduce_kernel(const RParams p, float *grads)
 {
+    __shared__ float sum[8][32];
     dependent_start();
     const int l = blockIdx.y;
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < p.n[l]; i += gridDim.x * 256) {
-        const float *q = p.part[l] + i;
+    const int n = p.n[l], ctas = p.ctas[l];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i0 = blockIdx.x * 32; i0 < n; i0 += gridDim.x * 32) {      // uniform
+        const int i = i0 + lane;
         float a = 0.f;
-#pragma unroll 8
-        for (int c = 0; c < p.ctas[l]; ++c) a += q[(long long)c * p.n[l]];
-        grads[p.off[l] + i] = a;
+        if (i < n) {
+#pragma unroll 4
+            for (int c = warp; c < ctas; c += 8) a += p.part[l][(long long)c * n + i];
+        }
+        sum[warp][lane] = a;
+        __syncthreads();
+        if (warp == 0 && i < n) {
+            for (int w = 1; w < 8; ++w) a += sum[w][lane];
+            grads[p.off[l] + i] = a;
+        }
+        __syncthreads();
     }
 }
 
@@ -484,7 +496,7 @@ void tc_wgrad_reduce(const float *partials, const int ctas[4], const long long w
         r.off[l] = w_off[l];
         off += (size_t)sm_count() * DW[l];
     }
-    launch_dependent(reduce_kernel, dim3((DW[1] + 255) / 256, 4), 256u, 0, stream, r, grads);
+    launch_dependent(reduce_kernel, dim3((DW[1] + 31) / 32, 4), 256u, 0, stream, r, grads);
     check_launch("weight gradient sum");
 }
 
