@@ -33,10 +33,13 @@
 // of input sits in shared memory as [channel group][row][8 voxels + 2 halo]
 // x 16 B: every 8-voxel core matrix brings its own halo, so tap (dy, dx) of
 // any tile is a start address and M may span rows.
-//   - warp 0: issues the MMAs, tile by tile;
-//   - warps 1 .. 16: epilogue of tile (w - 1) / 4, lane quarter w % 4;
-//   - warps 17 .. 20: fill the input slots (cp.async; FIRST and DLAST build
-//     their groups from the FP32 fields).
+//   - two warps (LAST: four) issue the MMAs, each for its share of the tiles;
+//   - 16 warps: epilogue, four to a tile, by lane quarter;
+//   - four warps fill the input slots (cp.async; FIRST and DLAST build their
+//     groups from the FP32 fields).
+// At 256^3 the layers take 450 (FIRST), 470 (MID) and 310 us (LAST).  MID is
+// bound by the MMAs' operand reads (80% of the cycles); FIRST by the
+// epilogue, 900 instructions per 32 voxels and about half of the FMA pipe.
 // Every wait is bounded and gives up early once another role has failed; a
 // CTA that gives up sets the error word, lets its copies and MMAs finish and
 // frees its tensor memory.
@@ -56,13 +59,19 @@ enum { ACT = 0, GRAD = 1, OUT = 2 };
 constexpr int TILES = 4;                    // accumulator tiles of 128 voxels per CTA
 constexpr int EPI_WARPS = 16;
 constexpr int LOAD_WARPS = 4;
-constexpr int THREADS = 32 * (1 + EPI_WARPS + LOAD_WARPS);
-constexpr int LOAD0 = 1 + EPI_WARPS;
 constexpr int S = 3;                        // input slots
 
 template<int SRC, int TXW>
 struct Geo {
     static constexpr bool WIDE = SRC == MID || SRC == LAST;     // 24 channels with halo, else one built group
+    // Between two tiles a warp waits and issues nothing for some 200 clocks; the
+    // MMAs of another warp fill that in.  LAST, with 36 clocks per MMA, gains up
+    // to four (clocks per plane with 1, 2, 4 warps: 3990, 2640, 2350); MID has
+    // its tiles finish together with four and the epilogues then wait for each
+    // other (4930, 3610, 3830).
+    static constexpr int MMA_WARPS = SRC == LAST ? 4 : 2;
+    static constexpr int LOAD0 = MMA_WARPS + EPI_WARPS;
+    static constexpr int THREADS = 32 * (LOAD0 + LOAD_WARPS);
     static constexpr int TY = 512 / TXW;
     static constexpr int ROWS = TY + 2;
     static constexpr int NG = TXW / 8;
@@ -89,22 +98,16 @@ struct Params {
     const bf16 *w;              // packed weights
     const float *bias;          // ACT, OUT
     bf16 *out;                  // ACT, GRAD: ghosted
-    float *g;                   // ACT: GELU' of the pre-activations out (or null); GRAD: in
+    float *g;                   // ACT: GELU' of the pre-activations out (or null); GRAD: in; FP32
+                                // [batch][nz][ny][6][nx][4], four channels to a float4
     float *db;                  // GRAD: bias gradient, added to
     float *fout;                // OUT
     int add;                    // OUT: add to fout
     int *err;
 };
 
-// position of voxel (x, y) of plane z in the saved GELU': FP32
-// [batch][nz][ny][6][nx][4], the float4 of channels 4 c .. 4 c + 3 at + c * nx
-__device__ __forceinline__ long long g_at(const Shape& s, int b, int z, int y, int x)
-{
-    return ((((long long)b * s.nz + z) * s.ny + y) * 6) * s.nx + x;
-}
-
 template<int SRC, int EPI, int TXW>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__((Geo<SRC, TXW>::THREADS), 1)
 conv_tc_kernel(const Params p)
 {
     typedef Geo<SRC, TXW> G;
@@ -116,7 +119,9 @@ conv_tc_kernel(const Params p)
     __shared__ __align__(8) uint64_t bar_free[TILES];   // its completed accumulator read and started over
     __shared__ uint32_t s_tmem;
     __shared__ int s_fail;
+    __shared__ int s_commits[TILES];                    // planes committed, by tile
     __shared__ float s_db[24];
+    __shared__ __align__(16) float s_bias[24];
     volatile int *fail = &s_fail;
 
     unsigned char *smem = smem_raw + ((128 - (saddr(smem_raw) & 127)) & 127);
@@ -145,7 +150,7 @@ conv_tc_kernel(const Params p)
         mbar_init(saddr(&bar_w), 1);
         for (int i = 0; i < S; ++i) {
             mbar_init(saddr(&bar_full[i]), LOAD_WARPS);
-            mbar_init(saddr(&bar_empty[i]), 1);
+            mbar_init(saddr(&bar_empty[i]), G::MMA_WARPS);
         }
         for (int i = 0; i < TILES; ++i) {
             mbar_init(saddr(&bar_mma[i]), 1);
@@ -154,6 +159,7 @@ conv_tc_kernel(const Params p)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (EPI == GRAD && tid < 24) s_db[tid] = 0.f;
+    if (EPI == ACT && tid < 24) s_bias[tid] = __ldg(p.bias + tid);
     dependent_start();
     if (tid == 0) {
         mbar_expect_tx(saddr(&bar_w), G::W_BYTES);
@@ -163,12 +169,11 @@ conv_tc_kernel(const Params p)
     __syncthreads();
     fence_after();
     const uint32_t tmem = s_tmem;
-    int committed = 0;                                  // warp 0: tiles committed, over all planes
-    bool w_ready = false;
 
-    if (warp == 0) {
+    if (warp < G::MMA_WARPS) {
+        constexpr int OWN = TILES / G::MMA_WARPS;          // tiles of this warp
+        int commits = 0;
         bool ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_w), 0, fail));
-        w_ready = ok;
         const uint32_t rbase = saddr(ring), wbase = saddr(wsm);
         constexpr uint32_t ID = idesc(128, G::N, false);
         constexpr uint32_t HI_A = desc_hi(G::GS), HI_B = desc_hi(128);
@@ -181,7 +186,7 @@ conv_tc_kernel(const Params p)
             const uint32_t rot = (uint32_t)((3 - q % 3) % 3);
             const uint32_t b0 = SRC == LAST ? desc_lo(wbase + rot * (G::KSTEPS * G::KS_BYTES), 2 * 128)
                                             : desc_lo(wbase + rot * 3 * 128, 16 * 128);
-            for (int m = 0; m < TILES; ++m) {
+            for (int m = warp * OWN; m < warp * OWN + OWN; ++m) {
                 ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_free[m]), (uint32_t)(q & 1), fail));
                 if (!ok) break;
                 fence_after();
@@ -210,16 +215,19 @@ conv_tc_kernel(const Params p)
                                   desc(b0 + (uint32_t)((k * G::KS_BYTES) >> 4), HI_B), ID);
                     }
                     mma_commit(saddr(&bar_mma[m]));
-                    if (m == TILES - 1) mma_commit(saddr(&bar_empty[q % S]));
+                    if (m == warp * OWN + OWN - 1) mma_commit(saddr(&bar_empty[q % S]));
                 }
                 __syncwarp();
-                ++committed;
+                ++commits;
             }
         }
-        if (!ok && lane == 0) s_fail = 1;
+        if (lane == 0) {
+            for (int i = 0; i < OWN; ++i) s_commits[warp * OWN + i] = (commits + OWN - 1 - i) / OWN;
+            if (!ok) s_fail = 1;
+        }
         __syncwarp();
-    } else if (warp >= LOAD0) {
-        const int lt = tid - LOAD0 * 32;
+    } else if (warp >= G::LOAD0) {
+        const int lt = tid - G::LOAD0 * 32;
         int published = 0;
         bool ok = true;
         auto publish = [&](int upto) {
@@ -229,6 +237,58 @@ conv_tc_kernel(const Params p)
                 if (lane == 0) mbar_arrive(saddr(&bar_full[published % S]));
             }
         };
+        // What a thread copies lies at the same place of every plane.
+        // Wide: its 16-byte voxels of the slot; else its warp's segments of 32
+        // voxels, all at the same x (LOAD_WARPS * 32 is a multiple of TXW).
+        constexpr int PER_ROW = G::NG * 10;
+        constexpr int SEGS = G::ROWS * TXW / 32;
+        constexpr int PER = G::WIDE ? (G::ROWS * PER_ROW + LOAD_WARPS * 32 - 1) / (LOAD_WARPS * 32)
+                                    : (SEGS + LOAD_WARPS - 1) / LOAD_WARPS;
+        const long long plane = G::WIDE ? (long long)(s.ny + 2) * 3 * (s.nx + 2) : (long long)s.ny * s.nx;
+        uint32_t src[PER];                                  // in 16-byte units / floats of a plane (a plane of
+                                                            // 2^32 would not fit the device's memory)
+        uint32_t dst[G::WIDE ? PER : 1];
+        int side = 0;                                       // to the neighbour beyond the segment's end
+        if (G::WIDE) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int v = lt + i * LOAD_WARPS * 32;
+                const int row = v / PER_ROW;
+                const int j = v - row * PER_ROW;            // group j / 10, voxel j % 10 of it
+                const int gy = min(y0 + row, s.ny + 1);     // ghosted row (rows past the grid: any)
+                src[i] = (uint32_t)gy * 3u * (uint32_t)(s.nx + 2) + (uint32_t)(x0 + (j / 10) * 8 + j % 10);
+                dst[i] = (uint32_t)(row * G::ROWP + j * 16);
+            }
+        } else {
+            const int x = x0 + (lt & ~31) % TXW + lane;
+            side = lane == 0 ? (x == 0 ? s.nx - 1 : -1) : (x == s.nx - 1 ? 1 - s.nx : 1);
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int seg = (lt >> 5) + i * LOAD_WARPS;
+                int y = y0 - 1 + min(seg * 32 / TXW, G::ROWS - 1);
+                y = y < 0 ? y + s.ny : (y >= s.ny ? (y - s.ny) % s.ny : y);
+                src[i] = (uint32_t)y * (uint32_t)s.nx + (uint32_t)x;
+            }
+        }
+        constexpr int PERF = G::WIDE ? 1 : PER;
+        float na[PERF], nc[PERF], ma[PERF], mc[PERF];       // FIRST, DLAST: the next plane's fields
+        auto load = [&](int q) {
+            int z = z0 - 1 + q;
+            z = z < 0 ? z + s.nz : (z >= s.nz ? z - s.nz : z);
+            const float *f0 = p.f0 + ((long long)b * s.nz + z) * plane;
+            const float *f1 = p.f1 + ((long long)b * s.nz + z) * plane;
+#pragma unroll
+            for (int i = 0; i < PERF; ++i) {
+                na[i] = f0[src[i]];
+                nc[i] = f1[src[i]];
+                ma[i] = mc[i] = 0.f;
+                if (lane == 0 || lane == 31) {
+                    ma[i] = f0[src[i] + side];
+                    mc[i] = f1[src[i] + side];
+                }
+            }
+        };
+        if (!G::WIDE) load(0);
         for (int q = 0; q < n + 2; ++q) {
             // publish what has landed before waiting for a slot: the MMAs that
             // free it never wait on this loader
@@ -245,45 +305,31 @@ conv_tc_kernel(const Params p)
             }
             const uint32_t slot = saddr(ring) + (uint32_t)((q % S) * G::SLOT);
             if (G::WIDE) {
-                constexpr int PER_ROW = G::NG * 10;
-                for (int v = lt; v < G::ROWS * PER_ROW; v += LOAD_WARPS * 32) {
-                    const int r = v / PER_ROW;
-                    const int i = v - r * PER_ROW;              // group i / 10, voxel i % 10 of it
-                    const int gy = min(y0 + r, s.ny + 1);       // ghosted row (rows past the grid: any)
-                    const bf16 *src = p.in + (ghost_row(s, b, z0 + q, gy) * (s.nx + 2) + x0 + (i / 10) * 8 + i % 10) * 8;
-                    const uint32_t d = slot + (uint32_t)(r * G::ROWP + i * 16);
+                const uint4 *in = reinterpret_cast<const uint4 *>(p.in) + ((long long)b * (s.nz + 2) + z0 + q) * plane;
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) copy16(d + c * G::CGS, src + (long long)c * (s.nx + 2) * 8);
+                for (int i = 0; i < PER; ++i) {
+                    if ((i + 1) * LOAD_WARPS * 32 <= G::ROWS * PER_ROW || lt + i * LOAD_WARPS * 32 < G::ROWS * PER_ROW) {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) copy16(slot + dst[i] + c * G::CGS, in + src[i] + c * (s.nx + 2));
+                    }
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
             } else {
+                float va[PERF], vc[PERF], ea[PERF], ec[PERF];
                 // a warp builds the groups of 32 consecutive voxels: neighbours
                 // by shuffle, the two beyond the ends by the end lanes; the
-                // loads of all its segments are in flight together
-                constexpr int SEGS = G::ROWS * TXW / 32;
-                constexpr int PER = (SEGS + LOAD_WARPS - 1) / LOAD_WARPS;
-                int z = z0 - 1 + q;
-                z = z < 0 ? z + s.nz : (z >= s.nz ? z - s.nz : z);
-                float va[PER], vc[PER], ea[PER], ec[PER];
+                // loads of all its segments and of the next plane are in flight
+                // together
 #pragma unroll
-                for (int i = 0; i < PER; ++i) {
-                    const int seg = (lt >> 5) + i * LOAD_WARPS;
-                    const int r = min(seg * 32 / TXW, G::ROWS - 1);
-                    const int x = x0 + seg * 32 % TXW + lane;
-                    int y = y0 - 1 + r;
-                    y = y < 0 ? y + s.ny : (y >= s.ny ? (y - s.ny) % s.ny : y);
-                    const long long row = (((long long)b * s.nz + z) * s.ny + y) * s.nx;
-                    va[i] = p.f0[row + x];
-                    vc[i] = p.f1[row + x];
-                    const int e = lane == 0 ? (x == 0 ? s.nx - 1 : x - 1) : (x == s.nx - 1 ? 0 : x + 1);
-                    ea[i] = ec[i] = 0.f;
-                    if (lane == 0 || lane == 31) {
-                        ea[i] = p.f0[row + e];
-                        ec[i] = p.f1[row + e];
-                    }
+                for (int i = 0; i < PERF; ++i) {
+                    va[i] = na[i];
+                    vc[i] = nc[i];
+                    ea[i] = ma[i];
+                    ec[i] = mc[i];
                 }
+                if (q < n + 1) load(q + 1);
 #pragma unroll
-                for (int i = 0; i < PER; ++i) {
+                for (int i = 0; i < PERF; ++i) {
                     const int seg = (lt >> 5) + i * LOAD_WARPS;
                     uint32_t mid, edge;                 // FIRST: the pair (u, kappa); DLAST: the gradient
                     if (SRC == FIRST) {
@@ -311,13 +357,21 @@ conv_tc_kernel(const Params p)
         if (ok) publish(n + 2);
         else if (lane == 0) s_fail = 1;
     } else {
-        const int m = (warp - 1) >> 2;                  // tile
+        const int m = (warp - G::MMA_WARPS) >> 2;                  // tile
         const int qd = warp & 3;                        // lane quarter this warp may read
         const int vt = m * 128 + qd * 32 + lane;        // voxel of the CTA's 512
         const int x = x0 + vt % TXW;
         const int y = y0 + vt / TXW;
         const bool live = y < s.ny;
         const uint32_t acc = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(m * G::TCOLS);
+        // this voxel in plane 0 of the ghosted output (16-byte units) and of
+        // GELU' (float4), and whether an axis repeats it among the ghosts
+        const long long oplane = (long long)(s.ny + 2) * 3 * (s.nx + 2);
+        uint4 *const out0 = reinterpret_cast<uint4 *>(p.out) + b * (s.nz + 2) * oplane + (y + 1) * 3 * (s.nx + 2LL) + x + 1;
+        const long long gplane = (long long)s.ny * 6 * s.nx;
+        float4 *const g0 = reinterpret_cast<float4 *>(p.g) + (long long)b * s.nz * gplane + y * 6LL * s.nx + x;
+        const bool edge_x = x == 0 || x == s.nx - 1, edge_y = y == 0 || y == s.ny - 1;
+        const int ghost_x = x == 0 ? s.nx : -s.nx;          // where its copy lies (nx >= 32: only one)
         float db[EPI == GRAD ? 24 : 1] = {};
         const float b1 = EPI == OUT ? __ldg(p.bias) : 0.f;
         // accumulator slot (columns) j % 3 starts at the bias (OUT adds it at the end)
@@ -329,7 +383,7 @@ conv_tc_kernel(const Params p)
                 for (int c = 0; c < 3; ++c) {
                     float v[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) v[i] = EPI == ACT ? __ldg(p.bias + c * 8 + i) : 0.f;
+                    for (int i = 0; i < 8; ++i) v[i] = EPI == ACT ? s_bias[c * 8 + i] : 0.f;
                     tmem_st8(acc + (uint32_t)(slot * 24 + c * 8), v);
                 }
             }
@@ -358,25 +412,19 @@ conv_tc_kernel(const Params p)
                 }
             } else {
                 float v[24];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    float t[8];
-                    tmem_ld8(acc + (uint32_t)(slot * 24 + c * 8), t);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) v[c * 8 + i] = t[i];
-                }
+                tmem_ld24(acc + (uint32_t)(slot * 24), v);
                 restart(slot);
                 if (q < 2 || !live) continue;
                 if constexpr (EPI == ACT) {
                     if (p.g) {
                         // training: GELU' for the backward pass, beside GELU
-                        float4 *gp = reinterpret_cast<float4 *>(p.g) + g_at(s, b, z, y, x);
+                        float4 *gp = g0 + z * gplane;
 #pragma unroll
                         for (int c = 0; c < 6; ++c) {
-                            float2 h0, h1, g0, g1;
-                            gelu_pair<true>(make_float2(v[4 * c], v[4 * c + 1]), h0, g0);
-                            gelu_pair<true>(make_float2(v[4 * c + 2], v[4 * c + 3]), h1, g1);
-                            gp[(long long)c * s.nx] = make_float4(g0.x, g0.y, g1.x, g1.y);
+                            float2 h0, h1, d0, d1;
+                            gelu_pair<true>(make_float2(v[4 * c], v[4 * c + 1]), h0, d0);
+                            gelu_pair<true>(make_float2(v[4 * c + 2], v[4 * c + 3]), h1, d1);
+                            gp[c * s.nx] = make_float4(d0.x, d0.y, d1.x, d1.y);
                             v[4 * c] = h0.x;
                             v[4 * c + 1] = h0.y;
                             v[4 * c + 2] = h1.x;
@@ -392,10 +440,10 @@ conv_tc_kernel(const Params p)
                         }
                     }
                 } else {
-                    const float4 *gp = reinterpret_cast<const float4 *>(p.g) + g_at(s, b, z, y, x);
+                    const float4 *gp = g0 + z * gplane;
 #pragma unroll
                     for (int c = 0; c < 6; ++c) {
-                        const float4 t = gp[(long long)c * s.nx];
+                        const float4 t = gp[c * s.nx];
                         v[4 * c] *= t.x;
                         v[4 * c + 1] *= t.y;
                         v[4 * c + 2] *= t.z;
@@ -410,26 +458,31 @@ conv_tc_kernel(const Params p)
                     w[c] = make_uint4(pack_bf16(v[8 * c], v[8 * c + 1]), pack_bf16(v[8 * c + 2], v[8 * c + 3]),
                                       pack_bf16(v[8 * c + 4], v[8 * c + 5]), pack_bf16(v[8 * c + 6], v[8 * c + 7]));
                 }
-                // the voxel and its ghost copies (an axis of extent 1 has both)
-                auto put = [&](int gz, int gy, int gx) {
-                    uint4 *o = reinterpret_cast<uint4 *>(p.out) + ghost_row(s, b, gz, gy) * (s.nx + 2) + gx;
+                // the voxel and its ghost copies
+                auto put = [&](uint4 *o) {
                     o[0] = w[0];
                     o[s.nx + 2] = w[1];
                     o[2 * (s.nx + 2)] = w[2];
                 };
-                auto put_x = [&](int gz, int gy) {
-                    put(gz, gy, x + 1);
-                    if (x == 0) put(gz, gy, s.nx + 1);
-                    if (x == s.nx - 1) put(gz, gy, 0);
+                auto put_x = [&](uint4 *o) {
+                    put(o);
+                    if (edge_x) put(o + ghost_x);
                 };
-                auto put_y = [&](int gz) {
-                    put_x(gz, y + 1);
-                    if (y == 0) put_x(gz, s.ny + 1);
-                    if (y == s.ny - 1) put_x(gz, 0);
-                };
-                put_y(z + 1);
-                if (z == 0) put_y(s.nz + 1);
-                if (z == s.nz - 1) put_y(0);
+                if (!edge_y && z != 0 && z != s.nz - 1) {
+                    put_x(out0 + (z + 1) * oplane);
+                } else {
+                    // in z and y: itself, the far ghost, the near ghost (an axis of extent 1 has both)
+#pragma unroll 1
+                    for (int i = 0; i < 9; ++i) {
+                        const int iz = i / 3, iy = i - 3 * iz;
+                        if ((iz == 1 && z != 0) || (iz == 2 && z != s.nz - 1) || (iy == 1 && y != 0) ||
+                            (iy == 2 && y != s.ny - 1)) {
+                            continue;
+                        }
+                        put_x(out0 + (iz == 0 ? z + 1 : (iz == 1 ? s.nz + 1 : 0)) * oplane +
+                              (iy == 0 ? 0 : (iy == 1 ? s.ny : -s.ny)) * 3LL * (s.nx + 2));
+                    }
+                }
             }
         }
         if constexpr (EPI == GRAD) {
@@ -451,10 +504,9 @@ conv_tc_kernel(const Params p)
         if (tid == 0) {
             atomicExch(p.err, 1);
             for (int m = 0; m < TILES; ++m) {
-                const int c = (committed + TILES - 1 - m) / TILES;      // commits of this tile
-                if (c > 0) mbar_wait(saddr(&bar_mma[m]), (uint32_t)((c - 1) & 1), nullptr);
+                if (s_commits[m] > 0) mbar_wait(saddr(&bar_mma[m]), (uint32_t)((s_commits[m] - 1) & 1), nullptr);
             }
-            if (!w_ready) mbar_wait(saddr(&bar_w), 0, nullptr);
+            mbar_wait(saddr(&bar_w), 0, nullptr);
         }
         fence_before();
         __syncthreads();
@@ -562,7 +614,7 @@ static void run(Params p, cudaStream_t stream)
     const int bx = p.s.nx / TXW, by = (p.s.ny + G::TY - 1) / G::TY;
     p.zchunk = pick_zchunk((long long)bx * by * p.s.batch, p.s.nz, sms);
     const int zsplit = (p.s.nz + p.zchunk - 1) / p.zchunk;
-    launch_dependent(conv_tc_kernel<SRC, EPI, TXW>, dim3(bx, by, p.s.batch * zsplit), THREADS, G::SMEM, stream, p);
+    launch_dependent(conv_tc_kernel<SRC, EPI, TXW>, dim3(bx, by, p.s.batch * zsplit), G::THREADS, G::SMEM, stream, p);
     check_launch("tensor-core convolution");
 }
 

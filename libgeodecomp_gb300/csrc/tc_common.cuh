@@ -78,7 +78,29 @@ __device__ __forceinline__ void mma_commit(uint32_t bar)
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// eight consecutive columns of this thread's tensor-memory lane
+// 24 consecutive columns of this thread's tensor-memory lane, and eight
+__device__ __forceinline__ void tmem_ld24(uint32_t taddr, float (&v)[24])
+{
+    uint32_t r[24];
+#pragma unroll
+    for (int c = 0; c < 24; c += 8) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[c]), "=r"(r[c + 1]), "=r"(r[c + 2]), "=r"(r[c + 3]), "=r"(r[c + 4]), "=r"(r[c + 5]),
+                       "=r"(r[c + 6]), "=r"(r[c + 7])
+                     : "r"(taddr + (uint32_t)c)
+                     : "memory");
+    }
+    // the values pass through the wait, so that none is used before it
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                   "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23])
+                 :
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 24; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
 {
     uint32_t r[8];
@@ -172,8 +194,8 @@ __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 {
-    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16(lo)) |
-           ((uint32_t)__bfloat16_as_ushort(__float2bfloat16(hi)) << 16);
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);     // one conversion for the pair
+    return *reinterpret_cast<const uint32_t *>(&v);
 }
 
 // GELU(z) = z Phi(z) of two values, and GELU'(z) = Phi(z) + z phi(z) where
