@@ -159,8 +159,8 @@ conv_tc_kernel(const Params p)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (EPI == GRAD && tid < 24) s_db[tid] = 0.f;
-    if (EPI == ACT && tid < 24) s_bias[tid] = __ldg(p.bias + tid);
     dependent_start();
+    if (EPI == ACT && tid < 24) s_bias[tid] = __ldg(p.bias + tid);
     if (tid == 0) {
         mbar_expect_tx(saddr(&bar_w), G::W_BYTES);
         bulk_copy(saddr(wsm), p.w, G::W_BYTES, saddr(&bar_w));
@@ -393,7 +393,21 @@ conv_tc_kernel(const Params p)
             if (lane == 0) mbar_arrive(saddr(&bar_free[m]));
         };
         restart(0);
+        // What the epilogue reads of a plane is loaded while its MMAs run.  In MID,
+        // where the MMAs set the pace, GELU' is not: multiplying before the
+        // accumulator is handed back costs more (101 -> 107 us at 64^3 x 8; DLAST
+        // 117 -> 97), and after it the registers do not suffice.
+        constexpr bool AHEAD = SRC == DLAST;
+        float *const fout0 = p.fout + ((long long)b * s.nz * s.ny + y) * s.nx + x;
+        const long long fplane = (long long)s.ny * s.nx;
+        float before = 0.f;
+        float4 g[AHEAD ? 6 : 1];
+        if (AHEAD && live) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) g[AHEAD ? c : 0] = g0[z0 * gplane + c * s.nx];
+        }
         for (int q = 0; q < n + 2; ++q) {
+            if (EPI == OUT && p.add && q >= 2 && live) before = fout0[(z0 + q - 2) * fplane];
             const bool ok = mbar_wait(saddr(&bar_mma[m]), (uint32_t)(q & 1), fail);
             if (!__all_sync(0xffffffffu, ok)) {
                 if (lane == 0) s_fail = 1;
@@ -406,17 +420,58 @@ conv_tc_kernel(const Params p)
                 const float v = tmem_ld1(acc + (uint32_t)slot);
                 restart(slot);
                 if (q >= 2 && live) {
-                    float *o = p.fout + (((long long)b * s.nz + z) * s.ny + y) * s.nx + x;
-                    if (p.add) *o += v + b1;
-                    else *o = v + b1;
+                    float *o = fout0 + z * fplane;
+                    *o = p.add ? before + (v + b1) : v + b1;
                 }
             } else {
-                float v[24];
-                tmem_ld24(acc + (uint32_t)(slot * 24), v);
-                restart(slot);
-                if (q < 2 || !live) continue;
-                if constexpr (EPI == ACT) {
-                    if (p.g) {
+                uint4 w[3];
+                if constexpr (AHEAD) {
+                    const bool use = q >= 2 && live;
+                    const float zero[8] = {};
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        float v[8];
+                        tmem_ld8(acc + (uint32_t)(slot * 24 + c * 8), v);
+                        tmem_st8(acc + (uint32_t)(slot * 24 + c * 8), zero);
+                        if (use) {
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const float4 t = g[2 * c + i];
+                                v[4 * i] *= t.x;
+                                v[4 * i + 1] *= t.y;
+                                v[4 * i + 2] *= t.z;
+                                v[4 * i + 3] *= t.w;
+                                if (q + 1 < n + 2) g[2 * c + i] = g0[(z + 1) * gplane + (2 * c + i) * s.nx];
+                            }
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) db[c * 8 + i] += v[i];
+                            w[c] = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]),
+                                              pack_bf16(v[6], v[7]));
+                        }
+                    }
+                    tmem_st_wait();
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(saddr(&bar_free[m]));
+                    if (!use) continue;
+                } else {
+                    float v[24];
+                    tmem_ld24(acc + (uint32_t)(slot * 24), v);
+                    restart(slot);
+                    if (q < 2 || !live) continue;
+                    if constexpr (EPI == GRAD) {
+                        const float4 *gp = g0 + z * gplane;
+#pragma unroll
+                        for (int c = 0; c < 6; ++c) {
+                            const float4 t = gp[c * s.nx];
+                            v[4 * c] *= t.x;
+                            v[4 * c + 1] *= t.y;
+                            v[4 * c + 2] *= t.z;
+                            v[4 * c + 3] *= t.w;
+                        }
+#pragma unroll
+                        for (int c = 0; c < 24; ++c) db[c] += v[c];
+                    } else if (p.g) {
                         // training: GELU' for the backward pass, beside GELU
                         float4 *gp = g0 + z * gplane;
 #pragma unroll
@@ -433,30 +488,17 @@ conv_tc_kernel(const Params p)
                     } else {
 #pragma unroll
                         for (int c = 0; c < 12; ++c) {
-                            float2 h, g;
-                            gelu_pair<false>(make_float2(v[2 * c], v[2 * c + 1]), h, g);
+                            float2 h, d;
+                            gelu_pair<false>(make_float2(v[2 * c], v[2 * c + 1]), h, d);
                             v[2 * c] = h.x;
                             v[2 * c + 1] = h.y;
                         }
                     }
-                } else {
-                    const float4 *gp = g0 + z * gplane;
 #pragma unroll
-                    for (int c = 0; c < 6; ++c) {
-                        const float4 t = gp[c * s.nx];
-                        v[4 * c] *= t.x;
-                        v[4 * c + 1] *= t.y;
-                        v[4 * c + 2] *= t.z;
-                        v[4 * c + 3] *= t.w;
+                    for (int c = 0; c < 3; ++c) {
+                        w[c] = make_uint4(pack_bf16(v[8 * c], v[8 * c + 1]), pack_bf16(v[8 * c + 2], v[8 * c + 3]),
+                                          pack_bf16(v[8 * c + 4], v[8 * c + 5]), pack_bf16(v[8 * c + 6], v[8 * c + 7]));
                     }
-#pragma unroll
-                    for (int c = 0; c < 24; ++c) db[c] += v[c];
-                }
-                uint4 w[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    w[c] = make_uint4(pack_bf16(v[8 * c], v[8 * c + 1]), pack_bf16(v[8 * c + 2], v[8 * c + 3]),
-                                      pack_bf16(v[8 * c + 4], v[8 * c + 5]), pack_bf16(v[8 * c + 6], v[8 * c + 7]));
                 }
                 // the voxel and its ghost copies
                 auto put = [&](uint4 *o) {

@@ -5,13 +5,16 @@
 // Operands lie in shared memory with the channels contiguous (16 bytes = 8
 // channels of a voxel, voxels 16 bytes apart), which is the tensor core's
 // MN-major form with K = voxels: a unit of eight M or N elements per (row,
-// channel group), all units a constant stride apart, and a tap in x is a start
-// address.  Per MMA (K = 16 voxels):
+// channel group), all units a constant stride apart.  Per MMA (K = 16 voxels):
 //   CC (layers 2, 3)  M = 16 units = five rows of h and a third (120 of the
-//                     128 rows of D used), N = two rows of dz (48): the pairs
-//                     (row of h, row of dz) with h at most one row away give
-//                     the taps in y, so that one MMA serves all three.  Nine
-//                     accumulators of 48 columns: taps in z times taps in x;
+//                     128 rows of D used), N = two rows of dz, each three
+//                     times, moved by the taps in x (144): the pairs (row of h,
+//                     row of dz) with h at most one row away give the taps in
+//                     y, so that one MMA serves nine taps.  Three accumulators,
+//                     the taps in z.  An MMA reads 4 KB of h and 32 N bytes of
+//                     dz at 128 B per clock and multiplies in N / 2 clocks: 72
+//                     either way.  One MMA per tap in x (N = 48) took 46 each,
+//                     138 for the three;
 //   L (layer 4)       the same h against two rows of the loss gradient, its
 //                     three x neighbours in one unit: N = 16, three
 //                     accumulators;
@@ -25,10 +28,13 @@
 // every tile's dW to the gradient with atomics.
 //
 // CTAs are persistent over (column of TXW x TY voxels, z chunk) items and
-// march each in z: h plane q meets dz planes q - 2, q - 1, q (two slots of h,
-// four of dz).  Warp 0 issues the MMAs, warps 1 .. 4 clear the accumulators
-// first and fold them at the end, warps 5 .. 12 fill the slots.  Waits are
-// bounded as in conv_tc.cu.
+// march each in z: a dz plane meets three h planes (five slots of h, three of
+// dz, so that two planes are on their way: with one the copies' latency set the
+// pace).  FL and LL build a field's groups from registers loaded a plane ahead.
+// At 64^3 x 8: CC 73 us (127 with one MMA per tap in x and one plane ahead), FL
+// 37 (87), LL 51 (69).  Three warps issue the MMAs, four clear the accumulators
+// first and fold them at the end, eight fill the slots.  Waits are bounded as in
+// conv_tc.cu.
 #include <algorithm>
 
 #include "lgd_internal.h"
@@ -42,24 +48,25 @@ namespace tc {
 enum { CC = 0, FL = 1, LL = 2 };            // layers 2 and 3; first; last
 
 constexpr int WG_LOADERS = 8;
-constexpr int WG_THREADS = 32 * (5 + WG_LOADERS);
-constexpr int SH = 2, SD = 4;               // slots of h and dz
+constexpr int WG_MMA = 3;                   // one per tap in z: the MMAs of one fill the waits of the others
+constexpr int WG_LOAD0 = WG_MMA + 4;
+constexpr int WG_THREADS = 32 * (WG_LOAD0 + WG_LOADERS);
+constexpr int SH = 5, SD = 3;               // slots of h (three in use) and dz (one): two planes ahead
 
 template<int MODE, int TXW>
 struct WGeo {
-    static constexpr int TY = 512 / TXW;
+    static constexpr int TY = (MODE == CC ? 256 : 512) / TXW;   // CC: three slots of dz, three times each, take 110 KB
     static constexpr int ROWS = TY + 2;
     static constexpr int NG = TXW / 8;
-    static constexpr int GS = MODE == FL ? 128 : 160;           // bytes of an 8-voxel group of h (with halo)
+    static constexpr int GS = 128;                              // bytes of an 8-voxel group
     static constexpr int UA = NG * GS;                          // M unit stride
     static constexpr int UPR = MODE == FL ? 1 : 3;              // M units per row
     static constexpr int HSLOT = ROWS * UPR * UA;
     static constexpr int UB = TXW * 16;                         // N unit stride
-    static constexpr int NPR = MODE == LL ? 1 : 3;              // N units per row
+    static constexpr int NPR = MODE == LL ? 1 : (MODE == FL ? 3 : 9);   // N units per row
     static constexpr int DSLOT = TY * NPR * UB;
     static constexpr int YB = MODE == FL ? 4 : 2;               // dz rows per MMA
-    static constexpr int N = YB * NPR * 8;                      // 48, 96, 16
-    static constexpr int DX = MODE == CC ? 3 : 1;
+    static constexpr int N = YB * NPR * 8;                      // 144, 96, 16
     static constexpr int TMEM = MODE == CC ? 512 : (MODE == FL ? 512 : 64);
     static constexpr int CIN = MODE == FL ? 2 : 24;
     static constexpr int COUT = MODE == LL ? 1 : 24;
@@ -85,7 +92,7 @@ struct WParams {
 
 __device__ __forceinline__ void copy16_or_zero(uint32_t dst, const void *src, bool copy)
 {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(copy ? 16 : 0) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(copy ? 16 : 0) : "memory");
 }
 
 __device__ __forceinline__ void st_shared16(uint32_t dst, uint4 v)
@@ -99,7 +106,7 @@ wgrad_tc_kernel(const WParams p)
 {
     typedef WGeo<MODE, TXW> G;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bar_full[SH];      // a step's h and dz planes there (one arrive per loader warp)
+    __shared__ __align__(8) uint64_t bar_full[SH];      // h plane q and dz plane q - 2 there (one arrive per loader warp)
     __shared__ __align__(8) uint64_t bar_empty[SH];     // h slot no longer read
     __shared__ __align__(8) uint64_t bar_dempty[SD];    // dz slot no longer read
     __shared__ __align__(8) uint64_t bar_clear;         // accumulators cleared
@@ -131,11 +138,11 @@ wgrad_tc_kernel(const WParams p)
         s_bad = 0;
         for (int i = 0; i < SH; ++i) {
             mbar_init(saddr(&bar_full[i]), WG_LOADERS);
-            mbar_init(saddr(&bar_empty[i]), 1);
+            mbar_init(saddr(&bar_empty[i]), WG_MMA);
         }
-        for (int i = 0; i < SD; ++i) mbar_init(saddr(&bar_dempty[i]), 1);
+        for (int i = 0; i < SD; ++i) mbar_init(saddr(&bar_dempty[i]), WG_MMA);
         mbar_init(saddr(&bar_clear), 4);
-        mbar_init(saddr(&bar_done), 1);
+        mbar_init(saddr(&bar_done), WG_MMA);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     dependent_start();
@@ -159,59 +166,56 @@ wgrad_tc_kernel(const WParams p)
         return t;
     };
 
-    if (warp == 0) {
+    if (warp < WG_MMA) {
+        const int dz = warp;        // tap in z
         bool ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_clear), 0, fail));
         fence_after();
         constexpr uint32_t ID = idesc(128, G::N, true);
         constexpr uint32_t HI_A = desc_hi(G::UA), HI_B = desc_hi(G::UB);
-        int step = 0;               // h planes so far
-        int dbase = 0;              // dz planes of the items before this one
+        int plane = 0;              // h planes so far
+        int dplane = 0;             // dz planes so far
         for (int it = blockIdx.x; ok && it < p.items; it += gridDim.x) {
             const Item t = item_of(it);
-            for (int q = 0; ok && q < t.n + 2; ++q, ++step) {
-                ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_full[step % SH]), (uint32_t)((step / SH) & 1), fail));
+            for (int q = 0; q < t.n + 2; ++q, ++plane) {
+                ok = __all_sync(0xffffffffu, mbar_wait(saddr(&bar_full[plane % SH]), (uint32_t)((plane / SH) & 1), fail));
                 if (!ok) break;
+                if (q < 2) continue;
                 fence_after();
-                const uint32_t a0 = desc_lo(hring + (uint32_t)((step % SH) * G::HSLOT), G::GS);
-                for (int dz = 0; dz < 3; ++dz) {
-                    const int j = q - dz;
-                    if (j < 0 || j >= t.n) continue;
-                    const uint32_t b0 = desc_lo(dring + (uint32_t)(((dbase + j) % SD) * G::DSLOT), 128);
-                    for (int y = 0; y < G::TY; y += G::YB) {
-                        if (elect_one()) {
-                            const uint32_t ay = a0 + (uint32_t)((y * G::UPR * G::UA) >> 4);
-                            const uint32_t bw = b0 + (uint32_t)((y * G::NPR * G::UB) >> 4);
-                            const uint32_t d = tmem + (uint32_t)(dz * G::DX * G::N);
+                // dz plane q - 2 against h planes q - 2, q - 1, q
+                const uint32_t a0 = desc_lo(hring + (uint32_t)(((plane - 2 + dz) % SH) * G::HSLOT), G::GS);
+                const uint32_t b0 = desc_lo(dring + (uint32_t)((dplane % SD) * G::DSLOT), 128);
+                const uint32_t d = tmem + (uint32_t)(dz * G::N);
+                for (int y = 0; y < G::TY; y += G::YB) {
+                    if (elect_one()) {
+                        const uint32_t ay = a0 + (uint32_t)((y * G::UPR * G::UA) >> 4);
+                        const uint32_t bw = b0 + (uint32_t)((y * G::NPR * G::UB) >> 4);
 #pragma unroll
-                            for (int dx = 0; dx < G::DX; ++dx) {
-                                // CC: tap dx; LL: the centre voxel; FL: x taps sit in the unit
-                                const int shift = MODE == CC ? dx : (MODE == LL ? 1 : 0);
-#pragma unroll
-                                for (int k = 0; k < TXW / 16; ++k) {
-                                    mma<true>(d + (uint32_t)(dx * G::N), desc(ay + (uint32_t)((2 * k * G::GS) / 16 + shift), HI_A),
-                                              desc(bw + (uint32_t)(2 * k * 8), HI_B), ID);
-                                }
-                            }
+                        for (int k = 0; k < TXW / 16; ++k) {
+                            mma<true>(d, desc(ay + (uint32_t)((2 * k * G::GS) / 16), HI_A), desc(bw + (uint32_t)(2 * k * 8), HI_B), ID);
                         }
-                        __syncwarp();
                     }
+                    __syncwarp();
                 }
                 if (elect_one()) {
-                    mma_commit(saddr(&bar_empty[step % SH]));
-                    if (q >= 2) mma_commit(saddr(&bar_dempty[(dbase + q - 2) % SD]));
+                    mma_commit(saddr(&bar_dempty[dplane % SD]));
+                    mma_commit(saddr(&bar_empty[(plane - 2) % SH]));
+                    if (q == t.n + 1) {
+                        mma_commit(saddr(&bar_empty[(plane - 1) % SH]));
+                        mma_commit(saddr(&bar_empty[plane % SH]));
+                    }
                 }
                 __syncwarp();
+                ++dplane;
             }
-            dbase += t.n;
         }
         if (elect_one()) mma_commit(saddr(&bar_done));
         if (!ok && lane == 0) s_fail = 1;
         __syncwarp();
-    } else if (warp >= 5) {
-        const int lt = tid - 5 * 32;
+    } else if (warp >= WG_LOAD0) {
+        const int lt = tid - WG_LOAD0 * 32;
         constexpr int LT = WG_LOADERS * 32;
         bool ok = true;
-        int step = 0, dcount = 0;
+        int plane = 0, dplane = 0;
         int published = 0;
         auto publish = [&](int upto) {
             fence_async_proxy();
@@ -220,92 +224,135 @@ wgrad_tc_kernel(const WParams p)
                 if (lane == 0) mbar_arrive(saddr(&bar_full[published % SH]));
             }
         };
+        // FL, LL: the fields of the next plane, loaded while this one's slots are awaited
+        constexpr int PERF = MODE == FL ? (G::ROWS * TXW + LT - 1) / LT : G::TY * TXW / LT;
+        uint32_t nx0[MODE == FL ? PERF : 1][3];
+        float ng[MODE == LL ? PERF : 1][6];
+        auto fetch = [&](const Item& t, int q) {
+            if (MODE == FL) {
+                int z = t.z0 - 1 + q;
+                z = z < 0 ? z + s.nz : (z >= s.nz ? z - s.nz : z);
+#pragma unroll
+                for (int i = 0; i < PERF; ++i) {
+                    const int v = lt + i * LT;
+                    const int x = t.x0 + v % TXW;
+                    int y = t.y0 - 1 + min(v / TXW, G::ROWS - 1);
+                    y = y < 0 ? y + s.ny : (y >= s.ny ? (y - s.ny) % s.ny : y);
+                    const uint32_t *row = p.x0 + (((long long)t.b * s.nz + z) * s.ny + y) * s.nx;
+                    nx0[i][0] = row[x == 0 ? s.nx - 1 : x - 1];
+                    nx0[i][1] = row[x];
+                    nx0[i][2] = row[x == s.nx - 1 ? 0 : x + 1];
+                }
+            }
+            if (MODE == LL && q >= 2) {
+#pragma unroll
+                for (int i = 0; i < PERF; ++i) {
+                    const int v = lt + i * LT;
+                    const int x = t.x0 + v % TXW;
+                    const int y = min(t.y0 + v / TXW, s.ny - 1);
+                    const long long row = (((long long)t.b * s.nz + t.z0 + q - 2) * s.ny + y) * s.nx;
+                    const int xw = x == 0 ? s.nx - 1 : x - 1, xe = x == s.nx - 1 ? 0 : x + 1;
+                    ng[i][0] = p.du[row + xe];
+                    ng[i][1] = p.target[row + xe];
+                    ng[i][2] = p.du[row + x];
+                    ng[i][3] = p.target[row + x];
+                    ng[i][4] = p.du[row + xw];
+                    ng[i][5] = p.target[row + xw];
+                }
+            }
+        };
+        if (blockIdx.x < p.items) fetch(item_of(blockIdx.x), 0);
         for (int it = blockIdx.x; ok && it < p.items; it += gridDim.x) {
             const Item t = item_of(it);
-            for (int q = 0; q < t.n + 2; ++q, ++step) {
+            for (int q = 0; q < t.n + 2; ++q, ++plane) {
                 bool got = true;
-                if (step >= SH) {
-                    // the step before has landed meanwhile: hand it over first
-                    asm volatile("cp.async.wait_all;" ::: "memory");
-                    publish(step);
-                    got = mbar_wait(saddr(&bar_empty[step % SH]), (uint32_t)(((step - SH) / SH) & 1), fail);
+                // hand over what has landed before waiting for a slot: the MMAs
+                // that free it need no more than the planes up to this one's
+                // second predecessor
+                if (plane >= 2) {
+                    asm volatile("cp.async.wait_group 1;" ::: "memory");
+                    publish(plane - 1);
                 }
-                const bool has_dz = q < t.n;
-                if (has_dz && dcount >= SD) {
-                    got = got && mbar_wait(saddr(&bar_dempty[dcount % SD]), (uint32_t)(((dcount - SD) / SD) & 1), fail);
+                if (plane >= SH) {
+                    got = mbar_wait(saddr(&bar_empty[plane % SH]), (uint32_t)(((plane - SH) / SH) & 1), fail);
+                }
+                const bool has_dz = q >= 2;
+                if (has_dz && dplane >= SD) {
+                    got = got && mbar_wait(saddr(&bar_dempty[dplane % SD]), (uint32_t)(((dplane - SD) / SD) & 1), fail);
                 }
                 if (!__all_sync(0xffffffffu, got)) {
                     ok = false;
                     break;
                 }
-                const uint32_t hs = hring + (uint32_t)((step % SH) * G::HSLOT);
-                const uint32_t ds = dring + (uint32_t)((dcount % SD) * G::DSLOT);
+                const uint32_t hs = hring + (uint32_t)((plane % SH) * G::HSLOT);
+                const uint32_t ds = dring + (uint32_t)((dplane % SD) * G::DSLOT);
                 if (MODE == FL) {
-                    int z = t.z0 - 1 + q;
-                    z = z < 0 ? z + s.nz : (z >= s.nz ? z - s.nz : z);
-                    for (int v = lt; v < G::ROWS * TXW; v += LT) {
-                        const int r = v / TXW;
-                        const int x = t.x0 + v % TXW;
-                        int y = t.y0 - 1 + r;
-                        y = y < 0 ? y + s.ny : (y >= s.ny ? (y - s.ny) % s.ny : y);
-                        const uint32_t *row = p.x0 + (((long long)t.b * s.nz + z) * s.ny + y) * s.nx;
-                        st_shared16(hs + (uint32_t)(v * 16), make_uint4(row[x == 0 ? s.nx - 1 : x - 1], row[x],
-                                                                        row[x == s.nx - 1 ? 0 : x + 1], 0u));
+#pragma unroll
+                    for (int i = 0; i < PERF; ++i) {
+                        const int v = lt + i * LT;
+                        if ((i + 1) * LT <= G::ROWS * TXW || v < G::ROWS * TXW) {
+                            st_shared16(hs + (uint32_t)(v * 16), make_uint4(nx0[i][0], nx0[i][1], nx0[i][2], 0u));
+                        }
                     }
                 } else {
-                    constexpr int PER_ROW = G::NG * 10;
-                    for (int v = lt; v < G::ROWS * PER_ROW; v += LT) {
-                        const int r = v / PER_ROW;
-                        const int i = v - r * PER_ROW;
-                        const int gy = min(t.y0 + r, s.ny + 1);
-                        const bf16 *src =
-                            p.h + (ghost_row(s, t.b, t.z0 + q, gy) * (s.nx + 2) + t.x0 + (i / 10) * 8 + i % 10) * 8;
-                        const uint32_t d = hs + (uint32_t)(r * 3 * G::UA + i * 16);
+                    const bf16 *from = p.h + ghost_row(s, t.b, t.z0 + q, 0) * (s.nx + 2) * 8;
+                    for (int v = lt; v < G::ROWS * TXW; v += LT) {
+                        const int row = v / TXW, x = v % TXW;
+                        const int gy = min(t.y0 + row, s.ny + 1);
+                        const bf16 *src = from + (gy * 3LL * (s.nx + 2) + t.x0 + x + 1) * 8;
+                        const uint32_t d = hs + (uint32_t)(row * 3 * G::UA + x * 16);
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) copy16(d + c * G::UA, src + (long long)c * (s.nx + 2) * 8);
+                        for (int c = 0; c < 3; ++c) copy16(d + c * G::UA, src + c * (s.nx + 2LL) * 8);
                     }
                 }
                 if (has_dz) {
                     // rows past the grid count nothing
-                    for (int v = lt; v < G::TY * TXW; v += LT) {
-                        const int r = v / TXW;
-                        const int x = t.x0 + v % TXW;
-                        const int y = t.y0 + r;
-                        const bool in = y < s.ny;
-                        const uint32_t d = ds + (uint32_t)(r * G::NPR * G::UB + v % TXW * 16);
+                    const bf16 *from = MODE == LL ? nullptr : p.dz + ghost_row(s, t.b, t.z0 + q - 1, 0) * (s.nx + 2) * 8;
+#pragma unroll
+                    for (int i = 0; i < G::TY * TXW / LT; ++i) {
+                        const int v = lt + i * LT;
+                        const int row = v / TXW, x = v % TXW;
+                        const bool in = t.y0 + row < s.ny;
+                        const uint32_t d = ds + (uint32_t)(row * G::NPR * G::UB + x * 16);
                         if (MODE == LL) {
                             // taps dx = 0, 1, 2 of voxel x of h meet g at x + 1, x, x - 1
                             uint4 g = make_uint4(0u, 0u, 0u, 0u);
                             if (in) {
-                                const long long row = (((long long)t.b * s.nz + t.z0 + q) * s.ny + y) * s.nx;
-                                const int xw = x == 0 ? s.nx - 1 : x - 1, xe = x == s.nx - 1 ? 0 : x + 1;
-                                g.x = pack_bf16(p.scale * (p.du[row + xe] - p.target[row + xe]),
-                                                p.scale * (p.du[row + x] - p.target[row + x]));
-                                g.y = pack_bf16(p.scale * (p.du[row + xw] - p.target[row + xw]), 0.f);
+                                g.x = pack_bf16(p.scale * (ng[i][0] - ng[i][1]), p.scale * (ng[i][2] - ng[i][3]));
+                                g.y = pack_bf16(p.scale * (ng[i][4] - ng[i][5]), 0.f);
                             }
                             st_shared16(d, g);
                         } else {
-                            const bf16 *src =
-                                p.dz + (ghost_row(s, t.b, t.z0 + q + 1, in ? y + 1 : 0) * (s.nx + 2) + x + 1) * 8;
+                            const bf16 *src = from + ((in ? t.y0 + row + 1 : 0) * 3LL * (s.nx + 2) + t.x0 + x + 1) * 8;
 #pragma unroll
                             for (int c = 0; c < 3; ++c) {
-                                copy16_or_zero(d + c * G::UB, src + (long long)c * (s.nx + 2) * 8, in);
+                                const bf16 *sc = src + c * (s.nx + 2LL) * 8;
+                                if (MODE == FL) {
+                                    copy16_or_zero(d + c * G::UB, sc, in);
+                                } else {
+                                    // tap dx of voxel x of h meets dz at x + 1 - dx
+#pragma unroll
+                                    for (int dx = 0; dx < 3; ++dx) copy16_or_zero(d + (dx * 3 + c) * G::UB, sc + (1 - dx) * 8, in);
+                                }
                             }
                         }
                     }
-                    ++dcount;
+                    ++dplane;
                 }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (q + 1 < t.n + 2) fetch(t, q + 1);
+                else if (it + (int)gridDim.x < p.items) fetch(item_of(it + gridDim.x), 0);
             }
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
-        if (ok) publish(step);
+        if (ok) publish(plane);
         else if (lane == 0) s_fail = 1;
     } else {
-        // warps 1 .. 4: lane quarter warp % 4
+        // the four warps between: lane quarter warp % 4
         const int qd = warp & 3;
         const uint32_t acc = tmem + ((uint32_t)(qd * 32) << 16);
         const float zero[8] = {};
-        for (int c = 0; c < 3 * G::DX * G::N; c += 8) tmem_st8(acc + (uint32_t)c, zero);
+        for (int c = 0; c < 3 * G::N; c += 8) tmem_st8(acc + (uint32_t)c, zero);
         tmem_st_wait();
         fence_before();
         __syncwarp();
@@ -317,7 +364,7 @@ wgrad_tc_kernel(const WParams p)
         if (!s_bad) {
             // every copy has been read by an MMA: the ring becomes dW
             float *dw = reinterpret_cast<float *>(smem);
-            const int ft = (warp - 1) * 32 + lane;
+            const int ft = (warp - WG_MMA) * 32 + lane;
             for (int i = ft; i < G::OUT; i += 128) dw[i] = 0.f;
             asm volatile("bar.sync 1, 128;" ::: "memory");
             const int m = qd * 32 + lane;               // row of D: unit m / 8, element m % 8
@@ -329,21 +376,18 @@ wgrad_tc_kernel(const WParams p)
                 const bool use = dy >= 0 && dy < 3 && (MODE != FL || e < 6);
                 for (int dz = 0; dz < 3; ++dz) {
 #pragma unroll
-                    for (int dx = 0; dx < G::DX; ++dx) {
+                    for (int c = 0; c < G::NPR; ++c) {
+                        float v[8];
+                        __syncwarp();
+                        tmem_ld8(acc + (uint32_t)(dz * G::N + (y * G::NPR + c) * 8), v);
 #pragma unroll
-                        for (int c = 0; c < G::NPR; ++c) {
-                            float v[8];
-                            __syncwarp();
-                            tmem_ld8(acc + (uint32_t)((dz * G::DX + dx) * G::N + (y * G::NPR + c) * 8), v);
-#pragma unroll
-                            for (int i = 0; i < 8 && use; ++i) {
-                                if (MODE == LL) {
-                                    if (i < 3) dw[((dz * 3 + dy) * 3 + i) * 24 + e] += v[i];
-                                } else if (MODE == FL) {
-                                    dw[(((dz * 3 + dy) * 3 + e / 2) * 2 + e % 2) * 24 + c * 8 + i] += v[i];
-                                } else {
-                                    dw[(((dz * 3 + dy) * 3 + dx) * 24 + e) * 24 + c * 8 + i] += v[i];
-                                }
+                        for (int i = 0; i < 8 && use; ++i) {
+                            if (MODE == LL) {
+                                if (i < 3) dw[((dz * 3 + dy) * 3 + i) * 24 + e] += v[i];
+                            } else if (MODE == FL) {
+                                dw[(((dz * 3 + dy) * 3 + e / 2) * 2 + e % 2) * 24 + c * 8 + i] += v[i];
+                            } else {        // c = 3 dx + channel group
+                                dw[(((dz * 3 + dy) * 3 + c / 3) * 24 + e) * 24 + c % 3 * 8 + i] += v[i];
                             }
                         }
                     }
@@ -448,7 +492,9 @@ static int run_w(WParams p, cudaStream_t stream)
 template<int MODE>
 static int run_w_any(const WParams& p, cudaStream_t stream)
 {
-    if (p.s.nx % 128 == 0) return run_w<MODE, 128>(p, stream);
+    if constexpr (MODE != CC) {             // 256 voxels of CC: 64 x 4 has fewer halo rows than 128 x 2
+        if (p.s.nx % 128 == 0) return run_w<MODE, 128>(p, stream);
+    }
     if (p.s.nx % 64 == 0) return run_w<MODE, 64>(p, stream);
     return run_w<MODE, 32>(p, stream);
 }
