@@ -4,18 +4,27 @@
 // independent additions measured 498 G operations per second on the whole
 // GPU.  Everything here serves to keep that pipe busy and to take work off it:
 //   - the multiplication by fl(1/7) runs on the integer pipes, bit for bit
-//     (mul_seventh): six FP64 operations per cell instead of seven.  The z
-//     loop stays rolled: unrolled, the compiler turns mul_seventh's rare
-//     branch into predicated code that pays the FP64 multiplication always
-//     (512^3: 72 GLUPS with the multiplication, 78 unrolled, 84 rolled);
+//     (mul_seventh), and so do the first three of the six additions (sum4):
+//     three FP64 operations per cell instead of seven.  Three is where the
+//     FP64 and the integer work take about the same time: at 512^3, in us per
+//     step, 1600 with no addition in integers, 1110 with two, 916 with three,
+//     1140 with four, 1376 with all six (measured without the one-sided
+//     neighbour's rule below and with plain launches).  Where sum4's condition
+//     fails in some lane the warp adds in FP64 after all, which costs what it
+//     cost before: smooth fields meet it but for the cells beside a zero edge
+//     in y; the zero east of the last column is dropped (drop_e);
+//   - the rare branches must stay branches: predicated, their FP64 operations
+//     would be paid always.  So the z loop stays rolled, and sum4's fallback is
+//     a loop;
 //   - every thread owns one cell of a plane and marches a few planes; the
 //     cells of a plane are numbered through (no idle lanes whatever nx is)
 //     and neighbours come straight from global memory (L1 / L2 hits), so
 //     there is no barrier and no tile, and a grid is cut into as many small
 //     CTAs as it takes to give every SM an even share.
-// Measured (us per step, against the TMA kernel of k_tma.cu before): 24 x 20
-// x 16 4.2 against 22.6, 64^3 8.2 against 22.6, 128^3 28.7 against 38.9,
-// 512^3 1598 against 1795 (84 GLUPS x 6 operations = 503 G/s: the pipe).
+// Measured (us per step; in brackets the kernel without sum4, then the TMA
+// kernel of k_tma.cu): 24 x 20 x 16 1.9 (2.2, 22.6), 64^3 4.0 (5.9, 22.6), 128^3
+// 17.1 (25.4, 38.9), 512^3 886 (1598, 1795): 151 GLUPS, 91% of the FP64 pipe's
+// rate at three operations per cell.
 // The sum's order is the cell's own: results are bit-identical to every
 // other kernel of the cell.
 #include <algorithm>
@@ -28,8 +37,9 @@ namespace lgd {
 namespace fp64k {
 
 constexpr int THREADS = 128;
+constexpr int CTAS = 8;        // per SM: 64 registers
 
-__global__ void __launch_bounds__(THREADS, 16)
+__global__ void __launch_bounds__(THREADS, CTAS)
 jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, int nz,
                    int zchunk, double edge)
 {
@@ -43,6 +53,7 @@ jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, in
     const int z1 = min(z0 + zchunk, nz);
     const long plane = pitch * ny;
     const bool has_n = y > 0, has_s = y + 1 < ny, has_w = x > 0, has_e = x + 1 < nx;
+    const bool drop_e = !has_e && edge == 0.0;      // the sum of the others is not zero where it is taken
     const double *p = in + (long)z0 * plane + (long)y * pitch + x;
     double *o = out + (long)z0 * plane + (long)y * pitch + x;
     double b = z0 > 0 ? *(p - plane) : edge;
@@ -54,9 +65,12 @@ jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, in
         const double s = has_s ? *(p + pitch) : edge;
         const double e = has_e ? *(p + 1) : edge;
         const double w = has_w ? *(p - 1) : edge;
-        double acc = __dadd_rn(m, n);
-        acc = __dadd_rn(acc, s);
-        acc = __dadd_rn(acc, e);
+        double acc;
+        if (!sum4(m, n, s, e, drop_e, acc)) {
+            acc = m;
+#pragma unroll 1
+            for (int i = 0; i < 3; ++i) acc = __dadd_rn(acc, i == 0 ? n : (i == 1 ? s : e));
+        }
         acc = __dadd_rn(acc, w);
         acc = __dadd_rn(acc, t);
         acc = __dadd_rn(acc, b);
@@ -78,10 +92,12 @@ bool jacobi7_f64_applicable(const Grid& g)
            (long long)g.desc.nx * g.desc.ny < (1ll << 31) - fp64k::THREADS;
 }
 
-// Planes per thread: 8 re-read least, but the grid must fall into many more
-// CTAs than the SMs hold at once (16), or the last wave leaves the pipe idle,
-// so small grids march fewer planes (128^3: 28.7 us at 2 and 4, 30.8 at 8
-// and 16; 512^3 does not care).
+// Planes per thread: 8 re-read least, but the grid must fall into more CTAs
+// than the SMs hold at once (8), or the last wave leaves the pipe idle, so small
+// grids march fewer planes until there are 20 CTAs per SM.  us per step with 1,
+// 2, 4, 8 planes: 64^3 4.0, 4.8, 7.3, 10.4 (13 CTAs per SM at one plane); 96^3
+// 9.3, 8.5, 9.0, 14.0 (23 at two); 128^3 19.7, 17.4, 17.1, 18.0 (27 at four);
+// 512^3 1189, 1005, 920, 886.
 void launch_jacobi7_f64(Grid& g)
 {
     static PerDevice<int> setup;
@@ -93,7 +109,7 @@ void launch_jacobi7_f64(Grid& g)
     });
     const long long xy = ((long long)g.desc.nx * g.desc.ny + fp64k::THREADS - 1) / fp64k::THREADS;
     int zchunk = 8;
-    while (zchunk > 1 && xy * ((g.desc.nz + zchunk - 1) / zchunk) < 40LL * sms) zchunk /= 2;
+    while (zchunk > 1 && xy * ((g.desc.nz + zchunk - 1) / zchunk) < 20LL * sms) zchunk /= 2;
     zchunk = std::max(zchunk, (g.desc.nz + 65534) / 65535);
     const dim3 grid((unsigned)xy, (unsigned)((g.desc.nz + zchunk - 1) / zchunk));
     launch_dependent(

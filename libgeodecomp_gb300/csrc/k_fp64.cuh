@@ -31,6 +31,50 @@ __device__ __forceinline__ double mul_seventh(double a)
     return __dmul_rn(a, 1.0 / 7.0);
 }
 
+// fl(fl(fl(a + b) + c) + d), the IEEE sum in that order, in integer arithmetic;
+// false where that does not hold (the caller adds in FP64): operands of
+// different sign or more than six binary exponents apart, zeros, subnormals,
+// infinities, NaN and the ends of the exponent range.  With drop_d, d stands
+// for +-0 and its value is not looked at.
+// The operands become integers in units of 2^-53 times the smallest one's
+// power of two (so that the first rounding already has a bit to drop); a sum of
+// four is below 2^62.  A sum of 53 + k bits drops k: half a unit minus one,
+// plus the last kept bit, rounds to nearest even.
+#define LGD_FP64_SUM_REACH 7
+__device__ __forceinline__ bool sum4(double a, double b, double c, double d, bool drop_d, double& sum)
+{
+    const unsigned ha = (unsigned)__double2hiint(a), sign = ha & 0x80000000u;
+    const unsigned h[4] = {ha ^ sign, (unsigned)__double2hiint(b) ^ sign, (unsigned)__double2hiint(c) ^ sign,
+                           drop_d ? ha ^ sign : (unsigned)__double2hiint(d) ^ sign};
+    const unsigned lo[4] = {(unsigned)__double2loint(a), (unsigned)__double2loint(b), (unsigned)__double2loint(c),
+                            (unsigned)__double2loint(d)};
+    const unsigned e0 = (min(min(h[0], h[1]), min(h[2], h[3])) >> 20) - 1u;
+    unsigned long long v[4];
+    unsigned reach = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const unsigned shift = (h[i] >> 20) - e0;           // 1 .. 7; another sign's exponent is far above
+        const unsigned m = (h[i] & 0xfffffu) | 0x100000u;
+        reach |= shift;
+        v[i] = ((unsigned long long)__funnelshift_l(lo[i], m, shift) << 32) | (lo[i] << (shift & 31u));
+    }
+    if (drop_d) v[3] = 0;
+    unsigned long long s = v[0];
+    unsigned k = 0;
+#pragma unroll
+    for (int i = 1; i < 4; ++i) {
+        s += v[i];
+        k = 11u - (unsigned)__clz((int)(s >> 32));
+        const unsigned unit = 1u << (k & 31u);
+        s += (unit >> 1) - 1u + (((unsigned)s >> (k & 31u)) & 1u);
+        s &= ~(unsigned long long)(unit - 1u);
+    }
+    // s >> k holds the leading bit, which adds one to the exponent field
+    const unsigned long long r = (s >> (k & 31u)) + ((unsigned long long)(e0 + k - 1u) << 52);
+    sum = __longlong_as_double((long long)(r | ((unsigned long long)sign << 32)));
+    return reach <= LGD_FP64_SUM_REACH && e0 - 1u < 2030u;
+}
+
 }  // namespace lgd
 
 #endif

@@ -37,3 +37,19 @@ def test_value_ranges(scale):
         ref = oracle.jacobi7(u0, 3)
     out = run(u0, 3)
     np.testing.assert_array_equal(out.view(np.uint64), ref.view(np.uint64))
+
+
+@pytest.mark.parametrize("reach", [0, 5, 6, 7, 40])
+@pytest.mark.parametrize("shape", [(3, 9, 33), (5, 6, 128)])
+def test_exponent_distances(reach, shape):
+    """The integer sum's condition met by all, some and none of a warp's
+    cells, with few significant bits (ties) and full significands, of one
+    sign and of both."""
+    rng = np.random.default_rng(reach)
+    for bits, both in [(3, False), (52, False), (52, True)]:
+        m = 1.0 + np.floor(rng.random(shape) * 2.0 ** bits) * 2.0 ** -bits
+        u0 = np.ldexp(m, rng.integers(0, reach + 1, shape))
+        if both:
+            u0 *= np.where(rng.random(shape) < 0.02, -1.0, 1.0)
+        np.testing.assert_array_equal(run(u0, 1).view(np.uint64), oracle.jacobi7(u0, 1).view(np.uint64))
+        np.testing.assert_array_equal(run(-u0, 4), oracle.jacobi7(-u0, 4))
