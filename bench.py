@@ -439,9 +439,8 @@ class VarcoefWorkload:
 
 class LbmWorkload:
     """512 D3Q19 lid-driven cavities, edges uniform in {32..192}, omega
-    uniform in [1.0, 1.9), lid 0.05, FP32; one persistent launch per step or
-    one two-step launch per pair of steps, launch shape and steps per launch
-    from the library's pattern-search tuner."""
+    uniform in [1.0, 1.9), lid 0.05, FP32; one launch per step or one two-step
+    launch per pair of steps, whichever the library's tuner finds fastest."""
     run_steps = 500
     bytes_per_unit = 152     # 19 FP32 reads + 19 FP32 writes per cell
 

@@ -36,15 +36,16 @@ typedef struct lgd_lbm lgd_lbm;
 int lgd_lbm_create(int count, const int32_t *edges, const double *omegas, double lid, int precision, lgd_lbm **out);
 int lgd_lbm_destroy(lgd_lbm *h);
 
-/* steps time steps of every instance: one persistent launch per step. */
+/* steps time steps of every instance: one launch per step (one thread per
+ * cell, or the persistent kernel once a launch shape has been set). */
 int lgd_lbm_step(lgd_lbm *h, int steps);
 
 /* the same steps with one launch per instance and step (comparison path). */
 int lgd_lbm_step_looped(lgd_lbm *h, int steps);
 
-/* Launch shape: tile_rows rows of one z plane per work item, threads per
- * CTA (64..1024, power of two), resident CTAs per SM (clamped to the
- * occupancy limit). */
+/* Single steps by the persistent kernel with this launch shape: tile_rows
+ * rows of one z plane per work item, threads per CTA (64..1024, power of
+ * two), resident CTAs per SM (clamped to the occupancy limit). */
 int lgd_lbm_set_config(lgd_lbm *h, int tile_rows, int threads, int ctas_per_sm);
 int lgd_lbm_get_config(lgd_lbm *h, int *tile_rows, int *threads, int *ctas_per_sm);
 
@@ -59,9 +60,10 @@ int lgd_lbm_get_config(lgd_lbm *h, int *tile_rows, int *threads, int *ctas_per_s
 int lgd_lbm_set_time_block(lgd_lbm *h, int depth, int shape, int ctas_per_sm);
 int lgd_lbm_get_time_block(lgd_lbm *h, int *depth, int *shape, int *ctas_per_sm);
 
-/* Pattern search over the launch shape of single steps, timing trial_steps
- * steps per candidate with CUDA events, then over the two-step kernel's
- * tile shape and residency; leaves the fastest per step set (read it back
+/* Times single steps with one thread per cell, then a pattern search over
+ * the persistent kernel's launch shape, timing trial_steps steps per
+ * candidate with CUDA events, then over the two-step kernel's tile shape
+ * and residency; leaves the fastest per step set (read it back
  * with lgd_lbm_get_config and lgd_lbm_get_time_block).  The trial steps
  * advance the ensemble: reset or upload afterwards.  (Precedent: the
  * reference's AutoTuningSimulator with PatternOptimizer,

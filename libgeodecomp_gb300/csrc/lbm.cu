@@ -7,12 +7,14 @@
 // population array starts on a 128-byte (FP32) boundary.  Warps walk the
 // cells of a work item in 32-cell groups aligned to that boundary (lanes
 // outside the item idle), so a warp's own-cell loads and stores are whole
-// sectors.  Every time step is one persistent
-// kernel launch: the CTAs pull work items - TY rows of one z plane of one
-// instance, largest instances first - from an atomic counter until the list
-// is exhausted, so instances of 32^3 and 192^3 cells share the GPU without
-// per-instance launches.  Two steps (A -> B, B -> A, each with its counter
-// reset) are captured once into a CUDA graph and replayed.  With temporal
+// sectors.  Every time step is one launch for all instances, so that 32^3 and
+// 192^3 cells share the GPU.  By default it has one thread per cell and one CTA
+// per 128 cells (lbm_flat_kernel: 132 us for 5.5 M cells of 40^3 to 115^3 in
+// FP32, 6.35 TB/s).  With a launch shape set by the caller, CTAs are persistent
+// and their warps pull work items - TY rows of one z plane of one instance,
+// largest instances first - from an atomic counter until the list is exhausted
+// (188 us at the best shape).  Two steps (A -> B, B -> A) are captured once into
+// a CUDA graph and replayed.  With temporal
 // blocking (lbm_tb2_kernel) one persistent launch advances two steps, and
 // two such launches (four steps) are captured and replayed the same way.
 //
@@ -23,9 +25,10 @@
 // lid (the wall beyond y = L-1).  Traffic: 19 reads + 19 writes per cell and
 // step (152 B in FP32), the bounce-back reads hit L1.
 //
-// The tile height TY, threads per CTA and CTAs per SM are chosen by a
-// pattern search (lgd_lbm_tune), the method of the reference's
-// PatternOptimizer (misc/patternoptimizer.h:13) applied to this kernel.
+// lgd_lbm_tune times the default, then searches the tile height TY, threads per
+// CTA and CTAs per SM of the persistent kernel by pattern search, the method of
+// the reference's PatternOptimizer (misc/patternoptimizer.h:13), and the
+// two-step kernel.
 #include <algorithm>
 #include <limits>
 #include <mutex>
@@ -47,6 +50,8 @@ struct LbmInstance {
     double omega;
     double lid;
 };
+
+struct FlatBlock;
 
 struct Lbm {
     int count;
@@ -83,6 +88,9 @@ struct Lbm {
     int4 *d_cols;       // (instance, x0 | y0 << 16, z0, z1)
     int n_cols;
     int cols_shape;
+    bool flat;          // single steps by lbm_flat_kernel (until a launch shape is set or found faster)
+    FlatBlock *d_blocks;
+    int n_blocks;
     double *d_stage;    // conversion staging of uploads and downloads (FP32; from the first one on)
 };
 
@@ -352,6 +360,70 @@ __global__ void lbm_persistent_kernel(const LbmInstance *__restrict__ inst, cons
     }
 }
 
+// ------------------------------------------- one thread per cell and step
+// A CTA takes FLAT consecutive cells of one instance, found in a table (an
+// entry holds all it needs: one load), and is gone: the next CTA's 19 loads per
+// cell overlap with this one's stores.  Warps that walk work items wait for a
+// cell's loads, collide, store, and only then load again; with 38 streams that
+// left DRAM at 5.0 of 6.8 TB/s whatever the registers, warps and item shapes.
+constexpr int FLAT = 128;
+
+struct FlatBlock {
+    long long base;
+    int L;
+    unsigned magic;
+    double omega, lid;
+    int first;          // cell
+    int pad[3];
+};
+
+// population I of a cell of which some may lie at a wall: one load, its address
+// selected, so that a warp's inner and wall cells stay together
+template<typename R, int I, typename IDX, int NC>
+__device__ __forceinline__ void pull_select(const R *src, IDX n3, IDX cell, int L, int x, int y, int z, R lid, R *f)
+{
+    if constexpr (I < 19) {
+        const bool inside = (unsigned)(x - Q<I>::ex) < (unsigned)L && (unsigned)(y - Q<I>::ey) < (unsigned)L &&
+                            (unsigned)(z - Q<I>::ez) < (unsigned)L;
+        const IDX at = inside ? I * n3 + cell - (Q<I>::ex + (IDX)Q<I>::ey * L + (IDX)Q<I>::ez * L * L) : Q<I>::opp * n3 + cell;
+        R v = Mem<NC>::ld(src + at);
+        if (Q<I>::ey == -1 && Q<I>::ex != 0) {              // see pull_one
+            const R from_lid = LbmArith<R>::add(
+                v, LbmArith<R>::mul(LbmArith<R>::mul((R)6.0, I < 7 ? (R)(1.0 / 18.0) : (R)(1.0 / 36.0)), (R)Q<I>::ex * lid));
+            v = !inside && y == L - 1 ? from_lid : v;
+        }
+        f[I] = v;
+        pull_select<R, I + 1, IDX, NC>(src, n3, cell, L, x, y, z, lid, f);
+    }
+}
+
+template<typename R, typename IDX, int NC>
+__global__ void __launch_bounds__(FLAT, sizeof(R) == 4 ? 8 : 5)
+lbm_flat_kernel(const FlatBlock *__restrict__ blocks, const R *A, R *B)
+{
+    dependent_start();
+    const FlatBlock in = blocks[blockIdx.x];
+    const unsigned L = (unsigned)in.L;
+    const unsigned c = (unsigned)in.first + threadIdx.x;
+    unsigned row = __umulhi(c, in.magic);                   // c below 2^30: at most one too many
+    if (row * L > c) --row;
+    unsigned plane = __umulhi(row, in.magic);
+    if (plane * L > row) --plane;
+    const int x = (int)(c - row * L), y = (int)(row - plane * L), z = (int)plane;
+    const IDX n3 = ((IDX)L * L * L + 31) & ~(IDX)31;
+    const bool live = plane < L;
+    const bool inner = (unsigned)(x - 1) < L - 2 && (unsigned)(y - 1) < L - 2 && (unsigned)(z - 1) < L - 2;
+    const R *src = A + in.base;
+    R f[19];
+    if (__all_sync(0xffffffffu, inner)) {
+        PullAll<R, 0, IDX, NC, true>::run(src, n3, (IDX)c, (int)L, x, y, z, (R)in.lid, f);
+    } else {
+        if (!live) return;
+        pull_select<R, 0, IDX, NC>(src, n3, (IDX)c, (int)L, x, y, z, (R)in.lid, f);
+    }
+    collide_store<R, IDX, NC>(f, (R)in.omega, B + in.base, n3, (IDX)c);
+}
+
 // one instance, one launch: the looped single-grid comparison
 template<typename R, typename IDX, int NC>
 __global__ void lbm_single_kernel(const LbmInstance *__restrict__ inst, int j, const R *__restrict__ A, R *__restrict__ B)
@@ -581,6 +653,28 @@ static void build_items(Lbm& e)
     e.n_items = (int)items.size();
 }
 
+static void build_blocks(Lbm& e)
+{
+    std::vector<FlatBlock> blocks;
+    for (const LbmInstance& in : e.inst) {
+        const long long n3 = (long long)in.L * in.L * in.L;
+        for (long long c = 0; c < n3; c += FLAT) {
+            FlatBlock b = {in.base, in.L, in.magic, in.omega, in.lid, (int)c, {}};
+            if (e.precision == 4) {
+                b.omega = in.omega_f;
+                b.lid = in.lid_f;
+            }
+            blocks.push_back(b);
+        }
+    }
+    LGD_REQUIRE(blocks.size() < (1ull << 31), LGD_ERR_RANGE, "ensemble too large");
+    LGD_CHECK_CUDA(cudaMalloc(&e.d_blocks, sizeof(FlatBlock) * blocks.size()));
+    LGD_CHECK_CUDA(
+        cudaMemcpyAsync(e.d_blocks, blocks.data(), sizeof(FlatBlock) * blocks.size(), cudaMemcpyHostToDevice, e.stream));
+    LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
+    e.n_blocks = (int)blocks.size();
+}
+
 // the persistent kernel for the ensemble's precision and index width
 template<int NC>
 static const void *persistent_fn_nc(const Lbm& e)
@@ -619,8 +713,29 @@ static void launch_single_nc(Lbm& e, int j, dim3 grid)
     }
 }
 
+template<typename R, typename IDX>
+static void launch_flat_as(Lbm& e, int src)
+{
+    const R *a = (const R *)e.buf[src];
+    R *b = (R *)e.buf[1 - src];
+    if (e.variant == 1) {       // reads through the read-only path: not while the step before still writes
+        lbm_flat_kernel<R, IDX, 1><<<e.n_blocks, FLAT, 0, e.stream>>>(e.d_blocks, a, b);
+    } else {
+        launch_dependent(lbm_flat_kernel<R, IDX, 0>, dim3(e.n_blocks), FLAT, 0, e.stream, (const FlatBlock *)e.d_blocks, a, b);
+    }
+}
+
 static void launch_step(Lbm& e, int which_counter, int src)
 {
+    if (e.flat) {
+        if (e.precision == 4) {
+            if (e.idx32) launch_flat_as<float, int>(e, src); else launch_flat_as<float, long long>(e, src);
+        } else {
+            if (e.idx32) launch_flat_as<double, int>(e, src); else launch_flat_as<double, long long>(e, src);
+        }
+        check_launch("lbm step");
+        return;
+    }
     LGD_CHECK_CUDA(cudaMemsetAsync(e.d_counter + which_counter, 0, sizeof(int), e.stream));
     const int grid = e.sms * e.ctas_per_sm;
     int *counter = e.d_counter + which_counter;
@@ -875,6 +990,7 @@ static void lbm_free(Lbm& e)
     cudaFree(e.d_inst);
     cudaFree(e.d_items);
     cudaFree(e.d_cols);
+    cudaFree(e.d_blocks);
     cudaFree(e.d_stage);
     cudaFree(e.d_counter);
     if (e.stream) cudaStreamDestroy(e.stream);
@@ -938,6 +1054,8 @@ int lgd_lbm_create(int count, const int32_t *edges, const double *omegas, double
             }
             check_launch("lbm rest state");
             ++e->launches;
+            build_blocks(*e);
+            e->flat = true;
             set_config(*e, 4, 256, 4);
         } catch (...) {
             lbm_free(*e);
@@ -986,7 +1104,17 @@ int lgd_lbm_step_looped(lgd_lbm *h, int steps)
 
 int lgd_lbm_set_config(lgd_lbm *h, int tile_rows, int threads, int ctas_per_sm)
 {
-    return guard([&] { set_config(lbm_of(h), tile_rows, threads, ctas_per_sm); });
+    return guard([&] {
+        Lbm& e = lbm_of(h);
+        const bool before = e.flat;
+        e.flat = false;
+        try {
+            set_config(e, tile_rows, threads, ctas_per_sm);
+        } catch (...) {
+            e.flat = before;
+            throw;
+        }
+    });
 }
 
 int lgd_lbm_get_config(lgd_lbm *h, int *tile_rows, int *threads, int *ctas_per_sm)
@@ -1022,7 +1150,11 @@ int lgd_lbm_tune(lgd_lbm *h, int trial_steps, int *tile_rows, int *threads, int 
             LGD_CHECK_CUDA(cudaEventElapsedTime(&ms, t0, t1));
             return ms / trial_steps;
         };
-        // pattern search over (log2 tile rows, log2 threads, CTAs per SM)
+        // one thread per cell, then a pattern search over (log2 tile rows,
+        // log2 threads, CTAs per SM)
+        e.flat = true;
+        const double flat_ms = measure(e.ty, e.threads, e.ctas_per_sm);
+        e.flat = false;
         const int tys[] = {1, 2, 4, 8, 16, 32};
         const int ths[] = {128, 256, 512};
         const int cts[] = {1, 2, 3, 4, 6, 8};
@@ -1053,6 +1185,11 @@ int lgd_lbm_tune(lgd_lbm *h, int trial_steps, int *tile_rows, int *threads, int 
             b = bb;
             c = bc;
         }
+        // the first measurement pays for the ensemble's first steps: repeated
+        e.flat = true;
+        const double flat_best = std::min(flat_ms, measure(tys[a], ths[b], cts[c]));
+        e.flat = flat_best <= best;
+        best = std::min(best, flat_best);
         set_config(e, tys[a], ths[b], cts[c]);
         // then temporal blocking: two steps per launch in each tile shape
         // and residency; the fastest per step wins, one step per launch
