@@ -12,7 +12,7 @@
 //     h = west + self + east           two bit planes (XOR3, majority)
 //     the sum of three rows' h         T = u0 + 2 k, the 3 x 3 total
 //     next = (T == 3) | (self & T == 4)
-// that is sixteen logic and shift instructions per 32 cells.  Summing across
+// that is two shuffles and eleven logic and shift instructions per 32 cells.  Summing across
 // the row before summing down needs the neighbours of one bit plane, not of
 // two as in gol_bits_kernel (k_gol.cu), and rows are independent of each
 // other, where that kernel's chain runs through all its generations in every
@@ -20,11 +20,13 @@
 // generation; with T generations per pass the inner W * R - 2 T rows and, for
 // T <= 32, lanes 1 .. 30 are right and are stored.
 //
-// Bound by the ALU pipe (64 lanes per clock and SM): 16 instructions per word
-// allow 38 T cell updates per second on 152 SMs.  A pass of 16 generations of
-// 8192^2 takes 44 us (24 T updates per second; gol_bits_kernel: 99 us); the
-// rest goes to the rim (6% of rows, 5% of words), 144 of 152 SMs at work, and
-// four warps per SM quarter that do not always have an instruction ready.
+// Bound by the ALU pipe (64 lanes per clock and SM): 11 instructions per word
+// allow 57 T cell updates per second on 152 SMs.  A pass of 16 generations of
+// 8192^2 takes 38 us (28 T updates per second; 44 with three instructions more
+// per word, gol_bits_kernel 99); the rest goes to the rim (6% of rows, 5% of
+// words), 144 of 152 SMs at work, 5 us of launch, loads and stores per pass,
+// and the exchange of rows.  More warps of fewer rows (24 x 23, 32 x 17) and
+// shifts moved to the multiplier pipe gained nothing.
 #include <algorithm>
 
 #include "lgd_internal.h"
@@ -98,20 +100,18 @@ __device__ __forceinline__ void row_sum(uint32_t v, uint32_t& h0, uint32_t& h1)
     h1 = maj(w, v, e);
 }
 
-// next state of the row m from the sums of the rows above, at and below
+// Next state of the row m from the sums of the rows above, at and below, in
+// seven three-input operations: T = u0 + 2 k with k = p + 2 q + cy, and the
+// cell lives if T == 3 (u0, k == 1) or, itself alive, T == 4 (~u0, k == 2).  The
+// last three use that T == 0 does not occur for a living cell.
 __device__ __forceinline__ uint32_t rule(uint32_t m, uint32_t a0, uint32_t a1, uint32_t m0, uint32_t m1, uint32_t c0,
                                          uint32_t c1)
 {
-    const uint32_t u0 = a0 ^ m0 ^ c0;
-    const uint32_t cy = maj(a0, m0, c0);
-    // k = a1 + m1 + c1 + cy from two half sums
-    const uint32_t p1 = a1 ^ m1, p2 = a1 & m1;
-    const uint32_t q1 = c1 ^ cy, q2 = c1 & cy;
-    const uint32_t two = p2 | q2;
-    const uint32_t k1 = (p1 ^ q1) & ~two;                           // k == 1
-    const uint32_t x2 = p2 ^ q2;
-    const uint32_t k2 = (p1 & q1) | (x2 & ~p1 & ~q1);               // k == 2
-    return (u0 & k1) | (~u0 & (m & k2));
+    const uint32_t u0 = a0 ^ m0 ^ c0, cy = maj(a0, m0, c0);
+    const uint32_t p = a1 ^ m1 ^ c1, q = maj(a1, m1, c1);
+    const uint32_t x = (u0 & ~q) | (~u0 & ~m);
+    const uint32_t even = (~cy & ~p) | (cy & p & ~q);           // k == 2, k == 0, not k == 1
+    return (u0 & x & ~even) | (~u0 & ~x & even);
 }
 
 // T generations; the tile's inner rows [T, T + out_rows) are the board's rows
@@ -236,9 +236,9 @@ gol_pack_kernel(const uint32_t *in, uint32_t *out, Board b, int T, int out_rows)
 
 // Tile height and generations per pass, by a model fitted to a sweep of all of
 // them on boards from 300^2 to 8192^2 (it finds the sweep's best or one within
-// 5%).  A generation takes the busiest SM's rows at 4.45 ns each (its four
+// 5%).  A generation takes the busiest SM's rows at 3.75 ns each (its four
 // quarters in step: the warps of the fullest count), or one warp's chain of
-// rows, 18 ns each, whichever is longer, and 45 ns of exchange; a pass adds
+// rows, 15 ns each, whichever is longer, and 45 ns of exchange; a pass adds
 // its launch, loads and stores.
 struct Plan {
     int R, W, T, out_rows;
@@ -266,7 +266,7 @@ static Plan plan(int nx, int ny, int sms, int steps)
                 const int out_rows = (int)((ny + bands - 1) / bands);
                 const long long per_sm = (xt * bands + sms - 1) / sms;
                 const double rows = (double)((per_sm * W + 3) / 4 * 4) * R;
-                const double gen = std::max(rows * 4.45, R * 18.0) + 45.0;
+                const double gen = std::max(rows * 3.75, R * 15.0) + 45.0;
                 const int passes = (steps + T - 1) / T;
                 const double ns = (passes * (1600.0 + 100.0 * R) + gen * steps) / steps;
                 if (ns < best.ns * 0.999) best = {R, W, T, out_rows, (int)per_sm, ns};
