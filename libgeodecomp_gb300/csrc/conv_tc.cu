@@ -99,7 +99,8 @@ struct Params {
     const float *bias;          // ACT, OUT
     bf16 *out;                  // ACT, GRAD: ghosted
     float *g;                   // ACT: GELU' of the pre-activations out (or null); GRAD: in; FP32
-                                // [batch][nz][ny][6][nx][4], four channels to a float4
+                                // [batch][nz][ny][6][nx][4], four channels to a float4.  OUT: receives fout too
+                                // (or null)
     float *db;                  // GRAD: bias gradient, added to
     float *fout;                // OUT
     int add;                    // OUT: add to fout
@@ -421,7 +422,9 @@ conv_tc_kernel(const Params p)
                 restart(slot);
                 if (q >= 2 && live) {
                     float *o = fout0 + z * fplane;
-                    *o = p.add ? before + (v + b1) : v + b1;
+                    const float r = p.add ? before + (v + b1) : v + b1;
+                    *o = r;
+                    if (p.g) p.g[o - p.fout] = r;
                 }
             } else {
                 uint4 w[3];
@@ -743,8 +746,8 @@ void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, f
     run_any<MID, ACT>(p, stream);
 }
 
-void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, const int dims[4], int *err,
-                   cudaStream_t stream)
+void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, float *copy, const int dims[4],
+                   int *err, cudaStream_t stream)
 {
     Params p = {};
     p.s = {dims[0], dims[1], dims[2], dims[3]};
@@ -752,6 +755,7 @@ void tc_layer_last(const void *in, const void *w, const float *bias, float *out,
     p.w = (const bf16 *)w;
     p.bias = bias;
     p.fout = out;
+    p.g = copy;
     p.add = add ? 1 : 0;
     p.err = err;
     run_any<LAST, OUT>(p, stream);

@@ -29,9 +29,10 @@ void tc_layer1(const float *u, const float *k, const void *w, const float *bias,
                int *err, cudaStream_t stream);
 void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, float *gelu_grad, const int dims[4], int *err,
                   cudaStream_t stream);
-// layer 4 (24 -> 1): out = conv + bias, or out += that
-void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, const int dims[4], int *err,
-                   cudaStream_t stream);
+// layer 4 (24 -> 1): out = conv + bias, or out += that; copy (or null)
+// receives out too
+void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, float *copy, const int dims[4],
+                   int *err, cudaStream_t stream);
 
 // input gradients: dz of the layer below = conv_t(dz) * gelu_grad, ghosted, and
 // its sum over the voxels added to db.  The last layer's takes the loss
@@ -44,10 +45,11 @@ void tc_grad_last(const float *du, const float *target, float scale, const void 
 // weight gradients of layer 0 (x0: BF16 pairs u, kappa; dz), 1 and 2 (h the
 // layer's input, dz), 3 (h, du, target, scale): each CTA's share into its
 // slice of partials (tc_partial_floats); returns the CTAs.  tc_wgrad_reduce
-// sums all layers' shares into grads.
+// sums all layers' shares into grads.  Layer 3 also adds the sum of (du -
+// target)^2 to loss and the output bias' gradient to db.
 size_t tc_partial_floats();
 int tc_wgrad(int layer, const void *h, const void *x0, const void *dz, const float *du, const float *target, float scale,
-             float *partials, const int dims[4], int *err, cudaStream_t stream);
+             double *loss, float *db, float *partials, const int dims[4], int *err, cudaStream_t stream);
 void tc_wgrad_reduce(const float *partials, const int ctas[4], const long long w_off[4], float *grads,
                      cudaStream_t stream);
 

@@ -454,7 +454,7 @@ struct Net {
     float *dh;          // [V][C] FP32 input gradient
     bf16 *dzb;          // [V][C] BF16 gradient
     bf16 *dz4;          // [V][2]
-    double *d_loss;
+    double *d_loss;     // one allocation with grads behind it
     int t;              // Adam step
     cudaStream_t stream;
     uint64_t launches;
@@ -558,7 +558,7 @@ static void sync_and_check(Net& n)
 // two ghosted buffers (three when training, which also keeps GELU' and the
 // packed input).  With add_to_u the last layer adds its
 // result to u instead (u <- u + du, the residual step).
-static void forward_fast(Net& n, const float *u, const float *k, float *du, bool add_to_u)
+static void forward_fast(Net& n, const float *u, const float *k, float *du, bool add_to_u, float *copy)
 {
     const int dims[4] = {n.g.nx, n.g.ny, n.g.nz, n.g.batch};
     const float *bias[4];
@@ -571,7 +571,8 @@ static void forward_fast(Net& n, const float *u, const float *k, float *du, bool
     tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], n.gt[0], dims, n.d_err, n.stream);
     tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], n.gt[1], dims, n.d_err, n.stream);
     tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], h3, n.gt[2], dims, n.d_err, n.stream);
-    tc_layer_last(h3, n.wtc.fwd[3], bias[3], add_to_u ? const_cast<float *>(u) : du, add_to_u, dims, n.d_err, n.stream);
+    tc_layer_last(h3, n.wtc.fwd[3], bias[3], add_to_u ? const_cast<float *>(u) : du, add_to_u, copy, dims, n.d_err,
+                  n.stream);
     n.launches += 4;
 }
 
@@ -582,21 +583,18 @@ static void backward_fast(Net& n, const float *target, double *loss_out)
 {
     const int dims[4] = {n.g.nx, n.g.ny, n.g.nz, n.g.batch};
     const float scale = 2.0f / (float)n.V;
-    LGD_CHECK_CUDA(cudaMemsetAsync(n.grads, 0, sizeof(float) * n.P, n.stream));
-    LGD_CHECK_CUDA(cudaMemsetAsync(n.d_loss, 0, sizeof(double), n.stream));
-    loss_kernel<<<grid_blocks(n.V), 256, 0, n.stream>>>(n.du, target, nullptr, n.grads + n.L[3].b_off, n.d_loss, n.V);
-    check_launch("loss");
+    LGD_CHECK_CUDA(cudaMemsetAsync(n.d_loss, 0, sizeof(double) + sizeof(float) * n.P, n.stream));     // and grads
     int ctas[4];
-    ctas[3] = tc_wgrad(3, n.hg[2], nullptr, nullptr, n.du, target, scale, n.part, dims, n.d_err, n.stream);
+    ctas[3] = tc_wgrad(3, n.hg[2], nullptr, nullptr, n.du, target, scale, n.d_loss, n.grads + n.L[3].b_off, n.part, dims, n.d_err, n.stream);
     tc_grad_last(n.du, target, scale, n.wtc.grad[3], n.gt[2], n.dzg[0], n.grads + n.L[2].b_off, dims, n.d_err, n.stream);
-    ctas[2] = tc_wgrad(2, n.hg[1], nullptr, n.dzg[0], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
+    ctas[2] = tc_wgrad(2, n.hg[1], nullptr, n.dzg[0], nullptr, nullptr, 0.f, nullptr, nullptr, n.part, dims, n.d_err, n.stream);
     tc_grad_mid(n.dzg[0], n.wtc.grad[2], n.gt[1], n.dzg[1], n.grads + n.L[1].b_off, dims, n.d_err, n.stream);
-    ctas[1] = tc_wgrad(1, n.hg[0], nullptr, n.dzg[1], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
+    ctas[1] = tc_wgrad(1, n.hg[0], nullptr, n.dzg[1], nullptr, nullptr, 0.f, nullptr, nullptr, n.part, dims, n.d_err, n.stream);
     tc_grad_mid(n.dzg[1], n.wtc.grad[1], n.gt[0], n.dzg[0], n.grads + n.L[0].b_off, dims, n.d_err, n.stream);
-    ctas[0] = tc_wgrad(0, nullptr, n.xt, n.dzg[0], nullptr, nullptr, 0.f, n.part, dims, n.d_err, n.stream);
+    ctas[0] = tc_wgrad(0, nullptr, n.xt, n.dzg[0], nullptr, nullptr, 0.f, nullptr, nullptr, n.part, dims, n.d_err, n.stream);
     const long long off[4] = {n.L[0].w_off, n.L[1].w_off, n.L[2].w_off, n.L[3].w_off};
     tc_wgrad_reduce(n.part, ctas, off, n.grads, n.stream);
-    n.launches += 9;
+    n.launches += 8;
     if (loss_out) {
         double l = 0.0;
         LGD_CHECK_CUDA(cudaMemcpyAsync(&l, n.d_loss, sizeof(double), cudaMemcpyDeviceToHost, n.stream));
@@ -674,11 +672,11 @@ static void backward_impl(Net& n, const float *target, double *loss_out)
 
 // du = net(u, k); with add_to_u the fast path may add du to u itself
 // (returns true when it did)
-static bool forward(Net& n, const float *u, const float *k, float *du, bool add_to_u = false)
+static bool forward(Net& n, const float *u, const float *k, float *du, bool add_to_u = false, float *copy = nullptr)
 {
     n.fast_forward = n.fast && n.variant == 0;
     if (n.fast_forward) {
-        forward_fast(n, u, k, du, add_to_u);
+        forward_fast(n, u, k, du, add_to_u, copy);
         return add_to_u;
     }
     ensure_dense(n);
@@ -687,6 +685,7 @@ static bool forward(Net& n, const float *u, const float *k, float *du, bool add_
     } else {
         if (n.TX == 64) forward_impl<8, 64>(n, u, k, du); else forward_impl<8, 32>(n, u, k, du);
     }
+    if (copy) LGD_CHECK_CUDA(cudaMemcpyAsync(copy, du, sizeof(float) * n.V, cudaMemcpyDeviceToDevice, n.stream));
     return false;
 }
 
@@ -708,7 +707,6 @@ static void net_free(Net& n)
 {
     if (n.stream) cudaStreamSynchronize(n.stream);
     cudaFree(n.params);
-    cudaFree(n.grads);
     cudaFree(n.m);
     cudaFree(n.v);
     for (int l = 0; l < 4; ++l) {
@@ -812,13 +810,13 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
             const long long V = n->V;
             LGD_CHECK_CUDA(cudaMalloc(&n->du, sizeof(float) * V));
             if (n->training) {
-                LGD_CHECK_CUDA(cudaMalloc(&n->grads, sizeof(float) * n->P));
+                LGD_CHECK_CUDA(cudaMalloc(&n->d_loss, sizeof(double) + sizeof(float) * n->P));
+                n->grads = reinterpret_cast<float *>(n->d_loss + 1);
                 LGD_CHECK_CUDA(cudaMalloc(&n->m, sizeof(float) * n->P));
                 LGD_CHECK_CUDA(cudaMalloc(&n->v, sizeof(float) * n->P));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->grads, 0, sizeof(float) * n->P, n->stream));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->m, 0, sizeof(float) * n->P, n->stream));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->v, 0, sizeof(float) * n->P, n->stream));
-                LGD_CHECK_CUDA(cudaMalloc(&n->d_loss, sizeof(double)));
             }
             n->fast = tc_applicable(nx, ny, C);
             if (n->fast) {
@@ -911,10 +909,7 @@ int lgd_net_forward(lgd_net *h, const float *d_u, const float *d_kappa, float *d
     return guard([&] {
         Net& n = net_of(h);
         LGD_REQUIRE(d_u && d_kappa, LGD_ERR_INVALID, "null input");
-        forward(n, d_u, d_kappa, d_du ? d_du : n.du);
-        if (d_du && n.training) {
-            LGD_CHECK_CUDA(cudaMemcpyAsync(n.du, d_du, sizeof(float) * n.V, cudaMemcpyDeviceToDevice, n.stream));
-        }
+        forward(n, d_u, d_kappa, d_du ? d_du : n.du, false, d_du && n.training ? n.du : nullptr);
     });
 }
 

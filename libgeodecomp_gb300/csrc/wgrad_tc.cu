@@ -86,6 +86,8 @@ struct WParams {
     const bf16 *dz;             // CC, FL: ghosted
     const float *du, *target;   // LL
     float scale;                // LL: 2 / N
+    double *loss;               // LL: the sum of (du - target)^2, added to
+    float *db;                  // LL: the bias gradient, added to
     float *part;                // [gridDim.x][OUT]
     int *err;
 };
@@ -261,6 +263,8 @@ wgrad_tc_kernel(const WParams p)
                 }
             }
         };
+        double loss = 0.0;
+        float db = 0.f;
         if (blockIdx.x < p.items) fetch(item_of(blockIdx.x), 0);
         for (int it = blockIdx.x; ok && it < p.items; it += gridDim.x) {
             const Item t = item_of(it);
@@ -320,6 +324,9 @@ wgrad_tc_kernel(const WParams p)
                             if (in) {
                                 g.x = pack_bf16(p.scale * (ng[i][0] - ng[i][1]), p.scale * (ng[i][2] - ng[i][3]));
                                 g.y = pack_bf16(p.scale * (ng[i][4] - ng[i][5]), 0.f);
+                                const float e = ng[i][2] - ng[i][3];
+                                loss = fma((double)e, (double)e, loss);
+                                db += p.scale * e;
                             }
                             st_shared16(d, g);
                         } else {
@@ -347,6 +354,16 @@ wgrad_tc_kernel(const WParams p)
         asm volatile("cp.async.wait_all;" ::: "memory");
         if (ok) publish(plane);
         else if (lane == 0) s_fail = 1;
+        if (MODE == LL) {
+            for (int o = 16; o > 0; o >>= 1) {
+                loss += __shfl_xor_sync(0xffffffffu, loss, o);
+                db += __shfl_xor_sync(0xffffffffu, db, o);
+            }
+            if (lane == 0) {
+                atomicAdd(p.loss, loss);
+                atomicAdd(p.db, db);
+            }
+        }
     } else {
         // the four warps between: lane quarter warp % 4
         const int qd = warp & 3;
@@ -512,7 +529,7 @@ size_t tc_partial_floats()
 }
 
 int tc_wgrad(int layer, const void *h, const void *x0, const void *dz, const float *du, const float *target, float scale,
-             float *partials, const int dims[4], int *err, cudaStream_t stream)
+             double *loss, float *db, float *partials, const int dims[4], int *err, cudaStream_t stream)
 {
     WParams p = {};
     p.s = {dims[0], dims[1], dims[2], dims[3]};
@@ -522,6 +539,8 @@ int tc_wgrad(int layer, const void *h, const void *x0, const void *dz, const flo
     p.du = du;
     p.target = target;
     p.scale = scale;
+    p.loss = loss;
+    p.db = db;
     size_t off = 0;
     for (int l = 0; l < layer; ++l) off += (size_t)sm_count() * DW[l];
     p.part = partials + off;
