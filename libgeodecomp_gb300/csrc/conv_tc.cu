@@ -570,8 +570,20 @@ conv_tc_kernel(const Params p)
 // output channel: columns 0, 1, 2 are the accumulators, one copy per rotation.
 // W: FP32 [tap][cin][cout]; mirror: the input-gradient convolution (taps
 // mirrored, channel roles swapped).
-__global__ void pack_kernel(const float *w, bf16 *out, int src, int mirror)
+struct PackJobs {               // by blockIdx.y
+    struct Job {
+        const float *w;
+        bf16 *out;
+        int src, mirror;
+    } job[7];
+};
+
+__global__ void pack_kernel(const PackJobs jobs)
 {
+    const PackJobs::Job& job = jobs.job[blockIdx.y];
+    const float *w = job.w;
+    bf16 *out = job.out;
+    const int src = job.src, mirror = job.mirror;
     const int ksteps = src == MID || src == LAST ? 14 : 2;
     const int ng = src == LAST ? 2 : 16;
     const int copies = src == LAST ? 3 : 1;
@@ -697,19 +709,16 @@ TcWeights tc_alloc_weights(bool training)
 
 void tc_free_weights(TcWeights& w) { cudaFree(w.base); }
 
-int tc_pack_weights(const float *const layer[4], const TcWeights& w, cudaStream_t stream)
+void tc_pack_weights(const float *const layer[4], const TcWeights& w, cudaStream_t stream)
 {
     const int src[4] = {FIRST, MID, MID, LAST};
-    int launches = 0;
-    for (int l = 0; l < 4; ++l, ++launches) pack_kernel<<<56, 256, 0, stream>>>(layer[l], (bf16 *)w.fwd[l], src[l], 0);
-    if (w.grad[1]) {
-        const int gsrc[4] = {0, MID, MID, DLAST};
-        for (int l = 1; l < 4; ++l, ++launches) {
-            pack_kernel<<<56, 256, 0, stream>>>(layer[l], (bf16 *)w.grad[l], gsrc[l], 1);
-        }
-    }
+    const int gsrc[4] = {0, MID, MID, DLAST};
+    PackJobs jobs;
+    int n = 0;
+    for (int l = 0; l < 4; ++l) jobs.job[n++] = {layer[l], (bf16 *)w.fwd[l], src[l], 0};
+    for (int l = 1; l < 4 && w.grad[1]; ++l) jobs.job[n++] = {layer[l], (bf16 *)w.grad[l], gsrc[l], 1};
+    pack_kernel<<<dim3(56, n), 256, 0, stream>>>(jobs);
     check_launch("pack tensor-core weights");
-    return launches;
 }
 
 size_t tc_ghost_bytes(int nx, int ny, int nz, int batch)

@@ -20,7 +20,7 @@ bool tc_applicable(int nx, int ny, int channels);
 size_t tc_ghost_bytes(int nx, int ny, int nz, int batch);
 TcWeights tc_alloc_weights(bool training);
 void tc_free_weights(TcWeights& w);
-int tc_pack_weights(const float *const layer[4], const TcWeights& w, cudaStream_t stream);   // launches made
+void tc_pack_weights(const float *const layer[4], const TcWeights& w, cudaStream_t stream);
 
 // layer 1 (u, kappa -> 24), layers 2 and 3 (24 -> 24): ghosted BF16 output;
 // gelu_grad (or null) receives GELU' of the pre-activations for the backward

@@ -376,9 +376,20 @@ __global__ void add_inplace_kernel(float *__restrict__ u, const float *__restric
 // Fragment packing.  Forward: B[k][n] = W[k][n] (W flat [27 * CIN][COUT]).
 // Input-gradient convolution: CIN' = COUTP, COUT' = CIN,
 // B'[k'][n'] = W[((26 - tap') * CIN + n') * COUT + co] with k' = tap' * CIN' + co.
-__global__ void pack_frag_kernel(const float *__restrict__ w, uint2 *__restrict__ frag, int cin, int cout, int mirror,
-                                 int cin_eff, int cout_eff)
+struct FragJobs {               // by blockIdx.y
+    struct Job {
+        const float *w;
+        uint2 *frag;
+        int cin, cout, mirror, cin_eff, cout_eff;
+    } job[8];
+};
+
+__global__ void pack_frag_kernel(const FragJobs jobs)
 {
+    const FragJobs::Job& job = jobs.job[blockIdx.y];
+    const float *w = job.w;
+    uint2 *frag = job.frag;
+    const int cin = job.cin, cout = job.cout, mirror = job.mirror, cin_eff = job.cin_eff, cout_eff = job.cout_eff;
     // cin_eff / cout_eff: the convolution's own channel counts (K = 27 * cin_eff)
     const int K = 27 * cin_eff;
     const int KS = (K + 15) / 16;
@@ -461,6 +472,7 @@ struct Net {
     // tensor-core (tcgen05) path: C = 24 (conv_tc.cu, wgrad_tc.cu)
     bool fast;
     bool fast_forward;  // the last forward pass took it (the backward pass follows)
+    bool frag_stale, tc_stale;  // packed weights older than params
     int variant;        // 0: tcgen05 path where it applies; 1: mma.sync for every layer
     void *hg[3];        // ghosted activations (two without training)
     void *dzg[2];       // ghosted gradients (training)
@@ -526,21 +538,35 @@ static int grid_blocks(long long n)
     return (int)std::min<long long>(b, 152LL * 16);
 }
 
-static void repack(Net& n)
+// The weights as the operands of the path that runs (fast: tcgen05, else
+// mma.sync), after they have changed.  The other path's are packed when it runs.
+static void ensure_packed(Net& n, bool fast)
 {
-    for (int l = 0; l < 4; ++l) {
-        Layer& L = n.L[l];
-        pack_frag_kernel<<<64, 256, 0, n.stream>>>(n.params + L.w_off, L.frag, L.cin, L.cout, 0, L.cin, L.cout);
-        const int coutp = (L.cout + 1) & ~1;
-        pack_frag_kernel<<<64, 256, 0, n.stream>>>(n.params + L.w_off, L.frag_t, L.cin, L.cout, 1, coutp, L.cin);
-        n.launches += 2;
-    }
-    check_launch("pack fragments");
-    if (n.fast) {
+    bool& stale = fast ? n.tc_stale : n.frag_stale;
+    if (!stale) return;
+    if (fast) {
         const float *w[4];
         for (int l = 0; l < 4; ++l) w[l] = n.params + n.L[l].w_off;
-        n.launches += tc_pack_weights(w, n.wtc, n.stream);
+        tc_pack_weights(w, n.wtc, n.stream);
+    } else {
+        FragJobs jobs;
+        for (int l = 0; l < 4; ++l) {
+            Layer& L = n.L[l];
+            const int coutp = (L.cout + 1) & ~1;
+            jobs.job[2 * l] = {n.params + L.w_off, L.frag, L.cin, L.cout, 0, L.cin, L.cout};
+            jobs.job[2 * l + 1] = {n.params + L.w_off, L.frag_t, L.cin, L.cout, 1, coutp, L.cin};
+        }
+        pack_frag_kernel<<<dim3(64, 8), 256, 0, n.stream>>>(jobs);
+        check_launch("pack fragments");
     }
+    ++n.launches;
+    stale = false;
+}
+
+static void repack(Net& n)
+{
+    n.frag_stale = n.tc_stale = true;
+    ensure_packed(n, n.fast && n.variant == 0);
 }
 
 // waits for the stream, then reports (and clears) a wait that gave up
@@ -675,6 +701,7 @@ static void backward_impl(Net& n, const float *target, double *loss_out)
 static bool forward(Net& n, const float *u, const float *k, float *du, bool add_to_u = false, float *copy = nullptr)
 {
     n.fast_forward = n.fast && n.variant == 0;
+    ensure_packed(n, n.fast_forward);
     if (n.fast_forward) {
         forward_fast(n, u, k, du, add_to_u, copy);
         return add_to_u;
@@ -691,6 +718,7 @@ static bool forward(Net& n, const float *u, const float *k, float *du, bool add_
 
 static void backward(Net& n, const float *target, double *loss)
 {
+    ensure_packed(n, n.fast_forward);
     if (n.fast_forward) {
         backward_fast(n, target, loss);
         return;

@@ -93,3 +93,32 @@ def test_batches_are_sums_of_their_samples(shape, batch):
         # the loss gradient is rounded to BF16 at another scale: 2^-8 relative
         # per voxel, averaged over the sums
         assert np.linalg.norm(a - b) / np.linalg.norm(b) < 1e-2
+
+
+@pytest.mark.parametrize("order", [(0, 1), (1, 0)])
+def test_changed_weights_reach_either_path(order):
+    """A path that did not run while the parameters changed packs them when
+    it does: the same output as a network that had them from the start."""
+    from libgeodecomp_gb300.surrogate import SurrogateNet
+    shape = (4, 8, 64)
+    u, k, target, p = inputs(shape, 1, 3)
+    t = [torch.tensor(a, dtype=torch.float32, device="cuda").contiguous() for a in (u, k, target)]
+    du = torch.empty_like(t[0])
+    torch.cuda.synchronize()
+    with SurrogateNet(shape, channels=24, training=True) as net:
+        net.set_variant(order[0])
+        net.set_params(p.astype(np.float32))
+        net.forward(t[0], t[1], du)
+        net.backward(t[2])
+        net.adam(0.01)
+        net.set_variant(order[1])
+        net.forward(t[0], t[1], du)
+        net.synchronize()
+        out, changed = du.cpu().numpy(), net.get_params()
+    assert np.max(np.abs(changed - p)) > 5e-3
+    with SurrogateNet(shape, channels=24) as net:
+        net.set_variant(order[1])
+        net.set_params(changed)
+        net.forward(t[0], t[1], du)
+        net.synchronize()
+        np.testing.assert_array_equal(out, du.cpu().numpy())
