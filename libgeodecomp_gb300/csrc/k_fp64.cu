@@ -1,4 +1,5 @@
-// Whole-grid kernel of the IEEE FP64 Jacobi-7 cell on cube grids.
+// Whole-grid kernel of the IEEE FP64 Jacobi-7 cell, for any edge value and any
+// axes that wrap.
 //
 // GB300's FP64 pipe bounds this cell, not memory and not issue: a chain of
 // independent additions measured 498 G operations per second on the whole
@@ -24,7 +25,8 @@
 // Measured (us per step; in brackets the kernel without sum4, then the TMA
 // kernel of k_tma.cu): 24 x 20 x 16 1.9 (2.2, 22.6), 64^3 4.0 (5.9, 22.6), 128^3
 // 17.1 (25.4, 38.9), 512^3 886 (1598, 1795): 151 GLUPS, 91% of the FP64 pipe's
-// rate at three operations per cell.
+// rate at three operations per cell.  On a torus, against the register kernel:
+// 64^3 4.3 (45), 128^3 18.9 (51), 512^3 1026 (1850).
 // The sum's order is the cell's own: results are bit-identical to every
 // other kernel of the cell.
 #include <algorithm>
@@ -39,9 +41,11 @@ namespace fp64k {
 constexpr int THREADS = 128;
 constexpr int CTAS = 8;        // per SM: 64 registers
 
+// WRAP: some axis wraps (a cube of 512^3 takes 886 us without, 1030 with)
+template<bool WRAP>
 __global__ void __launch_bounds__(THREADS, CTAS)
 jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, int nz,
-                   int zchunk, double edge)
+                   int zchunk, double edge, int periodic)
 {
     dependent_start();
     const unsigned cells = (unsigned)nx * (unsigned)ny;         // below 2^31 (host rule)
@@ -52,19 +56,25 @@ jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, in
     const int z0 = blockIdx.y * zchunk;
     const int z1 = min(z0 + zchunk, nz);
     const long plane = pitch * ny;
-    const bool has_n = y > 0, has_s = y + 1 < ny, has_w = x > 0, has_e = x + 1 < nx;
+    // the neighbours in the plane: a fixed distance, around the torus at its
+    // ends, or the edge value
+    const bool wrap_x = WRAP && (periodic & 1), wrap_y = WRAP && (periodic & 2), wrap_z = WRAP && (periodic & 4);
+    const bool has_n = wrap_y || y > 0, has_s = wrap_y || y + 1 < ny;
+    const bool has_w = wrap_x || x > 0, has_e = wrap_x || x + 1 < nx;
+    const long north = !WRAP || y > 0 ? -pitch : (ny - 1) * pitch, south = !WRAP || y + 1 < ny ? pitch : -(ny - 1) * pitch;
+    const int west = !WRAP || x > 0 ? -1 : nx - 1, east = !WRAP || x + 1 < nx ? 1 : 1 - nx;
     const bool drop_e = !has_e && edge == 0.0;      // the sum of the others is not zero where it is taken
     const double *p = in + (long)z0 * plane + (long)y * pitch + x;
     double *o = out + (long)z0 * plane + (long)y * pitch + x;
-    double b = z0 > 0 ? *(p - plane) : edge;
+    double b = z0 > 0 ? *(p - plane) : (wrap_z ? *(p + (nz - 1) * plane) : edge);
     double m = *p;
 #pragma unroll 1
     for (int z = z0; z < z1; ++z) {
-        const double t = z + 1 < nz ? *(p + plane) : edge;
-        const double n = has_n ? *(p - pitch) : edge;
-        const double s = has_s ? *(p + pitch) : edge;
-        const double e = has_e ? *(p + 1) : edge;
-        const double w = has_w ? *(p - 1) : edge;
+        const double t = z + 1 < nz ? *(p + plane) : (wrap_z ? *(p - (nz - 1) * plane) : edge);
+        const double n = has_n ? *(p + north) : edge;
+        const double s = has_s ? *(p + south) : edge;
+        const double e = has_e ? *(p + east) : edge;
+        const double w = has_w ? *(p + west) : edge;
         double acc;
         if (!sum4(m, n, s, e, drop_e, acc)) {
             acc = m;
@@ -84,11 +94,11 @@ jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, in
 
 }  // namespace fp64k
 
-// The rule: IEEE Jacobi on a cube (any edge value) whose plane fits 32-bit
-// numbering.  The TMA kernel keeps larger planes.
+// The rule: IEEE Jacobi whose plane fits 32-bit numbering.  The TMA kernel (cube,
+// zero edge) and the register kernels keep larger planes.
 bool jacobi7_f64_applicable(const Grid& g)
 {
-    return g.desc.cell == LGD_CELL_JACOBI7_F64 && g.desc.periodic == 0 &&
+    return g.desc.cell == LGD_CELL_JACOBI7_F64 &&
            (long long)g.desc.nx * g.desc.ny < (1ll << 31) - fp64k::THREADS;
 }
 
@@ -113,8 +123,8 @@ void launch_jacobi7_f64(Grid& g)
     zchunk = std::max(zchunk, (g.desc.nz + 65534) / 65535);
     const dim3 grid((unsigned)xy, (unsigned)((g.desc.nz + zchunk - 1) / zchunk));
     launch_dependent(
-        fp64k::jacobi7_f64_kernel, grid, fp64k::THREADS, 0, g.stream, (const double *)g.m[0].buf[g.cur], (double *)g.m[0].buf[1 - g.cur], (long)(g.pitch_bytes[0] / 8), g.desc.nx,
-        g.desc.ny, g.desc.nz, zchunk, g.desc.edge[0]);
+        g.desc.periodic & 7 ? fp64k::jacobi7_f64_kernel<true> : fp64k::jacobi7_f64_kernel<false>, grid, fp64k::THREADS, 0, g.stream, (const double *)g.m[0].buf[g.cur], (double *)g.m[0].buf[1 - g.cur], (long)(g.pitch_bytes[0] / 8), g.desc.nx,
+        g.desc.ny, g.desc.nz, zchunk, g.desc.edge[0], g.desc.periodic);
     check_launch("jacobi7 f64");
     ++g.launches;
     g.cur = 1 - g.cur;

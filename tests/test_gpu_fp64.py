@@ -11,8 +11,8 @@ from libgeodecomp_gb300 import lgd, workloads
 pytestmark = pytest.mark.gpu
 
 
-def run(u0, steps, edge=0.0):
-    with lgd.Grid(lgd.CELL_JACOBI7_F64, u0.shape, edge=(edge, 0, 0, 0)) as g:
+def run(u0, steps, edge=0.0, periodic=0):
+    with lgd.Grid(lgd.CELL_JACOBI7_F64, u0.shape, periodic=periodic, edge=(edge, 0, 0, 0)) as g:
         g.upload(0, u0)
         g.step(steps)
         return g.download(0)
@@ -53,3 +53,22 @@ def test_exponent_distances(reach, shape):
             u0 *= np.where(rng.random(shape) < 0.02, -1.0, 1.0)
         np.testing.assert_array_equal(run(u0, 1).view(np.uint64), oracle.jacobi7(u0, 1).view(np.uint64))
         np.testing.assert_array_equal(run(-u0, 4), oracle.jacobi7(-u0, 4))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 127), (3, 2, 1), (2, 16, 8), (17, 1, 129), (9, 33, 31), (130, 96, 64)])
+def test_torus(shape):
+    u0 = workloads.jacobi_initial(shape[2], shape[1], shape[0], seed=52)
+    np.testing.assert_array_equal(run(u0, 5, periodic=7), oracle.jacobi7(u0, 5, torus=True))
+
+
+@pytest.mark.parametrize("periodic", [1, 2, 3, 4, 5, 6])
+@pytest.mark.parametrize("shape", [(4, 7, 33), (2, 3, 40)])
+def test_some_axes_wrap(periodic, shape):
+    """A grid that wraps along some axes only, against one extended along
+    them by as many cells as steps."""
+    steps = 3
+    u0 = workloads.jacobi_initial(shape[2], shape[1], shape[0], seed=53)
+    pad = [(steps, steps) if periodic >> axis & 1 else (0, 0) for axis in (2, 1, 0)]
+    inner = tuple(slice(a, a + n) for (a, _), n in zip(pad, shape))
+    ref = oracle.jacobi7(np.pad(u0, pad, mode="wrap"), steps, edge=0.25)[inner]
+    np.testing.assert_array_equal(run(u0, steps, edge=0.25, periodic=periodic), ref)
