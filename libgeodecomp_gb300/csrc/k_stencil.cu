@@ -690,14 +690,19 @@ varcoef_pair_kernel(View<const R> u, View<const R> k, View<R> out, int periodic,
 
 void launch_varcoef(Grid& g, int steps)
 {
-    // default: the TMA kernel for FP32 cells (HBM-bound); FP64 cells are
-    // bound by the FP64 rate, where the register kernel measured faster
+    // default: two steps per pass for FP32 cells on a full torus, then the TMA
+    // kernel where it takes the grid; one cell of a plane per thread for other
+    // FP32 grids and for FP64
     const bool tma = (g.variant == 6) || (g.variant == 0 && g.desc.cell == LGD_CELL_VARCOEF_F32);
     if (g.variant == 0 && g.time_block != 1 && varcoef_tb2_applicable(g)) {
         for (; steps >= 2; steps -= 2) launch_varcoef_tb2(g);
     }
     if (tma && varcoef_tma_applicable(g)) {
         for (int s = 0; s < steps; ++s) launch_varcoef_tma(g);
+        return;
+    }
+    if (g.variant == 0 && varcoef_plane_applicable(g)) {
+        for (int s = 0; s < steps; ++s) launch_varcoef_plane(g);
         return;
     }
     if (g.variant != 1) {

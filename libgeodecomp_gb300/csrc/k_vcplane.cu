@@ -1,0 +1,175 @@
+// Variable-coefficient diffusion, one cell of a plane per thread: FP64 grids of
+// any shape and boundary, and the FP32 grids that no tiled kernel takes (rows not
+// a multiple of 16 bytes, axes that do not wrap).
+//
+// The cells of a plane are numbered through, so no lane idles whatever nx is, and
+// a thread marches a few planes with u and k of the centre and top in registers;
+// the neighbours in the plane are L1 hits.  A grid falls into as many small CTAs
+// as give every SM an even share.
+//
+// FP64 is bound by the FP64 pipe, so the cell's 30 operations become 21, bit for
+// bit: the face to the plane below is the exact negative of the face the thread
+// took to its top neighbour one plane earlier (4 operations, and a sum does not
+// see the sign of a zero), and the multiplication of k + k' by 1/2 is a
+// subtraction from the exponent (5 of them).  Where an exponent is at the range's
+// ends (k + k' zero, subnormal, infinite, NaN) the cell is computed as written.
+//
+// us per step, against the pair kernel of k_stencil.cu before (two x cells per
+// lane, whose blocks at a grid's ragged end loaded cell by cell): FP64 24^3 3.4
+// (159), 64^3 14.4 (70), 101 x 77 x 60 24 (246), 128^3 89 (133), 256^3 685 (888;
+// 24.5 GLUPS x 21 operations = 514 G/s, the pipe's rate); FP32 101 x 77 x 60 4.3
+// (162), 253 x 250 x 250 68 (517).
+#include <algorithm>
+
+#include "lgd_internal.h"
+#include "k_cells.cuh"
+#include "k_common.cuh"
+
+namespace lgd {
+namespace vcp {
+
+constexpr int THREADS = 128;
+
+// x / 2 by the exponent; ok becomes false where that is not the rounded product
+__device__ __forceinline__ double half_of(double x, bool& ok)
+{
+    const unsigned hi = (unsigned)__double2hiint(x);
+    const unsigned e = hi & 0x7ff00000u;
+    ok = ok && e - 0x00200000u < 0x7fd00000u;               // exponents 2 .. 2046
+    return __hiloint2double((int)(hi - 0x00100000u), __double2loint(x));
+}
+
+// the cell as written (a call: predicated, its operations would be paid always)
+__device__ __noinline__ double plain(double uc, double kc, double uw, double kw, double ue, double ke, double un, double kn,
+                                     double us, double ks, double ub, double kb, double ut, double kt)
+{
+    return VarCoef<double>::apply(uc, kc, uw, kw, ue, ke, un, kn, us, ks, ub, kb, ut, kt);
+}
+
+__device__ __noinline__ double plain_face(double uc, double kc, double un, double kn)
+{
+    return VarCoef<double>::face(uc, kc, un, kn);
+}
+
+template<typename R>
+struct Args {
+    const R *u, *k;
+    R *out;
+    long pitch;
+    int nx, ny, nz, zchunk, periodic;
+    R edge_u, edge_k;
+};
+
+template<typename R>
+__global__ void __launch_bounds__(THREADS, sizeof(R) == 8 ? 6 : 8)
+varcoef_plane_kernel(const Args<R> a)
+{
+    dependent_start();
+    const int nx = a.nx, ny = a.ny, nz = a.nz;
+    const unsigned c = blockIdx.x * THREADS + threadIdx.x;
+    if (c >= (unsigned)nx * (unsigned)ny) return;           // below 2^31 (host rule)
+    const int y = (int)(c / (unsigned)nx);
+    const int x = (int)(c - (unsigned)y * (unsigned)nx);
+    const int z0 = blockIdx.y * a.zchunk;
+    const int z1 = min(z0 + a.zchunk, nz);
+    const long plane = a.pitch * ny;
+    const bool wrap_z = a.periodic & 4;
+    const bool has_w = x > 0 || (a.periodic & 1), has_e = x + 1 < nx || (a.periodic & 1);
+    const bool has_n = y > 0 || (a.periodic & 2), has_s = y + 1 < ny || (a.periodic & 2);
+    const int west = x > 0 ? -1 : nx - 1, east = x + 1 < nx ? 1 : 1 - nx;
+    const long north = y > 0 ? -a.pitch : (ny - 1) * a.pitch, south = y + 1 < ny ? a.pitch : -(ny - 1) * a.pitch;
+    const long at = (long)z0 * plane + (long)y * a.pitch + x;
+    const R *u = a.u + at, *k = a.k + at;
+    R *o = a.out + at;
+    R uc = *u, kc = *k, ub, kb;
+    {
+        const bool has = z0 > 0 || wrap_z;
+        const long d = z0 > 0 ? -plane : (nz - 1) * plane;
+        ub = has ? u[d] : a.edge_u;
+        kb = has ? k[d] : a.edge_k;
+    }
+    R fb = 0;                                               // FP64: the face from the plane below to this one
+    if constexpr (sizeof(R) == 8) fb = VarCoef<R>::face(ub, kb, uc, kc);
+#pragma unroll 1
+    for (int z = z0; z < z1; ++z) {
+        const bool has = z + 1 < nz || wrap_z;
+        const long d = z + 1 < nz ? plane : -(nz - 1) * plane;
+        const R ut = has ? u[d] : a.edge_u, kt = has ? k[d] : a.edge_k;
+        const R un = has_n ? u[north] : a.edge_u, kn = has_n ? k[north] : a.edge_k;
+        const R us = has_s ? u[south] : a.edge_u, ks = has_s ? k[south] : a.edge_k;
+        const R ue = has_e ? u[east] : a.edge_u, ke = has_e ? k[east] : a.edge_k;
+        const R uw = has_w ? u[west] : a.edge_u, kw = has_w ? k[west] : a.edge_k;
+        R r;
+        if constexpr (sizeof(R) == 8) {
+            bool ok = true;
+            auto face = [&](double un, double kn) {
+                return __dmul_rn(half_of(__dadd_rn(kc, kn), ok), __dadd_rn(un, -uc));
+            };
+            double flux = face(uw, kw);
+            flux = __dadd_rn(flux, face(ue, ke));
+            flux = __dadd_rn(flux, face(un, kn));
+            flux = __dadd_rn(flux, face(us, ks));
+            flux = __dadd_rn(flux, -fb);
+            double ft = face(ut, kt);
+            r = __dadd_rn(uc, __dadd_rn(flux, ft));
+            if (!ok) {
+                r = plain(uc, kc, uw, kw, ue, ke, un, kn, us, ks, ub, kb, ut, kt);
+                ft = plain_face(uc, kc, ut, kt);
+            }
+            fb = ft;
+        } else {
+            r = VarCoef<R>::apply(uc, kc, uw, kw, ue, ke, un, kn, us, ks, ub, kb, ut, kt);
+        }
+        *o = r;
+        ub = uc;
+        kb = kc;
+        uc = ut;
+        kc = kt;
+        u += plane;
+        k += plane;
+        o += plane;
+    }
+}
+
+// Planes per thread: 8 re-read least, fewer until there are 10 CTAs per SM.  us per
+// step with 1, 2, 4, 8 planes, FP64: 64^3 14.4, 13.5, 21.6, 39.4; 120 x 96 x 100
+// 56.7, 52.3, 50.3, 53.2; 256^3 796, 732, 701, 685; FP32 101 x 77 x 60 5.1, 4.3,
+// 5.3, 5.6; 130 x 128 x 128 18.2, 12.4, 10.8, 10.7.
+template<typename R>
+static void launch(Grid& g, int sms)
+{
+    const long long xy = ((long long)g.desc.nx * g.desc.ny + THREADS - 1) / THREADS;
+    int zchunk = 8;
+    while (zchunk > 1 && xy * ((g.desc.nz + zchunk - 1) / zchunk) < 10LL * sms) zchunk /= 2;
+    zchunk = std::max(zchunk, (g.desc.nz + 65534) / 65535);
+    const Args<R> a = {(const R *)g.m[0].buf[g.cur], (const R *)g.m[1].buf[0], (R *)g.m[0].buf[1 - g.cur],
+                       (long)(g.pitch_bytes[0] / sizeof(R)), g.desc.nx, g.desc.ny, g.desc.nz, zchunk, g.desc.periodic,
+                       (R)g.desc.edge[0], (R)g.desc.edge[1]};
+    launch_dependent(varcoef_plane_kernel<R>, dim3((unsigned)xy, (unsigned)((g.desc.nz + zchunk - 1) / zchunk)), THREADS, 0,
+                     g.stream, a);
+}
+
+}  // namespace vcp
+
+bool varcoef_plane_applicable(const Grid& g)
+{
+    return (long long)g.desc.nx * g.desc.ny < (1ll << 31) - vcp::THREADS && g.pitch_bytes[0] == g.pitch_bytes[1];
+}
+
+void launch_varcoef_plane(Grid& g)
+{
+    static PerDevice<int> setup;
+    const int sms = setup.get([] {
+        int dev = 0, count = 0;
+        LGD_CHECK_CUDA(cudaGetDevice(&dev));
+        LGD_CHECK_CUDA(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev));
+        return count;
+    });
+    if (g.desc.cell == LGD_CELL_VARCOEF_F32) vcp::launch<float>(g, sms);
+    else vcp::launch<double>(g, sms);
+    check_launch("varcoef plane");
+    ++g.launches;
+    g.cur = 1 - g.cur;
+}
+
+}  // namespace lgd

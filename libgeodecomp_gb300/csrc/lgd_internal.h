@@ -213,6 +213,10 @@ void launch_varcoef_tma(Grid& g);
 // two var-coef steps per pass (k_vctb.cu)
 bool varcoef_tb2_applicable(const Grid& g);
 void launch_varcoef_tb2(Grid& g);
+
+// k_vcplane.cu: variable-coefficient diffusion, one cell of a plane per thread
+bool varcoef_plane_applicable(const Grid& g);
+void launch_varcoef_plane(Grid& g);
 // temporal blocking (k_tb.cu): depth time steps per pass, 2 .. LGD_TB_MAX_DEPTH
 bool tb_applicable(const Grid& g);
 int tb_default_depth(const Grid& g);

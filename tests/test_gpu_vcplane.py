@@ -1,0 +1,61 @@
+"""The one-cell-per-thread var-coef kernel (csrc/k_vcplane.cu): FP64 bit for bit
+against the oracle on tori and against the kernel of variant 1 for every set of
+wrapping axes and edge values, with coefficients and fields at the ends of the
+exponent range; FP32 grids of ragged rows against variant 1."""
+import numpy as np
+import pytest
+
+import oracle
+from libgeodecomp_gb300 import lgd
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1, 127), (3, 2, 1), (2, 16, 8), (17, 1, 129), (9, 33, 31), (40, 20, 66)]
+
+
+def run(cell, u, k, steps, variant, periodic, edge=(0.0, 0.0, 0.0, 0.0)):
+    with lgd.Grid(cell, u.shape, periodic=periodic, edge=edge) as g:
+        g.set_variant(variant)
+        g.upload(0, u)
+        g.upload(1, k)
+        g.step(steps)
+        return g.download(0)
+
+
+def fields(shape, seed):
+    rng = np.random.default_rng(seed)
+    return rng.random(shape), 0.02 + 0.13 * rng.random(shape)
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_fp64_torus_matches_oracle(shape):
+    u, k = fields(shape, 1)
+    np.testing.assert_array_equal(run(lgd.CELL_VARCOEF_F64, u, k, 5, 0, 7), oracle.varcoef(u, k, 5))
+
+
+@pytest.mark.parametrize("periodic", range(8))
+@pytest.mark.parametrize("shape", [(5, 9, 33), (12, 7, 130)])
+def test_fp64_any_boundary(periodic, shape):
+    u, k = fields(shape, 2)
+    edge = (0.3, 0.07, 0.0, 0.0)
+    np.testing.assert_array_equal(run(lgd.CELL_VARCOEF_F64, u, k, 4, 0, periodic, edge),
+                                  run(lgd.CELL_VARCOEF_F64, u, k, 4, 1, periodic, edge))
+
+
+@pytest.mark.parametrize("scale", [0.0, 5e-324, 1e-308, 4.5e-308, 1e-300, 1e300, 8e307, np.inf])
+def test_fp64_coefficients_at_the_ends_of_the_range(scale):
+    u, k = fields((4, 6, 40), 3)
+    k[1:3, 2:, ::3] = scale
+    u[2, :, 5] = -u[2, :, 5]
+    u[0] = 0.5
+    np.testing.assert_array_equal(run(lgd.CELL_VARCOEF_F64, u, k, 2, 0, 7), run(lgd.CELL_VARCOEF_F64, u, k, 2, 1, 7))
+
+
+@pytest.mark.parametrize("periodic", [0, 5, 7])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_fp32_ragged_rows(periodic, shape):
+    """Three steps of sums of 14 terms below one: within 40 roundings."""
+    u, k = (a.astype(np.float32) for a in fields(shape, 4))
+    edge = (0.25, 0.05, 0.0, 0.0)
+    np.testing.assert_allclose(run(lgd.CELL_VARCOEF_F32, u, k, 3, 0, periodic, edge),
+                               run(lgd.CELL_VARCOEF_F32, u, k, 3, 1, periodic, edge), rtol=0, atol=40 * 2.0 ** -24)
