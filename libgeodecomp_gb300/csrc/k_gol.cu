@@ -1,8 +1,10 @@
 // Game of Life on uint8 cells (one byte per cell, 0 or 1), Moore radius 1.
 //
-// Default path (torus, nx a multiple of 16): temporal blocking, several
-// generations per pass (gol_tb_kernel below).  Single-generation fast path
-// (the same conditions): SWAR on 32-bit words.  A thread
+// The kernels on byte rows: single generations, and the passes that an explicit
+// depth selects (gol_bits_kernel, gol_tb_kernel below).  Calls of more than a few
+// generations run on packed rows by default (k_golpack.cu).
+//
+// Single generation (torus, nx a multiple of 16): SWAR on 32-bit words.  A thread
 // owns 16 consecutive cells of one row (one 16-byte load per row for the
 // rows above, at and below) plus the 4-byte words left and right of them.
 // Column sums of the three rows are formed per byte lane (values <= 3),

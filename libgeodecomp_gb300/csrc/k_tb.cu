@@ -409,11 +409,12 @@ bool tb_applicable(const Grid& g)
 }
 
 // Default depth per cell, measured at 512^3 on GB300: FP32 (packed pairs)
-// 754 GLUPS at depth 1, 932 at 2, 1100 at 3 (16x4), 1026 at 4; fixed point
-// 403 at depth 1 (95% of HBM
-// bandwidth), 482 at depth 2 with exact two-step sums (a pass of two
+// 754 GLUPS at depth 1, 1226 at 3; fixed point 409 at depth 1 (97% of HBM
+// bandwidth), 557 at depth 2 with exact two-step sums (a pass of two
 // single-rounding steps took as long as two HBM-bound single steps: the
-// per-step division by 7 costs a 64-bit multiply-high).
+// per-step division by 7 costs a 64-bit multiply-high).  Before two CTAs of 8
+// warps shared an SM the depths measured, FP32, 932 (2), 1100 (3), 1026 (4),
+// fixed point 482 (2).
 int tb_default_depth(const Grid& g)
 {
     return g.desc.cell == LGD_CELL_JACOBI7_F32 ? 3 : 2;

@@ -1,5 +1,6 @@
-// Jacobi-7 with TMA-fed shared-memory planes (default whole-grid kernel on
-// cube grids whose edge cell is zero - the Jacobi configuration).
+// Jacobi-7 with TMA-fed shared-memory planes: single steps of the FP32 and
+// fixed-point cells on cube grids whose edge cell is zero (several steps per
+// pass: k_tb.cu; the IEEE FP64 cell: k_fp64.cu).
 //
 // A CTA owns a 64 x 16 tile of every z plane of its z chunk.  One thread
 // issues cp.async.bulk.tensor loads of the tile plus its one-cell rim

@@ -4,6 +4,10 @@
 // its forward pass, backward pass and Adam update as hand-written kernels.
 // No counterpart in the reference library.
 //
+// With C = 24 all layers, input gradients and weight gradients run on tcgen05
+// (conv_tc.cu, wgrad_tc.cu; forward_fast and backward_fast below).  The kernels
+// of this file serve C = 8 and variant 1:
+//
 // Convolutions are implicit GEMMs on the tensor cores (mma.sync
 // m16n8k16, BF16 operands, FP32 accumulation): one CTA computes a
 // TX x 4 x 1 tile of output voxels; the input halo (TX+2) x 6 x 3 voxels x
@@ -16,8 +20,8 @@
 // mirrored and the channel roles swapped (weights re-packed); the weight
 // gradient is a GEMM over the voxels of a tile (M = 27 * CIN, N = COUT,
 // K = voxels) accumulated in FP32 and added to the global gradient with
-// atomics.  Parameters stay in FP32 (master copy), Adam runs in FP32 and
-// re-packs the BF16 fragments after every update.
+// atomics.  Parameters stay in FP32 (master copy), Adam runs in FP32 and the
+// BF16 operands of the path in use are packed again after every update.
 #include <cuda_bf16.h>
 
 #include <cmath>
