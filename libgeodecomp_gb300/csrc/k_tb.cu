@@ -337,7 +337,10 @@ static long long tb_resident()
 }
 
 // Planes per CTA: minimise waves of resident CTAs times input planes per CTA
-// (the chunk plus the 2 TB halo planes); chunks of at least 8 planes.
+// (the chunk plus the 2 TB halo planes); chunks of at least 2 planes.  A grid of
+// few columns is latency bound, and its chunks run side by side: fixed point, us
+// per step with chunks of at least 8, 4, 2 planes, 20 x 24 x 30 6.6, 4.1, 2.7, 64^3
+// 5.8, 3.8, 3.3, 400 x 60 x 100 9.5, 6.8, 6.8; from 128^3 on no difference.
 struct TbPlan {
     int zchunk;
     double planes;          // of the launch: waves times planes per CTA
@@ -346,7 +349,7 @@ struct TbPlan {
 static TbPlan plan_tb(long long xy, int nz, long long resident, int halo)
 {
     TbPlan best = {nz, 1e300};
-    const int max_split = std::max(1, nz / 8);
+    const int max_split = std::max(1, nz / 2);
     for (int split = 1; split <= max_split; ++split) {
         const int chunk = (nz + split - 1) / split;
         const int s = (nz + chunk - 1) / chunk;

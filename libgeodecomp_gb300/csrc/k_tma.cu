@@ -451,14 +451,15 @@ namespace tmak {
 
 // Planes per CTA of a z-marching launch over xy tiles per plane: the split
 // that minimises the modelled time, waves of resident CTAs times planes per
-// CTA (including the two halo planes), with chunks of at least 8 planes.
+// CTA (including the two halo planes), with chunks of at least 2 planes (small
+// grids are latency bound).
 // A partial last wave costs a whole wave: the kernels are bound by the
 // copies each CTA keeps in flight, so fewer CTAs move fewer bytes.
 static int pick_zchunk(long long xy, int nz, long long resident)
 {
     int best_chunk = nz;
     double best = 1e300;
-    const int max_split = std::max(1, nz / 8);
+    const int max_split = std::max(1, nz / 2);
     for (int split = 1; split <= max_split; ++split) {
         const int chunk = (nz + split - 1) / split;
         const int s = (nz + chunk - 1) / chunk;
@@ -557,7 +558,10 @@ static void launch_tma_typed(Grid& g, CUtensorMapDataType dt)
         // keep the tail of the launch short (measured: 400 GLUPS at 512^3
         // against 387 with the wave-count model the var-coef kernel uses)
         zsplit = (int)((152LL * 16 + xy - 1) / xy);
-        zsplit = std::max(1, std::min(zsplit, (g.desc.nz + 15) / 16));
+        // chunks of at least 16 planes, but of 2 where those would not give
+        // every SM two CTAs
+        const int even = (int)std::min<long long>((2LL * 152 + xy - 1) / xy, g.desc.nz / 2);
+        zsplit = std::max(1, std::min(zsplit, std::max((g.desc.nz + 15) / 16, even)));
         zchunk = (g.desc.nz + zsplit - 1) / zsplit;
     }
     zsplit = (g.desc.nz + zchunk - 1) / zchunk;
