@@ -7,18 +7,18 @@
 // the neighbours in the plane are L1 hits.  A grid falls into as many small CTAs
 // as give every SM an even share.
 //
-// FP64 is bound by the FP64 pipe, so the cell's 30 operations become 21, bit for
-// bit: the face to the plane below is the exact negative of the face the thread
-// took to its top neighbour one plane earlier (4 operations, and a sum does not
-// see the sign of a zero), and the multiplication of k + k' by 1/2 is a
-// subtraction from the exponent (5 of them).  Where an exponent is at the range's
-// ends (k + k' zero, subnormal, infinite, NaN) the cell is computed as written.
+// FP64 is bound by the FP64 pipe, so of the cell's 30 operations it keeps 16, bit
+// for bit: the face to the plane below is the exact negative of the face the
+// thread took to its top neighbour one plane earlier (a sum does not see the sign
+// of a zero), and (k + k') / 2 of the other five is an integer sum.  Where that
+// does not hold the cell is computed as written.
 //
-// us per step, against the pair kernel of k_stencil.cu before (two x cells per
-// lane, whose blocks at a grid's ragged end loaded cell by cell): FP64 24^3 3.4
-// (159), 64^3 14.4 (70), 101 x 77 x 60 24 (246), 128^3 89 (133), 256^3 685 (888;
-// 24.5 GLUPS x 21 operations = 514 G/s, the pipe's rate); FP32 101 x 77 x 60 4.3
-// (162), 253 x 250 x 250 68 (517).
+// us per step (in brackets with a halving by the exponent but FP64 sums, 21
+// operations; then the pair kernel of k_stencil.cu: two x cells per lane, whose
+// blocks at a grid's ragged end loaded cell by cell): FP64 64^3 12 (14, 70), 101 x
+// 77 x 60 19 (24, 246), 128^3 74 (89, 133), 256^3 530 (685, 888): 31.7 GLUPS x 16
+// operations = 507 G/s, the pipe's rate; FP32 101 x 77 x 60 4.3 (162), 253 x 250 x
+// 250 68 (517).
 #include <algorithm>
 
 #include "lgd_internal.h"
@@ -30,13 +30,27 @@ namespace vcp {
 
 constexpr int THREADS = 128;
 
-// x / 2 by the exponent; ok becomes false where that is not the rounded product
-__device__ __forceinline__ double half_of(double x, bool& ok)
+// fl((a + b) / 2) of positive doubles in integer arithmetic, as sum4 (k_fp64.cuh)
+// adds, b possibly +0 (a zero edge coefficient: then the half is a subtraction from
+// the exponent); ok becomes false where that does not hold: other signs, more
+// than nine binary exponents apart and the ends of the exponent range
+__device__ __forceinline__ double half_sum(double a, double b, bool& ok)
 {
-    const unsigned hi = (unsigned)__double2hiint(x);
-    const unsigned e = hi & 0x7ff00000u;
-    ok = ok && e - 0x00200000u < 0x7fd00000u;               // exponents 2 .. 2046
-    return __hiloint2double((int)(hi - 0x00100000u), __double2loint(x));
+    const unsigned ha = (unsigned)__double2hiint(a), hb = (unsigned)__double2hiint(b);
+    const unsigned e0 = min(ha, hb) >> 20;
+    const unsigned sa = (ha >> 20) - e0, sb = (hb >> 20) - e0;          // one of them 0
+    const unsigned ma = (ha & 0xfffffu) | 0x100000u, mb = (hb & 0xfffffu) | 0x100000u;
+    const unsigned la = (unsigned)__double2loint(a), lb = (unsigned)__double2loint(b);
+    unsigned long long s = (((unsigned long long)__funnelshift_l(la, ma, sa) << 32) | (la << (sa & 31u))) +
+                           (((unsigned long long)__funnelshift_l(lb, mb, sb) << 32) | (lb << (sb & 31u)));
+    const unsigned k = 11u - (unsigned)__clz((int)(s >> 32));          // bits to drop, 1 .. 10
+    const unsigned unit = 1u << (k & 31u);
+    s += (unit >> 1) - 1u + (((unsigned)s >> (k & 31u)) & 1u);
+    // s >> k holds the leading bit, which adds one to the exponent field; the half takes it off again
+    const bool alone = (hb | lb) == 0u;
+    ok = ok && (alone ? (ha >> 20) - 3u < 2030u : (sa | sb) <= 9u && e0 - 3u < 2030u);
+    const double half = __longlong_as_double((long long)((s >> (k & 31u)) + ((unsigned long long)(e0 + k - 2u) << 52)));
+    return alone ? __hiloint2double((int)(ha - 0x00100000u), (int)la) : half;
 }
 
 // the cell as written (a call: predicated, its operations would be paid always)
@@ -103,7 +117,7 @@ varcoef_plane_kernel(const Args<R> a)
         if constexpr (sizeof(R) == 8) {
             bool ok = true;
             auto face = [&](double un, double kn) {
-                return __dmul_rn(half_of(__dadd_rn(kc, kn), ok), __dadd_rn(un, -uc));
+                return __dmul_rn(half_sum(kc, kn, ok), __dadd_rn(un, -uc));
             };
             double flux = face(uw, kw);
             flux = __dadd_rn(flux, face(ue, ke));
@@ -132,7 +146,7 @@ varcoef_plane_kernel(const Args<R> a)
 }
 
 // Planes per thread: 8 re-read least, fewer until there are 10 CTAs per SM.  us per
-// step with 1, 2, 4, 8 planes, FP64: 64^3 14.4, 13.5, 21.6, 39.4; 120 x 96 x 100
+// step with 1, 2, 4, 8 planes, FP64 (with 21 operations): 64^3 14.4, 13.5, 21.6, 39.4; 120 x 96 x 100
 // 56.7, 52.3, 50.3, 53.2; 256^3 796, 732, 701, 685; FP32 101 x 77 x 60 5.1, 4.3,
 // 5.3, 5.6; 130 x 128 x 128 18.2, 12.4, 10.8, 10.7.
 template<typename R>

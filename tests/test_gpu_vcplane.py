@@ -51,6 +51,17 @@ def test_fp64_coefficients_at_the_ends_of_the_range(scale):
     np.testing.assert_array_equal(run(lgd.CELL_VARCOEF_F64, u, k, 2, 0, 7), run(lgd.CELL_VARCOEF_F64, u, k, 2, 1, 7))
 
 
+@pytest.mark.parametrize("reach", [1, 9, 10, 30])
+@pytest.mark.parametrize("bits", [3, 52])
+def test_fp64_coefficients_far_apart(reach, bits):
+    """The integer sum's condition met by all, some and none of a warp's
+    faces; few significant bits (ties) and full significands."""
+    rng = np.random.default_rng(reach)
+    u = rng.random((6, 9, 40))
+    k = np.ldexp(1.0 + np.floor(rng.random(u.shape) * 2.0 ** bits) * 2.0 ** -bits, rng.integers(-reach - 2, -1, u.shape))
+    np.testing.assert_array_equal(run(lgd.CELL_VARCOEF_F64, u, k, 2, 0, 7), run(lgd.CELL_VARCOEF_F64, u, k, 2, 1, 7))
+
+
 @pytest.mark.parametrize("periodic", [0, 5, 7])
 @pytest.mark.parametrize("shape", SHAPES)
 def test_fp32_ragged_rows(periodic, shape):
