@@ -182,7 +182,7 @@ def workload_config(name: str, args, world: int = 1) -> dict:
     elif name == "gol_u8_8192":
         cfg = {"workload": name, "grid": [8192, 8192], "boundary": "torus", "cells": 8192 * 8192,
                "initial": "Bernoulli(0.3) seed 42", "run_steps": 1000,
-               "generations_per_pass": "library default (16, bit-sliced)",
+               "generations_per_pass": "library default (packed rows, planned for the board)",
                "l2": "both buffers (128 MiB) about L2-sized; no flush between steps"}
     elif name == "sell_f64_4m":
         cfg = {"workload": name, "nodes": 4194304, "C": 32, "sigma": 256, "degree": "power law alpha=2 on [4,64]",
