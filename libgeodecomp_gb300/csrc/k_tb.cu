@@ -349,14 +349,7 @@ struct TbPlan {
 static TbPlan plan_tb(long long xy, int nz, long long resident, int halo)
 {
     TbPlan best = {nz, 1e300};
-    const int max_split = std::max(1, nz / 2);
-    for (int split = 1; split <= max_split; ++split) {
-        const int chunk = (nz + split - 1) / split;
-        const int s = (nz + chunk - 1) / chunk;
-        const long long waves = (xy * s + resident - 1) / resident;
-        const double t = (double)waves * (chunk + halo);
-        if (t < best.planes * 0.999) best = {chunk, t};
-    }
+    best.zchunk = tmak::least_planes(xy, nz, resident, halo, &best.planes);
     return best;
 }
 

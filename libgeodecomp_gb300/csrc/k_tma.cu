@@ -457,20 +457,7 @@ namespace tmak {
 // copies each CTA keeps in flight, so fewer CTAs move fewer bytes.
 static int pick_zchunk(long long xy, int nz, long long resident)
 {
-    int best_chunk = nz;
-    double best = 1e300;
-    const int max_split = std::max(1, nz / 2);
-    for (int split = 1; split <= max_split; ++split) {
-        const int chunk = (nz + split - 1) / split;
-        const int s = (nz + chunk - 1) / chunk;
-        const long long waves = (xy * s + resident - 1) / resident;
-        const double t = (double)waves * (chunk + 2);
-        if (t < best * 0.999) {
-            best = t;
-            best_chunk = chunk;
-        }
-    }
-    return best_chunk;
+    return least_planes(xy, nz, resident, 2, nullptr);
 }
 
 // Planes per CTA for a kernel bound by its arithmetic pipe (the IEEE FP64
