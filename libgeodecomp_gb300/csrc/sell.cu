@@ -129,7 +129,9 @@ sell_diffusion_kernel(const int *__restrict__ chunk_offset, const int *__restric
 // row's iterations cost one memory round trip each instead of a DRAM trip
 // followed by a dependent L2 trip.  Slots below the chunk length exist for
 // every lane of the chunk, lanes load only their own row's entries; the
-// sum runs in slot order, as in the kernel above.
+// sum runs in slot order, as in the kernel above.  The first slots' entries load
+// before the wait for the step before (2000 nodes FP64 7.4 -> 6.9 us per step,
+// 100003 14.9 -> 14.1, 4.19 M 203.5 -> 201.7).
 template<typename R, bool EXACT, int D>
 __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offset, const int *__restrict__ row_length,
                                               const R *__restrict__ values, const int *__restrict__ column,
@@ -138,7 +140,6 @@ __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offs
     const long long cbase = chunk_offset[chunk];
     const long long base = cbase + (row - chunk * C);
     const int len = row_length[row];
-    const R xr = x[row];
     const R *v = values + base;
     const int *c = column + base;
     R w[D];
@@ -152,6 +153,8 @@ __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offs
             cc[j] = __ldg(c + (long long)j * C);
         }
     }
+    dependent_start();          // the matrix does not change between steps, x does
+    const R xr = x[row];
     R acc = (R)0;
     for (int k = 0; k < len; k += D) {
         R g[D];
@@ -197,7 +200,6 @@ sell_diffusion_pipe_kernel(const int *__restrict__ chunk_offset, const int *__re
                            const R *__restrict__ values, const int *__restrict__ column,
                            const R *x, R *xn, int n, int C, int row_begin, int row_end)
 {
-    dependent_start();
     const int row = row_begin + blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= row_end) return;
     sell_pipe_row<R, EXACT, D>(chunk_offset, row_length, values, column, x, xn, C, row, row / C);
@@ -210,20 +212,20 @@ sell_diffusion_pipe_kernel(const int *__restrict__ chunk_offset, const int *__re
 // from the others' registers - the same additions in the same order as above.
 // FP32 only: the L-fold repeated additions would fill the FP64 pipe.
 // Measured, FP32, us per step against the better single-lane form: 2000 nodes
-// 4.1 / 5.8, 20000 7.0 / 7.2, 100003 9.9 / 11.2, 300000 21.1 / 20.4.
-template<bool EXACT, int L, int D, int THREADS>
+// 3.7 / 5.8, 20000 6.5 / 7.2, 100003 9.9 / 11.2, 300000 21.1 / 20.4.
+template<bool EXACT, int L, int D, int THREADS, bool EARLY>
 __global__ void __launch_bounds__(THREADS)
 sell_diffusion_team_kernel(const int *__restrict__ chunk_offset, const int *__restrict__ row_length,
                            const float *__restrict__ values, const int *__restrict__ column, const float *x, float *xn,
                            int C, int row_begin, int row_end)
 {
-    dependent_start();
+    if (!EARLY) dependent_start();
     const int t = blockIdx.x * THREADS + threadIdx.x;
     const int q = t % L;
     const int row = min(row_begin + t / L, row_end - 1);            // idle teams repeat the last row (all lanes shuffle)
     const int chunk = row / C;
     const int len = row_length[row];
-    const float xr = x[row];
+    float xr = EARLY ? 0.f : x[row];
     const float *v = values + (long long)chunk_offset[chunk] + (row - chunk * C);
     const int *c = column + (long long)chunk_offset[chunk] + (row - chunk * C);
     // rounds of the warp's longest row
@@ -244,6 +246,10 @@ sell_diffusion_team_kernel(const int *__restrict__ chunk_offset, const int *__re
         }
     };
     load(0, w, cc);
+    if (EARLY) {                // the matrix does not change between steps, x does
+        dependent_start();
+        xr = x[row];
+    }
     float acc = 0.f;
     for (int k0 = 0; k0 < longest; k0 += D * L) {
         float g[D];
@@ -314,6 +320,10 @@ static void launch_pipe(Sell& s, int row_begin, int row_end, const R *x, R *xn, 
 }
 
 constexpr int SELL_TEAM_MAX_ROWS = 200000;
+// CTAs of one wave load their first slots while the step before still runs (20000
+// rows 6.5 us against 7.0); beyond one wave the loads only take the running step's
+// slots (100003 rows 10.2 against 9.9)
+constexpr int SELL_TEAM_EARLY_CTAS = 152 * 16;
 constexpr int SELL_DEEP_MAX_ROWS = 600000;
 
 template<bool EXACT>
@@ -321,8 +331,10 @@ static void launch_team(Sell& s, int row_begin, int row_end, const float *x, flo
 {
     constexpr int L = 4, D = 4, THREADS = 128;
     const int blocks = (int)(((long long)(row_end - row_begin) * L + THREADS - 1) / THREADS);
-    launch_dependent(sell_diffusion_team_kernel<EXACT, L, D, THREADS>, dim3(blocks), THREADS, 0, s.stream,
-                     s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.C, row_begin, row_end);
+    launch_dependent(blocks <= SELL_TEAM_EARLY_CTAS ? sell_diffusion_team_kernel<EXACT, L, D, THREADS, true>
+                                                    : sell_diffusion_team_kernel<EXACT, L, D, THREADS, false>,
+                     dim3(blocks), THREADS, 0, s.stream, s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.C,
+                     row_begin, row_end);
 }
 
 template<typename R, bool EXACT>
