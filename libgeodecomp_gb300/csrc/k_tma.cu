@@ -545,9 +545,10 @@ static void launch_tma_typed(Grid& g, CUtensorMapDataType dt)
         // keep the tail of the launch short (measured: 400 GLUPS at 512^3
         // against 387 with the wave-count model the var-coef kernel uses)
         zsplit = (int)((152LL * 16 + xy - 1) / xy);
-        // chunks of at least 16 planes, but of 2 where those would not give
-        // every SM two CTAs
-        const int even = (int)std::min<long long>((2LL * 152 + xy - 1) / xy, g.desc.nz / 2);
+        // chunks of at least 16 planes, but shorter ones where those would not
+        // fill the resident slots once: fixed point, us per step, 64^3 11.6 -> 4.3, 68 x 110
+        // x 322 20.3 -> 11.8; FP32 8.5 -> 2.7 and 17.9 -> 7.0
+        const int even = (int)std::min<long long>((resident + xy - 1) / xy, g.desc.nz / 2);
         zsplit = std::max(1, std::min(zsplit, std::max((g.desc.nz + 15) / 16, even)));
         zchunk = (g.desc.nz + zsplit - 1) / zsplit;
     }
