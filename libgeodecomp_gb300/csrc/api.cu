@@ -237,8 +237,9 @@ static void check_device_error(Grid& g)
 
 // Device staging buffer of the handle for conversions at the boundary,
 // allocated on first use and grown when needed (kept until destroy, so
-// repeated uploads and downloads do not allocate).
-static double *staging(Grid& g, size_t bytes)
+// repeated uploads and downloads do not allocate); null where the device has
+// no room for it.
+static double *try_staging(Grid& g, size_t bytes)
 {
     if (bytes > g.stage_bytes) {
         if (g.d_stage) {
@@ -247,10 +248,21 @@ static double *staging(Grid& g, size_t bytes)
             g.d_stage = nullptr;
             g.stage_bytes = 0;
         }
-        LGD_CHECK_CUDA(cudaMalloc(&g.d_stage, bytes));
+        if (cudaMalloc(&g.d_stage, bytes) != cudaSuccess) {
+            (void)cudaGetLastError();
+            g.d_stage = nullptr;
+            return nullptr;
+        }
         g.stage_bytes = bytes;
     }
     return (double *)g.d_stage;
+}
+
+static double *staging(Grid& g, size_t bytes)
+{
+    double *stage = try_staging(g, bytes);
+    if (stage == nullptr) throw Error(LGD_ERR_CUDA, "no device memory for the staging buffer");
+    return stage;
 }
 
 // Row chunks of a fixed-point transfer: the copy of chunk k overlaps the
@@ -321,7 +333,8 @@ static void repitch(Grid& g, void *dense, void *pitched, size_t row_bytes, long 
 }
 
 // Host <-> grid copy of one member: rows that fill their pitch go as one
-// dense copy, others through a bounded staging buffer and repitch.
+// dense copy, others through a bounded staging buffer and repitch (or row by row
+// where that does not fit).
 constexpr size_t HOST_STAGE_BYTES = 64u << 20;
 constexpr size_t REPITCH_MAX_ROW = 1u << 30;        // repitch_kernel numbers a row's words in 32 bits
 
@@ -335,13 +348,13 @@ static void host_copy(Grid& g, int member, void *buf, void *host, bool to_grid)
         LGD_CHECK_CUDA(cudaMemcpyAsync(to_grid ? buf : host, to_grid ? host : buf, row_bytes * rows, kind, g.stream));
         return;
     }
-    if (row_bytes > REPITCH_MAX_ROW) {
+    const size_t chunk = std::min(rows, std::max<size_t>(1, HOST_STAGE_BYTES / row_bytes));
+    unsigned char *stage = row_bytes > REPITCH_MAX_ROW ? nullptr : (unsigned char *)try_staging(g, chunk * row_bytes);
+    if (stage == nullptr) {
         LGD_CHECK_CUDA(cudaMemcpy2DAsync(to_grid ? buf : host, to_grid ? pitch : row_bytes, to_grid ? host : buf,
                                          to_grid ? row_bytes : pitch, row_bytes, rows, kind, g.stream));
         return;
     }
-    const size_t chunk = std::min(rows, std::max<size_t>(1, HOST_STAGE_BYTES / row_bytes));
-    unsigned char *stage = (unsigned char *)staging(g, chunk * row_bytes);
     for (size_t r = 0; r < rows; r += chunk) {
         const size_t n = std::min(chunk, rows - r);
         unsigned char *h = (unsigned char *)host + r * row_bytes;

@@ -466,7 +466,7 @@ void launch_gol(Grid& g, int steps)
     // their meaning, and leaves 0 and 1 behind
     const bool aligned_torus = gol_tb_applicable(g);
     if (g.variant == 0 && g.time_block == 0 && steps >= (aligned_torus ? GOL_PACK_MIN_TORUS : GOL_PACK_MIN) &&
-        gol_packed_applicable(g)) {
+        gol_packed_applicable(g) && gol_packed_ready(g)) {
         if (!aligned_torus) {
             gol_single(g, 1);
             --steps;

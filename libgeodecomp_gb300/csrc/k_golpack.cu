@@ -22,7 +22,7 @@
 //
 // Bound by the ALU pipe (64 lanes per clock and SM): 11 instructions per word
 // allow 57 T cell updates per second on 152 SMs.  A pass of 16 generations of
-// 8192^2 takes 38 us (28 T updates per second; 44 with three instructions more
+// 8192^2 takes 33 us (33 T updates per second; 44 with three instructions more
 // per word, gol_bits_kernel 99); the rest goes to the rim (6% of rows, 5% of
 // words), 144 of 152 SMs at work, 5 us of launch, loads and stores per pass,
 // and the exchange of rows.  More warps of fewer rows (24 x 23, 32 x 17) and
@@ -315,6 +315,30 @@ bool gol_packed_applicable(const Grid& g)
            g.desc.ny <= (1 << 24) && ((g.desc.periodic & 3) == 3 || edge == 0.0 || edge == 1.0);
 }
 
+static golp::Board board_of(const Grid& g)
+{
+    golp::Board b;
+    b.nx = g.desc.nx;
+    b.ny = g.desc.ny;
+    b.words = (b.nx + 31) / 32;
+    b.wpitch = round_up(b.words, 4);
+    b.periodic = g.desc.periodic & 3;
+    b.edge = (uint8_t)g.desc.edge[0] ? 0xffffffffu : 0u;
+    return b;
+}
+
+// A quarter of one byte board's memory, kept with the grid; a board that leaves
+// no room for it runs on bytes.
+bool gol_packed_ready(Grid& g)
+{
+    const golp::Board b = board_of(g);
+    if (g.d_bits == nullptr && cudaMalloc(&g.d_bits, 2 * (size_t)b.wpitch * b.ny * sizeof(uint32_t)) != cudaSuccess) {
+        (void)cudaGetLastError();
+        g.d_bits = nullptr;
+    }
+    return g.d_bits != nullptr;
+}
+
 // steps >= 1 generations of a board whose cells are 0 or 1
 void launch_gol_packed(Grid& g, int steps)
 {
@@ -326,15 +350,8 @@ void launch_gol_packed(Grid& g, int steps)
         LGD_CHECK_CUDA(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev));
         return count;
     });
-    Board b;
-    b.nx = g.desc.nx;
-    b.ny = g.desc.ny;
-    b.words = (b.nx + 31) / 32;
-    b.wpitch = round_up(b.words, 4);
-    b.periodic = g.desc.periodic & 3;
-    b.edge = (uint8_t)g.desc.edge[0] ? 0xffffffffu : 0u;
+    const Board b = board_of(g);
     const size_t elems = (size_t)b.wpitch * b.ny;
-    if (g.d_bits == nullptr) LGD_CHECK_CUDA(cudaMalloc(&g.d_bits, 2 * elems * sizeof(uint32_t)));
     uint32_t *bits[2] = {g.d_bits, g.d_bits + elems};
     const long pitch = (long)g.pitch_bytes[0];
     const unsigned blocks = (unsigned)std::min<long long>(152LL * 32, ((long long)elems + 255) / 256);

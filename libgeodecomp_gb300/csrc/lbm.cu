@@ -91,6 +91,7 @@ struct Lbm {
     bool flat;          // single steps by lbm_flat_kernel (until a launch shape is set or found faster)
     FlatBlock *d_blocks;
     int n_blocks;
+    long long stage_values;
     double *d_stage;    // conversion staging of uploads and downloads (FP32; from the first one on)
 };
 
@@ -604,11 +605,20 @@ static void copy_instance(Lbm& e, const LbmInstance& in, size_t n3, double *host
         LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
         return;
     }
-    if (e.d_stage == nullptr) LGD_CHECK_CUDA(cudaMalloc(&e.d_stage, CONVERT_CHUNK * sizeof(double)));
+    if (e.d_stage == nullptr) {
+        // shorter chunks where the populations leave little room
+        e.stage_values = CONVERT_CHUNK;
+        while (cudaMalloc(&e.d_stage, e.stage_values * sizeof(double)) != cudaSuccess) {
+            (void)cudaGetLastError();
+            e.d_stage = nullptr;
+            e.stage_values /= 16;
+            LGD_REQUIRE(e.stage_values >= 1024, LGD_ERR_CUDA, "no device memory for the conversion buffer");
+        }
+    }
     float *f = (float *)e.buf[e.cur] + in.base;
     const long long total = 19ll * (long long)n3;
-    for (long long first = 0; first < total; first += CONVERT_CHUNK) {
-        const long long n = std::min(CONVERT_CHUNK, total - first);
+    for (long long first = 0; first < total; first += e.stage_values) {
+        const long long n = std::min(e.stage_values, total - first);
         const unsigned blocks = (unsigned)std::min<long long>(152 * 16, (n + 255) / 256);
         if (up) {
             LGD_CHECK_CUDA(cudaMemcpyAsync(e.d_stage, host + first, n * 8, cudaMemcpyHostToDevice, e.stream));
@@ -668,7 +678,11 @@ static void build_blocks(Lbm& e)
         }
     }
     LGD_REQUIRE(blocks.size() < (1ull << 31), LGD_ERR_RANGE, "ensemble too large");
-    LGD_CHECK_CUDA(cudaMalloc(&e.d_blocks, sizeof(FlatBlock) * blocks.size()));
+    if (cudaMalloc(&e.d_blocks, sizeof(FlatBlock) * blocks.size()) != cudaSuccess) {
+        (void)cudaGetLastError();       // populations that leave no room: the persistent kernel
+        e.d_blocks = nullptr;
+        return;
+    }
     LGD_CHECK_CUDA(
         cudaMemcpyAsync(e.d_blocks, blocks.data(), sizeof(FlatBlock) * blocks.size(), cudaMemcpyHostToDevice, e.stream));
     LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
@@ -1055,7 +1069,7 @@ int lgd_lbm_create(int count, const int32_t *edges, const double *omegas, double
             check_launch("lbm rest state");
             ++e->launches;
             build_blocks(*e);
-            e->flat = true;
+            e->flat = e->d_blocks != nullptr;
             set_config(*e, 4, 256, 4);
         } catch (...) {
             lbm_free(*e);
@@ -1152,7 +1166,8 @@ int lgd_lbm_tune(lgd_lbm *h, int trial_steps, int *tile_rows, int *threads, int 
         };
         // one thread per cell, then a pattern search over (log2 tile rows,
         // log2 threads, CTAs per SM)
-        e.flat = true;
+        const bool flat = e.d_blocks != nullptr;
+        e.flat = flat;
         const double flat_ms = measure(e.ty, e.threads, e.ctas_per_sm);
         e.flat = false;
         const int tys[] = {1, 2, 4, 8, 16, 32};
@@ -1186,9 +1201,9 @@ int lgd_lbm_tune(lgd_lbm *h, int trial_steps, int *tile_rows, int *threads, int 
             c = bc;
         }
         // the first measurement pays for the ensemble's first steps: repeated
-        e.flat = true;
+        e.flat = flat;
         const double flat_best = std::min(flat_ms, measure(tys[a], ths[b], cts[c]));
-        e.flat = flat_best <= best;
+        e.flat = flat && flat_best <= best;
         best = std::min(best, flat_best);
         set_config(e, tys[a], ths[b], cts[c]);
         // then temporal blocking: two steps per launch in each tile shape

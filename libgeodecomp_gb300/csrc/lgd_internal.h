@@ -233,6 +233,7 @@ void encode_tensor_map(void *map, int dtype, int rank, void *base, const uint64_
 void launch_jacobi7(Grid& g, int steps);
 void launch_gol(Grid& g, int steps);
 bool gol_packed_applicable(const Grid& g);
+bool gol_packed_ready(Grid& g);             // the packed boards are there
 void launch_gol_packed(Grid& g, int steps);
 void launch_varcoef(Grid& g, int steps);
 void launch_region(Grid& g, const int *d_streaks, const long long *d_prefix, int n_streaks, long long cells,
