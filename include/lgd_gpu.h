@@ -257,14 +257,17 @@ int lgd_gpu_plane_bytes(lgd_handle *h, int member, size_t *bytes);
 int lgd_gpu_copy_planes(lgd_handle *h, int member, int which, int p0, int np, void *buf, size_t bytes, int to_grid);
 
 /* Kernel variant for the Jacobi cells (results are identical): 0 (default)
- * TMA-staged shared-memory planes on cube grids with a zero edge cell,
- * otherwise variant 5; 1 shared-memory plane tiles loaded by the threads;
+ * for IEEE FP64 one cell of a plane per thread, for the others TMA-staged
+ * shared-memory planes (several steps per pass, see below) on cube grids with a
+ * zero edge cell, otherwise variant 5; 1 shared-memory plane tiles loaded by the
+ * threads;
  * 2 one cell per lane in registers; 3 / 4 / 5 two cells per lane, 8 / 2 / 4
  * rows per warp, marching in z with register rotation and warp shuffles.
  * Var-coef cells: 0 (default) for FP32 TMA-staged planes of u and k, wrapped
  * neighbours copied into their own areas (3D grids whose non-wrapping axes
- * have zero edge values and, when x wraps, rows of a multiple of 16 bytes),
- * otherwise (and for FP64) variant 2; 1 shared-memory plane tiles; 2 .. 5
+ * have zero edge values and, when x wraps, rows of a multiple of 16 bytes; two
+ * steps per pass on a torus), otherwise (and for FP64) one cell of a plane per
+ * thread; 1 shared-memory plane tiles; 2 .. 5
  * two cells per lane in registers.  6: the TMA kernel wherever it applies
  * (either cell family), else the default.  For tuning and comparison. */
 int lgd_gpu_set_variant(lgd_handle *h, int variant);
