@@ -7,18 +7,19 @@
 // the neighbours in the plane are L1 hits.  A grid falls into as many small CTAs
 // as give every SM an even share.
 //
-// FP64 is bound by the FP64 pipe, so of the cell's 30 operations it keeps 16, bit
+// FP64 is bound by the FP64 pipe, so of the cell's 30 operations it keeps 11, bit
 // for bit: the face to the plane below is the exact negative of the face the
 // thread took to its top neighbour one plane earlier (a sum does not see the sign
-// of a zero), and (k + k') / 2 of the other five is an integer sum.  Where that
-// does not hold the cell is computed as written.
+// of a zero), and (k + k') / 2 of the other five and its product with the
+// difference of u are integer sums and products.  Where that does not hold the cell
+// is computed as written.
 //
-// us per step (in brackets with a halving by the exponent but FP64 sums, 21
-// operations; then the pair kernel of k_stencil.cu: two x cells per lane, whose
-// blocks at a grid's ragged end loaded cell by cell): FP64 64^3 12 (14, 70), 101 x
-// 77 x 60 19 (24, 246), 128^3 74 (89, 133), 256^3 530 (685, 888): 31.7 GLUPS x 16
-// operations = 507 G/s, the pipe's rate; FP32 101 x 77 x 60 4.3 (162), 253 x 250 x
-// 250 68 (517).
+// us per step with 11 operations on the FP64 pipe (in brackets with the products,
+// 16, with the sums too, 21; then the pair kernel of k_stencil.cu: two x cells per
+// lane, whose blocks at a grid's ragged end loaded cell by cell): FP64 64^3 9.4 (12,
+// 14, 70), 101 x 77 x 60 14 (19, 24, 246), 128^3 52 (74, 89, 133), 256^3 380 (530,
+// 685, 888): 44.2 GLUPS x 11 operations = 486 G/s of the pipe's 498; FP32 101 x 77
+// x 60 4.3 (162), 253 x 250 x 250 68 (517).
 #include <algorithm>
 
 #include "lgd_internal.h"
@@ -51,6 +52,28 @@ __device__ __forceinline__ double half_sum(double a, double b, bool& ok)
     ok = ok && (alone ? (ha >> 20) - 3u < 2030u : (sa | sb) <= 9u && e0 - 3u < 2030u);
     const double half = __longlong_as_double((long long)((s >> (k & 31u)) + ((unsigned long long)(e0 + k - 2u) << 52)));
     return alone ? __hiloint2double((int)(ha - 0x00100000u), (int)la) : half;
+}
+
+// fl(a b) of a positive a in integer arithmetic; ok becomes false where the
+// exponents or the result's leave the middle of the range.  A product of the
+// significands has 105 or 106 bits, hi its top 63 or 64; the rest only matters as
+// zero or not.
+__device__ __forceinline__ double product(double a, double b, bool& ok)
+{
+    const unsigned ha = (unsigned)__double2hiint(a), hb = (unsigned)__double2hiint(b);
+    const unsigned ea = ha >> 20, eb = (hb >> 20) & 0x7ffu;
+    const unsigned long long ma = ((unsigned long long)__double_as_longlong(a) << 11) | 0x8000000000000000ull;
+    const unsigned long long mb = ((unsigned long long)__double_as_longlong(b) << 11) | 0x8000000000000000ull;
+    const unsigned long long hi = __umul64hi(ma, mb), lo = ma * mb;
+    const unsigned big = (unsigned)(hi >> 63), drop = 10u + big;
+    const unsigned odd = ((unsigned)hi >> drop) & 1u;
+    const unsigned long long m = (hi + ((512u << big) - 1u) + (odd | (lo != 0))) >> drop;
+    // m holds its leading bit, which adds one to the exponent field
+    const unsigned e = ea + eb + big - 1024u;
+    const double r = __longlong_as_double((long long)((m + ((unsigned long long)e << 52)) | ((unsigned long long)(hb & 0x80000000u) << 32)));
+    const bool zero = ((hb & 0x7fffffffu) | (unsigned)__double2loint(b)) == 0u;
+    ok = ok && (zero || (eb - 1u < 2046u && e - 2u < 2040u));
+    return zero ? b : r;
 }
 
 // the cell as written (a call: predicated, its operations would be paid always)
@@ -117,7 +140,7 @@ varcoef_plane_kernel(const Args<R> a)
         if constexpr (sizeof(R) == 8) {
             bool ok = true;
             auto face = [&](double un, double kn) {
-                return __dmul_rn(half_sum(kc, kn, ok), __dadd_rn(un, -uc));
+                return product(half_sum(kc, kn, ok), __dadd_rn(un, -uc), ok);
             };
             double flux = face(uw, kw);
             flux = __dadd_rn(flux, face(ue, ke));
