@@ -75,6 +75,30 @@ __device__ __forceinline__ bool sum4(double a, double b, double c, double d, boo
     return reach <= LGD_FP64_SUM_REACH && e0 - 1u < 2030u;
 }
 
+// fl(a b) in integer arithmetic; ok becomes false where an operand is subnormal,
+// infinite or NaN or the result leaves the middle of the exponent range.  A product
+// of the significands has 105 or 106 bits, hi its top 63 or 64; of the rest only
+// whether it is zero matters.
+__device__ __forceinline__ double mul_integer(double a, double b, bool& ok)
+{
+    const unsigned ha = (unsigned)__double2hiint(a), hb = (unsigned)__double2hiint(b);
+    const unsigned ea = (ha >> 20) & 0x7ffu, eb = (hb >> 20) & 0x7ffu;
+    const unsigned sign = (ha ^ hb) & 0x80000000u;
+    const unsigned long long ma = ((unsigned long long)__double_as_longlong(a) << 11) | 0x8000000000000000ull;
+    const unsigned long long mb = ((unsigned long long)__double_as_longlong(b) << 11) | 0x8000000000000000ull;
+    const unsigned long long hi = __umul64hi(ma, mb), lo = ma * mb;
+    const unsigned big = (unsigned)(hi >> 63), drop = 10u + big;
+    const unsigned odd = ((unsigned)hi >> drop) & 1u;
+    const unsigned long long m = (hi + ((512u << big) - 1u) + (odd | (lo != 0))) >> drop;
+    // m holds its leading bit, which adds one to the exponent field
+    const unsigned e = ea + eb + big - 1024u;
+    const unsigned long long r = (m + ((unsigned long long)e << 52)) | ((unsigned long long)sign << 32);
+    const bool zero = ((ha & 0x7fffffffu) | (unsigned)__double2loint(a)) == 0u ||
+                      ((hb & 0x7fffffffu) | (unsigned)__double2loint(b)) == 0u;
+    ok = ok && ea < 2047u && eb < 2047u && (zero || (ea != 0u && eb != 0u && e - 2u < 2040u));
+    return __longlong_as_double((long long)(zero ? (unsigned long long)sign << 32 : r));
+}
+
 }  // namespace lgd
 
 #endif

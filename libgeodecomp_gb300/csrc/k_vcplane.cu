@@ -54,8 +54,9 @@ __device__ __forceinline__ double half_sum(double a, double b, bool& ok)
     return alone ? __hiloint2double((int)(ha - 0x00100000u), (int)la) : half;
 }
 
-// fl(a b) of a positive a in integer arithmetic; ok becomes false where the
-// exponents or the result's leave the middle of the range.  A product of the
+// fl(a b) of a positive normal a in integer arithmetic (mul_integer of k_fp64.cuh
+// takes any sign; 399 us at 256^3 with it, 380 with this one); ok becomes false
+// where the exponents or the result's leave the middle of the range.  A product of the
 // significands has 105 or 106 bits, hi its top 63 or 64; the rest only matters as
 // zero or not.
 __device__ __forceinline__ double product(double a, double b, bool& ok)

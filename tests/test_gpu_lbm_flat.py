@@ -44,3 +44,23 @@ def test_conversion_beyond_one_chunk():
     with lgd.LbmEnsemble([80], [1.3], precision=4) as e:
         e.upload(0, f)
         np.testing.assert_array_equal(e.download(0), f)
+
+
+@pytest.mark.parametrize("omega", [1.0, 0.5, 1.999])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -520, 1e-300, 1e160, 0.0])
+def test_fp64_products_at_the_ends_of_the_range(scale, omega):
+    """Populations whose products are zero, subnormal or overflow (the cell is
+    then computed with FP64 multiplications), mixed with ordinary ones; the
+    persistent kernel multiplies in FP64 throughout."""
+    rng = np.random.default_rng(7)
+    f = rng.random((19, 7, 7, 7)) * np.where(rng.random((1, 7, 7, 7)) < 0.5, scale, 1.0) * rng.choice([-1.0, 1.0], (19, 7, 7, 7))
+    f[:, :2] = 0.0
+    out = []
+    for persistent in (False, True):
+        with lgd.LbmEnsemble([7], [omega], lid=0.05, precision=8) as e:
+            if persistent:
+                e.set_config(2, 64, 1)
+            e.upload(0, f)
+            e.step(3)
+            out.append(e.download(0))
+    np.testing.assert_array_equal(out[0], out[1])
