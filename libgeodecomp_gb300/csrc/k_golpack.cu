@@ -153,8 +153,11 @@ gol_pack_kernel(const uint32_t *in, uint32_t *out, Board b, int T, int out_rows)
     const bool wraps = (b.periodic & 1) && fill < 32;
 
     // rows first .. first + R - 1 of the board (rowin: those that exist); all
-    // loads of a kind are in flight together, and only windows that reach
-    // around a row's end load more than one word per row
+    // loads of a kind are in flight together, and only warps with a window that
+    // is not one word of the row load more: windows that straddle two words, and
+    // the row's last, partial word, which the row's start completes.  That one is
+    // aligned and may be the only such window of its warp (lane 31 of a tile that
+    // ends there: rows of 1921 .. 1951 cells, and every 960 more)
     uint32_t v[R];
     uint32_t rowin[CUBE ? (R + 31) / 32 : 1] = {};
     int first = y0 - T + warp * R;
@@ -175,7 +178,7 @@ gol_pack_kernel(const uint32_t *in, uint32_t *out, Board b, int T, int out_rows)
     };
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = row_of(r)[wl];
-    if (__any_sync(0xffffffffu, sh != 0)) {
+    if (__any_sync(0xffffffffu, sh != 0 || wraps)) {
         const int wh = has_hi ? wl + 1 : wl;
 #pragma unroll
         for (int r = 0; r < R; ++r) {

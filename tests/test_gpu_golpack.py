@@ -45,3 +45,13 @@ def test_bytes_other_than_0_and_1_keep_their_meaning():
     c0 = workloads.gol_initial(101, 77, seed=63) * np.random.default_rng(1).integers(1, 4, (77, 101)).astype(np.uint8)
     for periodic in (0, 3):
         np.testing.assert_array_equal(run(c0, 20, periodic), run(c0, 20, periodic, pack=False))
+
+
+@pytest.mark.parametrize("nx", [961, 1921, 1936, 1951, 1952, 2881, 2911, 3850])
+@pytest.mark.parametrize("steps", [8, 33])
+def test_last_partial_word_in_a_tiles_last_lane(nx, steps):
+    """Rows that wrap and whose last, partial word is the one window of its tile
+    that takes more than one word: 1921 .. 1951 cells, and every 960 more."""
+    c0 = workloads.gol_initial(nx, 41, seed=64)
+    np.testing.assert_array_equal(run(c0, steps, 3), oracle.gol(c0, steps))
+    np.testing.assert_array_equal(run(c0, steps, 1), run(c0, steps, 1, pack=False))
