@@ -99,8 +99,8 @@ struct Params {
     const float *bias;          // ACT, OUT
     bf16 *out;                  // ACT, GRAD: ghosted
     float *g;                   // ACT: GELU' of the pre-activations out (or null); GRAD: in; FP32
-                                // [batch][nz][ny][6][nx][4], four channels to a float4.  OUT: receives fout too
-                                // (or null)
+                                // [batch][nz][ny][6][nx][4], four channels to a float4.  OUT: receives conv +
+                                // bias (or null)
     float *db;                  // GRAD: bias gradient, added to
     float *fout;                // OUT
     int add;                    // OUT: add to fout
@@ -422,9 +422,9 @@ conv_tc_kernel(const Params p)
                 restart(slot);
                 if (q >= 2 && live) {
                     float *o = fout0 + z * fplane;
-                    const float r = p.add ? before + (v + b1) : v + b1;
-                    *o = r;
-                    if (p.g) p.g[o - p.fout] = r;
+                    const float d = v + b1;
+                    *o = p.add ? before + d : d;
+                    if (p.g) p.g[o - p.fout] = d;
                 }
             } else {
                 uint4 w[3];

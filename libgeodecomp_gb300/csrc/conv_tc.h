@@ -30,7 +30,7 @@ void tc_layer1(const float *u, const float *k, const void *w, const float *bias,
 void tc_layer_mid(const void *in, const void *w, const float *bias, void *out, float *gelu_grad, const int dims[4], int *err,
                   cudaStream_t stream);
 // layer 4 (24 -> 1): out = conv + bias, or out += that; copy (or null)
-// receives out too
+// receives conv + bias
 void tc_layer_last(const void *in, const void *w, const float *bias, float *out, bool add, float *copy, const int dims[4],
                    int *err, cudaStream_t stream);
 

@@ -585,22 +585,25 @@ static void sync_and_check(Net& n)
 }
 
 // The forward pass on the tensor cores: four launches, the activations between
-// two ghosted buffers (three when training, which also keeps GELU' and the
-// packed input).  With add_to_u the last layer adds its
-// result to u instead (u <- u + du, the residual step).
-static void forward_fast(Net& n, const float *u, const float *k, float *du, bool add_to_u, float *copy)
+// two ghosted buffers.  keep: a backward pass may follow, which reads the three
+// layers' activations, GELU', the packed input and n.du.  With add_to_u the last
+// layer adds its result to u instead (u <- u + du, the residual step); copy (or
+// null) receives the result itself.
+static void forward_fast(Net& n, const float *u, const float *k, float *du, bool add_to_u, float *copy, bool keep)
 {
     const int dims[4] = {n.g.nx, n.g.ny, n.g.nz, n.g.batch};
     const float *bias[4];
     for (int l = 0; l < 4; ++l) bias[l] = n.params + n.L[l].b_off;
-    void *h3 = n.training ? n.hg[2] : n.hg[0];
-    if (n.training) {
+    void *h3 = keep ? n.hg[2] : n.hg[0];
+    float *const none[3] = {};
+    float *const *gt = keep ? n.gt : none;
+    if (keep) {
         pack_input_kernel<<<grid_blocks(n.V), 256, 0, n.stream>>>(u, k, (bf16 *)n.xt, n.V);
         ++n.launches;
     }
-    tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], n.gt[0], dims, n.d_err, n.stream);
-    tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], n.gt[1], dims, n.d_err, n.stream);
-    tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], h3, n.gt[2], dims, n.d_err, n.stream);
+    tc_layer1(u, k, n.wtc.fwd[0], bias[0], n.hg[0], gt[0], dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[0], n.wtc.fwd[1], bias[1], n.hg[1], gt[1], dims, n.d_err, n.stream);
+    tc_layer_mid(n.hg[1], n.wtc.fwd[2], bias[2], h3, gt[2], dims, n.d_err, n.stream);
     tc_layer_last(h3, n.wtc.fwd[3], bias[3], add_to_u ? const_cast<float *>(u) : du, add_to_u, copy, dims, n.d_err,
                   n.stream);
     n.launches += 4;
@@ -701,13 +704,14 @@ static void backward_impl(Net& n, const float *target, double *loss_out)
 }
 
 // du = net(u, k); with add_to_u the fast path may add du to u itself
-// (returns true when it did)
-static bool forward(Net& n, const float *u, const float *k, float *du, bool add_to_u = false, float *copy = nullptr)
+// (returns true when it did).  copy (or null) receives du too.  keep: leave
+// what a backward pass reads (training); the mma.sync path always does.
+static bool forward(Net& n, const float *u, const float *k, float *du, bool add_to_u, float *copy, bool keep)
 {
     n.fast_forward = n.fast && n.variant == 0;
     ensure_packed(n, n.fast_forward);
     if (n.fast_forward) {
-        forward_fast(n, u, k, du, add_to_u, copy);
+        forward_fast(n, u, k, du, add_to_u, copy, keep);
         return add_to_u;
     }
     ensure_dense(n);
@@ -716,7 +720,7 @@ static bool forward(Net& n, const float *u, const float *k, float *du, bool add_
     } else {
         if (n.TX == 64) forward_impl<8, 64>(n, u, k, du); else forward_impl<8, 32>(n, u, k, du);
     }
-    if (copy) LGD_CHECK_CUDA(cudaMemcpyAsync(copy, du, sizeof(float) * n.V, cudaMemcpyDeviceToDevice, n.stream));
+    if (copy && copy != du) LGD_CHECK_CUDA(cudaMemcpyAsync(copy, du, sizeof(float) * n.V, cudaMemcpyDeviceToDevice, n.stream));
     return false;
 }
 
@@ -941,7 +945,7 @@ int lgd_net_forward(lgd_net *h, const float *d_u, const float *d_kappa, float *d
     return guard([&] {
         Net& n = net_of(h);
         LGD_REQUIRE(d_u && d_kappa, LGD_ERR_INVALID, "null input");
-        forward(n, d_u, d_kappa, d_du ? d_du : n.du, false, d_du && n.training ? n.du : nullptr);
+        forward(n, d_u, d_kappa, d_du ? d_du : n.du, false, d_du && n.training ? n.du : nullptr, n.training);
     });
 }
 
@@ -977,7 +981,9 @@ int lgd_net_advance(lgd_net *h, float *d_u, const float *d_kappa, int calls)
         LGD_REQUIRE(d_u && d_kappa, LGD_ERR_INVALID, "null input");
         LGD_REQUIRE(calls >= 0, LGD_ERR_INVALID, "negative call count");
         for (int c = 0; c < calls; ++c) {
-            if (forward(n, d_u, d_kappa, n.du, true)) continue;
+            // a backward pass after this is about the last call, as after a forward
+            const bool keep = n.training && c + 1 == calls;
+            if (forward(n, d_u, d_kappa, n.du, true, keep ? n.du : nullptr, keep)) continue;
             add_inplace_kernel<<<grid_blocks(n.V), 256, 0, n.stream>>>(d_u, n.du, n.V);
             check_launch("residual update");
             ++n.launches;

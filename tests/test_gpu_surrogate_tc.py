@@ -122,3 +122,32 @@ def test_changed_weights_reach_either_path(order):
         net.forward(t[0], t[1], du)
         net.synchronize()
         np.testing.assert_array_equal(out, du.cpu().numpy())
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("calls", [1, 3])
+def test_backward_after_advance_is_about_its_last_call(variant, calls):
+    """advance leaves what a forward pass of its last call would: the same loss
+    and gradients (up to the order of the FP32 atomic sums, 1e-6 relative)."""
+    from libgeodecomp_gb300.surrogate import SurrogateNet
+    shape = (5, 12, 64)
+    u, k, target, p = inputs(shape, 2, 8)
+    before, v, kt, tt = (torch.tensor(a, dtype=torch.float32, device="cuda").contiguous() for a in (u, u, k, target))
+    du = torch.empty_like(v)
+    torch.cuda.synchronize()
+    out = []
+    for step in ("advance", "forward"):
+        with SurrogateNet(shape, batch=2, channels=24, training=True) as net:
+            net.set_params(p.astype(np.float32))
+            net.set_variant(variant)
+            if step == "advance":
+                net.advance(v, kt, calls)
+            else:
+                net.advance(before, kt, calls - 1)
+                net.forward(before, kt, du)
+            loss = net.backward(tt)
+            out.append((loss, net.get_grads().astype(np.float64)))
+    np.testing.assert_array_equal(v.cpu().numpy(), (before + du).cpu().numpy())
+    np.testing.assert_allclose(out[0][0], out[1][0], rtol=1e-6)
+    for a, b in zip(layers(out[0][1]), layers(out[1][1])):
+        assert np.linalg.norm(a - b) / np.linalg.norm(b) < 1e-5
