@@ -228,7 +228,7 @@ struct PullAll<R, 19, IDX, NC, INTERIOR> {
 // e . u for one of a pair of opposite directions, components added in the
 // oracle's order (x, y, z).  Its zero components drop out: adding 0 * u does
 // not change a sum but for the sign of a zero, which d + eu and eu * eu below
-// do not see.
+// do not see, and for an infinite u, which collide_with looks for.
 template<typename R, int I>
 __device__ __forceinline__ R dot_dir(R ux, R uy, R uz)
 {
@@ -254,9 +254,15 @@ __device__ __forceinline__ void collide_pair(const R *f, R keep, R w1, R w2, R d
     put(Q<I>::opp, A::add(mul(keep, f[Q<I>::opp]), mul(wi, A::add(A::sub(d, eu), sq))));
 }
 
+// not a number or infinite, without the FP64 pipe
+__device__ __forceinline__ bool non_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u; }
+__device__ __forceinline__ bool non_finite(double v) { return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u; }
+
 // BGK collision, operation order of the oracle's lgd_d3q19_collide; put(i,
-// v) stores post-collision population i, mul multiplies
-template<typename R, typename PUT, typename MUL>
+// v) stores post-collision population i, mul multiplies.  CHECK: velocities may
+// be infinite; 0 * u then makes every direction's e . u a NaN (without it mul
+// has to report them).
+template<typename R, bool CHECK, typename PUT, typename MUL>
 __device__ __forceinline__ void collide_with(const R *f, R omega, PUT put, MUL mul)
 {
     typedef LbmArith<R> A;
@@ -273,11 +279,12 @@ __device__ __forceinline__ void collide_with(const R *f, R omega, PUT put, MUL m
     const R uz = A::sub(A::add(A::add(A::add(A::add(f[5], f[11]), f[13]), f[15]), f[17]),
                         A::add(A::add(A::add(A::add(f[6], f[12]), f[14]), f[16]), f[18]));
     const R usq = A::add(A::add(mul(ux, ux), mul(uy, uy)), mul(uz, uz));
-    const R d = A::sub(mul(rho, (R)(1.0 / 3.0)), mul((R)0.5, usq));
+    R d = A::sub(mul(rho, (R)(1.0 / 3.0)), mul((R)0.5, usq));
     const R keep = A::sub((R)1.0, omega);
     const R w1 = mul(omega, (R)(1.0 / 6.0));
     const R w2 = mul(omega, (R)(1.0 / 12.0));
     put(0, A::add(mul(keep, f[0]), mul(omega, d)));
+    if (CHECK && (non_finite(ux) || non_finite(uy) || non_finite(uz))) d = (R)__int_as_float(0x7fffffff);
     collide_pair<R, 1>(f, keep, w1, w2, d, ux, uy, uz, put, mul);
     collide_pair<R, 2>(f, keep, w1, w2, d, ux, uy, uz, put, mul);
     collide_pair<R, 5>(f, keep, w1, w2, d, ux, uy, uz, put, mul);
@@ -292,7 +299,7 @@ __device__ __forceinline__ void collide_with(const R *f, R omega, PUT put, MUL m
 template<typename R, typename PUT>
 __device__ __forceinline__ void collide_to(const R *f, R omega, PUT put)
 {
-    collide_with<R>(f, omega, put, [](R a, R b) { return LbmArith<R>::mul(a, b); });
+    collide_with<R, true>(f, omega, put, [](R a, R b) { return LbmArith<R>::mul(a, b); });
 }
 
 template<typename R, typename IDX, int NC>
@@ -443,8 +450,8 @@ lbm_flat_kernel(const FlatBlock *__restrict__ blocks, const R *A, R *B)
     if constexpr (sizeof(R) == 8) {
         // FP64 is bound by the FP64 pipe: the collision's multiplications run on the
         // integer pipes, bit for bit (4 cavities of 32^3 to 96^3: 408 -> 287 us per step)
-        bool ok = true;
-        collide_with<R>(
+        bool ok = true;                 // mul_integer(u, u, ok) reports an infinite u
+        collide_with<R, false>(
             f, (R)in.omega, [&](int i, R v) { Mem<NC>::st(dst + ((IDX)i * n3 + (IDX)c), v); },
             [&](R a, R b) { return mul_integer(a, b, ok); });
         if (!ok) plain_cell<IDX, NC>(src, dst, n3, (IDX)c, (int)L, x, y, z, (R)in.lid, (R)in.omega);

@@ -64,3 +64,49 @@ def test_fp64_products_at_the_ends_of_the_range(scale, omega):
             e.step(3)
             out.append(e.download(0))
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("kernel", ["flat", "persistent", "looped", "two steps"])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("precision", [4, 8])
+def test_infinite_velocities(precision, axis, kernel):
+    """A density that is finite and a velocity component that overflows: 0 * u
+    makes every moving direction a NaN, the directions across the component
+    too, as in the oracle."""
+    L = 6
+    plus, minus = ((2, 3), (1, 4), (5, 6))[axis]        # E W, N S, T B
+    f = np.tile(0.05 + 0.01 * np.arange(19.0)[:, None, None, None], (1, L, L, L))
+    big = 3e38 if precision == 4 else 1.5e308
+    # what cell (2, 2, 2) pulls: the source cell is the cell minus the direction
+    for i, sign in ((plus, 1), (minus, -1)):
+        src = [2, 2, 2]
+        src[axis] -= sign                               # x, y, z
+        f[i, src[2], src[1], src[0]] = sign * big
+    with np.errstate(all="ignore"):
+        ref = oracle.lbm(L, 1, 1.2, 0.05, f)
+    assert np.isnan(ref[1:, 2, 2, 2]).all() or precision == 4
+    with lgd.LbmEnsemble([L], [1.2], lid=0.05, precision=precision) as e:
+        e.upload(0, f)
+        if kernel == "persistent":
+            e.set_config(2, 64, 1)
+        if kernel == "two steps":
+            e.set_time_block(2, 0, 1)
+        if kernel == "looped":
+            e.step_looped(1)
+        else:
+            e.step(2 if kernel == "two steps" else 1)
+        out = e.download(0)
+    if kernel == "two steps":
+        with np.errstate(all="ignore"):
+            ref = oracle.lbm(L, 2, 1.2, 0.05, f)
+        if precision == 4:
+            # the neighbours that pulled a NaN from the blown-up cell
+            assert np.isnan(out[1:, 2, 2, 1]).all() and np.isnan(out[1:, 3, 2, 2]).all()
+        else:
+            np.testing.assert_array_equal(out, ref)
+    elif precision == 4:
+        assert np.isnan(out[1:, 2, 2, 2]).all()
+        out[:, 2, 2, 2] = ref[:, 2, 2, 2] = 0.0
+        assert np.isfinite(out[:, 0]).all()
+    else:
+        np.testing.assert_array_equal(out, ref)
