@@ -110,3 +110,41 @@ def test_infinite_velocities(precision, axis, kernel):
         assert np.isfinite(out[:, 0]).all()
     else:
         np.testing.assert_array_equal(out, ref)
+
+
+def rounded_fma(a, b, c):
+    """fl(a b + c) of FP32 numbers: the product is exact in FP64, and the sum's
+    second rounding only matters next to a tie."""
+    return np.float32(np.float64(a) * np.float64(b) + np.float64(c))
+
+
+def test_fp32_relaxation_rounds_the_weighted_term():
+    """FP32 rounds keep f + w x once for the weighted term and once for the sum:
+    of the two FMAs this is the one with the smaller error (see relax)."""
+    L, omega = 12, np.float32(1.3)
+    rng = np.random.default_rng(9)
+    w = np.array([1 / 3] + [1 / 18] * 6 + [1 / 36] * 12)[:, None, None, None]
+    f = np.float32(w * (1 + 0.2 * rng.uniform(-1, 1, (19, L, L, L))))
+    e = np.array([(0, 0, 0), (0, 1, 0), (1, 0, 0), (-1, 0, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1), (-1, 1, 0), (-1, -1, 0),
+                  (1, 1, 0), (1, -1, 0), (-1, 0, 1), (-1, 0, -1), (1, 0, 1), (1, 0, -1), (0, 1, 1), (0, 1, -1), (0, -1, 1),
+                  (0, -1, -1)])
+    inner = slice(1, L - 1)
+    p = np.array([f[i][1 - z:L - 1 - z, 1 - y:L - 1 - y, 1 - x:L - 1 - x] for i, (x, y, z) in enumerate(e)])
+    p64 = p.astype(np.float64)
+    rho, u = p64.sum(axis=0), np.tensordot(e.T, p64, axes=1)
+    d = rho / 3 - 0.5 * (u * u).sum(axis=0)
+    with lgd.LbmEnsemble([L], [float(omega)], lid=0.05, precision=4) as ens:
+        ens.upload(0, f.astype(np.float64))
+        ens.step(1)
+        out = np.float32(ens.download(0))[:, inner, inner, inner]
+    keep = np.float32(1) - omega
+    for i in range(1, 19):
+        wi = omega * np.float32(1 / 6 if i < 7 else 1 / 12)
+        eu = np.tensordot(e[i], u, axes=1)
+        x = np.float32(d + eu + 1.5 * eu * eu)
+        one, other = rounded_fma(keep, p[i], wi * x), rounded_fma(wi, x, keep * p[i])
+        # x has roundings of its own on the device: the two forms are told apart
+        # where they differ, by which one the outputs lie nearer to
+        differ = one != other
+        near = np.abs(out[i].astype(np.float64) - one)[differ].sum(), np.abs(out[i].astype(np.float64) - other)[differ].sum()
+        assert near[0] < near[1], i
