@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "lgd_internal.h"
+#include "alloc_all.h"
 #include "conv_tc.h"
 #include "../../include/lgd_surrogate.h"
 
@@ -636,19 +637,23 @@ static void backward_fast(Net& n, const float *target, double *loss_out)
     }
 }
 
-// buffers of the mma.sync path, made when it first runs
+// buffers of the mma.sync path, made when it first runs: all of them (x0 says
+// that they exist), or none where there is no room
 static void ensure_dense(Net& n)
 {
     if (n.x0) return;
-    LGD_CHECK_CUDA(cudaMalloc(&n.x0, sizeof(bf16) * 2 * n.V));
-    const int nh = n.training ? 3 : 2;
-    for (int i = 0; i < nh; ++i) LGD_CHECK_CUDA(cudaMalloc(&n.h[i], sizeof(bf16) * n.C * n.V));
+    std::vector<BufferRequest> list = {{(void **)&n.x0, sizeof(bf16) * 2 * n.V}};
+    for (int i = 0; i < (n.training ? 3 : 2); ++i) list.push_back({(void **)&n.h[i], sizeof(bf16) * n.C * n.V});
     if (n.training) {
-        for (int i = 0; i < 3; ++i) LGD_CHECK_CUDA(cudaMalloc(&n.zb[i], sizeof(float) * n.C * n.V));
-        LGD_CHECK_CUDA(cudaMalloc(&n.dh, sizeof(float) * n.C * n.V));
-        LGD_CHECK_CUDA(cudaMalloc(&n.dzb, sizeof(bf16) * n.C * n.V));
-        LGD_CHECK_CUDA(cudaMalloc(&n.dz4, sizeof(bf16) * 2 * n.V));
+        for (int i = 0; i < 3; ++i) list.push_back({(void **)&n.zb[i], sizeof(float) * n.C * n.V});
+        list.push_back({(void **)&n.dh, sizeof(float) * n.C * n.V});
+        list.push_back({(void **)&n.dzb, sizeof(bf16) * n.C * n.V});
+        list.push_back({(void **)&n.dz4, sizeof(bf16) * 2 * n.V});
     }
+    const cudaError_t error = allocate_all(
+        list, [](void **p, size_t bytes) { return cudaMalloc(p, bytes); }, [](void *p) { cudaFree(p); });
+    if (error != cudaSuccess) (void)cudaGetLastError();     // reported here, not at the next launch
+    LGD_CHECK_CUDA(error);
 }
 
 // the network's channel count is a template parameter of the kernels; the
