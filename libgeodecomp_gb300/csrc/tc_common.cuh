@@ -78,7 +78,9 @@ __device__ __forceinline__ void mma_commit(uint32_t bar)
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// 24 consecutive columns of this thread's tensor-memory lane, and eight
+// 24 consecutive columns of this thread's tensor-memory lane, eight, and one.
+// The loaded values pass through the wait, so that none is used before it: the
+// order of volatile statements alone does not hold arithmetic on them back.
 __device__ __forceinline__ void tmem_ld24(uint32_t taddr, float (&v)[24])
 {
     uint32_t r[24];
@@ -90,7 +92,6 @@ __device__ __forceinline__ void tmem_ld24(uint32_t taddr, float (&v)[24])
                      : "r"(taddr + (uint32_t)c)
                      : "memory");
     }
-    // the values pass through the wait, so that none is used before it
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
                    "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
@@ -108,7 +109,10 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr)
                  : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 :
+                 : "memory");
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
@@ -126,7 +130,7 @@ __device__ __forceinline__ float tmem_ld1(uint32_t taddr)
 {
     uint32_t r;
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r) : : "memory");
     return __uint_as_float(r);
 }
 
