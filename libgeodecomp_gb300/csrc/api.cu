@@ -248,11 +248,7 @@ static double *try_staging(Grid& g, size_t bytes)
             g.d_stage = nullptr;
             g.stage_bytes = 0;
         }
-        if (cudaMalloc(&g.d_stage, bytes) != cudaSuccess) {
-            (void)cudaGetLastError();
-            g.d_stage = nullptr;
-            return nullptr;
-        }
+        if (malloc_on_first_use(&g.d_stage, bytes) != cudaSuccess) return nullptr;
         g.stage_bytes = bytes;
     }
     return (double *)g.d_stage;

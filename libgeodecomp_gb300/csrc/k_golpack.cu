@@ -335,10 +335,7 @@ static golp::Board board_of(const Grid& g)
 bool gol_packed_ready(Grid& g)
 {
     const golp::Board b = board_of(g);
-    if (g.d_bits == nullptr && cudaMalloc(&g.d_bits, 2 * (size_t)b.wpitch * b.ny * sizeof(uint32_t)) != cudaSuccess) {
-        (void)cudaGetLastError();
-        g.d_bits = nullptr;
-    }
+    if (g.d_bits == nullptr) (void)malloc_on_first_use((void **)&g.d_bits, 2 * (size_t)b.wpitch * b.ny * sizeof(uint32_t));
     return g.d_bits != nullptr;
 }
 

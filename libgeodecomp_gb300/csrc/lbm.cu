@@ -653,9 +653,7 @@ static void copy_instance(Lbm& e, const LbmInstance& in, size_t n3, double *host
     if (e.d_stage == nullptr) {
         // shorter chunks where the populations leave little room
         e.stage_values = CONVERT_CHUNK;
-        while (cudaMalloc(&e.d_stage, e.stage_values * sizeof(double)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            e.d_stage = nullptr;
+        while (malloc_on_first_use((void **)&e.d_stage, e.stage_values * sizeof(double)) != cudaSuccess) {
             e.stage_values /= 16;
             LGD_REQUIRE(e.stage_values >= 1024, LGD_ERR_CUDA, "no device memory for the conversion buffer");
         }

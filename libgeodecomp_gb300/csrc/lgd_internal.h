@@ -96,6 +96,24 @@ inline void check_launch(const char *what)
     }
 }
 
+// cudaMalloc for a buffer that a handle makes on its first use, in a call that
+// otherwise only launches or copies.  The caller may be capturing those launches
+// into a graph: the allocation is no part of it, but under the default mode it
+// would be refused and end the capture.  A failure is returned and not left
+// behind for the next check_launch.
+inline cudaError_t malloc_on_first_use(void **p, size_t bytes)
+{
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    LGD_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t error = cudaMalloc(p, bytes);
+    if (error != cudaSuccess) {
+        *p = nullptr;
+        (void)cudaGetLastError();
+    }
+    LGD_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    return error;
+}
+
 // Launches a kernel that may be scheduled while the kernel before it on the
 // stream still runs (programmatic dependent launch).  The kernel calls
 // dependent_start() before it touches global memory, which waits for that

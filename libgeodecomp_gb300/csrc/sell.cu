@@ -1050,7 +1050,7 @@ static void sell_copy_x(Sell& s, int which, double *host, size_t bytes, bool up,
     LGD_REQUIRE(!logical || s.d_perm != nullptr, LGD_ERR_INVALID, "no permutation was given at create");
     // kept by the handle: a pool allocation per copy cost 200 us, most of a
     // copy of 100000 nodes
-    if (s.d_stage == nullptr) LGD_CHECK_CUDA(cudaMalloc(&s.d_stage, bytes));
+    if (s.d_stage == nullptr) LGD_CHECK_CUDA(malloc_on_first_use((void **)&s.d_stage, bytes));
     double *tmp = s.d_stage;
     void *x = s.d_x[which ? 1 - s.cur : s.cur];
     const int *perm = logical ? s.d_perm : nullptr;

@@ -650,10 +650,7 @@ static void ensure_dense(Net& n)
         list.push_back({(void **)&n.dzb, sizeof(bf16) * n.C * n.V});
         list.push_back({(void **)&n.dz4, sizeof(bf16) * 2 * n.V});
     }
-    const cudaError_t error = allocate_all(
-        list, [](void **p, size_t bytes) { return cudaMalloc(p, bytes); }, [](void *p) { cudaFree(p); });
-    if (error != cudaSuccess) (void)cudaGetLastError();     // reported here, not at the next launch
-    LGD_CHECK_CUDA(error);
+    LGD_CHECK_CUDA(allocate_all(list, malloc_on_first_use, [](void *p) { cudaFree(p); }));
 }
 
 // the network's channel count is a template parameter of the kernels; the
