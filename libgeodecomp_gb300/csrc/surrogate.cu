@@ -545,6 +545,15 @@ static int grid_blocks(long long n)
 
 // The weights as the operands of the path that runs (fast: tcgen05, else
 // mma.sync), after they have changed.  The other path's are packed when it runs.
+// What a caller captures into a graph has not run yet, and may run any number of
+// times: it leaves the flags as they are.
+static bool capturing(const Net& n)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    LGD_CHECK_CUDA(cudaStreamIsCapturing(n.stream, &status));
+    return status != cudaStreamCaptureStatusNone;
+}
+
 static void ensure_packed(Net& n, bool fast)
 {
     bool& stale = fast ? n.tc_stale : n.frag_stale;
@@ -565,13 +574,16 @@ static void ensure_packed(Net& n, bool fast)
         check_launch("pack fragments");
     }
     ++n.launches;
-    stale = false;
+    stale = capturing(n);
 }
 
+// after the parameters have changed; a graph that changes them packs for both paths
 static void repack(Net& n)
 {
     n.frag_stale = n.tc_stale = true;
-    ensure_packed(n, n.fast && n.variant == 0);
+    const bool now = n.fast && n.variant == 0;
+    ensure_packed(n, now);
+    if (n.fast && capturing(n)) ensure_packed(n, !now);
 }
 
 // waits for the stream, then reports (and clears) a wait that gave up

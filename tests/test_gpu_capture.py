@@ -67,3 +67,47 @@ def test_mma_sync_forward_captured():
                 net.synchronize()
             out.append(du.cpu().numpy())
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+def test_packed_weights_of_a_graph_count_when_it_runs(variant):
+    """A captured first use of a path that is not replayed packs nothing, and a
+    captured update reaches the path that did not record it."""
+    from libgeodecomp_gb300 import surrogate
+    shape = (3, 8, 32)
+    u, k, t = (torch.rand((1,) + shape, device="cuda") for _ in range(3))
+    du, ref = torch.zeros_like(u), torch.zeros_like(u)
+    torch.cuda.synchronize()
+    with surrogate.SurrogateNet(shape, training=True) as net, surrogate.SurrogateNet(shape) as plain:
+        net.set_variant(1 - variant)
+        net.set_params(surrogate.init_params(24, 1))
+        stream = torch.cuda.ExternalStream(net.stream())
+        net.set_variant(variant)
+        unused = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(unused, stream=stream):
+            net.forward(u, k, du)
+        del unused
+
+        def compare():
+            net.set_variant(variant)
+            net.forward(u, k, du)
+            plain.set_variant(variant)
+            plain.set_params(net.get_params())
+            plain.forward(u, k, ref)
+            plain.synchronize()
+            np.testing.assert_array_equal(du.cpu().numpy(), ref.cpu().numpy())
+
+        compare()
+        before = net.get_params()
+        net.backward(t)
+        net.set_variant(1 - variant)
+        net.forward(u, k, du)
+        update = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(update, stream=stream):
+            net.adam(0.01)
+        compare()                                   # captured only: nothing has changed
+        update.replay()
+        torch.cuda.synchronize()
+        assert np.abs(net.get_params() - before).max() > 1e-3
+        compare()
+        del update
