@@ -45,7 +45,11 @@ int lgd_lbm_step_looped(lgd_lbm *h, int steps);
 
 /* Single steps by the persistent kernel with this launch shape: tile_rows
  * rows of one z plane per work item, threads per CTA (64..1024, power of
- * two), resident CTAs per SM (clamped to the occupancy limit). */
+ * two), resident CTAs per SM (clamped to the occupancy limit).  The shape
+ * 1, 128, 32 stands for one thread per cell instead (the default, where there
+ * is room for its table of a 48-byte entry per 128 cells); get_config reports
+ * it as that, so that a shape that was read can be set again, on this ensemble
+ * or another. */
 int lgd_lbm_set_config(lgd_lbm *h, int tile_rows, int threads, int ctas_per_sm);
 int lgd_lbm_get_config(lgd_lbm *h, int *tile_rows, int *threads, int *ctas_per_sm);
 

@@ -392,6 +392,9 @@ __global__ void lbm_persistent_kernel(const LbmInstance *__restrict__ inst, cons
 // cell's loads, collide, store, and only then load again; with 38 streams that
 // left DRAM at 5.0 of 6.8 TB/s whatever the registers, warps and item shapes.
 constexpr int FLAT = 128;
+// how a launch shape says it: more CTAs of 128 threads than an SM holds, which a
+// persistent shape is clamped to and never reports
+constexpr int FLAT_ROWS = 1, FLAT_CTAS = 32;
 
 struct FlatBlock {
     long long base;
@@ -990,6 +993,13 @@ static void set_config(Lbm& e, int ty, int threads, int ctas)
     rebuild_graph(e);
 }
 
+static void report_config(const Lbm& e, int *tile_rows, int *threads, int *ctas_per_sm)
+{
+    if (tile_rows) *tile_rows = e.flat ? FLAT_ROWS : e.ty;
+    if (threads) *threads = e.flat ? FLAT : e.threads;
+    if (ctas_per_sm) *ctas_per_sm = e.flat ? FLAT_CTAS : e.ctas_per_sm;
+}
+
 static void run_steps(Lbm& e, int steps)
 {
     if (e.depth == 2) {
@@ -1035,6 +1045,118 @@ static void run_steps(Lbm& e, int steps)
         ++e.launches;
         e.cur = 1;
     }
+}
+
+// the fastest kernel of single steps, then of two steps per launch; returns its
+// milliseconds per step
+static double tune(Lbm& e, int trial_steps)
+{
+    struct Events {
+        cudaEvent_t t[2] = {};
+        ~Events()
+        {
+            for (cudaEvent_t ev : t) {
+                if (ev) cudaEventDestroy(ev);
+            }
+        }
+    } events;
+    for (cudaEvent_t& ev : events.t) LGD_CHECK_CUDA(cudaEventCreate(&ev));
+    const cudaEvent_t t0 = events.t[0], t1 = events.t[1];
+    // the trial runs advance the ensemble: callers reset or upload afterwards
+    auto measure = [&](int ty, int th, int ct) -> double {
+        int fits = 0;
+        LGD_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fits, persistent_fn(e), th, 0));
+        if (fits < 1) return std::numeric_limits<double>::infinity();   // too many registers for th threads
+        set_config(e, ty, th, ct);
+        run_steps(e, 2);   // warm
+        LGD_CHECK_CUDA(cudaEventRecord(t0, e.stream));
+        run_steps(e, trial_steps);
+        LGD_CHECK_CUDA(cudaEventRecord(t1, e.stream));
+        LGD_CHECK_CUDA(cudaEventSynchronize(t1));
+        float ms = 0.f;
+        LGD_CHECK_CUDA(cudaEventElapsedTime(&ms, t0, t1));
+        return ms / trial_steps;
+    };
+    // one thread per cell, then a pattern search over (log2 tile rows,
+    // log2 threads, CTAs per SM)
+    const bool flat = e.d_blocks != nullptr;
+    e.flat = flat;
+    const double flat_ms = measure(e.ty, e.threads, e.ctas_per_sm);
+    e.flat = false;
+    const int tys[] = {1, 2, 4, 8, 16, 32};
+    const int ths[] = {128, 256, 512};
+    const int cts[] = {1, 2, 3, 4, 6, 8};
+    int a = 2, b = 1, c = 3;   // start at (4, 256, 4)
+    double best = measure(tys[a], ths[b], cts[c]);
+    bool moved = true;
+    int evals = 1;
+    while (moved && evals < 40) {
+        moved = false;
+        const int da[6] = {-1, 1, 0, 0, 0, 0};
+        const int db[6] = {0, 0, -1, 1, 0, 0};
+        const int dc[6] = {0, 0, 0, 0, -1, 1};
+        int ba = a, bb = b, bc = c;
+        for (int k = 0; k < 6; ++k) {
+            const int na = a + da[k], nb = b + db[k], nc = c + dc[k];
+            if (na < 0 || na >= 6 || nb < 0 || nb >= 3 || nc < 0 || nc >= 6) continue;
+            const double t = measure(tys[na], ths[nb], cts[nc]);
+            ++evals;
+            if (t < best * 0.99) {
+                best = t;
+                ba = na;
+                bb = nb;
+                bc = nc;
+                moved = true;
+            }
+        }
+        a = ba;
+        b = bb;
+        c = bc;
+    }
+    // the first measurement pays for the ensemble's first steps: repeated
+    e.flat = flat;
+    const double flat_best = std::min(flat_ms, measure(tys[a], ths[b], cts[c]));
+    e.flat = flat && flat_best <= best;
+    best = std::min(best, flat_best);
+    set_config(e, tys[a], ths[b], cts[c]);
+    // then temporal blocking: two steps per launch in each tile shape
+    // and residency; the fastest per step wins, one step per launch
+    // included (the reference's autotuner tunes the pipeline length of
+    // its cache-blocking simulator the same way,
+    // misc/cacheblockingsimulationfactory.h:26-28)
+    e.depth = 1;
+    int best_depth = 1, best_shape = 0, best_ctas = 1;
+    for (int shape = 0; shape < TB2_SHAPES; ++shape) {
+        int threads = 0;
+        size_t smem = 0;
+        const void *fn = tb2_kernel(e, shape, &threads, &smem);
+        const int per_sm = tb2_resident(fn, threads, smem);
+        for (int ct = 1; ct <= std::min(per_sm, 8); ++ct) {
+            e.depth = 2;
+            e.tb_shape = shape;
+            e.tb_ctas = ct;
+            run_steps(e, 2);   // warm (builds the columns)
+            const int n = 2 * ((trial_steps + 1) / 2);
+            LGD_CHECK_CUDA(cudaEventRecord(t0, e.stream));
+            run_steps(e, n);
+            LGD_CHECK_CUDA(cudaEventRecord(t1, e.stream));
+            LGD_CHECK_CUDA(cudaEventSynchronize(t1));
+            float ms = 0.f;
+            LGD_CHECK_CUDA(cudaEventElapsedTime(&ms, t0, t1));
+            const double t = ms / n;
+            if (t < best * 0.99) {
+                best = t;
+                best_depth = 2;
+                best_shape = shape;
+                best_ctas = ct;
+            }
+        }
+    }
+    e.depth = best_depth;
+    e.tb_shape = best_shape;
+    e.tb_ctas = best_ctas;
+    LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
+    return best;
 }
 
 static void lbm_free(Lbm& e)
@@ -1164,9 +1286,10 @@ int lgd_lbm_set_config(lgd_lbm *h, int tile_rows, int threads, int ctas_per_sm)
     return guard([&] {
         Lbm& e = lbm_of(h);
         const bool before = e.flat;
-        e.flat = false;
+        e.flat = e.d_blocks != nullptr && tile_rows == FLAT_ROWS && threads == FLAT && ctas_per_sm == FLAT_CTAS;
         try {
-            set_config(e, tile_rows, threads, ctas_per_sm);
+            if (e.flat) rebuild_graph(e);
+            else set_config(e, tile_rows, threads, ctas_per_sm);
         } catch (...) {
             e.flat = before;
             throw;
@@ -1177,10 +1300,7 @@ int lgd_lbm_set_config(lgd_lbm *h, int tile_rows, int threads, int ctas_per_sm)
 int lgd_lbm_get_config(lgd_lbm *h, int *tile_rows, int *threads, int *ctas_per_sm)
 {
     return guard([&] {
-        Lbm& e = lbm_of(h);
-        if (tile_rows) *tile_rows = e.ty;
-        if (threads) *threads = e.threads;
-        if (ctas_per_sm) *ctas_per_sm = e.ctas_per_sm;
+        report_config(lbm_of(h), tile_rows, threads, ctas_per_sm);
     });
 }
 
@@ -1189,108 +1309,22 @@ int lgd_lbm_tune(lgd_lbm *h, int trial_steps, int *tile_rows, int *threads, int 
     return guard([&] {
         Lbm& e = lbm_of(h);
         LGD_REQUIRE(trial_steps >= 2, LGD_ERR_INVALID, "trial_steps must be at least 2");
-        cudaEvent_t t0, t1;
-        LGD_CHECK_CUDA(cudaEventCreate(&t0));
-        LGD_CHECK_CUDA(cudaEventCreate(&t1));
-        // the trial runs advance the ensemble: callers reset or upload afterwards
-        auto measure = [&](int ty, int th, int ct) -> double {
-            int fits = 0;
-            LGD_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fits, persistent_fn(e), th, 0));
-            if (fits < 1) return std::numeric_limits<double>::infinity();   // too many registers for th threads
-            set_config(e, ty, th, ct);
-            run_steps(e, 2);   // warm
-            LGD_CHECK_CUDA(cudaEventRecord(t0, e.stream));
-            run_steps(e, trial_steps);
-            LGD_CHECK_CUDA(cudaEventRecord(t1, e.stream));
-            LGD_CHECK_CUDA(cudaEventSynchronize(t1));
-            float ms = 0.f;
-            LGD_CHECK_CUDA(cudaEventElapsedTime(&ms, t0, t1));
-            return ms / trial_steps;
-        };
-        // one thread per cell, then a pattern search over (log2 tile rows,
-        // log2 threads, CTAs per SM)
-        const bool flat = e.d_blocks != nullptr;
-        e.flat = flat;
-        const double flat_ms = measure(e.ty, e.threads, e.ctas_per_sm);
-        e.flat = false;
-        const int tys[] = {1, 2, 4, 8, 16, 32};
-        const int ths[] = {128, 256, 512};
-        const int cts[] = {1, 2, 3, 4, 6, 8};
-        int a = 2, b = 1, c = 3;   // start at (4, 256, 4)
-        double best = measure(tys[a], ths[b], cts[c]);
-        bool moved = true;
-        int evals = 1;
-        while (moved && evals < 40) {
-            moved = false;
-            const int da[6] = {-1, 1, 0, 0, 0, 0};
-            const int db[6] = {0, 0, -1, 1, 0, 0};
-            const int dc[6] = {0, 0, 0, 0, -1, 1};
-            int ba = a, bb = b, bc = c;
-            for (int k = 0; k < 6; ++k) {
-                const int na = a + da[k], nb = b + db[k], nc = c + dc[k];
-                if (na < 0 || na >= 6 || nb < 0 || nb >= 3 || nc < 0 || nc >= 6) continue;
-                const double t = measure(tys[na], ths[nb], cts[nc]);
-                ++evals;
-                if (t < best * 0.99) {
-                    best = t;
-                    ba = na;
-                    bb = nb;
-                    bc = nc;
-                    moved = true;
-                }
+        const bool flat = e.flat;
+        const int depth = e.depth;
+        double best = 0.0;
+        try {
+            best = tune(e, trial_steps);
+        } catch (...) {
+            // the kernels as they were (the persistent kernel's shape is the search's last)
+            e.flat = flat;
+            e.depth = depth;
+            try {
+                rebuild_graph(e);
+            } catch (...) {
             }
-            a = ba;
-            b = bb;
-            c = bc;
+            throw;
         }
-        // the first measurement pays for the ensemble's first steps: repeated
-        e.flat = flat;
-        const double flat_best = std::min(flat_ms, measure(tys[a], ths[b], cts[c]));
-        e.flat = flat && flat_best <= best;
-        best = std::min(best, flat_best);
-        set_config(e, tys[a], ths[b], cts[c]);
-        // then temporal blocking: two steps per launch in each tile shape
-        // and residency; the fastest per step wins, one step per launch
-        // included (the reference's autotuner tunes the pipeline length of
-        // its cache-blocking simulator the same way,
-        // misc/cacheblockingsimulationfactory.h:26-28)
-        e.depth = 1;
-        int best_depth = 1, best_shape = 0, best_ctas = 1;
-        for (int shape = 0; shape < TB2_SHAPES; ++shape) {
-            int threads = 0;
-            size_t smem = 0;
-            const void *fn = tb2_kernel(e, shape, &threads, &smem);
-            const int per_sm = tb2_resident(fn, threads, smem);
-            for (int ct = 1; ct <= std::min(per_sm, 8); ++ct) {
-                e.depth = 2;
-                e.tb_shape = shape;
-                e.tb_ctas = ct;
-                run_steps(e, 2);   // warm (builds the columns)
-                const int n = 2 * ((trial_steps + 1) / 2);
-                LGD_CHECK_CUDA(cudaEventRecord(t0, e.stream));
-                run_steps(e, n);
-                LGD_CHECK_CUDA(cudaEventRecord(t1, e.stream));
-                LGD_CHECK_CUDA(cudaEventSynchronize(t1));
-                float ms = 0.f;
-                LGD_CHECK_CUDA(cudaEventElapsedTime(&ms, t0, t1));
-                const double t = ms / n;
-                if (t < best * 0.99) {
-                    best = t;
-                    best_depth = 2;
-                    best_shape = shape;
-                    best_ctas = ct;
-                }
-            }
-        }
-        e.depth = best_depth;
-        e.tb_shape = best_shape;
-        e.tb_ctas = best_ctas;
-        LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
-        cudaEventDestroy(t0);
-        cudaEventDestroy(t1);
-        if (tile_rows) *tile_rows = e.ty;
-        if (threads) *threads = e.threads;
-        if (ctas_per_sm) *ctas_per_sm = e.ctas_per_sm;
+        report_config(e, tile_rows, threads, ctas_per_sm);
         if (best_ms) *best_ms = best;
     });
 }

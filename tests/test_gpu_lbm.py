@@ -185,3 +185,34 @@ def test_lbm_tuner_reports_depth_and_results_stay_exact():
             e.set_time_block(3, 0, 1)
         with pytest.raises(lgd.LGDError):
             e.set_time_block(2, 2, 1)
+
+
+def test_lbm_a_reported_launch_shape_selects_the_same_kernel():
+    """What get_config and tune report, set again on this ensemble or another,
+    is reported again: the kernel with one thread per cell as 1, 128, 32, which
+    a persistent shape (at most 16 CTAs of 128 threads fit an SM) never is."""
+    edges, omegas = [20, 24, 33], [1.1, 1.3, 1.7]
+    with lgd.LbmEnsemble(edges, omegas) as a, lgd.LbmEnsemble(edges, omegas) as b:
+        default = a.config()
+        assert default == (1, 128, 32)
+        a.set_config(*default)
+        assert a.config() == default
+        a.set_config(1, 128, 16)
+        persistent = a.config()
+        assert persistent[:2] == (1, 128) and 1 <= persistent[2] <= 16
+        with pytest.raises(lgd.LGDError):
+            a.set_config(0, 128, 32)
+        assert a.config() == persistent
+        a.set_config(*default)
+        assert a.config() == default
+        shape, _ = a.tune(trial_steps=2)
+        assert a.config() == shape
+        b.set_config(4, 256, 4)
+        b.set_config(*shape)
+        b.set_time_block(*a.time_block())
+        assert b.config() == shape
+        for e in (a, b):
+            e.reset()
+            e.step(7)
+        for j in range(len(edges)):
+            np.testing.assert_array_equal(a.download(j), b.download(j))
