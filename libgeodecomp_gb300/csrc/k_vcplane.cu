@@ -9,17 +9,22 @@
 //
 // FP64 is bound by the FP64 pipe, so of the cell's 30 operations it keeps 11, bit
 // for bit: the face to the plane below is the exact negative of the face the
-// thread took to its top neighbour one plane earlier (a sum does not see the sign
-// of a zero), and (k + k') / 2 of the other five and its product with the
-// difference of u are integer sums and products.  Where that does not hold the cell
-// is computed as written.
+// thread took to its top neighbour one plane earlier, and (k + k') / 2 of the other
+// five and its product with the difference of u are integer sums and products.
+// Where that does not hold for some cell of a warp (coefficients of zero, negative,
+// at the ends of the range or more than nine binary exponents from a neighbour's,
+// differences of u at the ends of the range), the warp computes this plane and its
+// next ones as written, 26 operations a cell: trying each plane again cost such grids
+// more than the pair kernel below (256^3 with half of the coefficients zero, of both
+// signs or 2^20 apart 1450 us against its 889; now 880, and 679 with insulating blocks).
+// The votes that this takes cost a field that never fails 7% (256^3 380 -> 406 us).
 //
-// us per step with 11 operations on the FP64 pipe (in brackets with the products,
-// 16, with the sums too, 21; then the pair kernel of k_stencil.cu: two x cells per
-// lane, whose blocks at a grid's ragged end loaded cell by cell): FP64 64^3 9.4 (12,
-// 14, 70), 101 x 77 x 60 14 (19, 24, 246), 128^3 52 (74, 89, 133), 256^3 380 (530,
-// 685, 888): 44.2 GLUPS x 11 operations = 486 G/s of the pipe's 498; FP32 101 x 77
-// x 60 4.3 (162), 253 x 250 x 250 68 (517).
+// us per step (in brackets the pair kernel of k_stencil.cu: two x cells per lane,
+// whose blocks at a grid's ragged end loaded cell by cell): FP64 64^3 10.2 (70), 101 x
+// 77 x 60 15.6 (246), 128^3 56 (133), 256^3 406 (888): 41.3 GLUPS x 11 operations =
+// 454 G/s of the pipe's 498; FP32 101 x 77 x 60 4.3 (162), 253 x 250 x 250 68 (517).
+// Without the votes the products in integers gave 256^3 530 -> 380, the sums before
+// them 685 -> 530.
 #include <algorithm>
 
 #include "lgd_internal.h"
@@ -31,15 +36,25 @@ namespace vcp {
 
 constexpr int THREADS = 128;
 
-// fl((a + b) / 2) of positive doubles in integer arithmetic, as sum4 (k_fp64.cuh)
-// adds, b possibly +0 (a zero edge coefficient: then the half is a subtraction from
-// the exponent); ok becomes false where that does not hold: other signs, more
-// than nine binary exponents apart and the ends of the exponent range
-__device__ __forceinline__ double half_sum(double a, double b, bool& ok)
+// whether half_sum takes a and b
+__device__ __forceinline__ bool summable(double a, double b)
 {
     const unsigned ha = (unsigned)__double2hiint(a), hb = (unsigned)__double2hiint(b);
     const unsigned e0 = min(ha, hb) >> 20;
     const unsigned sa = (ha >> 20) - e0, sb = (hb >> 20) - e0;          // one of them 0
+    const bool alone = (hb | (unsigned)__double2loint(b)) == 0u;
+    return alone ? (ha >> 20) - 3u < 2030u : (sa | sb) <= 9u && e0 - 3u < 2030u;
+}
+
+// fl((a + b) / 2) of positive doubles in integer arithmetic, as sum4 (k_fp64.cuh)
+// adds, b possibly +0 (a zero edge coefficient: then the half is a subtraction from
+// the exponent).  Not (summable) for other signs, more than nine binary exponents
+// apart and the ends of the exponent range.
+__device__ __forceinline__ double half_sum(double a, double b)
+{
+    const unsigned ha = (unsigned)__double2hiint(a), hb = (unsigned)__double2hiint(b);
+    const unsigned e0 = min(ha, hb) >> 20;
+    const unsigned sa = (ha >> 20) - e0, sb = (hb >> 20) - e0;
     const unsigned ma = (ha & 0xfffffu) | 0x100000u, mb = (hb & 0xfffffu) | 0x100000u;
     const unsigned la = (unsigned)__double2loint(a), lb = (unsigned)__double2loint(b);
     unsigned long long s = (((unsigned long long)__funnelshift_l(la, ma, sa) << 32) | (la << (sa & 31u))) +
@@ -49,7 +64,6 @@ __device__ __forceinline__ double half_sum(double a, double b, bool& ok)
     s += (unit >> 1) - 1u + (((unsigned)s >> (k & 31u)) & 1u);
     // s >> k holds the leading bit, which adds one to the exponent field; the half takes it off again
     const bool alone = (hb | lb) == 0u;
-    ok = ok && (alone ? (ha >> 20) - 3u < 2030u : (sa | sb) <= 9u && e0 - 3u < 2030u);
     const double half = __longlong_as_double((long long)((s >> (k & 31u)) + ((unsigned long long)(e0 + k - 2u) << 52)));
     return alone ? __hiloint2double((int)(ha - 0x00100000u), (int)la) : half;
 }
@@ -77,16 +91,26 @@ __device__ __forceinline__ double product(double a, double b, bool& ok)
     return zero ? b : r;
 }
 
-// the cell as written (a call: predicated, its operations would be paid always)
-__device__ __noinline__ double plain(double uc, double kc, double uw, double kw, double ue, double ke, double un, double kn,
-                                     double us, double ks, double ub, double kb, double ut, double kt)
+// the cell as written (a call: predicated, its operations would be paid always),
+// given the face to the plane below
+struct Written {
+    double r, above;        // the cell, the face to the plane above
+};
+__device__ __noinline__ Written as_written(double uc, double kc, double uw, double kw, double ue, double ke, double un, double kn,
+                                           double us, double ks, double below, double ut, double kt)
 {
-    return VarCoef<double>::apply(uc, kc, uw, kw, ue, ke, un, kn, us, ks, ub, kb, ut, kt);
+    double flux = VarCoef<double>::face(uc, kc, uw, kw);
+    flux = __dadd_rn(flux, VarCoef<double>::face(uc, kc, ue, ke));
+    flux = __dadd_rn(flux, VarCoef<double>::face(uc, kc, un, kn));
+    flux = __dadd_rn(flux, VarCoef<double>::face(uc, kc, us, ks));
+    flux = __dadd_rn(flux, below);
+    const double above = VarCoef<double>::face(uc, kc, ut, kt);
+    return {__dadd_rn(uc, __dadd_rn(flux, above)), above};
 }
 
-__device__ __noinline__ double plain_face(double uc, double kc, double un, double kn)
+__device__ __forceinline__ bool same_bits(double a, double b)
 {
-    return VarCoef<double>::face(uc, kc, un, kn);
+    return __double_as_longlong(a) == __double_as_longlong(b);
 }
 
 template<typename R>
@@ -105,7 +129,8 @@ varcoef_plane_kernel(const Args<R> a)
     dependent_start();
     const int nx = a.nx, ny = a.ny, nz = a.nz;
     const unsigned c = blockIdx.x * THREADS + threadIdx.x;
-    if (c >= (unsigned)nx * (unsigned)ny) return;           // below 2^31 (host rule)
+    const unsigned lanes = __ballot_sync(0xffffffffu, c < (unsigned)nx * (unsigned)ny);     // below 2^31 (host rule)
+    if (c >= (unsigned)nx * (unsigned)ny) return;
     const int y = (int)(c / (unsigned)nx);
     const int x = (int)(c - (unsigned)y * (unsigned)nx);
     const int z0 = blockIdx.y * a.zchunk;
@@ -126,8 +151,9 @@ varcoef_plane_kernel(const Args<R> a)
         ub = has ? u[d] : a.edge_u;
         kb = has ? k[d] : a.edge_k;
     }
-    R fb = 0;                                               // FP64: the face from the plane below to this one
-    if constexpr (sizeof(R) == 8) fb = VarCoef<R>::face(ub, kb, uc, kc);
+    R below = 0;                                            // FP64: the face to the plane below
+    if constexpr (sizeof(R) == 8) below = VarCoef<R>::face(uc, kc, ub, kb);
+    bool written = false;       // a cell of the warp was computed as written: so are all of its next ones
 #pragma unroll 1
     for (int z = z0; z < z1; ++z) {
         const bool has = z + 1 < nz || wrap_z;
@@ -139,22 +165,31 @@ varcoef_plane_kernel(const Args<R> a)
         const R uw = has_w ? u[west] : a.edge_u, kw = has_w ? k[west] : a.edge_k;
         R r;
         if constexpr (sizeof(R) == 8) {
-            bool ok = true;
-            auto face = [&](double un, double kn) {
-                return product(half_sum(kc, kn, ok), __dadd_rn(un, -uc), ok);
-            };
-            double flux = face(uw, kw);
-            flux = __dadd_rn(flux, face(ue, ke));
-            flux = __dadd_rn(flux, face(un, kn));
-            flux = __dadd_rn(flux, face(us, ks));
-            flux = __dadd_rn(flux, -fb);
-            double ft = face(ut, kt);
-            r = __dadd_rn(uc, __dadd_rn(flux, ft));
-            if (!ok) {
-                r = plain(uc, kc, uw, kw, ue, ke, un, kn, us, ks, ub, kb, ut, kt);
-                ft = plain_face(uc, kc, ut, kt);
+            double above = 0.0;
+            if (!written) {
+                written = __any_sync(lanes, !(summable(kc, kw) && summable(kc, ke) && summable(kc, kn) && summable(kc, ks) &&
+                                              summable(kc, kt)));
             }
-            fb = ft;
+            if (!written) {
+                bool ok = true;
+                auto face = [&](double un, double kn) { return product(half_sum(kc, kn), __dadd_rn(un, -uc), ok); };
+                double flux = face(uw, kw);
+                flux = __dadd_rn(flux, face(ue, ke));
+                flux = __dadd_rn(flux, face(un, kn));
+                flux = __dadd_rn(flux, face(us, ks));
+                flux = __dadd_rn(flux, below);
+                above = face(ut, kt);
+                r = __dadd_rn(uc, __dadd_rn(flux, above));
+                written = __any_sync(lanes, !ok);
+            }
+            if (written) {
+                const Written w = as_written(uc, kc, uw, kw, ue, ke, un, kn, us, ks, below, ut, kt);
+                r = w.r;
+                above = w.above;
+            }
+            // the same face from its other side: the difference of u is the exact
+            // negative, but for equal values (+0, or NaN, from both sides)
+            below = same_bits(ut, uc) ? above : -above;
         } else {
             r = VarCoef<R>::apply(uc, kc, uw, kw, ue, ke, un, kn, us, ks, ub, kb, ut, kt);
         }

@@ -1,0 +1,45 @@
+"""The default kernel is not the slower one where another can be selected for
+the same call: the least of several timings each, with room for their spread."""
+import time
+
+import numpy as np
+import pytest
+
+from libgeodecomp_gb300 import lgd
+
+pytestmark = pytest.mark.gpu
+
+
+def least(grid, steps, setups, rounds=5):
+    """Seconds per call of steps steps, the least of rounds timings, for each setup in turn."""
+    best = [float("inf")] * len(setups)
+    for _ in range(rounds):
+        for i, setup in enumerate(setups):
+            setup(grid)
+            grid.step(steps)
+            grid.synchronize()
+            t = time.perf_counter()
+            grid.step(steps)
+            grid.synchronize()
+            best[i] = min(best[i], time.perf_counter() - t)
+    return best
+
+
+@pytest.mark.parametrize("kind", ["zeros", "blocks", "both signs"])
+def test_fp64_varcoef_of_any_coefficients(kind):
+    """Against the pair kernel, whose time does not depend on them."""
+    shape = (128, 128, 128)
+    rng = np.random.default_rng(1)
+    k = 0.02 + 0.13 * rng.random(shape)
+    if kind == "zeros":
+        k[rng.random(shape) < 0.5] = 0.0
+    elif kind == "blocks":
+        k[:, 64:] = 0.0
+        k[64:, :, :32] = 0.0
+    else:
+        k -= 0.08
+    with lgd.Grid(lgd.CELL_VARCOEF_F64, shape, periodic=7) as g:
+        g.upload(0, rng.random(shape))
+        g.upload(1, k)
+        default, pair = least(g, 20, [lambda g: g.set_variant(0), lambda g: g.set_variant(2)])
+    assert default < 1.15 * pair

@@ -70,3 +70,32 @@ def test_fp32_ragged_rows(periodic, shape):
     edge = (0.25, 0.05, 0.0, 0.0)
     np.testing.assert_allclose(run(lgd.CELL_VARCOEF_F32, u, k, 3, 0, periodic, edge),
                                run(lgd.CELL_VARCOEF_F32, u, k, 3, 1, periodic, edge), rtol=0, atol=40 * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("kind", ["zeros", "blocks", "both signs", "far apart", "one cell"])
+@pytest.mark.parametrize("periodic", [0, 7])
+def test_fp64_warps_that_fall_back(kind, periodic):
+    """Grids whose threads march several planes (chunks of 8 here), where a warp
+    computes planes as written after some that it did not: every bit that of
+    variant 1, signs of zeros too."""
+    shape = (100, 128, 128)
+    rng = np.random.default_rng(6)
+    u, k = fields(shape, 6)
+    u[rng.random(shape) < 0.2] = 0.0
+    u[rng.random(shape) < 0.2] *= -1.0              # and -0
+    u[20:40, 20:60] = -0.0
+    if kind == "zeros":
+        k[rng.random(shape) < 0.5] = 0.0
+    elif kind == "blocks":
+        k[30:50, 10:70] = 0.0
+        k[60:, :, 40:] = 0.0
+    elif kind == "both signs":
+        k[rng.random(shape) < 0.01] *= -1.0
+    elif kind == "far apart":
+        k[:, 40:] *= 2.0 ** -14
+        k[13:, :, 70:] *= 2.0 ** -20
+    else:
+        k[51, 64, 77] = -0.05
+    edge = (0.0, 0.07, 0.0, 0.0)
+    a, b = (run(lgd.CELL_VARCOEF_F64, u, k, 3, variant, periodic, edge) for variant in (0, 1))
+    np.testing.assert_array_equal(a.view(np.uint64), b.view(np.uint64))
