@@ -48,6 +48,7 @@
 #include "lgd_internal.h"
 #include "tc_common.cuh"
 #include "conv_tc.h"
+#include "z_chunks.h"
 
 namespace lgd {
 namespace sur {
@@ -637,24 +638,6 @@ __global__ void pack_kernel(const PackJobs jobs)
     }
 }
 
-// planes per CTA: waves of one CTA per SM times planes per CTA (two of them
-// halo, and about two planes' time to start and to drain)
-static int pick_zchunk(long long xy, int nz, int sms)
-{
-    int best_chunk = nz;
-    double best = 1e300;
-    for (int split = 1; split <= std::max(1, nz / 2); ++split) {
-        const int chunk = (nz + split - 1) / split;
-        const int c = (nz + chunk - 1) / chunk;
-        const double t = (double)((xy * c + sms - 1) / sms) * (chunk + 4);
-        if (t < best * 0.999) {
-            best = t;
-            best_chunk = chunk;
-        }
-    }
-    return best_chunk;
-}
-
 template<int SRC, int EPI, int TXW>
 static void run(Params p, cudaStream_t stream)
 {
@@ -669,7 +652,8 @@ static void run(Params p, cudaStream_t stream)
         return count;
     });
     const int bx = p.s.nx / TXW, by = (p.s.ny + G::TY - 1) / G::TY;
-    p.zchunk = pick_zchunk((long long)bx * by * p.s.batch, p.s.nz, sms);
+    // one CTA per SM; of its planes two are halo, and about two planes' time to start and to drain
+    p.zchunk = least_planes((long long)bx * by * p.s.batch, p.s.nz, sms, 4, nullptr);
     const int zsplit = (p.s.nz + p.zchunk - 1) / p.zchunk;
     launch_dependent(conv_tc_kernel<SRC, EPI, TXW>, dim3(bx, by, p.s.batch * zsplit), G::THREADS, G::SMEM, stream, p);
     check_launch("tensor-core convolution");

@@ -349,7 +349,7 @@ struct TbPlan {
 static TbPlan plan_tb(long long xy, int nz, long long resident, int halo)
 {
     TbPlan best = {nz, 1e300};
-    best.zchunk = tmak::least_planes(xy, nz, resident, halo, &best.planes);
+    best.zchunk = least_planes(xy, nz, resident, halo, &best.planes);
     return best;
 }
 

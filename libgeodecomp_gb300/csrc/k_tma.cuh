@@ -3,6 +3,7 @@
 #ifndef LGD_K_TMA_CUH
 #define LGD_K_TMA_CUH
 
+#include "z_chunks.h"
 #include <cuda.h>
 #include <stdint.h>
 
@@ -91,32 +92,6 @@ __device__ __forceinline__ void st_pair(void *p, T a, T b)
         v.y = *reinterpret_cast<const int *>(&b);
         *reinterpret_cast<int2 *>(p) = v;
     }
-}
-
-// Planes per CTA of a z-marching launch over xy tiles per plane: the least waves
-// of resident CTAs times planes per CTA (its chunk and halo planes), chunks of at
-// least two planes; that product into *planes.  Per number of waves the most
-// chunks are best, and more waves only add halo planes, so a few waves beyond the
-// fewest suffice (a grid of thousands of planes is planned as fast as a small one).
-inline int least_planes(long long xy, int nz, long long resident, int halo, double *planes)
-{
-    const long long cap = nz / 2 > 1 ? nz / 2 : 1;
-    const long long fewest = (xy + resident - 1) / resident;
-    int best_chunk = nz;
-    double best = 1e300;
-    for (long long w = fewest; w < fewest + 64; ++w) {
-        const long long split = w * resident / xy < cap ? w * resident / xy : cap;
-        const int chunk = (int)((nz + split - 1) / split);
-        const long long waves = (xy * ((nz + chunk - 1) / chunk) + resident - 1) / resident;
-        const double t = (double)waves * (chunk + halo);
-        if (t < best * 0.999) {
-            best = t;
-            best_chunk = chunk;
-        }
-        if (split == cap) break;
-    }
-    if (planes) *planes = best;
-    return best_chunk;
 }
 
 }  // namespace tmak

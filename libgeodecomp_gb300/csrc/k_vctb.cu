@@ -34,6 +34,7 @@
 
 #include "lgd_internal.h"
 #include "k_cells.cuh"
+#include "z_chunks.h"
 
 namespace lgd {
 namespace vctb {
@@ -245,13 +246,10 @@ static Plan plan(const Grid& g, double us_per_plane)
         return count * std::max(1, per_sm);
     });
     const long long xy = (long long)((g.desc.nx + OX - 1) / OX) * ((g.desc.ny + G::OY - 1) / G::OY);
-    Plan best = {g.desc.nz, 1e300};
-    for (int split = 1; split <= std::max(1, g.desc.nz / 4); ++split) {
-        const int chunk = (g.desc.nz + split - 1) / split;
-        const int s = (g.desc.nz + chunk - 1) / chunk;
-        const double t = (double)((xy * s + resident - 1) / resident) * (chunk + 5) * us_per_plane;
-        if (t < best.us * 0.999) best = {chunk, t};
-    }
+    Plan best;
+    double planes;
+    best.zchunk = least_planes(xy, g.desc.nz, resident, 5, &planes, 4);
+    best.us = planes * us_per_plane;
     return best;
 }
 
@@ -279,8 +277,8 @@ bool varcoef_tb2_applicable(const Grid& g)
 }
 
 // Two boxes: 48 rows, one CTA per SM, or 24 rows, two per SM (finer bands of
-// y); the one whose waves of CTAs times planes per CTA (four of them halo)
-// take less by the measured time per plane.
+// y); the one whose waves of CTAs times planes per CTA (five of them halo) take
+// less by the measured time per plane.
 void launch_varcoef_tb2(Grid& g)
 {
     const vctb::Plan tall = vctb::plan<12, 4, 1>(g, 1.17), low = vctb::plan<8, 3, 2>(g, 1.03);

@@ -40,6 +40,7 @@
 #include "lgd_internal.h"
 #include "tc_common.cuh"
 #include "conv_tc.h"
+#include "z_chunks.h"
 
 namespace lgd {
 namespace sur {
@@ -489,17 +490,8 @@ static int run_w(WParams p, cudaStream_t stream)
     });
     const int sms = sm_count();
     const long long cols = (long long)(p.s.nx / TXW) * ((p.s.ny + G::TY - 1) / G::TY) * p.s.batch;
-    double best = 1e300;
-    for (int split = 1; split <= std::max(1, p.s.nz / 2); ++split) {
-        const int chunk = (p.s.nz + split - 1) / split;
-        const long long items = cols * ((p.s.nz + chunk - 1) / chunk);
-        const double t = (double)((items + sms - 1) / sms) * (chunk + 2);
-        if (t < best * 0.999) {
-            best = t;
-            p.zchunk = chunk;
-            p.items = (int)items;
-        }
-    }
+    p.zchunk = least_planes(cols, p.s.nz, sms, 2, nullptr);
+    p.items = (int)(cols * ((p.s.nz + p.zchunk - 1) / p.zchunk));
     const int ctas = std::min(sms, p.items);
     launch_dependent(wgrad_tc_kernel<MODE, TXW>, dim3(ctas), WG_THREADS, G::SMEM, stream, p);
     check_launch("tensor-core weight gradient");
