@@ -695,7 +695,8 @@ void launch_varcoef(Grid& g, int steps)
     // FP32 grids and for FP64
     const bool tma = (g.variant == 6) || (g.variant == 0 && g.desc.cell == LGD_CELL_VARCOEF_F32);
     if (g.variant == 0 && g.time_block != 1 && varcoef_tb2_applicable(g)) {
-        for (; steps >= 2; steps -= 2) launch_varcoef_tb2(g);
+        const double single_us = g.time_block == 0 && varcoef_tma_applicable(g) ? varcoef_tma_us(g) : 0.0;
+        while (steps >= 2 && launch_varcoef_tb2(g, single_us)) steps -= 2;
     }
     if (tma && varcoef_tma_applicable(g)) {
         for (int s = 0; s < steps; ++s) launch_varcoef_tma(g);

@@ -573,6 +573,28 @@ bool varcoef_tma_applicable(const Grid& g)
 }
 
 template<typename R>
+static long long varcoef_tma_resident()
+{
+    static PerDevice<long long> setup;
+    return setup.get([] {
+        const int smem = tmak::VC_S * tmak::vc::Lay<R>::SLOT;
+        LGD_CHECK_CUDA(cudaFuncSetAttribute(tmak::varcoef_tma_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        return tmak::resident_ctas((const void *)tmak::varcoef_tma_kernel<R>, tmak::THREADS, smem);
+    });
+}
+
+// FP32: waves of CTAs times planes per CTA, two of them halo, at 1.1 us a plane (as
+// fitted beside the two-step pass, see launch_varcoef_tb2), 0.9 where a plane fills less
+// than a quarter of one box (100000 x 4 x 4: single steps 169 us, two per pass 189)
+double varcoef_tma_us(const Grid& g)
+{
+    const long long xy = (long long)((g.desc.nx + tmak::TX - 1) / tmak::TX) * ((g.desc.ny + tmak::TY - 1) / tmak::TY);
+    double planes;
+    least_planes(xy, g.desc.nz, varcoef_tma_resident<float>(), 2, &planes);
+    return planes * ((long long)g.desc.nx * g.desc.ny < tmak::TX * tmak::TY / 4 ? 0.9 : 1.1);
+}
+
+template<typename R>
 static void launch_varcoef_tma_typed(Grid& g, CUtensorMapDataType dt)
 {
     typedef tmak::Box<R> B;
@@ -592,11 +614,7 @@ static void launch_varcoef_tma_typed(Grid& g, CUtensorMapDataType dt)
         g.vtmap_base[src][1] = kbuf;
     }
     const int smem = tmak::VC_S * tmak::vc::Lay<R>::SLOT;
-    static PerDevice<long long> setup;
-    const long long resident = setup.get([smem] {
-        LGD_CHECK_CUDA(cudaFuncSetAttribute(tmak::varcoef_tma_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        return tmak::resident_ctas((const void *)tmak::varcoef_tma_kernel<R>, tmak::THREADS, smem);
-    });
+    const long long resident = varcoef_tma_resident<R>();
     const int bx = (g.desc.nx + tmak::TX - 1) / tmak::TX;
     const int by = (g.desc.ny + tmak::TY - 1) / tmak::TY;
     const int zchunk = tmak::pick_zchunk((long long)bx * by, g.desc.nz, resident);

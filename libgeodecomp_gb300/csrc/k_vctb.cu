@@ -228,7 +228,8 @@ varcoef_tb2_kernel(const float *u, const float *k, float *out, long pitch, int n
 
 struct Plan {
     int zchunk;
-    double us;
+    double us;          // of a pass, with the input planes that only load counted in full
+    double pass_us;     // of a pass
 };
 
 template<int WY, int ROWS, int CTAS>
@@ -250,6 +251,8 @@ static Plan plan(const Grid& g, double us_per_plane)
     double planes;
     best.zchunk = least_planes(xy, g.desc.nz, resident, 5, &planes, 4);
     best.us = planes * us_per_plane;
+    const long long waves = (xy * ((g.desc.nz + best.zchunk - 1) / best.zchunk) + resident - 1) / resident;
+    best.pass_us = (double)waves * (best.zchunk + 2.5) * us_per_plane;
     return best;
 }
 
@@ -278,12 +281,21 @@ bool varcoef_tb2_applicable(const Grid& g)
 
 // Two boxes: 48 rows, one CTA per SM, or 24 rows, two per SM (finer bands of
 // y); the one whose waves of CTAs times planes per CTA (five of them halo) take
-// less by the measured time per plane.
-void launch_varcoef_tb2(Grid& g)
+// less by the measured time per plane.  Beside two single steps of single_us by the
+// TMA kernel's 64 x 16 boxes, which waste less of thin grids, where the caller asked
+// for no depth: false (nothing launched) where those take less.  us per step, two
+// steps per pass / single: 1 x 2048 x 4096 48 / 37, 256 x 1 x 4096 33 / 22, 3000 x 64 x
+// 64 41 / 32, but 256^3 30 / 40; of 250 grids of 1 to 4096 cells along an axis the rule is
+// 1% off the better one on average, and at the worst 25% (256 x 16 x 4096 34 / 42).
+bool launch_varcoef_tb2(Grid& g, double single_us)
 {
     const vctb::Plan tall = vctb::plan<12, 4, 1>(g, 1.17), low = vctb::plan<8, 3, 2>(g, 1.03);
-    if (tall.us <= low.us) vctb::launch<12, 4, 1>(g, tall.zchunk);
+    const vctb::Plan& best = tall.us <= low.us ? tall : low;
+    constexpr double LEAST_US = 4.0;            // any dependent launch
+    if (single_us > 0.0 && std::max(best.pass_us, LEAST_US) > 2.0 * std::max(single_us, LEAST_US)) return false;
+    if (&best == &tall) vctb::launch<12, 4, 1>(g, tall.zchunk);
     else vctb::launch<8, 3, 2>(g, low.zchunk);
+    return true;
 }
 
 }  // namespace lgd

@@ -228,9 +228,10 @@ bool tma_applicable(const Grid& g);
 void launch_jacobi7_tma(Grid& g);
 bool varcoef_tma_applicable(const Grid& g);
 void launch_varcoef_tma(Grid& g);
+double varcoef_tma_us(const Grid& g);       // a step's modelled time
 // two var-coef steps per pass (k_vctb.cu)
 bool varcoef_tb2_applicable(const Grid& g);
-void launch_varcoef_tb2(Grid& g);
+bool launch_varcoef_tb2(Grid& g, double single_us);
 
 // k_vcplane.cu: variable-coefficient diffusion, one cell of a plane per thread
 bool varcoef_plane_applicable(const Grid& g);

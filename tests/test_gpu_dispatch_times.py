@@ -43,3 +43,14 @@ def test_fp64_varcoef_of_any_coefficients(kind):
         g.upload(1, k)
         default, pair = least(g, 20, [lambda g: g.set_variant(0), lambda g: g.set_variant(2)])
     assert default < 1.15 * pair
+
+
+@pytest.mark.parametrize("shape", [(1, 2048, 4096), (256, 2, 4096), (3000, 64, 64), (256, 256, 256), (40, 33, 64)])
+def test_fp32_varcoef_of_any_shape(shape):
+    """Two steps per pass where that is the faster, against single steps."""
+    rng = np.random.default_rng(2)
+    with lgd.Grid(lgd.CELL_VARCOEF_F32, shape, periodic=7) as g:
+        g.upload(0, rng.random(shape))
+        g.upload(1, 0.1 * rng.random(shape))
+        default, single = least(g, 40, [lambda g: g.set_time_block(0), lambda g: g.set_time_block(1)])
+    assert default < 1.1 * single
