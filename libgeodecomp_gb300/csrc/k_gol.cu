@@ -293,12 +293,26 @@ gol_bits_kernel(const uint8_t *__restrict__ in, uint8_t *__restrict__ out, int n
 constexpr int GOL_BITS_DEFAULT_DEPTH = 16;
 
 // generations of a call from which the packed board pays for packing and
-// unpacking: on a torus of aligned rows (the alternative is a bit-sliced pass
-// over bytes), and on other boards (one launch per generation).  us per call,
-// packed against not: 8192^2 x 4 43 / 38, x 8 54 / 54, x 16 70 / 100; 1024^2 x
-// 4 11 / 15, x 16 12 / 83; 1001 x 777 x 4 17 / 34
-constexpr int GOL_PACK_MIN_TORUS = 6;
+// unpacking: on boards whose alternative is one launch per generation, and on a
+// torus of aligned rows, whose alternative is a bit-sliced pass over bytes.  us per
+// call, packed against not: 1001 x 777 x 4 17 / 34; 1024^2 x 6 10 / 21, 8192^2 x 6 44 /
+// 49, x 16 60 / 100.  Beyond L2 the passes over bytes, which do their few generations
+// in one read and write, win longer: 8192 x 16384 x 6 95 / 75, x 8 104 / 89, x 10 104 / 137; 23168^2 x 12 428 / 409, x
+// 14 464 / 586; 32768^2 x 16 1079 / 1011, x 20 1236 / 1449.  Boards of a few long rows
+// fill little of a tile of 32 rows or more: 1 x 1000000 x 8 15.6 / 11.5, x 16 25 / 26, 1 x
+// 4000000 x 32 132 / 120
 constexpr int GOL_PACK_MIN = 4;
+
+static int gol_pack_min(const Grid& g, bool aligned_torus)
+{
+    if (!aligned_torus) return GOL_PACK_MIN;
+    const int nx = g.desc.nx, ny = g.desc.ny;
+    const long long cells = (long long)nx * ny;
+    if (nx % 32 != 0) return 6;
+    if (ny < 16 && nx > 1 << 18) return ny < 4 && nx > 1 << 21 ? 96 : 16;
+    if (ny < 4) return 8;
+    return cells <= 1ll << 26 ? 6 : (cells < 1ll << 28 ? 10 : (cells < 1ll << 30 ? 14 : 20));
+}
 
 bool gol_tb_applicable(const Grid& g)
 {
@@ -465,7 +479,7 @@ void launch_gol(Grid& g, int steps)
     // counts cells by their byte values, so bytes other than 0 and 1 keep
     // their meaning, and leaves 0 and 1 behind
     const bool aligned_torus = gol_tb_applicable(g);
-    if (g.variant == 0 && g.time_block == 0 && steps >= (aligned_torus ? GOL_PACK_MIN_TORUS : GOL_PACK_MIN) &&
+    if (g.variant == 0 && g.time_block == 0 && steps >= gol_pack_min(g, aligned_torus) &&
         gol_packed_applicable(g) && gol_packed_ready(g)) {
         if (!aligned_torus) {
             gol_single(g, 1);

@@ -54,3 +54,14 @@ def test_fp32_varcoef_of_any_shape(shape):
         g.upload(1, 0.1 * rng.random(shape))
         default, single = least(g, 40, [lambda g: g.set_time_block(0), lambda g: g.set_time_block(1)])
     assert default < 1.1 * single
+
+
+@pytest.mark.parametrize("shape,steps", [((1, 1000000), 6), ((4, 1000000), 8), ((8192, 16384), 6), ((8192, 16384), 12),
+                                         ((1024, 1024), 6), ((16384, 16384), 8)])
+def test_gol_calls_of_a_few_generations(shape, steps):
+    """Packed rows where packing pays, against the bit-sliced passes over bytes."""
+    board = (np.random.default_rng(3).integers(0, 3, shape, dtype=np.uint8) == 0).astype(np.uint8)
+    with lgd.Grid(lgd.CELL_GOL_U8, shape, periodic=3) as g:
+        g.upload(0, board)
+        default, passes = least(g, steps, [lambda g: g.set_time_block(0), lambda g: g.set_time_block(16)], rounds=9)
+    assert default < 1.12 * passes
