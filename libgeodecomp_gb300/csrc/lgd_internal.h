@@ -140,13 +140,14 @@ void launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t 
 #ifdef __CUDACC__
 // In a kernel launched by launch_dependent, before its first access to memory
 // that an earlier kernel writes or reads: lets the next kernel be scheduled
-// and waits until the one before has finished.  What that kernel wrote must
+// (TRIGGER; else that waits for this one's end) and waits until the one before has finished.  What that kernel wrote must
 // be read by plain loads or TMA: read-only loads (__ldg, const __restrict__)
 // promise memory that does not change while the kernel is resident, and
 // resident it is before its predecessor's last store.
+template<bool TRIGGER = true>
 __device__ __forceinline__ void dependent_start()
 {
-    cudaTriggerProgrammaticLaunchCompletion();
+    if (TRIGGER) cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
     asm volatile("" ::: "memory");
 }

@@ -132,7 +132,7 @@ sell_diffusion_kernel(const int *__restrict__ chunk_offset, const int *__restric
 // sum runs in slot order, as in the kernel above.  The first slots' entries load
 // before the wait for the step before (2000 nodes FP64 7.4 -> 6.9 us per step,
 // 100003 14.9 -> 14.1, 4.19 M 203.5 -> 201.7).
-template<typename R, bool EXACT, int D>
+template<typename R, bool EXACT, int D, bool TRIGGER>
 __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offset, const int *__restrict__ row_length,
                                               const R *__restrict__ values, const int *__restrict__ column,
                                               const R *x, R *xn, int C, int row, int chunk)
@@ -153,7 +153,7 @@ __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offs
             cc[j] = __ldg(c + (long long)j * C);
         }
     }
-    dependent_start();          // the matrix does not change between steps, x does
+    dependent_start<TRIGGER>();          // the matrix does not change between steps, x does
     const R xr = x[row];
     R acc = (R)0;
     for (int k = 0; k < len; k += D) {
@@ -194,7 +194,7 @@ __device__ __forceinline__ void sell_pipe_row(const int *__restrict__ chunk_offs
 // Loads stay on the read-only path: hints that skip L1 on the gathers,
 // keep x in L2 with evict_last or stream the matrix with evict_first, and
 // an L2 bulk prefetch of each chunk, all measured slower.
-template<typename R, bool EXACT, int D, int THREADS>
+template<typename R, bool EXACT, int D, int THREADS, bool TRIGGER>
 __global__ void __launch_bounds__(THREADS)
 sell_diffusion_pipe_kernel(const int *__restrict__ chunk_offset, const int *__restrict__ row_length,
                            const R *__restrict__ values, const int *__restrict__ column,
@@ -202,7 +202,7 @@ sell_diffusion_pipe_kernel(const int *__restrict__ chunk_offset, const int *__re
 {
     const int row = row_begin + blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= row_end) return;
-    sell_pipe_row<R, EXACT, D>(chunk_offset, row_length, values, column, x, xn, C, row, row / C);
+    sell_pipe_row<R, EXACT, D, TRIGGER>(chunk_offset, row_length, values, column, x, xn, C, row, row / C);
 }
 
 // L lanes per row, for matrices that leave the GPU's warps idle: a row is a
@@ -311,12 +311,12 @@ static void sell_free(Sell& s)
     if (s.stream) cudaStreamDestroy(s.stream);
 }
 
-template<typename R, bool EXACT, int D, int THREADS>
+template<typename R, bool EXACT, int D, int THREADS, bool TRIGGER = true>
 static void launch_pipe(Sell& s, int row_begin, int row_end, const R *x, R *xn, const R *vals)
 {
     const int blocks = (row_end - row_begin + THREADS - 1) / THREADS;
     launch_dependent(
-        sell_diffusion_pipe_kernel<R, EXACT, D, THREADS>, dim3(blocks), THREADS, 0, s.stream, s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.n, s.C, row_begin, row_end);
+        sell_diffusion_pipe_kernel<R, EXACT, D, THREADS, TRIGGER>, dim3(blocks), THREADS, 0, s.stream, s.d_chunk_offset, s.d_row_length, vals, s.d_column, x, xn, s.n, s.C, row_begin, row_end);
 }
 
 constexpr int SELL_TEAM_MAX_ROWS = 200000;
@@ -356,11 +356,18 @@ static void launch_sell_typed(Sell& s, int row_begin, int row_end)
     case 4: launch_pipe<R, EXACT, 4, 256>(s, row_begin, row_end, x, xn, vals); break;
     case 5: launch_pipe<R, EXACT, 8, 64>(s, row_begin, row_end, x, xn, vals); break;
     default:
-        // small matrices: teams of lanes (FP32), deeper pipelines (FP64;
-        // 20000 nodes 8.6 us per step against 10.2, 400000 27.2 against
-        // 29.3, one million 61.6 against 60.6)
+        // small matrices: teams of lanes (FP32), deeper pipelines (FP64, us per
+        // step beside four deep: 20000 nodes 7.6 / 9.8, 400000 26.5 / 29.0, one
+        // million 61.4 / 59.7; exact 9.6 / 12.6, 41 / 45).  In FP64 the next step's
+        // CTAs are not placed while this one runs: they would go where there is
+        // room now, and pile up on some SMs, whose FP64 pipes the others then
+        // wait for (exact, 8 / 64 with that and 8 / 128 without: 30000 nodes
+        // 16.1 / 10.2, 60000 20.5 / 12.9, 100003 21.8 / 17.5, 250000 29.7 / 26.4; not
+        // exact, 60000 12.7 / 9.4)
         if (sizeof(R) == 4 && row_end - row_begin <= SELL_TEAM_MAX_ROWS) {
             launch_team<EXACT>(s, row_begin, row_end, (const float *)x, (float *)xn, (const float *)vals);
+        } else if (sizeof(R) == 8 && row_end - row_begin <= SELL_DEEP_MAX_ROWS) {
+            launch_pipe<R, EXACT, 8, 128, false>(s, row_begin, row_end, x, xn, vals);
         } else if (row_end - row_begin <= SELL_DEEP_MAX_ROWS) {
             launch_pipe<R, EXACT, 8, 64>(s, row_begin, row_end, x, xn, vals);
         } else {

@@ -5,7 +5,7 @@ import time
 import numpy as np
 import pytest
 
-from libgeodecomp_gb300 import lgd
+from libgeodecomp_gb300 import lgd, workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,17 @@ def test_gol_calls_of_a_few_generations(shape, steps):
         g.upload(0, board)
         default, passes = least(g, steps, [lambda g: g.set_time_block(0), lambda g: g.set_time_block(16)], rounds=9)
     assert default < 1.12 * passes
+
+
+@pytest.mark.parametrize("exact", [False, True])
+def test_fp64_sell_steps_grow_with_the_rows(exact):
+    """A step's CTAs spread over the SMs: half as many rows again never take
+    more than 30% longer among small matrices (piled up on some SMs they took 50%)."""
+    times = {}
+    for n in (20000, 30000, 40000, 60000, 90000):
+        g = lgd.SellGrid.from_csr(n, *workloads.powerlaw_graph(n, seed=1), 32, 256, exact=exact)
+        g.upload(np.random.default_rng(0).random(n))
+        times[n], = least(g, 200, [lambda g: None])
+        g.close()
+    for a, b in ((20000, 30000), (40000, 60000), (60000, 90000)):
+        assert times[b] < 1.3 * times[a], (a, b, times)
