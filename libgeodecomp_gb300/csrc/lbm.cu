@@ -636,8 +636,11 @@ convert_kernel(float *f, double *dense, unsigned n3, long long pitch, long long 
 
 // Host copy of one instance as 19 * L^3 doubles.  FP32 populations convert on
 // the device in bounded chunks (on one host core the conversion took 0.5 ns a
-// value, ten times the copy).
+// value, ten times the copy), small instances on the host, where that is less than
+// the launch (us by host / device: up 8^3 14.6 / 22.9, 12^3 18.9 / 24.3, 16^3 28.9 / 25.9;
+// down 8^3 16.2 / 18.4, 12^3 21.1 / 19.7).
 constexpr long long CONVERT_CHUNK = 8ll << 20;
+constexpr long long HOST_UP_VALUES = 56 << 10, HOST_DOWN_VALUES = 16 << 10;
 
 static void copy_instance(Lbm& e, const LbmInstance& in, size_t n3, double *host, bool up)
 {
@@ -653,6 +656,23 @@ static void copy_instance(Lbm& e, const LbmInstance& in, size_t n3, double *host
         LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
         return;
     }
+    float *f = (float *)e.buf[e.cur] + in.base;
+    const long long total = 19ll * (long long)n3;
+    if (total <= (up ? HOST_UP_VALUES : HOST_DOWN_VALUES)) {
+        if (up) {
+            const std::vector<float> values(host, host + total);
+            LGD_CHECK_CUDA(cudaMemcpy2DAsync(f, (size_t)in.pitch * 4, values.data(), n3 * 4, n3 * 4, 19, cudaMemcpyHostToDevice,
+                                             e.stream));
+            LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
+        } else {
+            std::vector<float> values(total);
+            LGD_CHECK_CUDA(cudaMemcpy2DAsync(values.data(), n3 * 4, f, (size_t)in.pitch * 4, n3 * 4, 19, cudaMemcpyDeviceToHost,
+                                             e.stream));
+            LGD_CHECK_CUDA(cudaStreamSynchronize(e.stream));
+            std::copy(values.begin(), values.end(), host);
+        }
+        return;
+    }
     if (e.d_stage == nullptr) {
         // shorter chunks where the populations leave little room
         e.stage_values = CONVERT_CHUNK;
@@ -661,8 +681,6 @@ static void copy_instance(Lbm& e, const LbmInstance& in, size_t n3, double *host
             LGD_REQUIRE(e.stage_values >= 1024, LGD_ERR_CUDA, "no device memory for the conversion buffer");
         }
     }
-    float *f = (float *)e.buf[e.cur] + in.base;
-    const long long total = 19ll * (long long)n3;
     for (long long first = 0; first < total; first += e.stage_values) {
         const long long n = std::min(e.stage_values, total - first);
         const unsigned blocks = (unsigned)std::min<long long>(152 * 16, (n + 255) / 256);

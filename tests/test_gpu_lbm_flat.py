@@ -2,6 +2,8 @@
 blocks of 128 cells end, against the oracle (FP64, bit for bit) and against the
 persistent kernel (FP32, bit for bit), and the device conversion of instances
 larger than one staging chunk."""
+import time
+
 import numpy as np
 import pytest
 
@@ -148,3 +150,34 @@ def test_fp32_relaxation_rounds_the_weighted_term():
         differ = one != other
         near = np.abs(out[i].astype(np.float64) - one)[differ].sum(), np.abs(out[i].astype(np.float64) - other)[differ].sum()
         assert near[0] < near[1], i
+
+
+@pytest.mark.parametrize("L", [2, 5, 9, 10, 14, 15])
+def test_conversion_on_host_or_device(L):
+    """Instances around the sizes up to which FP32 populations convert on the
+    host (19 * 9^3 values down, 14^3 up)."""
+    rng = np.random.default_rng(L)
+    f = rng.uniform(-1, 1, (19, L, L, L))
+    with lgd.LbmEnsemble([L, 3, L], [1.3, 1.0, 0.7], precision=4) as e:
+        e.upload(2, f)
+        np.testing.assert_array_equal(e.download(2), f.astype(np.float32).astype(np.float64))
+        np.testing.assert_array_equal(e.download(0), oracle.lbm_rest(L).astype(np.float32).astype(np.float64))
+
+
+@pytest.mark.parametrize("L", [3, 8])
+def test_copies_of_small_fp32_instances(L):
+    """They take no longer than 1.2 times FP64 ones, which need no conversion,
+    and 0.3 ns a value (with a kernel each 1.3 to 1.6 times FP64's time)."""
+    best = {}
+    for precision in (4, 8):
+        with lgd.LbmEnsemble([L], [1.3], precision=precision) as e:
+            f = e.download(0)
+            times = []
+            for _ in range(30):
+                t = time.perf_counter()
+                for _ in range(20):
+                    e.upload(0, f)
+                    e.download(0)
+                times.append(time.perf_counter() - t)
+            best[precision] = min(times)
+    assert best[4] < 1.2 * best[8] + 20 * 2 * 19 * L ** 3 * 0.3e-9, best
