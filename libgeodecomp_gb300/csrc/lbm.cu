@@ -187,6 +187,18 @@ struct Mem {
     }
 };
 
+// FP32 rounds the same in every kernel: the products whose bits an FMA keeps
+// are written out here and below (as the compiler had chosen them for separate
+// directions), not left to what else a kernel does with them.
+// Population I back from the lid: + 6 w_i (e_i . u_lid), u_lid = (lid, 0, 0).
+template<typename R, int I>
+__device__ __forceinline__ R from_lid(R v, R lid)
+{
+    const R w6 = LbmArith<R>::mul((R)6.0, I < 7 ? (R)(1.0 / 18.0) : (R)(1.0 / 36.0));
+    if constexpr (sizeof(R) == 4) return fmaf(w6, (R)Q<I>::ex * lid, v);
+    else return LbmArith<R>::add(v, LbmArith<R>::mul(w6, (R)Q<I>::ex * lid));
+}
+
 // INTERIOR: the cell is at least one cell away from every wall, so every
 // source cell exists (no wall tests)
 template<typename R, int I, typename IDX, int NC, bool INTERIOR>
@@ -200,14 +212,9 @@ __device__ __forceinline__ void pull_one(const R *__restrict__ src, IDX n3, IDX 
         ((unsigned)sx < (unsigned)L && (unsigned)sy < (unsigned)L && (unsigned)sz < (unsigned)L)) {
         f[I] = Mem<NC>::ld(src + (I * n3 + cell - (Q<I>::ex + (IDX)Q<I>::ey * L + (IDX)Q<I>::ez * L * L)));
     } else {
-        const R w = (I == 0) ? (R)(1.0 / 3.0) : ((I < 7) ? (R)(1.0 / 18.0) : (R)(1.0 / 36.0));
-        R v = Mem<NC>::ld(src + (Q<I>::opp * n3 + cell));
-        if (Q<I>::ey == -1 && Q<I>::ex != 0 && y == L - 1) {
-            // population from the lid: + 6 w_i (e_i . u_lid), u_lid = (lid, 0, 0);
-            // for every other wall the added term is exactly zero
-            v = LbmArith<R>::add(v, LbmArith<R>::mul(LbmArith<R>::mul((R)6.0, w), (R)Q<I>::ex * lid));
-        }
-        f[I] = v;
+        const R v = Mem<NC>::ld(src + (Q<I>::opp * n3 + cell));
+        // for every wall but the lid the added term is exactly zero
+        f[I] = Q<I>::ey == -1 && Q<I>::ex != 0 && y == L - 1 ? from_lid<R, I>(v, lid) : v;
     }
 }
 
@@ -240,9 +247,9 @@ __device__ __forceinline__ R dot_dir(R ux, R uy, R uz)
     return A::add(x, y);
 }
 
-// keep f + w x.  FP32: which product keeps its bits in the FMA is stated, not
-// left to the compiler (keep f: the error of 20 steps against FP64 is 2 to 3%
-// smaller than with w x, rms over cavities of 9^3 to 33^3)
+// keep f + w x.  FP32: the FMA keeps the bits of keep f (the error of 20 steps
+// against FP64 is 2 to 3% smaller than with those of w x, rms over cavities of 9^3
+// to 33^3)
 template<typename R, typename MUL>
 __device__ __forceinline__ R relax(R keep, R f, R w, R x, MUL mul)
 {
@@ -259,9 +266,18 @@ __device__ __forceinline__ void collide_pair(const R *f, R keep, R w1, R w2, R d
     typedef LbmArith<R> A;
     const R wi = (I < 7) ? w1 : w2;
     const R eu = dot_dir<R, I>(ux, uy, uz);
-    const R sq = mul((R)1.5, mul(eu, eu));
-    put(I, relax(keep, f[I], wi, A::add(A::add(d, eu), sq), mul));
-    put(Q<I>::opp, relax(keep, f[Q<I>::opp], wi, A::add(A::sub(d, eu), sq), mul));
+    R there, back;
+    if constexpr (sizeof(R) == 4) {
+        const R e2 = __fmul_rn(eu, eu);
+        there = fmaf(1.5f, e2, d + eu);
+        back = fmaf(1.5f, e2, d - eu);
+    } else {
+        const R sq = mul((R)1.5, mul(eu, eu));
+        there = A::add(A::add(d, eu), sq);
+        back = A::add(A::sub(d, eu), sq);
+    }
+    put(I, relax(keep, f[I], wi, there, mul));
+    put(Q<I>::opp, relax(keep, f[Q<I>::opp], wi, back, mul));
 }
 
 // not a number or infinite, without the FP64 pipe
@@ -288,8 +304,14 @@ __device__ __forceinline__ void collide_with(const R *f, R omega, PUT put, MUL m
     // T + TW + TE + TN + TS - (B + BW + BE + BN + BS)
     const R uz = A::sub(A::add(A::add(A::add(A::add(f[5], f[11]), f[13]), f[15]), f[17]),
                         A::add(A::add(A::add(A::add(f[6], f[12]), f[14]), f[16]), f[18]));
-    const R usq = A::add(A::add(mul(ux, ux), mul(uy, uy)), mul(uz, uz));
-    R d = A::sub(mul(rho, (R)(1.0 / 3.0)), mul((R)0.5, usq));
+    R d;
+    if constexpr (sizeof(R) == 4) {
+        const R usq = fmaf(uz, uz, fmaf(ux, ux, __fmul_rn(uy, uy)));
+        d = fmaf(rho, (R)(1.0 / 3.0), -0.5f * usq);
+    } else {
+        const R usq = A::add(A::add(mul(ux, ux), mul(uy, uy)), mul(uz, uz));
+        d = A::sub(mul(rho, (R)(1.0 / 3.0)), mul((R)0.5, usq));
+    }
     const R keep = A::sub((R)1.0, omega);
     const R w1 = mul(omega, (R)(1.0 / 6.0));
     const R w2 = mul(omega, (R)(1.0 / 12.0));
@@ -416,9 +438,8 @@ __device__ __forceinline__ void pull_select(const R *src, IDX n3, IDX cell, int 
         const IDX at = inside ? I * n3 + cell - (Q<I>::ex + (IDX)Q<I>::ey * L + (IDX)Q<I>::ez * L * L) : Q<I>::opp * n3 + cell;
         R v = Mem<NC>::ld(src + at);
         if (Q<I>::ey == -1 && Q<I>::ex != 0) {              // see pull_one
-            const R from_lid = LbmArith<R>::add(
-                v, LbmArith<R>::mul(LbmArith<R>::mul((R)6.0, I < 7 ? (R)(1.0 / 18.0) : (R)(1.0 / 36.0)), (R)Q<I>::ex * lid));
-            v = !inside && y == L - 1 ? from_lid : v;
+            const R lid_v = from_lid<R, I>(v, lid);
+            v = !inside && y == L - 1 ? lid_v : v;
         }
         f[I] = v;
         pull_select<R, I + 1, IDX, NC>(src, n3, cell, L, x, y, z, lid, f);
@@ -517,12 +538,8 @@ __device__ __forceinline__ R tb2_pull(const R *__restrict__ ring, int L, int x, 
     if ((unsigned)sx < (unsigned)L && (unsigned)sy < (unsigned)L && (unsigned)sz < (unsigned)L) {
         return ring[((sz % 3) * 19 + I) * G::HC + (ty + 1 - Q<I>::ey) * G::HX + (tx + 1 - Q<I>::ex)];
     }
-    R v = ring[((zz % 3) * 19 + Q<I>::opp) * G::HC + (ty + 1) * G::HX + (tx + 1)];
-    if (Q<I>::ey == -1 && Q<I>::ex != 0 && y == L - 1) {
-        const R w = (I < 7) ? (R)(1.0 / 18.0) : (R)(1.0 / 36.0);
-        v = LbmArith<R>::add(v, LbmArith<R>::mul(LbmArith<R>::mul((R)6.0, w), (R)Q<I>::ex * lid));
-    }
-    return v;
+    const R v = ring[((zz % 3) * 19 + Q<I>::opp) * G::HC + (ty + 1) * G::HX + (tx + 1)];
+    return Q<I>::ey == -1 && Q<I>::ex != 0 && y == L - 1 ? from_lid<R, I>(v, lid) : v;
 }
 
 template<typename R, int I, int TX, int TY>

@@ -181,3 +181,54 @@ def test_copies_of_small_fp32_instances(L):
                 times.append(time.perf_counter() - t)
             best[precision] = min(times)
     assert best[4] < 1.2 * best[8] + 20 * 2 * 19 * L ** 3 * 0.3e-9, best
+
+
+@pytest.mark.parametrize("kernel", ["flat", "read-only", "persistent", "looped"])
+def test_fp32_rounding_of_a_step(kernel):
+    """One step of populations of both signs, every rounding restated: squares of
+    u, the density's third, 1.5 (e . u)^2, the lid's share and the old population
+    inside an FMA each; the other products rounded."""
+    L, omega, lid = 12, np.float32(1.3), np.float32(0.05)
+    f = np.random.default_rng(9).uniform(-1, 1, (19, L, L, L)).astype(np.float32)
+    e = [(0, 0, 0), (0, 1, 0), (1, 0, 0), (-1, 0, 0), (0, -1, 0), (0, 0, 1), (0, 0, -1), (-1, 1, 0), (-1, -1, 0), (1, 1, 0),
+         (1, -1, 0), (-1, 0, 1), (-1, 0, -1), (1, 0, 1), (1, 0, -1), (0, 1, 1), (0, 1, -1), (0, -1, 1), (0, -1, -1)]
+    z, y, x = np.meshgrid(*[np.arange(L)] * 3, indexing="ij")
+    p = np.empty_like(f)
+    for i, (ex, ey, ez) in enumerate(e):
+        sx, sy, sz = x - ex, y - ey, z - ez
+        inside = (sx >= 0) & (sx < L) & (sy >= 0) & (sy < L) & (sz >= 0) & (sz < L)
+        back = f[e.index((-ex, -ey, -ez))]
+        if ey == -1 and ex != 0:
+            lidded = rounded_fma(np.float32(6) * np.float32(1 / 36), np.float32(ex) * lid, back)
+            back = np.where(y == L - 1, lidded, back)
+        p[i] = np.where(inside, f[i, sz % L, sy % L, sx % L], back)
+
+    def total(*idx):
+        s = p[idx[0]]
+        for i in idx[1:]:
+            s = s + p[i]
+        return s
+
+    rho = total(*range(19))
+    ux = total(2, 9, 10, 13, 14) - total(3, 7, 8, 11, 12)
+    uy = total(1, 7, 9, 15, 16) - total(4, 8, 10, 17, 18)
+    uz = total(5, 11, 13, 15, 17) - total(6, 12, 14, 16, 18)
+    assert all(a.dtype == np.float32 for a in (rho, ux, uy, uz))
+    usq = rounded_fma(uz, uz, rounded_fma(ux, ux, uy * uy))
+    d = rounded_fma(rho, np.float32(1 / 3), np.float32(-0.5) * usq)
+    keep = np.float32(1) - omega
+    ref = np.empty_like(f)
+    ref[0] = rounded_fma(keep, p[0], omega * d)
+    for i, (ex, ey, ez) in enumerate(e[1:], 1):
+        eu = np.float32(ex) * ux + np.float32(ey) * uy + np.float32(ez) * uz
+        w = omega * np.float32(1 / 6 if i < 7 else 1 / 12)
+        ref[i] = rounded_fma(keep, p[i], w * rounded_fma(np.float32(1.5), eu * eu, d + eu))
+    with lgd.LbmEnsemble([L], [float(omega)], lid=float(lid), precision=4) as ens:
+        if kernel == "read-only":
+            ens.set_variant(1)
+        if kernel == "persistent":
+            ens.set_config(4, 256, 4)
+        ens.upload(0, f.astype(np.float64))
+        ens.step_looped(1) if kernel == "looped" else ens.step(1)
+        out = ens.download(0).astype(np.float32)
+    np.testing.assert_array_equal(out, ref)
