@@ -216,3 +216,18 @@ def test_lbm_a_reported_launch_shape_selects_the_same_kernel():
             e.step(7)
         for j in range(len(edges)):
             np.testing.assert_array_equal(a.download(j), b.download(j))
+
+
+@pytest.mark.parametrize("precision", [4, 8])
+@pytest.mark.parametrize("edges", [[8] * 40, [24] * 100, [12] * 64, [90], [64, 20, 33]])
+def test_lbm_two_steps_whole_columns_and_chunks(edges, precision):
+    """Columns that stay whole and columns cut in z, by the ensemble and the
+    resident CTAs (changed between calls): the values of single steps."""
+    omegas = [0.8 + 0.9 * j / len(edges) for j in range(len(edges))]
+    with lgd.LbmEnsemble(edges, omegas, precision=precision) as a, lgd.LbmEnsemble(edges, omegas, precision=precision) as b:
+        for shape, ctas in ((0, 1), (0, 2), (1, 4), (1, 1)):
+            a.set_time_block(2, shape, ctas)
+            a.step(6)
+            b.step(6)
+        for j in {0, len(edges) // 2, len(edges) - 1}:
+            np.testing.assert_array_equal(a.download(j), b.download(j))
