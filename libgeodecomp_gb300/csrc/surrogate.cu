@@ -454,6 +454,12 @@ struct Layer {
     int frag_n, frag_t_n;
 };
 
+// the gradients start on a line of their own: the mma.sync weight gradients add
+// whole lines by atomics (8 bytes off, 20000 x 4 x 32 voxels of 8 channels trained in 3.56
+// ms per iteration instead of 3.29)
+constexpr size_t GRADS_AT = 256;
+static_assert(GRADS_AT >= sizeof(double) && GRADS_AT % 128 == 0, "the loss, then a line of its own");
+
 struct Net {
     Geo g;
     int C;
@@ -470,7 +476,7 @@ struct Net {
     float *dh;          // [V][C] FP32 input gradient
     bf16 *dzb;          // [V][C] BF16 gradient
     bf16 *dz4;          // [V][2]
-    double *d_loss;     // one allocation with grads behind it
+    double *d_loss;     // one allocation with grads, GRADS_AT bytes on
     int t;              // Adam step
     cudaStream_t stream;
     uint64_t launches;
@@ -629,7 +635,7 @@ static void backward_fast(Net& n, const float *target, double *loss_out)
 {
     const int dims[4] = {n.g.nx, n.g.ny, n.g.nz, n.g.batch};
     const float scale = 2.0f / (float)n.V;
-    LGD_CHECK_CUDA(cudaMemsetAsync(n.d_loss, 0, sizeof(double) + sizeof(float) * n.P, n.stream));     // and grads
+    LGD_CHECK_CUDA(cudaMemsetAsync(n.d_loss, 0, GRADS_AT + sizeof(float) * n.P, n.stream));     // and grads
     int ctas[4];
     ctas[3] = tc_wgrad(3, n.hg[2], nullptr, nullptr, n.du, target, scale, n.d_loss, n.grads + n.L[3].b_off, n.part, dims, n.d_err, n.stream);
     tc_grad_last(n.du, target, scale, n.wtc.grad[3], n.gt[2], n.dzg[0], n.grads + n.L[2].b_off, dims, n.d_err, n.stream);
@@ -860,8 +866,8 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
             const long long V = n->V;
             LGD_CHECK_CUDA(cudaMalloc(&n->du, sizeof(float) * V));
             if (n->training) {
-                LGD_CHECK_CUDA(cudaMalloc(&n->d_loss, sizeof(double) + sizeof(float) * n->P));
-                n->grads = reinterpret_cast<float *>(n->d_loss + 1);
+                LGD_CHECK_CUDA(cudaMalloc(&n->d_loss, GRADS_AT + sizeof(float) * n->P));
+                n->grads = reinterpret_cast<float *>(reinterpret_cast<char *>(n->d_loss) + GRADS_AT);
                 LGD_CHECK_CUDA(cudaMalloc(&n->m, sizeof(float) * n->P));
                 LGD_CHECK_CUDA(cudaMalloc(&n->v, sizeof(float) * n->P));
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->grads, 0, sizeof(float) * n->P, n->stream));

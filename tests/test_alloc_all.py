@@ -22,3 +22,11 @@ def test_the_networks_mma_buffers_are_made_together():
     src = open(os.path.join(CSRC, "surrogate.cu")).read()
     body = re.search(r"static void ensure_dense\(Net& n\)\n\{(.*?)\n\}", src, re.S).group(1)
     assert "allocate_all(" in body and "LGD_CHECK_CUDA(cudaMalloc" not in body
+
+
+def test_gradients_share_no_line_with_the_loss():
+    """They are one allocation; the gradients' atomics add whole 128-byte lines."""
+    src = open(os.path.join(CSRC, "surrogate.cu")).read()
+    at = re.search(r"constexpr size_t GRADS_AT = (\d+);", src)
+    assert at and int(at.group(1)) % 128 == 0 and int(at.group(1)) >= 128
+    assert re.search(r"n->grads = .*n->d_loss\) \+ GRADS_AT\)", src)
