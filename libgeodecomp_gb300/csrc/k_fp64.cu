@@ -11,9 +11,10 @@
 //     step, 1600 with no addition in integers, 1110 with two, 916 with three,
 //     1140 with four, 1376 with all six (measured without the one-sided
 //     neighbour's rule below and with plain launches).  Where sum4's condition
-//     fails in some lane the warp adds in FP64 after all, which costs what it
-//     cost before: smooth fields meet it but for the cells beside a zero edge
-//     in y; the zero east of the last column is dropped (drop_e);
+//     fails in some lane (both signs, zeros, far apart) the warp adds in FP64
+//     after all; four +0, an empty part of the field, it does not add.  Smooth
+//     fields meet the condition but for the cells beside a zero edge in y; the zero
+//     east of the last column is dropped (drop_e);
 //   - the rare branches must stay branches: predicated, their FP64 operations
 //     would be paid always.  So the z loop stays rolled, and sum4's fallback is
 //     a loop;
@@ -22,11 +23,13 @@
 //     and neighbours come straight from global memory (L1 / L2 hits), so
 //     there is no barrier and no tile, and a grid is cut into as many small
 //     CTAs as it takes to give every SM an even share.
-// Measured (us per step; in brackets the kernel without sum4, then the TMA
-// kernel of k_tma.cu): 24 x 20 x 16 1.9 (2.2, 22.6), 64^3 4.0 (5.9, 22.6), 128^3
-// 17.1 (25.4, 38.9), 512^3 886 (1598, 1795): 151 GLUPS, 91% of the FP64 pipe's
-// rate at three operations per cell.  On a torus, against the register kernel:
-// 64^3 4.3 (45), 128^3 18.9 (51), 512^3 1026 (1850).
+// Measured (us per step, uniform in [0, 1); in brackets the kernel without sum4, then
+// the TMA kernel of k_tma.cu): 24 x 20 x 16 1.9 (2.2, 22.6), 64^3 4.0 (5.9, 22.6), 128^3
+// 17.2 (25.4, 39.1), 512^3 914 (1598, 1795): 147 GLUPS, 88% of the FP64 pipe's rate at
+// three operations per cell.  On a torus, against the register kernel: 64^3 4.3 (45),
+// 128^3 19.0 (51), 512^3 1066 (1851).  Other fields, 512^3, cube / torus: of both signs
+// 1566 / 1786, a hot spot in an empty field 1058 / 1278 (adding its zeros 1822 / 2040),
+// exponents up to 30 apart 1083 / 1252.
 // The sum's order is the cell's own: results are bit-identical to every
 // other kernel of the cell.
 #include <algorithm>
@@ -40,6 +43,11 @@ namespace fp64k {
 
 constexpr int THREADS = 128;
 constexpr int CTAS = 8;        // per SM: 64 registers
+
+__device__ __forceinline__ bool any_bit(double a, double b, double c, double d)
+{
+    return ((__double_as_longlong(a) | __double_as_longlong(b)) | (__double_as_longlong(c) | __double_as_longlong(d))) != 0;
+}
 
 // WRAP: some axis wraps (a cube of 512^3 takes 886 us without, 1030 with)
 template<bool WRAP>
@@ -78,8 +86,9 @@ jacobi7_f64_kernel(const double *in, double *out, long pitch, int nx, int ny, in
         double acc;
         if (!sum4(m, n, s, e, drop_e, acc)) {
             acc = m;
+            const int adds = any_bit(m, n, s, e) ? 3 : 0;               // +0 four times sum to +0
 #pragma unroll 1
-            for (int i = 0; i < 3; ++i) acc = __dadd_rn(acc, i == 0 ? n : (i == 1 ? s : e));
+            for (int i = 0; i < adds; ++i) acc = __dadd_rn(acc, i == 0 ? n : (i == 1 ? s : e));
         }
         acc = __dadd_rn(acc, w);
         acc = __dadd_rn(acc, t);

@@ -79,3 +79,18 @@ def test_fp64_sell_steps_grow_with_the_rows(exact):
         g.close()
     for a, b in ((20000, 30000), (40000, 60000), (60000, 90000)):
         assert times[b] < 1.3 * times[a], (a, b, times)
+
+
+@pytest.mark.parametrize("kind", ["hot spot", "both signs", "uniform"])
+@pytest.mark.parametrize("periodic", [0, 7])
+def test_fp64_jacobi_of_any_field(kind, periodic):
+    """Against the register kernel, whose time does not depend on the values."""
+    n = 512 if kind == "hot spot" else 256
+    shape = (n, n, n)
+    rng = np.random.default_rng(5)
+    u = np.zeros(shape) if kind == "hot spot" else rng.random(shape) - (0.5 if kind == "both signs" else 0.0)
+    u[n // 2, n // 2, n // 2] = 1.0
+    with lgd.Grid(lgd.CELL_JACOBI7_F64, shape, periodic=periodic) as g:
+        g.upload(0, u)
+        default, register = least(g, 5, [lambda g: g.set_variant(0), lambda g: g.set_variant(5)])
+    assert default < 1.03 * register

@@ -72,3 +72,25 @@ def test_some_axes_wrap(periodic, shape):
     inner = tuple(slice(a, a + n) for (a, _), n in zip(pad, shape))
     ref = oracle.jacobi7(np.pad(u0, pad, mode="wrap"), steps, edge=0.25)[inner]
     np.testing.assert_array_equal(run(u0, steps, edge=0.25, periodic=periodic), ref)
+
+
+@pytest.mark.parametrize("periodic", [0, 7])
+@pytest.mark.parametrize("edge", [0.0, -0.0, 0.25])
+def test_empty_parts(periodic, edge):
+    """Zeros of either sign next to each other, to subnormals and to a hot spot:
+    the sign of every zero sum, too (grids whose threads march eight planes)."""
+    shape = (100, 128, 128)
+    rng = np.random.default_rng(8)
+    u0 = np.zeros(shape)
+    u0[50, 64, 64] = 1.0
+    u0[20:30, 10:20] = -0.0
+    u0[40:44, :, 30:33] = np.where(rng.random((4, 128, 3)) < 0.5, -0.0, 0.0)
+    u0[70:, 100:, 100:] = rng.integers(-2, 3, (30, 28, 28)) * 5e-324
+    out = []
+    for variant in (0, 2):
+        with lgd.Grid(lgd.CELL_JACOBI7_F64, shape, periodic=periodic, edge=(edge, 0, 0, 0)) as g:
+            g.set_variant(variant)
+            g.upload(0, u0)
+            g.step(4)
+            out.append(g.download(0).view(np.uint64))
+    np.testing.assert_array_equal(out[0], out[1])
