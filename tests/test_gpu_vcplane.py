@@ -99,3 +99,22 @@ def test_fp64_warps_that_fall_back(kind, periodic):
     edge = (0.0, 0.07, 0.0, 0.0)
     a, b = (run(lgd.CELL_VARCOEF_F64, u, k, 3, variant, periodic, edge) for variant in (0, 1))
     np.testing.assert_array_equal(a.view(np.uint64), b.view(np.uint64))
+
+
+@pytest.mark.parametrize("scale", [5e-324, 1e-308, 4.5e-308, 1e-300, 1.0, 1e300, 8e307, np.inf])
+@pytest.mark.parametrize("bits", [2, 52])
+def test_fp64_differences_of_u_at_the_ends_of_the_range(scale, bits):
+    """The product's other operand: subnormal, overflowing and infinite
+    differences, zeros of both signs, few significant bits (ties)."""
+    rng = np.random.default_rng(bits)
+    shape = (6, 9, 40)
+    m = (1.0 + np.floor(rng.random(shape) * 2.0 ** bits) * 2.0 ** -bits) * rng.choice([-1.0, 1.0], shape)
+    with np.errstate(over="ignore"):
+        u = np.where(rng.random(shape) < 0.4, m * scale, m)
+        u[2] = m[2] * scale
+    u[rng.random(shape) < 0.1] = 0.0
+    u[rng.random(shape) < 0.1] = -0.0
+    k = np.ldexp(1.0 + np.floor(rng.random(shape) * 2.0 ** bits) * 2.0 ** -bits, rng.integers(-6, -2, shape))
+    a, b = (run(lgd.CELL_VARCOEF_F64, u, k, 2, variant, 7) for variant in (0, 1))
+    same = np.isnan(a) & np.isnan(b)                            # any NaN is a NaN
+    np.testing.assert_array_equal(np.where(same, 0.0, a).view(np.uint64), np.where(same, 0.0, b).view(np.uint64))
