@@ -204,14 +204,17 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 
 // GELU(z) = z Phi(z) of two values, and GELU'(z) = Phi(z) + z phi(z) where
 // asked for, each from packed FMAs, one reciprocal and one exponential:
-//   |z| < 1   Phi = 1/2 + z Q(z^2), Q of degree 4 (largest error 7e-9)
+//   |z| < 1   Phi = 1/2 + z Q(z^2), Q of degree 4 (error of the fit below 1.3e-8)
 //   else      Phi(-|z|) = exp(-z^2 / 2) t P(t) with t = 1 / (1 + p |z|): the
 //             function exp(z^2 / 2) Phi(-z) / t is smooth in t, and P its
-//             polynomial of degree 6 (relative error 8e-8 up to z = 14; p chosen
-//             for the smallest)
+//             polynomial of degree 6 (relative error of the fit below 1.0e-7 up to
+//             z = 14; p chosen for the smallest)
 // Both are least-squares fits with weights moved towards the largest error until
-// that stopped falling.  erff and expf took twice the instructions, which set the
-// time of a layer's epilogue.
+// that stopped falling.  In FP32, over -16 .. 16, GELU is within 4e-7 (4.5e-7 with
+// erff) and GELU' within 1.4e-7; relative to itself Phi's lower tail is within 1.0e-6
+// to z = -4 and 9e-6 to z = -13.2, where the exponential's result is flushed to
+// zero.  erff and expf took twice the instructions, which set the time of a layer's
+// epilogue.
 template<bool GRAD>
 __device__ __forceinline__ void gelu_pair(float2 z, float2& h, float2& g)
 {
