@@ -338,8 +338,7 @@ __global__ void gelu_bwd_kernel(const float *__restrict__ dh, const float *__res
 }
 
 // MSE loss of du against target: g = 2 (du - t) / N as the BF16 gradient of
-// the last layer ([V][2], channel 1 zero; or null), db4 += sum g, loss += sum
-// diff^2
+// the last layer ([V][2], channel 1 zero), db4 += sum g, loss += sum diff^2
 __global__ void loss_kernel(const float *__restrict__ du, const float *__restrict__ target, bf16 *__restrict__ dz4,
                             float *__restrict__ db4, double *__restrict__ loss, long long nvox)
 {
@@ -353,7 +352,7 @@ __global__ void loss_kernel(const float *__restrict__ du, const float *__restric
         l = fma((double)d, (double)d, l);
         const float gv = scale * d;
         gs += gv;
-        if (dz4) *reinterpret_cast<uint32_t *>(dz4 + 2 * v) = pack2(__float2bfloat16(gv), __float2bfloat16(0.f));
+        *reinterpret_cast<uint32_t *>(dz4 + 2 * v) = pack2(__float2bfloat16(gv), __float2bfloat16(0.f));
     }
     sl[threadIdx.x] = l;
     sg[threadIdx.x] = gs;
