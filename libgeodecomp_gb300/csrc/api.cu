@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "lgd_internal.h"
+#include "error_words.h"
 #include "k_common.cuh"
 
 namespace lgd {
@@ -220,6 +221,38 @@ static void lower_fix_exp(Grid& g)
     g.fix_exp -= shift;
     LGD_CHECK_CUDA(cudaStreamSynchronize(g.stream));
 }
+
+// ------------------------------------------------------------ error words
+namespace {
+
+int *alloc_words(size_t bytes)
+{
+    int *p = nullptr;
+    LGD_CHECK_CUDA(cudaHostAlloc(&p, bytes, cudaHostAllocMapped | cudaHostAllocPortable));
+    return p;
+}
+
+void release_words(int *p) { cudaFreeHost(p); }
+
+bool words_alive(int *p)
+{
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, p) == cudaSuccess && attr.type == cudaMemoryTypeHost) return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
+// never destroyed: no CUDA call may run at exit
+ErrorWords<int *(*)(size_t), void (*)(int *), bool (*)(int *)>& error_words()
+{
+    static auto *pool = new ErrorWords<int *(*)(size_t), void (*)(int *), bool (*)(int *)>(alloc_words, release_words, words_alive);
+    return *pool;
+}
+
+}  // namespace
+
+int *take_error_word() { return error_words().take(); }
+void give_error_word(int *word) { error_words().give(word); }
 
 // --------------------------------------------------------------- helpers
 // Reads (and clears) the error word that kernels with bounded waits set when
@@ -492,9 +525,7 @@ static void create_grid(const lgd_grid_desc *desc, size_t record_bytes, const vo
         LGD_CHECK_CUDA(cudaGetDevice(&g.device));
         try {
             LGD_CHECK_CUDA(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
-            // unified addressing: the host pointer is the device's, too
-            LGD_CHECK_CUDA(cudaHostAlloc(&g.d_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-            *g.d_err = 0;
+            g.d_err = take_error_word();
             for (int m = 0; m < ci.n_members; ++m) {
                 g.m[m].elem = ci.elem[m];
                 g.m[m].is_static = ci.is_static[m];
@@ -528,7 +559,7 @@ static void create_grid(const lgd_grid_desc *desc, size_t record_bytes, const vo
                     if (g.m[m].buf[b]) cudaFree(g.m[m].buf[b]);
                 }
             }
-            if (g.d_err) cudaFreeHost(g.d_err);
+            if (g.d_err) give_error_word(g.d_err);
             if (g.d_fixmax) cudaFree(g.d_fixmax);
             if (g.d_edge_record) cudaFree(g.d_edge_record);
             std::free(g.edge_record);
@@ -680,7 +711,7 @@ int lgd_gpu_destroy(lgd_handle *h)
         if (g.d_streaks) cudaFree(g.d_streaks);
         if (g.d_streak_prefix) cudaFree(g.d_streak_prefix);
         if (g.d_partials) cudaFree(g.d_partials);
-        if (g.d_err) cudaFreeHost(g.d_err);
+        if (g.d_err) give_error_word(g.d_err);
         if (g.d_fixmax) cudaFree(g.d_fixmax);
         if (g.d_edge_record) cudaFree(g.d_edge_record);
         std::free(g.edge_record);

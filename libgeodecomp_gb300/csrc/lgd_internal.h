@@ -114,6 +114,12 @@ inline cudaError_t malloc_on_first_use(void **p, size_t bytes)
     return error;
 }
 
+// A zeroed error word in mapped host memory, which kernels with bounded waits write
+// (unified addressing: the pointer is the device's, too), and its return once no
+// kernel may write it any more.
+int *take_error_word();
+void give_error_word(int *word);
+
 // Launches a kernel that may be scheduled while the kernel before it on the
 // stream still runs (programmatic dependent launch).  The kernel calls
 // dependent_start() before it touches global memory, which waits for that

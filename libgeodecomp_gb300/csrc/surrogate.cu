@@ -787,7 +787,7 @@ static void net_free(Net& n)
     cudaFree(n.xt);
     cudaFree(n.part);
     tc_free_weights(n.wtc);
-    if (n.d_err) cudaFreeHost(n.d_err);
+    if (n.d_err) give_error_word(n.d_err);
     if (n.stream) cudaStreamDestroy(n.stream);
 }
 
@@ -886,9 +886,7 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
                     LGD_CHECK_CUDA(cudaMalloc(&n->part, sizeof(float) * tc_partial_floats()));
                 }
                 n->wtc = tc_alloc_weights(n->training);
-                // mapped host memory: written by a failing kernel, read by the host
-                LGD_CHECK_CUDA(cudaHostAlloc(&n->d_err, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
-                *n->d_err = 0;
+                n->d_err = take_error_word();
             }
             repack(*n);
             LGD_CHECK_CUDA(cudaStreamSynchronize(n->stream));

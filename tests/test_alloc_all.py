@@ -30,3 +30,15 @@ def test_gradients_share_no_line_with_the_loss():
     at = re.search(r"constexpr size_t GRADS_AT = (\d+);", src)
     assert at and int(at.group(1)) % 128 == 0 and int(at.group(1)) >= 128
     assert re.search(r"n->grads = .*n->d_loss\) \+ GRADS_AT\)", src)
+
+
+def test_error_words(tmp_path):
+    """The pool of the handles' error words (csrc/error_words.h), and that handles use it."""
+    exe = str(tmp_path / "t")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", CSRC,
+                    os.path.join(ROOT, "tests", "cpp", "error_words_test.cpp"), "-o", exe], check=True)
+    res = subprocess.run([exe], capture_output=True, text=True)
+    assert res.returncode == 0 and res.stdout == "ok\n", res.returncode
+    for name in ("api.cu", "surrogate.cu"):
+        src = open(os.path.join(CSRC, name)).read()
+        assert "= take_error_word()" in src and not re.search(r"cudaHostAlloc\(&(g\.|n->)", src)
