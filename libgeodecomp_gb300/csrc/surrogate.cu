@@ -874,7 +874,9 @@ int lgd_net_create(int nx, int ny, int nz, int batch, int channels, int training
                 LGD_CHECK_CUDA(cudaMemsetAsync(n->v, 0, sizeof(float) * n->P, n->stream));
             }
             n->fast = tc_applicable(nx, ny, C);
-            if (n->fast) {
+            if (!n->fast) {
+                ensure_dense(*n);           // its only path
+            } else {
                 const size_t gbytes = tc_ghost_bytes(nx, ny, nz, batch);
                 for (int i = 0; i < (n->training ? 3 : 2); ++i) LGD_CHECK_CUDA(cudaMalloc(&n->hg[i], gbytes));
                 if (n->training) {

@@ -199,3 +199,31 @@ def test_advance_equals_forward_plus_residual(shape):
         net.advance(ut, kt, 1)
         net.synchronize()
         assert torch.equal(ut, expect)
+
+
+@pytest.mark.parametrize("channels", [8, 24])
+@pytest.mark.parametrize("training", [False, True])
+def test_buffers_of_the_default_path_exist_from_the_start(channels, training):
+    """A network that does not fit is refused by create: neither its first
+    forward pass nor its first backward pass takes device memory."""
+    shape, batch = (64, 64, 64), 4
+    u, k, t = (torch.rand((batch,) + shape, device="cuda") for _ in range(3))
+    du = torch.empty_like(u)
+    with _net((4, 4, 32), channels, training) as warm:         # modules load on first use
+        warm.forward(u, k, du)
+        if training:
+            warm.backward(t)
+        warm.synchronize()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    with _net(shape, channels, training, batch) as net:
+        net.set_params(sr.init_params(channels, seed=1).astype(np.float32))
+        net.synchronize()
+        created = torch.cuda.mem_get_info()[0]
+        net.forward(u, k, du)
+        if training:
+            net.backward(t)
+        net.synchronize()
+        assert torch.cuda.mem_get_info()[0] == created
+    # two layers' BF16 activations at the least
+    assert before - created > 2 * 2 * channels * batch * 64 ** 3
