@@ -232,3 +232,16 @@ def test_fp32_rounding_of_a_step(kernel):
         ens.step_looped(1) if kernel == "looped" else ens.step(1)
         out = ens.download(0).astype(np.float32)
     np.testing.assert_array_equal(out, ref)
+
+
+def test_table_of_a_large_ensemble_is_made_on_the_device():
+    """Its 131072 entries (64 cavities of 64^3) took the host and the copy 1.3 ms of
+    create's 1.8."""
+    times = []
+    for _ in range(15):
+        t = time.perf_counter()
+        e = lgd.LbmEnsemble([64] * 64, [1.2] * 64)
+        times.append(time.perf_counter() - t)
+        assert e.config() == (1, 128, 32)
+        e.close()
+    assert min(times) < 1.2e-3, times
