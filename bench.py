@@ -67,7 +67,7 @@ import numpy as np  # noqa: E402
 
 JACOBI_METRIC = "Jacobi3D GLUPS & HBM GB/s vs 8 TB/s"
 METRICS = {"gol_u8_8192": "Game of Life GLUPS", "sell_f64_4m": "SELL-C-sigma diffusion GB/s and s/step",
-           "lbm_d3q19_ensemble_512": "D3Q19 ensemble GLUPS (persistent launches, autotuned steps per launch)",
+           "lbm_d3q19_ensemble_512": "D3Q19 ensemble GLUPS (one launch for all cavities, autotuned kernel and steps per launch)",
            "varcoef_f32_256": "variable-coefficient diffusion GLUPS"}
 DTYPES = {"gol_u8_8192": "u8", "lbm_d3q19_ensemble_512": "f32", "varcoef_f32_256": "f32", "jacobi7_f32_512": "f32",
           "sell_f64_4m": "f64", "jacobi7_f64_ieee_512": "f64",

@@ -352,8 +352,9 @@ int lgd_gpu_launch_count(lgd_handle *h, uint64_t *count);
 /* Temporal blocking depth used by lgd_gpu_step (time steps fused into one
  * pass over memory): 0 = library default (3 for LGD_CELL_JACOBI7_F32, 2 for
  * LGD_CELL_JACOBI7_F64_FIX, 2 for LGD_CELL_VARCOEF_F32 on a torus with rows of
- * a multiple of 16 bytes, passes of up to 32 generations on packed rows for
- * calls of several generations of LGD_CELL_GOL_U8, 1 for the others),
+ * a multiple of 16 bytes where that is the faster, passes of up to 32 generations
+ * on packed rows for calls of several generations of LGD_CELL_GOL_U8 (16 over
+ * bytes for short calls on large boards), 1 for the others),
  * 1 = one step per pass, 2 .. LGD_TB_MAX_DEPTH.  It applies to
  *   - the FP32 Jacobi cell (at most 4; results bit-identical for every depth)
  *     and the fixed-point Jacobi cell (at most 2: its pass sums two steps
