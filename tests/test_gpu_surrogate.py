@@ -209,7 +209,7 @@ def test_buffers_of_the_default_path_exist_from_the_start(channels, training):
     shape, batch = (64, 64, 64), 4
     u, k, t = (torch.rand((batch,) + shape, device="cuda") for _ in range(3))
     du = torch.empty_like(u)
-    with _net((4, 4, 32), channels, training) as warm:         # modules load on first use
+    with _net(shape, channels, training, batch) as warm:       # kernels load on first use
         warm.forward(u, k, du)
         if training:
             warm.backward(t)
