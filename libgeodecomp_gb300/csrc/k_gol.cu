@@ -297,10 +297,10 @@ constexpr int GOL_BITS_DEFAULT_DEPTH = 16;
 // torus of aligned rows, whose alternative is a bit-sliced pass over bytes.  us per
 // call, packed against not: 1001 x 777 x 4 17 / 34; 1024^2 x 6 10 / 21, 8192^2 x 6 44 /
 // 49, x 16 60 / 100.  Beyond L2 the passes over bytes, which do their few generations
-// in one read and write, win longer: 8192 x 16384 x 6 95 / 75, x 8 104 / 89, x 10 104 / 137; 23168^2 x 12 428 / 409, x
-// 14 464 / 586; 32768^2 x 16 1079 / 1011, x 20 1236 / 1449.  Boards of a few long rows
-// fill little of a tile of 32 rows or more: 1 x 1000000 x 8 15.6 / 11.5, x 16 25 / 26, 1 x
-// 4000000 x 32 132 / 120
+// in one read and write, win longer: 8192 x 16384 x 6 95 / 75, x 8 104 / 89, x 10 104 /
+// 137; 23168^2 x 12 428 / 409, x 14 464 / 586; 32768^2 x 16 1079 / 1011, x 20 1236 / 1449.
+// Boards of a few long rows fill little of a tile of 32 rows or more: 1 x 1000000 x 8
+// 15.6 / 11.5, x 16 25 / 26, 1 x 4000000 x 32 132 / 120
 constexpr int GOL_PACK_MIN = 4;
 
 static int gol_pack_min(const Grid& g, bool aligned_torus)

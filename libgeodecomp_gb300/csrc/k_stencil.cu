@@ -690,8 +690,8 @@ varcoef_pair_kernel(View<const R> u, View<const R> k, View<R> out, int periodic,
 
 void launch_varcoef(Grid& g, int steps)
 {
-    // default: two steps per pass for FP32 cells on a full torus, then the TMA
-    // kernel where it takes the grid; one cell of a plane per thread for other
+    // default: two steps per pass for FP32 cells on a full torus where that is the
+    // faster, then the TMA kernel where it takes the grid; one cell of a plane per thread for other
     // FP32 grids and for FP64
     const bool tma = (g.variant == 6) || (g.variant == 0 && g.desc.cell == LGD_CELL_VARCOEF_F32);
     if (g.variant == 0 && g.time_block != 1 && varcoef_tb2_applicable(g)) {

@@ -1,6 +1,6 @@
 """The default kernel is not the slower one where another can be selected for
 the same call: the least of several timings each, with room for their spread, and
-measured again before it counts as slower (the host is shared)."""
+measured again before it counts as slower."""
 import time
 
 import numpy as np

@@ -168,7 +168,7 @@ def test_conversion_on_host_or_device(L):
 def test_copies_of_small_fp32_instances(L):
     """They take no longer than 1.2 times FP64 ones, which need no conversion,
     and 0.3 ns a value (with a kernel each 1.3 to 1.6 times FP64's time)."""
-    for _ in range(5):                      # again before it counts: the host is shared
+    for _ in range(5):                      # again before it counts as slower
         best = {}
         for precision in (4, 8):
             with lgd.LbmEnsemble([L], [1.3], precision=precision) as e:
